@@ -3,21 +3,39 @@
 // bits here), and the product for any operand types the tensor-core kernel
 // does not take (a weight stored in 32-bit under bfloat16 activations).
 //
-// fastllm-py calls cuBLAS for `x @ w.T` (fastllm_py/model.py:63).  This kernel
-// is slower and has one property cuBLAS lacks: each output element is one
-// thread's sum over k = 0..K-1 in that order, whatever M is, so a token's
-// result does not depend on how many other tokens share the step.
+// fastllm-py calls cuBLAS for `x @ w.T` (fastllm_py/model.py:63).  These kernels
+// have one property cuBLAS lacks: the order of every sum depends on K alone,
+// whatever M is and whichever kernel runs, so a token's result does not depend
+// on how many other tokens share the step.  The order: K is cut into GS_SLICES
+// slices of gs_slice(K) inputs, a slice is summed from its first input to its last
+// with fused multiply-adds, and the slices' sums are added from the first to
+// the last.  (Eight short chains instead of one of K: the rounding error falls
+// too, and the slices are what the kernels share out among threads and CTAs.)
+//
+// Three kernels:
+//   gemm_f32_skinny_kernel  float operands, up to 16 rows: bound by streaming W from memory
+//   gemm_f32_tile_kernel    float operands, more rows: bound by the multiply-adds
+//   gemm_simt_kernel        any operand types, alignments and batches
+// The last one served everything before: 350 us a product for 4 rows and 590 us for 300 rows of a layer with 2048 and
+// 5504 columns (10 TFLOP/s); the others take 12 to 37 us (1.4 to 3.4 TB/s of W, out of a cold cache) and 88 to 416 us (29
+// to 32 TFLOP/s, 38 with 32256 features).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 #define GS_BM 64
 #define GS_BN 64
 #define GS_BK 16
+#define GS_SLICES 8
+
+// Inputs per slice: a multiple of 32, which every kernel's K step divides.
+static inline int gs_slice(int K) { return ((K + GS_SLICES - 1) / GS_SLICES + 31) / 32 * 32; }
 
 template <typename TA, typename TW, typename TC>
 __global__ void __launch_bounds__(256) gemm_simt_kernel(const TA* __restrict__ A, long lda,
                                                         const TW* __restrict__ W, long ldw,
                                                         TC* __restrict__ C, long ldc, int M, int N,
-                                                        int K, long a_batch, long w_batch, long c_batch) {
+                                                        int K, int slice, long a_batch, long w_batch, long c_batch) {
     pdl_wait();
     pdl_trigger();
     A += blockIdx.z * a_batch;                // a batch of products over column blocks of wider buffers
@@ -28,8 +46,8 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const TA* __restrict__ A
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;
     const int m0 = blockIdx.y * GS_BM, n0 = blockIdx.x * GS_BN;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += GS_BK) {
+    float acc[4][4] = {}, total[4][4] = {};
+    for (int k0 = 0, left = slice; k0 < K; k0 += GS_BK) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int idx = tid + i * 256;
@@ -49,7 +67,18 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const TA* __restrict__ A
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] += a[i] * b[j];
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        }
+        left -= GS_BK;
+        if (left == 0 || k0 + GS_BK >= K) {   // the slice is complete
+            left = slice;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    total[i][j] += acc[i][j];
+                    acc[i][j] = 0.0f;
+                }
         }
         __syncthreads();
     }
@@ -60,19 +89,324 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const TA* __restrict__ A
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int n = n0 + tx * 4 + j;
-            if (n < N) C[(long)m * ldc + n] = from_f32<TC>(acc[i][j]);
+            if (n < N) C[(long)m * ldc + n] = from_f32<TC>(total[i][j]);
         }
     }
 }
 
+// ------------------------------------------------------------ up to 16 rows
+// A CTA of 64 threads serves 8 x RT features: thread (slice s, row r) sums slice s of features r, r + 8, ... for all MT
+// rows of A.  W and A pass through a ring of shared-memory stages, 32 inputs of every slice each, filled by 16-byte
+// cp.async: what bounds the product is the stream of W, so the ring keeps 3 of 4 stages (24 KB a CTA, several CTAs an
+// SM) in flight and W's first stages are asked for before the preceding kernel has ended.  A staged row of W is padded
+// to 36 floats: the eight lanes of a quarter warp, on eight rows, then read all 32 banks.  MT rows of A are read
+// (rows past M repeat the last one and are not written).  RT = 2 above four rows of A, so that a value of A that has
+// been read from shared memory serves two features.
+#define SK_BK 32
+#define SK_PITCH 36
+
+template <int MT> struct Skinny {
+    static constexpr int RT = MT > 4 ? 2 : 1;
+    static constexpr int R = 8 * RT;
+    static constexpr int STAGES = MT > 8 ? 3 : 4;
+    static constexpr int A_PITCH = MT * SK_BK + 4;                     // floats of a slice's rows of A
+    static constexpr int W_FLOATS = GS_SLICES * R * SK_PITCH;
+    static constexpr int STAGE_FLOATS = W_FLOATS + GS_SLICES * A_PITCH;
+    static constexpr int SMEM = STAGES * STAGE_FLOATS * 4;
+};
+
+__device__ __forceinline__ void sk_cp16(float* smem, const float* gmem, bool valid) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(valid ? 16 : 0) : "memory");
+}
+
+template <typename TC, int MT>
+__global__ void __launch_bounds__(64) gemm_f32_skinny_kernel(const float* __restrict__ A, long lda,
+                                                             const float* __restrict__ W, long ldw,
+                                                             TC* __restrict__ C, long ldc, int M, int N, int K, int slice) {
+    using L = Skinny<MT>;
+    constexpr int RT = L::RT, R = L::R, STAGES = L::STAGES;
+    extern __shared__ __align__(16) float sk_smem[];
+    const int tid = threadIdx.x, row = tid & 7, s = tid >> 3;
+    const int n0 = blockIdx.x * R;
+    const int n_st = slice / SK_BK;
+    // this thread copies 16-byte piece `row` of a stage's 32 inputs, of slice `s`, for every row of W and A
+    auto load_w = [&](int t) {
+        const int k = s * slice + t * SK_BK + row * 4;
+        float* dst = sk_smem + (t % STAGES) * L::STAGE_FLOATS + s * R * SK_PITCH + row * 4;
+#pragma unroll
+        for (int r = 0; r < R; ++r) sk_cp16(dst + r * SK_PITCH, k < K ? W + (long)min(n0 + r, N - 1) * ldw + k : W, k < K);
+    };
+    auto load_a = [&](int t) {
+        const int k = s * slice + t * SK_BK + row * 4;
+        float* dst = sk_smem + (t % STAGES) * L::STAGE_FLOATS + L::W_FLOATS + s * L::A_PITCH + row * 4;
+#pragma unroll
+        for (int m = 0; m < MT; ++m) sk_cp16(dst + m * SK_BK, k < K ? A + (long)min(m, M - 1) * lda + k : A, k < K);
+    };
+    for (int t = 0; t < STAGES - 1 && t < n_st; ++t) load_w(t);
+    pdl_wait();
+    pdl_trigger();
+    for (int t = 0; t < STAGES - 1; ++t) {
+        if (t < n_st) load_a(t);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    float acc[RT][MT] = {};
+    for (int t = 0; t < n_st; ++t) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();                                               // stage t is there, stage t - 1 has been read
+        if (t + STAGES - 1 < n_st) {
+            load_w(t + STAGES - 1);
+            load_a(t + STAGES - 1);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float* w_s = sk_smem + (t % STAGES) * L::STAGE_FLOATS + (s * R + row) * SK_PITCH;
+        const float* a_s = sk_smem + (t % STAGES) * L::STAGE_FLOATS + L::W_FLOATS + s * L::A_PITCH;
+#pragma unroll(MT > 8 ? 1 : 4)
+        for (int k = 0; k < SK_BK; k += 4) {
+            float4 w[RT];
+#pragma unroll
+            for (int r = 0; r < RT; ++r) w[r] = *reinterpret_cast<const float4*>(w_s + r * 8 * SK_PITCH + k);
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const float4 a = *reinterpret_cast<const float4*>(a_s + m * SK_BK + k);
+#pragma unroll
+                for (int r = 0; r < RT; ++r) {
+                    acc[r][m] = fmaf(a.x, w[r].x, acc[r][m]);
+                    acc[r][m] = fmaf(a.y, w[r].y, acc[r][m]);
+                    acc[r][m] = fmaf(a.z, w[r].z, acc[r][m]);
+                    acc[r][m] = fmaf(a.w, w[r].w, acc[r][m]);
+                }
+            }
+        }
+    }
+    __syncthreads();
+    float* red = sk_smem;                                              // [slice][row of A][feature]
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+#pragma unroll
+        for (int m = 0; m < MT; ++m) red[(s * MT + m) * R + r * 8 + row] = acc[r][m];
+    __syncthreads();
+    for (int i = tid; i < MT * R; i += 64) {
+        const int m = i / R, n = n0 + i % R;
+        float total = 0.0f;
+#pragma unroll
+        for (int z = 0; z < GS_SLICES; ++z) total += red[z * MT * R + i];
+        if (m < M && n < N) C[(long)m * ldc + n] = from_f32<TC>(total);
+    }
+}
+
+// ------------------------------------------------------------ more rows
+// 64 rows x 128 features per CTA of 128 threads, 8 x 8 results a thread (four 16-byte reads of shared memory per 64
+// multiply-adds: with 4 x 8 a thread the reads took longer than the multiply-adds), two CTAs an SM; both operands are
+// turned to [input][row] on their way into shared memory (columns exchanged by a pattern of the input's index, so that
+// neither the turned stores nor the 16-byte reads meet in a bank), the next 16 inputs wait in registers meanwhile.  Bound
+// by the multiply-adds: they are issued in pairs (fma.rn.f32x2, the same rounding), which leaves issue slots for the reads.
+// SPLIT: a cluster of GS_SLICES CTAs shares a tile, each sums one slice, and each adds up an eighth of the rows from the
+// others' shared memory, in the order of the slices; no partial sum goes to global memory.
+#define TL_BM 64
+#define TL_BN 128
+#define TL_BK 16
+#define TL_THREADS 128
+
+__device__ __forceinline__ void fma2(float2& d, const float2 a, const float2 b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;"
+        : "+l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+}
+
+template <typename TC, bool SPLIT>
+__device__ __forceinline__ void gemm_f32_tile(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw,
+                                              TC* __restrict__ C, long ldc, int M, int N, int K, int slice) {
+    constexpr int STAGE = TL_BK * (TL_BM + TL_BN);
+    __shared__ __align__(16) float smem[SPLIT ? (2 * STAGE > TL_BM * TL_BN ? 2 * STAGE : TL_BM * TL_BN) : 2 * STAGE];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int m0 = blockIdx.y * TL_BM, n0 = blockIdx.x * TL_BN;
+    const int k_begin = SPLIT ? min(K, (int)blockIdx.z * slice) : 0;
+    const int k_end = SPLIT ? min(K, k_begin + slice) : K;
+    // this thread's 16-byte pieces of a stage: rows lr, lr + 32, ... of A (two) and W (four), inputs 4 lk .. 4 lk + 3
+    const int lr = tid >> 2, lk = tid & 3;
+    const float* src[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+        src[i] = (i < 2 ? A + (long)min(m0 + lr + 32 * i, M - 1) * lda : W + (long)min(n0 + lr + 32 * (i - 2), N - 1) * ldw) + lk * 4;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 next[6];
+    auto fetch = [&](int k0) {
+        const bool in = k0 + lk * 4 < k_end;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) next[i] = in ? *reinterpret_cast<const float4*>(src[i] + k0) : zero;
+    };
+    auto put = [&](int buf) {
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            constexpr int PA = TL_BM, PW = TL_BN;
+            const int pitch = i < 2 ? PA : PW;
+            float* d = smem + buf * STAGE + (i < 2 ? 0 : TL_BK * TL_BM) + lk * 4 * pitch + ((lr + 32 * (i < 2 ? i : i - 2)) ^ (lk << 3));
+            d[0] = next[i].x, d[pitch] = next[i].y, d[2 * pitch] = next[i].z, d[3 * pitch] = next[i].w;
+        }
+    };
+    float2 acc[8][4], total[SPLIT ? 1 : 8][4];                          // 8 rows x 4 pairs of features
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            acc[i][j] = make_float2(0.0f, 0.0f);
+            if (!SPLIT) total[i][j] = make_float2(0.0f, 0.0f);
+        }
+    if (k_begin < k_end) {
+        fetch(k_begin);
+        put(0);
+    }
+    __syncthreads();
+    int buf = 0, left = slice;
+    for (int k0 = k_begin; k0 < k_end; k0 += TL_BK) {
+        const bool more = k0 + TL_BK < k_end;
+        if (more) fetch(k0 + TL_BK);
+        const float* a_s = smem + buf * STAGE;
+        const float* w_s = a_s + TL_BK * TL_BM;
+#pragma unroll
+        for (int kk = 0; kk < TL_BK; ++kk) {
+            const int x = (kk >> 2) << 3;
+            const float4 a0 = *reinterpret_cast<const float4*>(a_s + kk * TL_BM + ((ty * 4) ^ x));
+            const float4 a1 = *reinterpret_cast<const float4*>(a_s + kk * TL_BM + 32 + ((ty * 4) ^ x));
+            const float4 b0 = *reinterpret_cast<const float4*>(w_s + kk * TL_BN + ((tx * 4) ^ x));
+            const float4 b1 = *reinterpret_cast<const float4*>(w_s + kk * TL_BN + 64 + ((tx * 4) ^ x));
+            const float2 b[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w), make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
+            const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float2 aa = make_float2(a[i], a[i]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) fma2(acc[i][j], aa, b[j]);
+            }
+        }
+        if (!SPLIT) {
+            left -= TL_BK;
+            if (left == 0 || !more) {                                   // the slice is complete
+                left = slice;
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        total[i][j].x += acc[i][j].x;
+                        total[i][j].y += acc[i][j].y;
+                        acc[i][j] = make_float2(0.0f, 0.0f);
+                    }
+            }
+        }
+        if (more) put(buf ^ 1);
+        __syncthreads();
+        buf ^= 1;
+    }
+    auto store = [&](int m, int n, const float4 v) {                    // four features of one row
+        if (m >= M) return;
+        TC* c = C + (long)m * ldc + n;
+        const float x[4] = {v.x, v.y, v.z, v.w};
+        if (sizeof(TC) == 4 && n + 4 <= N && ((uintptr_t)c & 15) == 0) {
+            *reinterpret_cast<float4*>(c) = v;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (n + j < N) c[j] = from_f32<TC>(x[j]);
+        }
+    };
+    if constexpr (!SPLIT) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                store(m0 + (i >> 2) * 32 + ty * 4 + (i & 3), n0 + h * 64 + tx * 4,
+                      make_float4(total[i][2 * h].x, total[i][2 * h].y, total[i][2 * h + 1].x, total[i][2 * h + 1].y));
+    } else {
+        namespace cg = cooperative_groups;
+        cg::cluster_group cluster = cg::this_cluster();
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                *reinterpret_cast<float4*>(smem + ((i >> 2) * 32 + ty * 4 + (i & 3)) * TL_BN + h * 64 + tx * 4) =
+                    make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x, acc[i][2 * h + 1].y);
+        cluster.sync();
+        // 8 rows x 128 features of the tile are this CTA's to add up: four features a thread
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int r = (int)blockIdx.z * (TL_BM / GS_SLICES) + half * 4 + (tid >> 5), c = (tid & 31) * 4;
+            float4 sum = zero;
+#pragma unroll
+            for (int z = 0; z < GS_SLICES; ++z) {
+                const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(smem, z) + r * TL_BN + c);
+                sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
+            }
+            store(m0 + r, n0 + c, sum);
+        }
+        cluster.sync();                                                 // no CTA leaves while another reads its sums
+    }
+}
+
+template <typename TC>
+__global__ void __launch_bounds__(TL_THREADS, 2) gemm_f32_tile_kernel(const float* __restrict__ A, long lda,
+                                                               const float* __restrict__ W, long ldw, TC* __restrict__ C,
+                                                               long ldc, int M, int N, int K, int slice) {
+    pdl_wait();
+    pdl_trigger();
+    gemm_f32_tile<TC, false>(A, lda, W, ldw, C, ldc, M, N, K, slice);
+}
+
+template <typename TC>
+__global__ void __cluster_dims__(1, 1, GS_SLICES) __launch_bounds__(TL_THREADS, 2)
+    gemm_f32_tile_split_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw,
+                               TC* __restrict__ C, long ldc, int M, int N, int K, int slice) {
+    pdl_wait();
+    pdl_trigger();
+    gemm_f32_tile<TC, true>(A, lda, W, ldw, C, ldc, M, N, K, slice);
+}
+
+// ------------------------------------------------------------ host side
+template <typename TC, int MT>
+static int gs_skinny(const float* A, long lda, const float* W, long ldw, TC* C, long ldc, int M, int N, int K, cudaStream_t stream) {
+    using L = Skinny<MT>;
+    auto kernel = gemm_f32_skinny_kernel<TC, MT>;
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
+    if (err != cudaSuccess) return (int)err;
+    return fl_launch(kernel, dim3((N + L::R - 1) / L::R), dim3(64), L::SMEM, stream, A, lda, W, ldw, C, ldc, M, N, K, gs_slice(K));
+}
+
+// Float operands that 16-byte loads can read.  Up to 16 rows W's bytes decide and the skinny kernel streams them; above,
+// the multiply-adds do.  A tile is split over a cluster when that fills the SMs better: what is compared is the waves of
+// CTAs (two an SM) times the inputs that a CTA goes through, a split CTA paying about 40 inputs' time for the exchange.
+template <typename TC>
+static int gs_f32(const float* A, long lda, const float* W, long ldw, TC* C, long ldc, int M, int N, int K, int sms,
+                  cudaStream_t stream) {
+    if (M <= 1) return gs_skinny<TC, 1>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+    if (M <= 2) return gs_skinny<TC, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+    if (M <= 4) return gs_skinny<TC, 4>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+    if (M <= 8) return gs_skinny<TC, 8>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+    if (M <= 16) return gs_skinny<TC, 16>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+    const int slice = gs_slice(K);
+    dim3 grid((N + TL_BN - 1) / TL_BN, (M + TL_BM - 1) / TL_BM);
+    if (grid.y > 65535) return (int)cudaErrorInvalidValue;
+    const long tiles = (long)grid.x * grid.y, slots = 2L * sms;
+    const long whole = (tiles + slots - 1) / slots * K;
+    const long split = (tiles * GS_SLICES + slots - 1) / slots * (slice + 40);
+    if (split < whole) {
+        grid.z = GS_SLICES;
+        return fl_launch(gemm_f32_tile_split_kernel<TC>, grid, dim3(TL_THREADS), 0, stream, A, lda, W, ldw, C, ldc, M, N, K, slice);
+    }
+    return fl_launch(gemm_f32_tile_kernel<TC>, grid, dim3(TL_THREADS), 0, stream, A, lda, W, ldw, C, ldc, M, N, K, slice);
+}
+
 FL_API int fl_gemm_simt(const void* A, int a_dtype, long lda, const void* W, int w_dtype, long ldw,
-                        void* C, int c_dtype, long ldc, int M, int N, int K, cudaStream_t stream) {
+                        void* C, int c_dtype, long ldc, int M, int N, int K, int sms, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
+    if (a_dtype == FL_F32 && w_dtype == FL_F32 && K > 0 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
+        ((uintptr_t)A | (uintptr_t)W) % 16 == 0) {
+        FL_DISPATCH(c_dtype, TC, return gs_f32<TC>((const float*)A, lda, (const float*)W, ldw, (TC*)C, ldc, M, N, K, sms, stream));
+    }
     dim3 grid((N + GS_BN - 1) / GS_BN, (M + GS_BM - 1) / GS_BM);
     if (grid.y > 65535) return (int)cudaErrorInvalidValue;
     FL_DISPATCH(a_dtype, TA, FL_DISPATCH(w_dtype, TW, FL_DISPATCH(c_dtype, TC,
         return fl_launch(gemm_simt_kernel<TA, TW, TC>, grid, dim3(256), 0, stream, (const TA*)A, lda,
-                         (const TW*)W, ldw, (TC*)C, ldc, M, N, K, 0L, 0L, 0L))));
+                         (const TW*)W, ldw, (TC*)C, ldc, M, N, K, gs_slice(K), 0L, 0L, 0L))));
     return 0;
 }
 
@@ -87,6 +421,6 @@ FL_API int fl_gemm_simt_batched(const void* A, int a_dtype, long lda, long a_bat
     if (grid.y > 65535 || batch > 65535) return (int)cudaErrorInvalidValue;
     FL_DISPATCH(a_dtype, TA, FL_DISPATCH(w_dtype, TW, FL_DISPATCH(c_dtype, TC,
         return fl_launch(gemm_simt_kernel<TA, TW, TC>, grid, dim3(256), 0, stream, (const TA*)A, lda,
-                         (const TW*)W, ldw, (TC*)C, ldc, M, N, K, a_batch, w_batch, c_batch))));
+                         (const TW*)W, ldw, (TC*)C, ldc, M, N, K, gs_slice(K), a_batch, w_batch, c_batch))));
     return 0;
 }

@@ -51,6 +51,16 @@ def _stream():
     return c_void_p(_raw_stream(_device_index))
 
 
+_sm_counts: dict = {}
+
+
+def _sms(device) -> int:
+    n = _sm_counts.get(device)
+    if n is None:
+        n = _sm_counts[device] = torch.cuda.get_device_properties(device).multi_processor_count
+    return n
+
+
 def _ld(t: torch.Tensor) -> int:
     """Leading dimension (elements between rows) of a 2-D view with a dense last axis."""
     if t.dim() != 2:
@@ -1329,9 +1339,9 @@ def gemm_simt(a, w, out):
     if a.shape[1] != w.shape[1] or out.shape[0] != a.shape[0] or out.shape[1] != w.shape[0]:
         raise KernelError(f"gemm: shapes {tuple(a.shape)} x {tuple(w.shape)}^T -> {tuple(out.shape)}")
     fn = _fn("gemm_simt", "fl_gemm_simt", [c_void_p, c_int, c_long, c_void_p, c_int, c_long, c_void_p,
-                                           c_int, c_long, c_int, c_int, c_int, c_void_p])
-    _check(fn(_ptr(a), dtype_code(a), _ld(a), _ptr(w), dtype_code(w), _ld(w), _ptr(out),
-              dtype_code(out), _ld(out), a.shape[0], w.shape[0], a.shape[1], _stream()), "gemm_simt")
+                                           c_int, c_long, c_int, c_int, c_int, c_int, c_void_p])
+    _check(fn(_ptr(a), dtype_code(a), _ld(a), _ptr(w), dtype_code(w), _ld(w), _ptr(out), dtype_code(out), _ld(out),
+              a.shape[0], w.shape[0], a.shape[1], _sms(a.device), _stream()), "gemm_simt")
 
 
 # ------------------------------------------------------------------- sampling

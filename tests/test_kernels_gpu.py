@@ -169,6 +169,38 @@ def test_cuda_core_gemm(a_dt, w_dt, c_dt):
         assert float((out.double().cpu() - ref).abs().max()) <= tol
 
 
+def sliced_sum_bound(a, w):
+    """What float sums of a @ w^T may be off: eight chains of at most k / 8 + 32 fused multiply-adds, then eight additions."""
+    terms = a.double().abs() @ w.double().abs().t()
+    return (a.shape[1] / 8 + 32 + 8) * 2.0 ** -24 * terms + 1e-30
+
+
+@pytest.mark.parametrize("n, k", [(1, 4), (9, 36), (130, 172), (127, 256), (2049, 2052), (384, 2048), (700, 5504)])
+def test_float_gemm_kernels(n, k):
+    """The kernels for few rows, for tiles and for tiles shared by a cluster against 64 bits, and a row's result is the same
+    bit for bit in all of them and in the kernel for any operands (an unaligned copy goes there)."""
+    from fastllm_py_b200.native import ops
+
+    g = torch.Generator().manual_seed(n + k)
+    a = torch.randn(330, k, generator=g)
+    w = torch.randn(n, k, generator=g)
+    ref, tol = a.double() @ w.double().t(), sliced_sum_bound(a, w)
+    ad, wd = a.to(DEV), w.to(DEV)
+    shifted = torch.zeros(330, k + 1, device=DEV)[:, 1:]
+    shifted.copy_(ad)
+    general = torch.empty(330, n, device=DEV)
+    ops.gemm_simt(shifted, wd, general)
+    assert bool(((general.double().cpu() - ref).abs() <= tol).all())
+    for m in (1, 2, 3, 4, 5, 8, 9, 16, 17, 63, 64, 65, 300, 330):
+        out = torch.full((m + 1, n + 3), 7.0, device=DEV)                # rows and columns beyond stay as they are
+        ops.gemm_simt(ad[:m], wd, out[:m, :n])
+        assert torch.equal(out[:m, :n], general[:m]), m
+        assert bool((out[m:] == 7.0).all()) and bool((out[:, n:] == 7.0).all())
+        half = torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
+        ops.gemm_simt(ad[:m], wd, half)
+        assert torch.equal(half, general[:m].to(torch.bfloat16)), m
+
+
 # ------------------------------------------------------------------ attention
 
 class AttentionCase:
