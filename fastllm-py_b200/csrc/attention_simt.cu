@@ -1,110 +1,337 @@
 // Paged causal attention on CUDA cores, for any mix of prompt portions and
 // single decoded tokens, in bfloat16 or true 32-bit.
 //
-// One block serves one (token, query head): it walks that token's visible keys
-// through the request's block table in tiles of 128 keys, keeps a running
-// maximum and sum (softmax in float, exact expf) and accumulates the weighted
-// values.  Tiles start at multiples of 128 of the absolute key position, so the
-// order of every sum depends only on the token's own position: the result is
-// the same bit for bit however the sequence was cut into steps and whatever
-// else is in the batch.  This is the reference kernel of the engine: slow,
-// simple, and the 32-bit path's attention.
+// The keys of a token are taken in tiles of 64 that start at multiples of 64 of
+// the absolute key position.  A tile has a result of its own (its maximum, the
+// sum of exp(score - maximum) and the weighted values, softmax in float with the
+// exact expf; a score is summed over the head's columns in order, the weighted
+// values over the tile's keys in order), and the tiles' results are folded from
+// the first to the last.  So the order of every sum depends only on the token's
+// own position: the result is the same bit for bit however the sequence was cut
+// into steps, whatever else is in the batch and however many CTAs share the
+// tiles.  This is the reference kernel of the engine and the 32-bit path's
+// attention.
+//
+// A cluster of CL CTAs serves QT neighbouring tokens of the step and one query
+// head.  QT is 8 for prompts (a tile that has been fetched serves 8 tokens; where
+// requests meet inside the 8, one request's tokens follow the other's) and 1
+// for steps in which every request brings one token.  Prompts are bound by the
+// multiply-adds and shared-memory reads, single tokens by latency: with few
+// (token, head) pairs in the step the tiles are dealt out to the cluster's CTAs
+// (tile t to CTA t mod CL), which hand their results over through distributed
+// shared memory.  One block a (token, head) pair, each thread walking a key row
+// in global memory, took 196 us a layer for 4 tokens over 700 keys and 16 heads
+// of 128 in 32 bits, and 450 us for a prompt of 300 tokens; this takes 50 and 146
+// (profiled inside a step, with the wait for the product before it).
 //
 // fastllm-py's counterparts: `_sdpa` (fastllm_py/model.py:341-353: scores scaled
 // by head_dim^-1/2, keys beyond the query masked, softmax and the weighted sum in
 // float) and the decode kernels `attn_decode` (fastllm_py/graph_decode.py:378-420)
 // and `battn` (fastllm_py/batched.py:48-92).  Grouped heads are index
 // arithmetic, h / (H / KVH), never a materialised repeat (model.py:426-428).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
-#define ATT_TILE 128
+#define ATT_THREADS 128
+#define ATT_TILE 64              // keys
 
-template <typename T>
-__global__ void __launch_bounds__(ATT_TILE) paged_attention_simt_kernel(
+template <int QT> struct AttHold { static constexpr int TILES = QT == 1 ? 8 : 2; };     // tiles a CTA holds before they are folded
+
+// floats of shared memory of a CTA: queries, keys, values, scores, weights, tile results
+__host__ __device__ constexpr int att_pad(int head_dim) { return (head_dim + 3) / 4 * 4; }
+__host__ __device__ constexpr int att_floats(int qt, int hold, int dp) {
+    return qt * dp + ATT_TILE * (dp + 4) + ATT_TILE * dp + 2 * qt * ATT_TILE + hold * qt * (dp + 2);
+}
+
+__device__ __forceinline__ void att_cp16(float* smem, const float* gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+}
+
+template <typename T, int QT, int CL>
+__global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
     const T* __restrict__ q, long q_ld, T* __restrict__ out, long out_ld,
     const T* __restrict__ k_cache, const T* __restrict__ v_cache, long page_stride, int page_size,
     const int* __restrict__ block_table, int bt_stride, const int* __restrict__ tok_req,
-    const int* __restrict__ positions, int n_heads, int n_kv_heads, int head_dim, int window,
-    float scale) {
+    const int* __restrict__ positions, int n_tokens, int n_heads, int n_kv_heads, int head_dim, int window,
+    float scale, int vec) {
     pdl_wait();
     pdl_trigger();
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    long* off_s = reinterpret_cast<long*>(smem_raw);                  // [ATT_TILE] element offset of each key row
-    float* p_s = reinterpret_cast<float*>(off_s + ATT_TILE);          // [ATT_TILE] softmax numerators of the tile
-    float* q_s = p_s + ATT_TILE;                                      // [head_dim]
-    __shared__ float scratch[32];
+    namespace cg = cooperative_groups;
+    constexpr int HOLD = AttHold<QT>::TILES;
+    extern __shared__ __align__(16) float att_smem[];
+    const int dp = att_pad(head_dim), kp = dp + 4;
+    float* q_s = att_smem;                              // [QT][dp]
+    float* k_s = q_s + QT * dp;                         // [tile][kp]: eight neighbouring rows lie in all 32 banks
+    float* v_s = k_s + ATT_TILE * kp;                   // [tile][dp]
+    float* s_s = v_s + ATT_TILE * dp;                   // [QT][tile] scores
+    float* p_s = s_s + QT * ATT_TILE;                   // [tile][QT] softmax numerators
+    float* hold_acc = p_s + QT * ATT_TILE;              // [HOLD][QT][dp]
+    float* hold_ml = hold_acc + HOLD * QT * dp;         // [HOLD][QT] maximum, sum
 
-    const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = CL == 1 ? 0 : (int)(blockIdx.x % CL), h = blockIdx.y;
+    const int t_begin = (int)(blockIdx.x / CL) * QT, t_end = min(n_tokens, t_begin + QT);
     const int kvh = h / (n_heads / n_kv_heads);
-    const int pos = positions[t];
-    const int* bt = block_table + (long)tok_req[t] * bt_stride;
-    const int lo = window > 0 ? max(0, pos - window + 1) : 0;
     const long head_off = (long)kvh * page_size * head_dim;
 
-    const T* qr = q + (long)t * q_ld + (long)h * head_dim;
-    for (int d = tid; d < head_dim; d += ATT_TILE) q_s[d] = to_f32<T>(qr[d]);
-    __syncthreads();
+    for (int t0 = t_begin, nq; t0 < t_end; t0 += nq) {  // tokens of one request at a time
+        const int req = tok_req[t0];
+        nq = 1;
+        while (QT > 1 && t0 + nq < t_end && tok_req[t0 + nq] == req) ++nq;
+        const int* bt = block_table + (long)req * bt_stride;
+        int pos[QT], first = 0x7fffffff, last = -1;
+#pragma unroll
+        for (int i = 0; i < QT; ++i) {
+            pos[i] = i < nq ? positions[t0 + i] : -1;
+            if (i < nq) {
+                first = min(first, window > 0 ? max(0, pos[i] - window + 1) : 0);
+                last = max(last, pos[i]);
+            }
+        }
+        for (int i = tid; i < nq * dp; i += ATT_THREADS) {
+            const int r = i / dp, d = i - r * dp;
+            q_s[i] = d < head_dim ? to_f32<T>(q[(long)(t0 + r) * q_ld + (long)h * head_dim + d]) : 0.0f;
+        }
+        float acc[QT][2] = {}, m[QT], l[QT];
+        bool begun[QT];
+#pragma unroll
+        for (int i = 0; i < QT; ++i) m[i] = -CUDART_INF_F, l[i] = 0.0f, begun[i] = false;
+        const int d0 = tid, d1 = tid + ATT_THREADS;
 
-    float m = -CUDART_INF_F, l = 0.0f, acc0 = 0.0f, acc1 = 0.0f;
-    const int d0 = tid, d1 = tid + ATT_TILE;
-    for (int tile = (lo / ATT_TILE) * ATT_TILE; tile <= pos; tile += ATT_TILE) {
-        const int j = tile + tid;
-        const bool valid = j >= lo && j <= pos;
-        float s = -CUDART_INF_F;
-        long off = 0;
-        if (valid) {
-            const long page = bt[j / page_size];
-            off = page * page_stride + head_off + (long)(j % page_size) * head_dim;
-            const T* kp = k_cache + off;
-            float dot = 0.0f;
-            for (int d = 0; d < head_dim; ++d) dot += q_s[d] * to_f32<T>(kp[d]);
-            s = dot * scale;
+        auto lowest = [&](int i) { return window > 0 ? max(0, pos[i] - window + 1) : 0; };
+        auto sees = [&](int i, int tile) { return i < nq && pos[i] >= tile * ATT_TILE && lowest(i) < (tile + 1) * ATT_TILE; };
+
+        // The result of one tile: maximum and sum of query i in ml[2 i], ml[2 i + 1], the weighted values in `a`.
+        auto do_tile = [&](int tile, float* ml, float (&a)[QT][2]) {
+            const int base = tile * ATT_TILE, keys = min(ATT_TILE, last + 1 - base);
+            // keys and values of the tile, rows past the last visible key left as zeros (their pages may hold anything)
+            if (sizeof(T) == 4 && vec) {
+                const int per = head_dim / 4;
+#pragma unroll 1
+                for (int side = 0; side < 2; ++side) {
+                    float* dst = side == 0 ? k_s : v_s;
+                    const int pitch = side == 0 ? kp : dp;
+                    const float* src = reinterpret_cast<const float*>(side == 0 ? k_cache : v_cache);
+                    for (int i = tid; i < ATT_TILE * per; i += ATT_THREADS) {
+                        const int r = i / per, c = (i - r * per) * 4, j = base + r;
+                        if (r < keys) {
+                            const long off = (long)bt[j / page_size] * page_stride + head_off + (long)(j % page_size) * head_dim;
+                            att_cp16(dst + r * pitch + c, src + off + c);
+                        } else {
+                            *reinterpret_cast<float4*>(dst + r * pitch + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        }
+                    }
+                    asm volatile("cp.async.commit_group;" ::: "memory");
+                }
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                for (int i = tid; i < ATT_TILE * dp; i += ATT_THREADS) {
+                    const int r = i / dp, c = i - r * dp, j = base + r;
+                    float kv = 0.0f, vv = 0.0f;
+                    if (r < keys && c < head_dim) {
+                        const long off = (long)bt[j / page_size] * page_stride + head_off + (long)(j % page_size) * head_dim + c;
+                        kv = to_f32<T>(k_cache[off]);
+                        vv = to_f32<T>(v_cache[off]);
+                    }
+                    k_s[r * kp + c] = kv;
+                    v_s[i] = vv;
+                }
+            }
+            __syncthreads();
+            // scores: a thread takes one key and every other group of queries
+            constexpr int HALF = QT > 1 ? QT / 2 : 1;
+            const int key = tid & (ATT_TILE - 1), i0 = (tid / ATT_TILE) * HALF;
+            if (QT > 1 || tid < ATT_TILE) {
+                float dot[HALF] = {};
+#pragma unroll 4
+                for (int d = 0; d < dp; d += 4) {
+                    const float4 k4 = *reinterpret_cast<const float4*>(k_s + key * kp + d);
+#pragma unroll
+                    for (int i = 0; i < HALF; ++i) {
+                        const float4 q4 = *reinterpret_cast<const float4*>(q_s + (i0 + i) * dp + d);
+                        dot[i] = fmaf(q4.x, k4.x, dot[i]);
+                        dot[i] = fmaf(q4.y, k4.y, dot[i]);
+                        dot[i] = fmaf(q4.z, k4.z, dot[i]);
+                        dot[i] = fmaf(q4.w, k4.w, dot[i]);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < HALF; ++i) s_s[(i0 + i) * ATT_TILE + key] = dot[i] * scale;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < QT; ++i) {
+                if ((i & 3) != warp || !sees(i, tile)) continue;
+                const int ja = base + lane, jb = ja + 32;
+                const bool va = ja >= lowest(i) && ja <= pos[i], vb = jb >= lowest(i) && jb <= pos[i];
+                const float sa = va ? s_s[i * ATT_TILE + lane] : -CUDART_INF_F, sb = vb ? s_s[i * ATT_TILE + lane + 32] : -CUDART_INF_F;
+                const float mt = warp_max(fmaxf(sa, sb));
+                const float pa = va ? expf(sa - mt) : 0.0f, pb = vb ? expf(sb - mt) : 0.0f;
+                p_s[lane * QT + i] = pa;
+                p_s[(lane + 32) * QT + i] = pb;
+                const float lt = warp_sum(pa + pb);
+                if (lane == 0) ml[2 * i] = mt, ml[2 * i + 1] = lt;
+            }
+            if (sizeof(T) == 4 && vec) asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            // keys outside a query's range are left out rather than weighted by zero: they may hold infinities
+#pragma unroll
+            for (int i = 0; i < QT; ++i) a[i][0] = a[i][1] = 0.0f;
+            bool all = true;
+#pragma unroll
+            for (int i = 0; i < QT; ++i)
+                if (i < nq) all = all && lowest(i) <= base && pos[i] >= base + ATT_TILE - 1;
+            if (all && nq == QT) {
+#pragma unroll 4
+                for (int j = 0; j < ATT_TILE; ++j) {
+                    const float v0 = d0 < head_dim ? v_s[j * dp + d0] : 0.0f, v1 = d1 < head_dim ? v_s[j * dp + d1] : 0.0f;
+#pragma unroll
+                    for (int i = 0; i < QT; ++i) {
+                        const float p = p_s[j * QT + i];
+                        a[i][0] = fmaf(p, v0, a[i][0]);
+                        if (d1 < head_dim) a[i][1] = fmaf(p, v1, a[i][1]);
+                    }
+                }
+            } else {
+                for (int j = 0; j < keys; ++j) {
+                    const float v0 = d0 < head_dim ? v_s[j * dp + d0] : 0.0f, v1 = d1 < head_dim ? v_s[j * dp + d1] : 0.0f;
+#pragma unroll
+                    for (int i = 0; i < QT; ++i) {
+                        if (i >= nq || base + j < lowest(i) || base + j > pos[i]) continue;
+                        const float p = p_s[j * QT + i];
+                        a[i][0] = fmaf(p, v0, a[i][0]);
+                        if (d1 < head_dim) a[i][1] = fmaf(p, v1, a[i][1]);
+                    }
+                }
+            }
+        };
+        auto fold = [&](int i, float mt, float lt, float a0, float a1) {
+            if (!begun[i]) {
+                begun[i] = true;
+                m[i] = mt, l[i] = lt, acc[i][0] = a0, acc[i][1] = a1;
+                return;
+            }
+            const float m_new = fmaxf(m[i], mt), c = expf(m[i] - m_new), ct = expf(mt - m_new);
+            m[i] = m_new;
+            l[i] = l[i] * c + lt * ct;
+            acc[i][0] = acc[i][0] * c + a0 * ct;
+            acc[i][1] = acc[i][1] * c + a1 * ct;
+        };
+
+        const int tile0 = first / ATT_TILE, tile1 = last / ATT_TILE + 1;
+        __syncthreads();                                 // the queries are there
+        if constexpr (CL == 1) {
+            for (int tile = tile0; tile < tile1; ++tile) {
+                float a[QT][2];
+                do_tile(tile, hold_ml, a);
+#pragma unroll
+                for (int i = 0; i < QT; ++i)
+                    if (sees(i, tile)) fold(i, hold_ml[2 * i], hold_ml[2 * i + 1], a[i][0], a[i][1]);
+                __syncthreads();                         // the tile's shared memory is read, the next one may come
+            }
+        } else {
+            cg::cluster_group cluster = cg::this_cluster();
+            for (int round = tile0; round < tile1; round += CL * HOLD) {
+#pragma unroll 1
+                for (int slot = 0; slot < HOLD; ++slot) {
+                    const int tile = round + slot * CL + rank;
+                    if (tile >= tile1) break;
+                    float a[QT][2];
+                    do_tile(tile, hold_ml + slot * 2 * QT, a);
+#pragma unroll
+                    for (int i = 0; i < QT; ++i) {
+                        if (d0 < head_dim) hold_acc[(slot * QT + i) * dp + d0] = a[i][0];
+                        if (d1 < head_dim) hold_acc[(slot * QT + i) * dp + d1] = a[i][1];
+                    }
+                    __syncthreads();
+                }
+                cluster.sync();
+                // query i is folded by CTA i mod CL
+                const int stop = min(tile1, round + CL * HOLD);
+                for (int tile = round; tile < stop; ++tile) {
+                    const int slot = (tile - round) / CL, from = (tile - round) % CL;
+                    const float* ml = cluster.map_shared_rank(hold_ml, from) + slot * 2 * QT;
+                    const float* ha = cluster.map_shared_rank(hold_acc, from) + slot * QT * dp;
+#pragma unroll
+                    for (int i = 0; i < QT; ++i)
+                        if (i % CL == rank && sees(i, tile))
+                            fold(i, ml[2 * i], ml[2 * i + 1], d0 < head_dim ? ha[i * dp + d0] : 0.0f,
+                                 d1 < head_dim ? ha[i * dp + d1] : 0.0f);
+                }
+                cluster.sync();
+            }
         }
-        off_s[tid] = off;
-        const float m_new = fmaxf(m, block_max(s, scratch));
-        const float p = valid ? expf(s - m_new) : 0.0f;
-        p_s[tid] = p;
-        const float tile_sum = block_sum(p, scratch);     // its barriers also publish p_s / off_s
-        const float corr = expf(m - m_new);               // 0 at the first tile (m = -inf)
-        l = l * corr + tile_sum;
-        const int j_begin = max(0, lo - tile);
-        const int j_end = min(ATT_TILE, pos - tile + 1);
-        if (d0 < head_dim) {
-            float a = acc0 * corr;
-            for (int jj = j_begin; jj < j_end; ++jj) a += p_s[jj] * to_f32<T>(v_cache[off_s[jj] + d0]);
-            acc0 = a;
+#pragma unroll
+        for (int i = 0; i < QT; ++i) {
+            if (i >= nq || (CL > 1 && i % CL != rank)) continue;
+            T* o = out + (long)(t0 + i) * out_ld + (long)h * head_dim;
+            if (d0 < head_dim) o[d0] = from_f32<T>(acc[i][0] / l[i]);
+            if (d1 < head_dim) o[d1] = from_f32<T>(acc[i][1] / l[i]);
         }
-        if (d1 < head_dim) {
-            float a = acc1 * corr;
-            for (int jj = j_begin; jj < j_end; ++jj) a += p_s[jj] * to_f32<T>(v_cache[off_s[jj] + d1]);
-            acc1 = a;
-        }
-        m = m_new;
-        __syncthreads();                                  // p_s / off_s are rewritten by the next tile
+        __syncthreads();                                 // the queries are read, the next request's may come
     }
-    T* o = out + (long)t * out_ld + (long)h * head_dim;
-    if (d0 < head_dim) o[d0] = from_f32<T>(acc0 / l);
-    if (d1 < head_dim) o[d1] = from_f32<T>(acc1 / l);
+}
+
+template <typename T, int QT, int CL>
+static int att_launch(const T* q, long q_ld, T* out, long out_ld, const T* k_cache, const T* v_cache, long page_stride,
+                      int page_size, const int* block_table, int bt_stride, const int* tok_req, const int* positions,
+                      int n_tokens, int n_heads, int n_kv_heads, int head_dim, int window, float scale, cudaStream_t stream) {
+    auto kernel = paged_attention_simt_kernel<T, QT, CL>;
+    const size_t smem = 4 * (size_t)att_floats(QT, AttHold<QT>::TILES, att_pad(head_dim));
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return (int)err;
+    const int vec = head_dim % 4 == 0 && page_stride % 4 == 0 && (((uintptr_t)k_cache | (uintptr_t)v_cache) % 16) == 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((n_tokens + QT - 1) / QT) * CL, n_heads);
+    cfg.blockDim = dim3(ATT_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CL;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = fl_pdl_enabled() ? 2 : 1;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, q, q_ld, out, out_ld, k_cache, v_cache, page_stride, page_size, block_table,
+                                   bt_stride, tok_req, positions, n_tokens, n_heads, n_kv_heads, head_dim, window, scale, vec);
 }
 
 // q: [n_tokens, q_ld] with head h at columns [h*head_dim, (h+1)*head_dim);
 // out likewise.  tok_req[t] is the row of `block_table` that token t's request
 // uses; positions[t] is the token's absolute position, whose key (already in
-// the cache) is the last one it sees.  window <= 0 means all keys.
+// the cache) is the last one it sees.  window <= 0 means all keys.  `single`: neighbouring tokens belong to
+// different requests (a hint, results do not depend on it).
 FL_API int fl_paged_attention_simt(const void* q, int dtype, long q_ld, void* out, long out_ld,
                                    const void* k_cache, const void* v_cache, long page_stride,
                                    int page_size, const int* block_table, int bt_stride,
                                    const int* tok_req, const int* positions, int n_tokens,
-                                   int n_heads, int n_kv_heads, int head_dim, int window, float scale,
+                                   int n_heads, int n_kv_heads, int head_dim, int window, float scale, int single, int sms,
                                    cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
-    if (head_dim < 1 || head_dim > 2 * ATT_TILE || n_heads > 65535 || n_heads % n_kv_heads)
+    if (head_dim < 1 || head_dim > 2 * ATT_THREADS || n_heads > 65535 || n_heads % n_kv_heads)
         return (int)cudaErrorInvalidValue;
-    const size_t smem = ATT_TILE * (sizeof(long) + sizeof(float)) + (size_t)head_dim * sizeof(float);
-    dim3 grid(n_tokens, n_heads);
-    FL_DISPATCH(dtype, T, return fl_launch(paged_attention_simt_kernel<T>, grid, dim3(ATT_TILE), smem, stream,
-                                           (const T*)q, q_ld, (T*)out, out_ld, (const T*)k_cache,
-                                           (const T*)v_cache, page_stride, page_size, block_table, bt_stride,
-                                           tok_req, positions, n_heads, n_kv_heads, head_dim, window, scale));
-    return 0;
+    // As many CTAs a cluster as keep the launch within two CTAs an SM or so: more only wait for one another.
+    const long units = (long)((n_tokens + (single ? 0 : 7)) / (single ? 1 : 8)) * n_heads;
+    const int cl = units * 4 <= 2L * sms ? 8 : units <= sms ? 4 : units <= 2L * sms ? 2 : 1;
+#define ATT_GO(QT, CL)                                                                                                    \
+    FL_DISPATCH(dtype, T, return (att_launch<T, QT, CL>((const T*)q, q_ld, (T*)out, out_ld, (const T*)k_cache,            \
+                                                        (const T*)v_cache, page_stride, page_size, block_table, bt_stride, \
+                                                        tok_req, positions, n_tokens, n_heads, n_kv_heads, head_dim,      \
+                                                        window, scale, stream)))
+    if (single) {
+        if (cl == 8) ATT_GO(1, 8);
+        if (cl == 4) ATT_GO(1, 4);
+        if (cl == 2) ATT_GO(1, 2);
+        ATT_GO(1, 1);
+    }
+    if (cl == 8) ATT_GO(8, 8);
+    if (cl == 4) ATT_GO(8, 4);
+    if (cl == 2) ATT_GO(8, 2);
+    ATT_GO(8, 1);
+#undef ATT_GO
 }

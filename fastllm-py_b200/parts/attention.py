@@ -157,4 +157,4 @@ class Attention(Part):
         else:
             ops.paged_attention_simt(q, ctx, cache.tensor, cache.block_table, step.tok_req,
                                      step.positions, self.heads, self.kv_heads, self.head_dim,
-                                     self.window, self.scale, cache.page_size)
+                                     self.window, self.scale, cache.page_size, single=step.max_q_len == 1)

@@ -390,6 +390,29 @@ def run_fast_cuda_core_decode(case, window=None):
     return run_fast(case, window, 0, 1)
 
 
+@pytest.mark.parametrize("head_dim, window, dtype", [(128, None, torch.float32), (48, 100, torch.float32),
+                                                     (256, None, torch.float32), (128, 70, torch.bfloat16)])
+def test_cuda_core_attention_order(head_dim, window, dtype):
+    """A token's result is the same bit for bit whether neighbours share its tiles or not and for every number of CTAs
+    that the tiles are dealt out to (16 heads: 330, 100, 70 and 16 tokens take 1, 2, 4 and 8 CTAs, 330, 18, 9 and 4
+    single ones too), where requests meet inside a group of eight, and it is right."""
+    from fastllm_py_b200.native import ops
+
+    case = AttentionCase([203, 1, 126], [700, 63, 0], 16, 4, head_dim, 16, dtype, seed=3)
+
+    def run(a, b, single):
+        out = torch.zeros_like(case.q[a:b])
+        ops.paged_attention_simt(case.q[a:b], out, case.cache, case.block_table, case.tok_req[a:b], case.positions[a:b],
+                                 case.heads, case.kv_heads, head_dim, window, head_dim ** -0.5, case.page_size, single)
+        return out
+
+    base = run(0, 330, False)
+    assert float((base.float().cpu() - case.reference(window)).abs().max()) <= case.tolerance()
+    for a, n in ((0, 330), (190, 100), (130, 100), (200, 16), (145, 70), (196, 18), (198, 9), (201, 4), (329, 1)):
+        for single in (False, True):
+            assert torch.equal(run(a, a + n, single), base[a:a + n]), (a, n, single)
+
+
 @pytest.mark.parametrize("runner", [run_simt, run_fast, run_fast_tcgen05, run_fast_cuda_core_decode])
 def test_a_far_key_among_hundreds_is_found(runner):
     """One key far back (and one right at a page edge, one at a split edge) gets
