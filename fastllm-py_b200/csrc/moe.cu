@@ -18,7 +18,7 @@
 // steps, where tokens are few and the matrices stream from memory.  A token's weight multiplies its expert's output, or
 // (weight_on_input) what the expert reads: the gate and up sums then, which are linear in it, before the activation.  All sums are float and depend only
 // on the token itself.
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 // One warp per token; z: float logits [n_tokens, experts] (the router's product, made by the caller).
 template <typename TW>
@@ -204,277 +204,440 @@ FL_API int fl_moe_experts(const void* h, int dtype, long h_ld, const void* w_gu,
 
 // ----------------------------------------------------------------- many tokens: grouped products
 // With many tokens the per-token kernels above would read each expert's matrices once per token.  Here
-// the (token, choice) pairs are ordered by expert, each expert's rows padded to whole tiles of 64, and
-// two tensor-core products run over the tiles: a tile's rows share one expert's matrix.
+// the (token, choice) pairs are ordered by expert, and two tensor-core products run over tiles of up to 256 pairs
+// that share an expert's matrix.
 //
-//   moe_sort        one block: counts per expert, padded offsets, row -> pair, pair -> row, tile -> expert
-//   moe_group_mma   bfloat16 mma.sync m16n8k16, 64 rows x 128 weight rows per block, K in steps of 32 through
-//                   a three-stage cp.async ring.  GATED: the 128 weight rows are 64 gate rows and the 64 up rows
-//                   of the same features, A rows are gathered token rows, the epilogue writes act(g) * u
-//                   (bfloat16, in row order); UP: experts without a gate, A gathered, 128 up rows, the epilogue
-//                   writes the unit's f(x, 1); DOWN: A is that buffer and the output float [rows, width]
+//   moe_sort        one block: counts per expert, row -> pair, pair -> row, and the list of tiles: an expert's rows are
+//                   cut into as few tiles of at most 256 as will do, equally wide (a multiple of 64)
+//   moe_gather      the tokens' rows in the order of the pairs
+//   moe_group       tcgen05.mma over CTA pairs.  GATED: a pair's 256 weight rows are 128 gate rows and the 128 up rows of
+//                   the same features, the epilogue writes f(g, u) (bfloat16, in row order); UP: experts without a gate,
+//                   256 up rows, the epilogue writes the unit's f(x, 1); DOWN: A is that buffer and the output
+//                   float [rows, width]
 //   moe_combine     out[t] = sum_k weight[t, k] * y[row of pair (t, k)], in order of choice
 //
 // A row's sums do not depend on the other rows of its tile, so the order of rows within an expert (it
 // comes from atomics) does not show in the results.
-#define MOE_TM 64
+#define MOE_TN 256               // rows (pairs) of a tile at most
+
+struct MoeTile {
+    int expert, row0, rows, n;   // n: rows in the MMA, a multiple of 64
+};
 
 __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ chosen, int n_pairs, int experts,
                                                        int* __restrict__ row_pair, int* __restrict__ pair_row,
-                                                       int* __restrict__ tile_expert, int* __restrict__ n_tiles_out,
-                                                       int max_tiles) {
+                                                       int4* __restrict__ tiles, int* __restrict__ n_tiles_out) {
     pdl_wait();
     pdl_trigger();
-    extern __shared__ int sort_s[];                      // [experts] counts -> cursors, [experts + 1] first rows
-    int* count = sort_s;
-    int* first = sort_s + experts;
+    extern __shared__ int count[];                       // [experts] counts, then cursors
     for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
     __syncthreads();
     for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) atomicAdd(&count[chosen[p]], 1);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int at = 0;
-        for (int e = 0; e < experts; ++e) {
-            first[e] = at;
-            const int tiles = (count[e] + MOE_TM - 1) / MOE_TM;
-            for (int i = 0; i < tiles; ++i) tile_expert[at / MOE_TM + i] = e;
-            at += tiles * MOE_TM;
-            count[e] = 0;
+    if (threadIdx.x < 32) {                              // running sums of rows and tiles, 32 experts at a time
+        const int lane = threadIdx.x;
+        int rows_before = 0, tiles_before = 0;
+        for (int e0 = 0; e0 < experts; e0 += 32) {
+            const int c = e0 + lane < experts ? count[e0 + lane] : 0, nt = (c + MOE_TN - 1) / MOE_TN;
+            int row = c, tile = nt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int r = __shfl_up_sync(0xffffffffu, row, o), t = __shfl_up_sync(0xffffffffu, tile, o);
+                if (lane >= o) row += r, tile += t;
+            }
+            const int first = rows_before + row - c, at = tiles_before + tile - nt;
+            if (e0 + lane < experts) count[e0 + lane] = first;
+            const int n = nt > 0 ? ((c + nt - 1) / nt + 63) / 64 * 64 : 0;
+            for (int i = 0; i < nt; ++i) tiles[at + i] = make_int4(e0 + lane, first + i * n, min(n, c - i * n), n);
+            rows_before += __shfl_sync(0xffffffffu, row, 31);
+            tiles_before += __shfl_sync(0xffffffffu, tile, 31);
         }
-        first[experts] = at;
-        *n_tiles_out = at / MOE_TM;
+        if (lane == 0) *n_tiles_out = tiles_before;
     }
     __syncthreads();
-    const int total = first[experts];
-    for (int r = threadIdx.x; r < max_tiles * MOE_TM; r += blockDim.x) row_pair[r] = -1;
-    __syncthreads();
     for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {
-        const int e = chosen[p];
-        const int r = first[e] + atomicAdd(&count[e], 1);
+        const int r = atomicAdd(&count[chosen[p]], 1);
         row_pair[r] = p;
         pair_row[p] = r;
     }
-    (void)total;
 }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
-
-#define MOE_BK 32
-#define MOE_STAGES 3
-#define MOE_PITCH (MOE_BK + 8)   // bfloat16 elements between rows of a staged tile: ldmatrix without bank conflicts
-#define MOE_PIECES (MOE_BK / 32) // 16-byte pieces of a row that a thread copies per stage
-#define MOE_SMEM (MOE_STAGES * (MOE_TM + 128) * MOE_PITCH * 2)
-
-// grid: (tiles of rows, blocks of 64 features (GATED) or 128 columns).  K % 32 == 0, rows 16-byte aligned.
-enum { MOE_DOWN = 0, MOE_GATED = 1, MOE_UP = 2 };
-template <int MODE>
-__global__ void __launch_bounds__(256) moe_group_mma_kernel(
-    const bf16* __restrict__ a, long a_ld, const bf16* __restrict__ w, int n_out, int K, const int* __restrict__ row_pair,
-    const int* __restrict__ tile_expert, const int* __restrict__ n_tiles, int top, bf16* __restrict__ act_out,
-    float* __restrict__ y_out, long out_ld, FlGate act, const float* __restrict__ in_weights) {
+// a[r] = h[token of row r]: 16 bytes a thread (a pass of its own costs 2 x rows x width bytes, 10 us at 8192 rows of 2048;
+// in return the products fetch both operands with plain TMA boxes; measured with its launch: 16 us)
+__global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict__ h, long h_ld, const int* __restrict__ row_pair,
+                                                         int n_pairs, int top, bf16* __restrict__ a, int width) {
     pdl_wait();
     pdl_trigger();
-    constexpr bool GATED = MODE == MOE_GATED;
-    extern __shared__ __align__(16) unsigned char moe_smem[];
-    bf16 (*a_s)[MOE_TM][MOE_PITCH] = reinterpret_cast<bf16 (*)[MOE_TM][MOE_PITCH]>(moe_smem);
-    bf16 (*w_s)[128][MOE_PITCH] = reinterpret_cast<bf16 (*)[128][MOE_PITCH]>(moe_smem + MOE_STAGES * MOE_TM * MOE_PITCH * 2);
-    __shared__ int pair_s[MOE_TM];
-    const int tile = blockIdx.x;
-    if (tile >= *n_tiles) return;
-    const int e = tile_expert[tile];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp >> 2, wn = warp & 3;                    // 2 x 4 warps: 32 rows x (GATED: 16 + 16, else 32) columns
-    if (tid < MOE_TM) pair_s[tid] = row_pair[tile * MOE_TM + tid];
-    __syncthreads();
-    // sources of this thread's 16-byte pieces of a stage: its part of one row of A and of two rows of W
-    const int ar = tid >> 2, ac = (tid & 3) * 8 * MOE_PIECES;
-    const bf16* a_src;
-    if (MODE != MOE_DOWN) {
-        const int pair = pair_s[ar];
-        a_src = a + (long)(pair < 0 ? 0 : pair / top) * a_ld + ac;
-    } else {
-        a_src = a + ((long)tile * MOE_TM + ar) * a_ld + ac;
-    }
-    const bf16* w_src[2];
-    bool w_ok[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int wr = (tid >> 2) + i * 64;
-        long row;                                               // row of this expert's matrix
-        if (GATED) {
-            const int f = blockIdx.y * 64 + (wr & 63);          // rows 0..63 gate features, 64..127 their up rows
-            w_ok[i] = f < n_out;
-            row = (long)e * 2 * n_out + (wr < 64 ? 0 : n_out) + (w_ok[i] ? f : 0);
-        } else {
-            const int c = blockIdx.y * 128 + wr;
-            w_ok[i] = c < n_out;
-            row = (long)e * n_out + (w_ok[i] ? c : 0);
-        }
-        w_src[i] = w + row * K + ac;
-    }
-    auto stage = [&](int buf, int k0) {
-#pragma unroll
-        for (int half = 0; half < MOE_PIECES; ++half) {
-            cp_async16(&a_s[buf][ar][ac + half * 8], a_src + k0 + half * 8);
-#pragma unroll
-            for (int i = 0; i < 2; ++i) cp_async16(&w_s[buf][(tid >> 2) + i * 64][ac + half * 8], w_src[i] + k0 + half * 8);
-        }
-        cp_async_commit();
-    };
-    float acc[2][4][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) acc[i][j][c] = 0.0f;
-    const int n_k = K / MOE_BK;
-    stage(0, 0);
-    if (n_k > 1) stage(1, MOE_BK);
-    for (int kb = 0; kb < n_k; ++kb) {
-        const int buf = kb % MOE_STAGES;
-        if (kb + 1 < n_k) cp_async_wait<1>(); else cp_async_wait<0>();
-        __syncthreads();                                            // stage kb has landed; stage kb - 1 is read by no one
-        if (kb + 2 < n_k) stage((kb + 2) % MOE_STAGES, (kb + 2) * MOE_BK);
-#pragma unroll
-        for (int ks = 0; ks < MOE_BK; ks += 16) {
-            unsigned af[2][4], bfr[4][2];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const bf16* p = &a_s[buf][wm * 32 + i * 16 + (lane & 15)][ks + (lane >> 4) * 8];
-                const unsigned s = (unsigned)__cvta_generic_to_shared(p);
-                asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(af[i][0]), "=r"(af[i][1]), "=r"(af[i][2]), "=r"(af[i][3]) : "r"(s));
-            }
-#pragma unroll
-            for (int j2 = 0; j2 < 2; ++j2) {
-                // GATED: column blocks 0, 1 are 16 gate features, 2, 3 the same features' up rows
-                const int n0 = GATED ? (j2 * 64 + wn * 16) : (wn * 32 + j2 * 16);
-                const bf16* p = &w_s[buf][n0 + (lane & 7) + (lane >> 4) * 8][ks + ((lane >> 3) & 1) * 8];
-                const unsigned s = (unsigned)__cvta_generic_to_shared(p);
-                asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(bfr[j2 * 2][0]), "=r"(bfr[j2 * 2][1]), "=r"(bfr[j2 * 2 + 1][0]), "=r"(bfr[j2 * 2 + 1][1])
-                             : "r"(s));
-            }
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                                 : "+f"(acc[i][j][0]), "+f"(acc[i][j][1]), "+f"(acc[i][j][2]), "+f"(acc[i][j][3])
-                                 : "r"(af[i][0]), "r"(af[i][1]), "r"(af[i][2]), "r"(af[i][3]), "r"(bfr[j][0]), "r"(bfr[j][1]));
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int r = wm * 32 + i * 16 + (lane >> 2) + half * 8;
-            const long row = (long)tile * MOE_TM + r;
-            float win = 1.0f;                                   // what multiplies the row's input
-            if (MODE != MOE_DOWN && in_weights != nullptr) win = pair_s[r] < 0 ? 0.0f : in_weights[pair_s[r]];
-            if (GATED) {
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-#pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        const int f = blockIdx.y * 64 + wn * 16 + j * 8 + (lane & 3) * 2 + c;
-                        if (f < n_out)
-                            act_out[row * out_ld + f] = __float2bfloat16_rn(fl_gated(acc[i][j][half * 2 + c] * win,
-                                                                                     acc[i][j + 2][half * 2 + c] * win, act));
-                    }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-#pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        const int col = blockIdx.y * 128 + wn * 32 + j * 8 + (lane & 3) * 2 + c;
-                        if (col >= n_out) continue;
-                        if (MODE == MOE_UP) act_out[row * out_ld + col] = __float2bfloat16_rn(fl_gated(acc[i][j][half * 2 + c] * win, 1.0f, act));
-                        else y_out[row * out_ld + col] = acc[i][j][half * 2 + c];
-                    }
-            }
-        }
+    const int per_row = width / 8;
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = (int)(i / per_row), c = (int)(i - (long)r * per_row) * 8;
+    if (r >= n_pairs) return;
+    *reinterpret_cast<uint4*>(a + (long)r * width + c) = *reinterpret_cast<const uint4*>(h + (long)(row_pair[r] / top) * h_ld + c);
 }
 
+// The CTA-pair product of gemm_tcgen05.cu (see there for the roles, the barriers and why a pair) over the list of tiles:
+// a unit of work is (tile, 256 weight rows), weight rows going fastest so that a tile's rows stay in L2 while its
+// expert's matrix streams by once; a tile's width is its own, so the MMA's N, the 32-row boxes of A and the bytes of a
+// stage are per unit.  64 rows x 128 weight rows a block on mma.sync took 452 + 300 us for 8192 pairs, 32 experts of
+// 2048 x 1408 (142 GFLOP: 190 TFLOP/s), its operands fetched six times as often from L2; this takes 119 + 66 us (770
+// TFLOP/s).  The accumulator's bits are the same: K in steps of 16 from the first to the last.
+enum { MOE_DOWN = 0, MOE_GATED = 1, MOE_UP = 2 };
+enum { MOE_ERR_WAIT = 131 };
+
+// g[j] = f(g[j], v[j]) as `fl_gated` has it (the exact exponential and division), the unit chosen once for all N values
+template <int N> __device__ __forceinline__ void moe_act(float (&g)[N], const float (&v)[N], const FlGate act) {
+#define MOE_ACT(ACT)                                                                                 \
+    {                                                                                                \
+        _Pragma("unroll") for (int j = 0; j < N; ++j) g[j] = fl_gated(g[j], v[j], FlGate{ACT, act.p0, act.p1}); \
+    }
+    switch (act.act) {
+        case FL_ACT_RELU: MOE_ACT(FL_ACT_RELU) break;
+        case FL_ACT_RELU_SQUARED: MOE_ACT(FL_ACT_RELU_SQUARED) break;
+        case FL_ACT_GELU_TANH: MOE_ACT(FL_ACT_GELU_TANH) break;
+        case FL_ACT_CLAMPED_SWISH: MOE_ACT(FL_ACT_CLAMPED_SWISH) break;
+        default: MOE_ACT(FL_ACT_SILU)
+    }
+#undef MOE_ACT
+}
+
+#define MOE_EPILOGUE_BYTES (2 * 32 * 128 * 4)            // GATED: 2 x (32 x 64 up values | 32 x 64 results); else 2 x 32 x 128
+#define MOE_SMEM (Tc2<256>::SMEM + MOE_EPILOGUE_BYTES + 2 * 32 * 4)
+
+template <int MODE>
+__global__ void __launch_bounds__(TC_THREADS) moe_group_kernel(
+    const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const int4* __restrict__ tiles,
+    const int* __restrict__ n_tiles, const int* __restrict__ row_pair, int n_out, int K, bf16* __restrict__ act_out,
+    float* __restrict__ y_out, FlGate act, const float* __restrict__ in_weights, int* __restrict__ status) {
+    using L = Tc2<256>;
+    constexpr bool GATED = MODE == MOE_GATED;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* ring = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* full_bar = (uint64_t*)(ring + L::TILE_BYTES);
+    uint64_t* empty_bar = full_bar + L::STAGES;
+    uint64_t* acc_full = empty_bar + L::STAGES;
+    uint64_t* acc_empty = acc_full + 2;
+    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    unsigned char* staged = ring + L::TILE_BYTES + 256;
+    float* win_s = reinterpret_cast<float*>(staged + MOE_EPILOGUE_BYTES);          // [2][32] what multiplies a row's input
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();                   // 0: leader
+    const int pair = (int)blockIdx.x >> 1, num_pairs = (int)gridDim.x >> 1;
+    const int num_kb = (K + TC_BK - 1) / TC_BK;
+    constexpr int FEATURES = GATED ? 128 : 256;             // of a unit; half of them are this CTA's
+    const int tiles_n = (n_out + FEATURES - 1) / FEATURES;
+    const int num_units = *n_tiles * tiles_n;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < L::STAGES; ++s) {
+            mbar_init(&full_bar[s], 1);
+            mbar_init(&empty_bar[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], 8);                    // four epilogue warps in each of the two CTAs
+        }
+        *abort_flag = (*(volatile int*)status != 0) ? 1 : 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(512u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();                                     // both CTAs' barriers exist before anyone signals them
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    // (launched in plain stream order, and no pdl_trigger: see the pair kernel of gemm_tcgen05.cu)
+
+    auto give_up = [&]() {
+        if (!*abort_flag) { *abort_flag = 1; atomicCAS(status, 0, MOE_ERR_WAIT); }
+    };
+    if (warp == 0) {
+        if (lane == 0 && !*abort_flag) {
+            // ---- producer (both CTAs): this CTA's 128 weight rows and half of the tile's rows, k-block after k-block
+            int s = 0;
+            uint32_t ph = 0;
+            bool ok = true;
+            for (int u = pair; u < num_units && ok; u += num_pairs) {
+                const int4 t = tiles[u / tiles_n];
+                const int tn = u % tiles_n, half = t.w / 2;
+                for (int kb = 0; kb < num_kb; ++kb) {
+                    if (!mbar_wait(&empty_bar[s], ph ^ 1u, abort_flag)) {
+                        give_up();
+                        ok = false;
+                        break;
+                    }
+                    unsigned char* dst = ring + s * L::STAGE_BYTES;
+                    if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * (L::W_BYTES + half * TC_BK * 2));
+                    if (GATED) {                            // 64 gate rows and the 64 up rows of the same features
+                        const int f0 = t.x * 2 * n_out + tn * 128 + (int)rank * 64;
+                        tma_load_2d_pair(dst, &map_w, &full_bar[s], kb * TC_BK, f0);
+                        tma_load_2d_pair(dst + L::W_BYTES / 2, &map_w, &full_bar[s], kb * TC_BK, f0 + n_out);
+                    } else {
+                        tma_load_2d_pair(dst, &map_w, &full_bar[s], kb * TC_BK, t.x * n_out + tn * 256 + (int)rank * 128);
+                    }
+                    for (int r = 0; r < half; r += 32)
+                        tma_load_2d_pair(dst + L::W_BYTES + r * TC_BK * 2, &map_a, &full_bar[s], kb * TC_BK,
+                                         t.y + (int)rank * half + r);
+                    if (++s == L::STAGES) { s = 0; ph ^= 1u; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {
+            // ---- MMA issuer (leader only): one 256 x n x 16 MMA per 16 columns of K, for both CTAs
+            int s = 0, i = 0;
+            uint32_t ph = 0;
+            bool ok = !*abort_flag;
+            for (int u = pair; u < num_units && ok; u += num_pairs, ++i) {
+                const uint32_t idesc = instr_desc_bf16(256, tiles[u / tiles_n].w);
+                const int buf = i & 1;
+                const uint32_t use = (uint32_t)(i >> 1);
+                if (!mbar_wait(&acc_empty[buf], (use & 1u) ^ 1u, abort_flag)) {
+                    give_up();
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * 256);
+                for (int kb = 0; kb < num_kb; ++kb) {
+                    if (!mbar_wait(&full_bar[s], ph, abort_flag)) {
+                        give_up();
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t w_addr = smem_u32(ring + s * L::STAGE_BYTES);
+                    const uint64_t adesc = smem_desc_sw128(w_addr);
+                    const uint64_t bdesc = smem_desc_sw128(w_addr + L::W_BYTES);
+#pragma unroll
+                    for (int k = 0; k < TC_BK / 16; ++k)
+                        umma_bf16_pair(tmem_acc, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc,
+                                       (kb > 0 || k > 0) ? 1u : 0u);
+                    umma_commit_pair(&empty_bar[s]);
+                    if (++s == L::STAGES) { s = 0; ph ^= 1u; }
+                }
+                if (ok) umma_commit_pair(&acc_full[buf]);
+            }
+        }
+    } else {
+        // ---- epilogue warps 2..5 of both CTAs: this CTA's 128 accumulator rows of the unit, 32 tile rows at a time
+        const int quarter = warp & 3, e = quarter * 32 + lane;
+        uint32_t rounds_out = 0;                            // picks the staging half
+        int i = 0;
+        for (int u = pair; u < num_units; u += num_pairs, ++i) {
+            const int buf = i & 1;
+            const uint32_t use = (uint32_t)(i >> 1);
+            if (!mbar_wait(&acc_full[buf], use & 1u, abort_flag)) give_up();
+            epilogue_sync();                                // the four warps decide together (they share barriers below)
+            if (*abort_flag) break;
+            tc_fence_after();
+            const int4 t = tiles[u / tiles_n];
+            const int f0 = (u % tiles_n) * FEATURES + (int)rank * (FEATURES / 2), cols = n_out - f0;
+            const uint32_t t_base = tmem_base + (uint32_t)(buf * 256) + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll 1
+            for (int c = 0; c < t.z; c += 32) {
+                const int rows = min(32, t.z - c);
+                uint32_t r[32];
+                tmem_ld16(t_base + (uint32_t)c, r);
+                tmem_ld16(t_base + (uint32_t)c + 16u, r + 16);
+                const uint32_t half = rounds_out++ & 1u;
+                float* win = win_s + half * 32;
+                if (MODE != MOE_DOWN && in_weights != nullptr && quarter == 0)
+                    win[lane] = lane < rows ? in_weights[row_pair[t.y + c + lane]] : 0.0f;
+                unsigned char* area = staged + half * (MOE_EPILOGUE_BYTES / 2);
+                tmem_ld_wait();
+                if constexpr (GATED) {
+                    // accumulator lanes 0..63: gate features, 64..127: the same features' up values; the gate warps
+                    // finish the even rows, the up warps the odd ones, trading values through shared memory
+                    const bool is_up = quarter >= 2;
+                    const int mine = is_up ? 1 : 0, col = (quarter & 1) * 32 + lane;
+                    float* x = reinterpret_cast<float*>(area);
+                    bf16* st = reinterpret_cast<bf16*>(area + 32 * 64 * 4);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        x[(2 * j + 1 - mine) * 64 + col] = __uint_as_float(is_up ? r[2 * j] : r[2 * j + 1]);
+                    epilogue_sync();
+                    float g[16], v[16];                     // rows 2 j + mine
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        const float own = __uint_as_float(is_up ? r[2 * j + 1] : r[2 * j]), other = x[(2 * j + mine) * 64 + col];
+                        g[j] = is_up ? other : own;
+                        v[j] = is_up ? own : other;
+                    }
+                    if (in_weights != nullptr) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const float w = win[2 * j + mine];
+                            g[j] *= w;
+                            v[j] *= w;
+                        }
+                    }
+                    moe_act(g, v, act);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) st[(2 * j + mine) * 64 + col] = __float2bfloat16_rn(g[j]);
+                    epilogue_sync();
+                    if (cols > 0)
+                        tc_copy_rows<bf16, 64>(act_out + (long)(t.y + c) * n_out + f0, n_out, st, rows, min(cols, 64), e, true);
+                } else if constexpr (MODE == MOE_UP) {
+                    if (in_weights != nullptr) epilogue_sync();
+                    float g[32], one[32];
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        g[j] = __uint_as_float(r[j]) * (in_weights != nullptr ? win[j] : 1.0f);
+                        one[j] = 1.0f;
+                    }
+                    moe_act(g, one, act);
+                    bf16* st = reinterpret_cast<bf16*>(area);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) st[j * 128 + e] = __float2bfloat16_rn(g[j]);
+                    epilogue_sync();
+                    if (cols > 0)
+                        tc_copy_rows<bf16, 128>(act_out + (long)(t.y + c) * n_out + f0, n_out, st, rows, min(cols, 128), e, true);
+                } else {
+                    float* st = reinterpret_cast<float*>(area);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) st[j * 128 + e] = __uint_as_float(r[j]);
+                    epilogue_sync();
+                    if (cols > 0)
+                        tc_copy_rows<float, 128>(y_out + (long)(t.y + c) * n_out + f0, n_out, st, rows, min(cols, 128), e, true);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_leader(&acc_empty[buf]);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();                                     // the peer is done with this CTA's barriers and memory
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    }
+    cluster_sync_all();                                     // both have given their tensor memory back before either leaves
+}
+
+// Four columns a thread and the rows of all choices asked for at once: one column a thread, each load behind its row's
+// index, took 62 us for 2048 tokens x 4 choices of 2048 columns (67 MB); this takes 12.
 template <typename T>
 __global__ void __launch_bounds__(256) moe_combine_kernel(const float* __restrict__ y, long y_ld, const int* __restrict__ pair_row,
                                                           const float* __restrict__ weights, T* __restrict__ out, long out_ld,
                                                           int width, int top, int accumulate) {
     pdl_wait();
     pdl_trigger();
-    const int t = blockIdx.x;
-    for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < width; c += gridDim.y * blockDim.x) {
-        float sum = 0.0f;
-        for (int k = 0; k < top; ++k) sum += (weights != nullptr ? weights[(long)t * top + k] : 1.0f) * y[(long)pair_row[(long)t * top + k] * y_ld + c];
-        out[(long)t * out_ld + c] = from_f32<T>(accumulate ? to_f32<T>(out[(long)t * out_ld + c]) + sum : sum);
+    const int t = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+    if (c >= width) return;
+    const int* rows = pair_row + (long)t * top;
+    const float* w = weights != nullptr ? weights + (long)t * top : nullptr;
+    float sum[4] = {};
+    for (int k0 = 0; k0 < top; k0 += 4) {                   // (width is a multiple of 32)
+        float4 v[4];
+        float wk[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (k0 + k >= top) continue;
+            v[k] = *reinterpret_cast<const float4*>(y + (long)rows[k0 + k] * y_ld + c);
+            wk[k] = w != nullptr ? w[k0 + k] : 1.0f;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (k0 + k >= top) continue;
+            sum[0] += wk[k] * v[k].x;
+            sum[1] += wk[k] * v[k].y;
+            sum[2] += wk[k] * v[k].z;
+            sum[3] += wk[k] * v[k].w;
+        }
     }
+    T* o = out + (long)t * out_ld + c;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = from_f32<T>(accumulate ? to_f32<T>(o[j]) + sum[j] : sum[j]);
 }
 
-// Rows of the ordered buffers a step of n_tokens needs: every expert may end with a partly filled tile.
+// Rows of the ordered buffers that a step of n_tokens is given: one a pair, and 64 an expert, which the products do not
+// need but the list of tiles (one for every 256 pairs and one per expert, 16 bytes each) does.
 FL_API long fl_moe_group_rows(int n_tokens, int top, int experts) {
-    return (((long)n_tokens * top + MOE_TM - 1) / MOE_TM + experts) * MOE_TM;
+    return (((long)n_tokens * top + 63) / 64 + experts) * 64;
 }
 
 // Does the grouped path take this problem?  (bfloat16 everywhere, K of both products a multiple of 32.)
 FL_API int fl_moe_group_takes(int dtype, int w_dtype, int width, int ff) {
-    return dtype == FL_BF16 && w_dtype == FL_BF16 && width % MOE_BK == 0 && ff % MOE_BK == 0;
+    return dtype == FL_BF16 && w_dtype == FL_BF16 && width % 32 == 0 && ff % 32 == 0;
 }
 
-static int moe_group_smem_ready() {
-    static int rc = -1;
-    if (rc < 0) {
-        rc = (int)cudaFuncSetAttribute(moe_group_mma_kernel<MOE_GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOE_SMEM);
-        if (rc == 0)
-            rc = (int)cudaFuncSetAttribute(moe_group_mma_kernel<MOE_DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOE_SMEM);
-        if (rc == 0)
-            rc = (int)cudaFuncSetAttribute(moe_group_mma_kernel<MOE_UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOE_SMEM);
-    }
-    return rc;
+template <int MODE>
+static int moe_group_launch(const void* a, const void* w, long w_rows, int n_pairs, int max_tiles, const int4* tiles, const int* n_tiles,
+                            const int* row_pair, int n_out, int K, void* act_out, float* y_out, FlGate act,
+                            const float* in_weights, int num_sms, int* status, cudaStream_t stream) {
+    auto kernel = moe_group_kernel<MODE>;
+    CUtensorMap map_w, map_a;
+    int rc = make_map(&map_w, w, w_rows, K, K, MODE == MOE_GATED ? 64 : 128);
+    if (rc == 0) rc = make_map(&map_a, a, n_pairs, K, K, 32);
+    if (rc == 0) rc = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MOE_SMEM);
+    if (rc) return rc;
+    static_assert(MOE_SMEM <= 232448, "more shared memory than a CTA can have");
+    const int features = MODE == MOE_GATED ? 128 : 256;
+    const long units = (long)max_tiles * ((n_out + features - 1) / features);
+    const int pairs = units < num_sms / 2 ? (int)units : num_sms / 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * pairs);
+    cfg.blockDim = dim3(TC_THREADS);
+    cfg.dynamicSmemBytes = MOE_SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, map_w, map_a, tiles, n_tiles, row_pair, n_out, K, (bf16*)act_out, y_out, act,
+                                   in_weights, status);
 }
 
-// ints: row_pair [rows] | pair_row [n_tokens * top] | tile_expert [rows / 64] | n_tiles [1];
-// act: bfloat16 [rows, ff]; y: float [rows, width].
+// ints: rows + n_tokens * top + rows / 64 + 1 of them, rows = fl_moe_group_rows: row -> pair, pair -> row, the list of tiles
+// (from a multiple of four) and its length, 2 pairs + pairs / 64 + 4 experts + 4 at most;
+// act: bfloat16 [rows, ff]; y: float [rows, width], which holds the gathered tokens before it holds the results.
 FL_API int fl_moe_experts_grouped(const void* h, long h_ld, const void* w_gu, const void* w_down, const int* chosen,
                                   const float* weights, int* ints, void* act, float* y, void* out, long out_ld,
                                   int n_tokens, int width, int ff, int top, int experts, int act_code, float act_p0, float act_p1,
-                                  int gated, int accumulate, int weight_on_input, cudaStream_t stream) {
+                                  int gated, int accumulate, int weight_on_input, int num_sms, int* status, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     const float* in_weights = weight_on_input ? weights : nullptr;
     if (act_code < 0 || act_code >= FL_ACT_COUNT) return (int)cudaErrorInvalidValue;
     const FlGate gate{act_code, act_p0, act_p1};
-    const long rows = fl_moe_group_rows(n_tokens, top, experts);
-    const int max_tiles = (int)(rows / MOE_TM);
+    const int n_pairs = n_tokens * top;
     int* row_pair = ints;
-    int* pair_row = row_pair + rows;
-    int* tile_expert = pair_row + (long)n_tokens * top;
-    int* n_tiles = tile_expert + max_tiles;
-    if ((size_t)(2 * experts + 1) * sizeof(int) > 48 * 1024 || ((uintptr_t)h % 16) || (h_ld % 8)) return (int)cudaErrorInvalidValue;
-    int rc = moe_group_smem_ready();
+    int* pair_row = ints + n_pairs;
+    int4* tiles = reinterpret_cast<int4*>(ints + (2L * n_pairs + 3) / 4 * 4);
+    const int max_tiles = n_pairs / MOE_TN + (experts < n_pairs ? experts : n_pairs);
+    int* n_tiles = reinterpret_cast<int*>(tiles + max_tiles);
+    if ((size_t)experts * sizeof(int) > 48 * 1024 || width % 32 || ff % 32 || num_sms < 2 ||
+        (((uintptr_t)h | (uintptr_t)ints | (uintptr_t)act | (uintptr_t)y) % 16) || (h_ld % 8))
+        return (int)cudaErrorInvalidValue;
+    int rc = fl_launch(moe_sort_kernel, dim3(1), dim3(1024), (size_t)experts * sizeof(int), stream, chosen, n_pairs, experts,
+                       row_pair, pair_row, tiles, n_tiles);
     if (rc) return rc;
-    rc = fl_launch(moe_sort_kernel, dim3(1), dim3(1024), (size_t)(2 * experts + 1) * sizeof(int), stream, chosen,
-                       n_tokens * top, experts, row_pair, pair_row, tile_expert, n_tiles, max_tiles);
+    const long pieces = (long)n_pairs * (width / 8);
+    rc = fl_launch(moe_gather_kernel, dim3((unsigned)((pieces + 255) / 256)), dim3(256), 0, stream, (const bf16*)h, h_ld,
+                   (const int*)row_pair, n_pairs, top, (bf16*)y, width);
     if (rc) return rc;
     if (gated)
-        rc = fl_launch(moe_group_mma_kernel<MOE_GATED>, dim3(max_tiles, (ff + 63) / 64), dim3(256), MOE_SMEM, stream, (const bf16*)h, h_ld,
-                       (const bf16*)w_gu, ff, width, (const int*)row_pair, (const int*)tile_expert, (const int*)n_tiles, top,
-                       (bf16*)act, (float*)nullptr, (long)ff, gate, in_weights);
+        rc = moe_group_launch<MOE_GATED>(y, w_gu, 2L * experts * ff, n_pairs, max_tiles, tiles, n_tiles, row_pair, ff, width, act,
+                                         nullptr, gate, in_weights, num_sms, status, stream);
     else
-        rc = fl_launch(moe_group_mma_kernel<MOE_UP>, dim3(max_tiles, (ff + 127) / 128), dim3(256), MOE_SMEM, stream, (const bf16*)h, h_ld,
-                       (const bf16*)w_gu, ff, width, (const int*)row_pair, (const int*)tile_expert, (const int*)n_tiles, top,
-                       (bf16*)act, (float*)nullptr, (long)ff, gate, in_weights);
+        rc = moe_group_launch<MOE_UP>(y, w_gu, (long)experts * ff, n_pairs, max_tiles, tiles, n_tiles, row_pair, ff, width, act,
+                                      nullptr, gate, in_weights, num_sms, status, stream);
     if (rc) return rc;
-    rc = fl_launch(moe_group_mma_kernel<MOE_DOWN>, dim3(max_tiles, (width + 127) / 128), dim3(256), MOE_SMEM, stream,
-                   (const bf16*)act, (long)ff, (const bf16*)w_down, width, ff, (const int*)row_pair,
-                   (const int*)tile_expert, (const int*)n_tiles, top, (bf16*)nullptr, y, (long)width, gate, (const float*)nullptr);
+    rc = moe_group_launch<MOE_DOWN>(act, w_down, (long)experts * width, n_pairs, max_tiles, tiles, n_tiles, row_pair, width, ff,
+                                    nullptr, y, gate, nullptr, num_sms, status, stream);
     if (rc) return rc;
-    int col_blocks = (width + 255) / 256;
-    if (col_blocks > 8) col_blocks = 8;
-    return fl_launch(moe_combine_kernel<bf16>, dim3(n_tokens, col_blocks), dim3(256), 0, stream, (const float*)y,
+    return fl_launch(moe_combine_kernel<bf16>, dim3(n_tokens, (width + 1023) / 1024), dim3(256), 0, stream, (const float*)y,
                      (long)width, (const int*)pair_row, weight_on_input ? nullptr : weights, (bf16*)out, out_ld, width, top, accumulate);
 }

@@ -1251,7 +1251,7 @@ def moe_experts(h, w_gate_up, w_down, chosen, weights, act_buf, out, activation=
 
 
 def moe_group_rows(n_tokens: int, top: int, experts: int) -> int:
-    """Rows of the expert-ordered buffers for a step of `n_tokens` (every expert's rows end on a tile)."""
+    """Rows of the expert-ordered buffers for a step of `n_tokens`."""
     fn = load_library("moe").fl_moe_group_rows
     fn.argtypes, fn.restype = [c_int, c_int, c_int], c_long
     return int(fn(n_tokens, top, experts))
@@ -1269,7 +1269,7 @@ def moe_group_takes(h_dtype, w_dtype, width: int, ff: int) -> bool:
 def moe_experts_grouped(h, w_gate_up, w_down, chosen, weights, ints, act, y, out, activation="silu", params=(0.0, 0.0),
                         gated=True, accumulate=False, weight_on_input=False):
     """The same sum as `moe_experts` for many tokens: pairs ordered by expert, two tensor-core products
-    over tiles of 64 rows, then the weighted sum per token.  All bfloat16; `ints` int32
+    over tiles of up to 256 rows, then the weighted sum per token.  All bfloat16; `ints` int32
     [rows + N * top + rows / 64 + 1], `act` bfloat16 [rows, ff], `y` float32 [rows, width] with
     rows = moe_group_rows(N, top, experts).  `gated=False` and `weight_on_input`: as in
     `moe_experts`."""
@@ -1279,11 +1279,12 @@ def moe_experts_grouped(h, w_gate_up, w_down, chosen, weights, ints, act, y, out
         ff2 *= 2
     fn = _fn("moe", "fl_moe_experts_grouped", [c_void_p, c_long, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                                c_void_p, c_void_p, c_void_p, c_long, c_int, c_int, c_int, c_int, c_int,
-                                               c_int, c_float, c_float, c_int, c_int, c_int, c_void_p])
+                                               c_int, c_float, c_float, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    from .gemm_tc import status_word
     _check(fn(_ptr(h), _ld(h), _ptr(w_gate_up), _ptr(w_down), _ptr(chosen), _ptr(weights), _ptr(ints), _ptr(act),
               _ptr(y), _ptr(out), _ld(out), h.shape[0], width, ff2 // 2, chosen.shape[1], experts,
               activation_code(activation), float(params[0]), float(params[1]), int(gated), int(accumulate),
-              int(weight_on_input), _stream()), "moe_experts_grouped", 4)
+              int(weight_on_input), _sms(h.device), _ptr(status_word(h.device)), _stream()), "moe_experts_grouped", 5)
 
 
 # -------------------------------------------------------------- rope + cache

@@ -20,7 +20,7 @@ Two ways through the experts.  Few tokens (decode steps): one launch over
 (token, choice) pairs, each streaming its expert's rows; the matrices are read
 about once and the step is bound by that.  Many tokens in bfloat16: the pairs
 are ordered by expert on the device and two tensor-core products run over tiles
-of 64 rows that share an expert (`GROUP_FROM` pairs and up).  Neither path asks
+of up to 256 rows that share an expert (`GROUP_FROM` pairs and up).  Neither path asks
 the host anything, so steps with this part can be captured.
 """
 from __future__ import annotations

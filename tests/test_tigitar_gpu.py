@@ -262,6 +262,45 @@ def test_command_line_on_a_random_weights_folder(tmp_path):
 
 # ------------------------------------------------------------------ kernels alone
 
+@pytest.mark.parametrize("width, ff, counts, top, gated, on_input", [
+    (32, 32, [1], 1, True, False), (96, 160, [255, 0, 257, 1], 1, True, True), (256, 224, [64, 65, 256, 600], 2, True, False),
+    (544, 416, [300, 31, 513], 3, False, True), (128, 96, [3] * 70, 2, False, False), (2048, 1408, [250, 270, 8], 1, True, False)])
+def test_grouped_expert_products_against_64_bits(width, ff, counts, top, gated, on_input):
+    """Experts with one, few, many and no rows, at and beside the tiles' edges, in the order of the pairs or not.  What may
+    differ from 64 bits: the unit's result is rounded to bfloat16 (2^-9 of each term of the second product), the output
+    too, and float sums (2^-24 per term, far less)."""
+    from fastllm_py_b200.native import ops
+
+    g = torch.Generator(device="cuda").manual_seed(width + ff)
+    randn = lambda *shape: torch.randn(*shape, device="cuda", generator=g)
+    experts, n = len(counts), sum(counts)
+    flat = torch.cat([torch.full((c,), e) for e, c in enumerate(counts)]).cuda()
+    # choice 0 follows `counts`, the others go round the experts behind it
+    chosen = torch.stack([(flat + k) % experts for k in range(top)], 1).to(torch.int32)[torch.randperm(n, device="cuda", generator=g)].contiguous()
+    h = randn(n, width).to(torch.bfloat16)
+    up = (randn(experts, (2 if gated else 1) * ff, width) * width ** -0.5).to(torch.bfloat16)
+    down = (randn(experts, width, ff) * ff ** -0.5).to(torch.bfloat16)
+    weights = torch.rand(n, top, device="cuda", generator=g) + 0.1
+    want, size = torch.zeros(n, width, device="cuda", dtype=torch.float64), torch.zeros(n, width, device="cuda", dtype=torch.float64)
+    for k in range(top):
+        for e in range(experts):
+            at = (chosen[:, k] == e).nonzero()[:, 0]
+            w = weights[at, k:k + 1].double()
+            z = h[at].double() @ up[e].double().T * (w if on_input else 1.0)
+            a = torch.nn.functional.silu(z[:, :ff]) * z[:, ff:] if gated else torch.relu(z) ** 2
+            o = 1.0 if on_input else w
+            want[at] += o * (a @ down[e].double().T)
+            size[at] += o * (a.abs() @ down[e].double().abs().T)
+    rows = ops.moe_group_rows(n, top, experts)
+    ints = torch.empty(rows + n * top + rows // 64 + 1, dtype=torch.int32, device="cuda")
+    out = torch.empty(n, width, device="cuda", dtype=torch.bfloat16)
+    ops.moe_experts_grouped(h, up, down, chosen, weights, ints, torch.empty(rows, ff, device="cuda", dtype=torch.bfloat16),
+                            torch.empty(rows, width, device="cuda"), out, "silu" if gated else "relu_squared", gated=gated,
+                            weight_on_input=on_input)
+    off = (out.double() - want).abs()
+    assert bool((off <= 2.0 ** -8 * want.abs() + 1.1 * 2.0 ** -9 * size + 1e-5 * size.max()).all()), float((off / size).max())
+
+
 def test_grouped_expert_products_against_the_per_token_kernels():
     from fastllm_py_b200.native import ops
 
