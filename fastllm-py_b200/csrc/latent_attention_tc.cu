@@ -292,3 +292,405 @@ FL_API int fl_latent_attention_tc(const void* q, long q_ld, void* out, int out_d
                          (TO*)out, out_ld, heads, n_splits, sink));
     return 0;
 }
+
+// ----------------------------------------------------------------- prompts: tcgen05
+// Eight neighbouring tokens of a request x 16 heads are the 128 rows of tcgen05.mma, where the kernel above has 16 rows of
+// mma.sync: a cache row that has been fetched serves 8 tokens.  (Prompt of 2048 tokens, 16 heads, rank 512, window 1024:
+// 971 us with mma.sync, which fetched 1.8 GB of rows from L2 and kept its tensor cores 4 % busy, 416 us so.)  The sums are the other
+// kernel's, one by one: the same tiles of 32 keys, scores and value sums in K steps of 16 from the first to the last, the
+// weights' sums in the same tree, a rescaling at every tile where the maximum moved (where it did not, the other kernel
+// multiplies by one), so results are the same bit for bit.
+//
+// Tensor memory holds 512 columns, so a CTA accumulates LP_VC = 256 value columns at most, and the CTAs of a tile's two
+// halves both compute its scores.  Roles in a CTA of 320 threads:
+//   warps 0-3  a row's weights: scores from tensor memory, maximum, exponentials, the weights as bfloat16 back into tensor
+//              memory (the A operand of the second product)
+//   warps 4-7  the same rows' accumulators: rescaled (read, multiplied, written) while the exponentials are made; output
+//   warp 8     TMA: queries once, then the keys' pages, LP_STAGES tiles ahead; a page that no row sees is fetched from
+//              beyond the tensor, which gives zeros
+//   warp 9     the MMAs: scores of tile i + 1, then values of tile i
+// What bounds it: the keys' way through L2, two tiles being all that fits beside the queries (without the copies 243 us),
+// and the 36 narrow MMAs of a tile's scores (110 us); exponentials and rescaling cost 25 us together.
+#if LT_WIDTH % 64 == 0 && LAT_RANK % 64 == 0 && LT_WIDTH <= 576 && (LAT_RANK <= 256 || LAT_RANK == 512)
+#define LP_BUILT 1
+#include "tcgen05.cuh"
+
+#define LP_VC (LAT_RANK <= 256 ? LAT_RANK : 256)         // value columns of a CTA
+#define LP_HALVES (LAT_RANK / LP_VC)
+#define LP_ATOMS (LT_WIDTH / 64)                          // 64-column swizzle atoms of a row
+#define LP_STAGES 2
+#define LP_Q_ATOM (128 * 128)                             // bytes of an atom of the 128 query rows
+#define LP_K_ATOM (LT_KEYS * 128)
+#define LP_STAGE_BYTES (LP_ATOMS * LP_K_ATOM)
+#define LP_TOKENS 8
+#define LP_THREADS 320
+#define LP_SMEM (LP_ATOMS * LP_Q_ATOM + LP_STAGES * LP_STAGE_BYTES + 256 + 3 * 128 * 4 + 1024)
+enum { LP_ERR_WAIT = 141 };
+static_assert(LP_SMEM <= 232448, "more shared memory than a CTA can have");
+
+__device__ __forceinline__ void lp_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ bool lp_warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    uint32_t ok = 1;
+    if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, abort_flag) ? 1u : 0u;
+    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+__device__ __forceinline__ void lp_warp_arrive(uint64_t* bar) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) lp_arrive(bar);
+}
+__device__ __forceinline__ void lp_tma_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+        "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D[tmem] (+)= A[tmem] * B[smem]
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// the staged rows as the second product's B operand, the contiguous axis being its N: 64-column blocks of N an atom apart
+__device__ __forceinline__ uint64_t lp_desc_values(uint32_t saddr) {
+    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(LP_K_ATOM >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+           ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+
+template <typename TO>
+__global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
+    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, TO* __restrict__ out, long out_ld,
+    int page_size, int cache_rows, const int* __restrict__ block_table, int bt_stride, const int* __restrict__ req_start,
+    const int* __restrict__ req_ctx, const int* __restrict__ req_qlen, int n_requests, int window, float scale,
+    const float* __restrict__ sink, int* __restrict__ status) {
+    extern __shared__ unsigned char lp_raw[];
+    unsigned char* q_s = (unsigned char*)(((uintptr_t)lp_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* k_s = q_s + LP_ATOMS * LP_Q_ATOM;
+    uint64_t* bars = (uint64_t*)(k_s + LP_STAGES * LP_STAGE_BYTES);
+    uint64_t* q_full = bars;
+    uint64_t* k_full = bars + 1;                          // [LP_STAGES]
+    uint64_t* k_empty = k_full + LP_STAGES;
+    uint64_t* s_full = k_empty + LP_STAGES;               // [2]
+    uint64_t* c_full = s_full + 2;                        // [2] the rows' rescaling factors are there
+    uint64_t* p_full = c_full + 2;                        // [2] weights written and accumulators rescaled
+    uint64_t* o_done = p_full + 2;
+    uint32_t* tmem_slot = (uint32_t*)(o_done + 1);
+    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    volatile int* never = abort_flag + 1;                 // stays 0: for waits that must not be cut short
+    float* corr_s = reinterpret_cast<float*>((unsigned char*)bars + 256);                // [2][128]
+    float* inv_s = corr_s + 2 * 128;                                                     // [128]
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int req = -1, tile = 0;                               // a request's last (longest) tile first
+    for (int r = 0, acc = 0; r < n_requests; ++r) {
+        const int nt = (req_qlen[r] + LP_TOKENS - 1) / LP_TOKENS;
+        if ((int)blockIdx.x < acc + nt) {
+            req = r;
+            tile = nt - 1 - ((int)blockIdx.x - acc);
+            break;
+        }
+        acc += nt;
+    }
+    if (req < 0) return;
+    const int head0 = (int)(blockIdx.y / LP_HALVES) * 16, half = (int)(blockIdx.y % LP_HALVES);
+    const int ctx = req_ctx[req], tok0 = req_start[req] + tile * LP_TOKENS;
+    const int tokens = min(LP_TOKENS, req_qlen[req] - tile * LP_TOKENS);
+    const int pos_first = ctx + tile * LP_TOKENS, pos_last = pos_first + tokens - 1;
+    const int lo_first = window > 0 ? max(0, pos_first - window + 1) : 0;
+    const int t_begin = lo_first / LT_KEYS, n_tiles = pos_last / LT_KEYS + 1 - t_begin;
+
+    if (threadIdx.x == 0) {
+        mbar_init(q_full, 1);
+        for (int s = 0; s < LP_STAGES; ++s) {
+            mbar_init(&k_full[s], 1);
+            mbar_init(&k_empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&s_full[b], 1);
+            mbar_init(&c_full[b], 4);
+            mbar_init(&p_full[b], 8);
+        }
+        mbar_init(o_done, 1);
+        *abort_flag = (*(volatile int*)status != 0) ? 1 : 0;
+        *never = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 9) {
+        tmem_alloc(tmem_slot, 512u);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_o = *tmem_slot, tmem_s = tmem_o + 256;          // two score buffers of 32 columns
+    auto give_up = [&]() {
+        if (!*abort_flag) { *abort_flag = 1; atomicCAS(status, 0, LP_ERR_WAIT); }
+    };
+
+    if (warp == 8) {
+        // ---- producer: a lane issues one box, the part of a page that lies in the tile x 64 columns
+        const int* bt = block_table + (long)req * bt_stride;
+        const int box = min(page_size, LT_KEYS), boxes = LT_KEYS / box;
+        if (lane == 0 && !*abort_flag) {
+            mbar_expect_tx(q_full, LP_ATOMS * LP_Q_ATOM);
+            for (int a = 0; a < LP_ATOMS; ++a) lp_tma_3d(q_s + a * LP_Q_ATOM, &map_q, q_full, a * 64, head0, tok0);
+        }
+        __syncwarp();
+        int i = 0;
+        for (; i < n_tiles && !*abort_flag; ++i) {
+            const int s = i % LP_STAGES;
+            if (!lp_warp_wait(&k_empty[s], ((uint32_t)(i / LP_STAGES) & 1u) ^ 1u, abort_flag)) {
+                if (lane == 0) give_up();
+                break;
+            }
+            if (lane == 0) mbar_expect_tx(&k_full[s], LP_STAGE_BYTES);
+            __syncwarp();
+            for (int op = lane; op < boxes * LP_ATOMS; op += 32) {
+                const int b = op / LP_ATOMS, a = op - b * LP_ATOMS;
+                const int key = (t_begin + i) * LT_KEYS + b * box;
+                int row = cache_rows;
+                if (key <= pos_last && key + box > lo_first) row = bt[key / page_size] * page_size + key % page_size;
+                tma_load_2d(k_s + s * LP_STAGE_BYTES + a * LP_K_ATOM + b * box * 128, &map_k, &k_full[s], a * 64, row);
+            }
+        }
+        if (*abort_flag) {                                // copies on their way land before the memory goes to another CTA
+            for (int k = max(0, i - LP_STAGES); k < i; ++k) lp_warp_wait(&k_full[k % LP_STAGES], (uint32_t)(k / LP_STAGES) & 1u, never);
+        }
+    } else if (warp == 9) {
+        // ---- MMA issuer
+        constexpr uint32_t idesc_s = instr_desc_bf16(128, LT_KEYS);
+        constexpr uint32_t idesc_o = instr_desc_bf16(128, LP_VC) | (1u << 16);          // B: the contiguous axis is N
+        bool ok = !*abort_flag;
+        auto scores = [&](int i) -> bool {
+            const int s = i % LP_STAGES, b = i & 1;
+            if (!lp_warp_wait(&k_full[s], (uint32_t)(i / LP_STAGES) & 1u, abort_flag)) return false;
+            __syncwarp();
+            const int here = pos_last + 1 - (t_begin + i) * LT_KEYS;                     // rows that are keys of the request
+            if (here < LT_KEYS) {                         // the last tile: rows never written may hold anything, also NaN
+                for (int p = here * 8 + lane; p < LT_KEYS * 8; p += 32)
+                    for (int a = 0; a < LP_ATOMS; ++a)
+                        *reinterpret_cast<uint4*>(k_s + s * LP_STAGE_BYTES + a * LP_K_ATOM + p * 16) = make_uint4(0, 0, 0, 0);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+            }
+            tc_fence_after();
+            if (lane == 0) {
+                const uint32_t qa = smem_u32(q_s), ka = smem_u32(k_s + s * LP_STAGE_BYTES);
+#pragma unroll 4
+                for (int k = 0; k < LT_WIDTH / 16; ++k)
+                    umma_bf16(tmem_s + (uint32_t)(b * LT_KEYS), smem_desc_sw128(qa + (uint32_t)((k >> 2) * LP_Q_ATOM + (k & 3) * 32)),
+                              smem_desc_sw128(ka + (uint32_t)((k >> 2) * LP_K_ATOM + (k & 3) * 32)), idesc_s, k > 0 ? 1u : 0u);
+                umma_commit(&s_full[b]);
+            }
+            __syncwarp();
+            return true;
+        };
+        if (ok) ok = lp_warp_wait(q_full, 0, abort_flag);
+        if (ok) ok = scores(0);
+        for (int i = 0; i < n_tiles && ok; ++i) {
+            // the scores of tile i + 1 go where those of tile i - 1 and then its weights were: the values of tile i - 1 were
+            // issued before, and the tensor cores work in order
+            if (i + 1 < n_tiles && !scores(i + 1)) { ok = false; break; }
+            const int b = i & 1, s = i % LP_STAGES;
+            if (!lp_warp_wait(&p_full[b], (uint32_t)(i >> 1) & 1u, abort_flag)) { ok = false; break; }
+            tc_fence_after();
+            if (lane == 0) {
+                const uint32_t va = smem_u32(k_s + s * LP_STAGE_BYTES + half * (LP_VC / 64) * LP_K_ATOM);
+#pragma unroll
+                for (int k = 0; k < LT_KEYS / 16; ++k)
+                    umma_bf16_ts(tmem_o, tmem_s + (uint32_t)(b * LT_KEYS + k * 8), lp_desc_values(va + (uint32_t)(k * 16 * 128)), idesc_o,
+                                 (i > 0 || k > 0) ? 1u : 0u);
+                umma_commit(&k_empty[s]);
+                umma_commit(o_done);                      // phase i: the accumulators hold the tiles up to i
+            }
+            __syncwarp();
+        }
+        if (!ok && lane == 0) give_up();
+    } else if (warp < 4) {
+        // ---- weights of row r: token r / 16, head head0 + r % 16
+        const int r = threadIdx.x, token = r >> 4;
+        const uint32_t lanes = (uint32_t)(warp * 32) << 16;
+        const int pos = token < tokens ? pos_first + token : -1;
+        const int lo = window > 0 ? max(0, pos - window + 1) : 0;
+        float m = -CUDART_INF_F, l = 0.0f;
+        if (sink != nullptr) {
+            m = sink[head0 + (r & 15)];
+            l = 1.0f;
+        }
+        bool ok = !*abort_flag;
+        for (int i = 0; i < n_tiles; ++i) {
+            const int b = i & 1;
+            if (!lp_warp_wait(&s_full[b], (uint32_t)(i >> 1) & 1u, abort_flag)) {
+                if (lane == 0) give_up();
+                ok = false;
+                break;
+            }
+            tc_fence_after();
+            uint32_t v[32];
+            tmem_ld16(tmem_s + (uint32_t)(b * LT_KEYS) + lanes, v);
+            tmem_ld16(tmem_s + (uint32_t)(b * LT_KEYS) + 16u + lanes, v + 16);
+            tmem_ld_wait();
+            const int key0 = (t_begin + i) * LT_KEYS;
+            float p[32], mx[4];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                p[j] = key0 + j >= lo && key0 + j <= pos ? __fmul_rn(__uint_as_float(v[j]), scale) : -CUDART_INF_F;
+                mx[j & 3] = j < 4 ? p[j] : fmaxf(mx[j & 3], p[j]);
+            }
+            const float m_new = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
+            const bool out_of_sight = pos < key0 || lo >= key0 + LT_KEYS;
+            const float corr = out_of_sight ? 1.0f : expf(m - m_new);     // 0 at a row's first tile without a sink
+            corr_s[b * 128 + r] = m == -CUDART_INF_F ? 1.0f : corr;       // (nothing has been added up yet)
+            lp_warp_arrive(&c_full[b]);
+            uint32_t w[16];
+            if (out_of_sight) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) w[j] = 0u;
+            } else {
+                float sum = 0.0f;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    float e[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) e[j] = expf(__fsub_rn(p[g * 8 + j], m_new));
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const __nv_bfloat162 pair = __floats2bfloat162_rn(e[2 * j], e[2 * j + 1]);
+                        w[g * 4 + j] = *reinterpret_cast<const uint32_t*>(&pair);
+                    }
+                    sum += ((e[0] + e[1]) + (e[2] + e[3])) + ((e[4] + e[5]) + (e[6] + e[7]));
+                }
+                m = m_new;
+                l = l * corr + sum;
+            }
+            tmem_st16(tmem_s + (uint32_t)(b * LT_KEYS) + lanes, w);
+            tmem_st_wait();
+            tc_fence_before();
+            lp_warp_arrive(&p_full[b]);
+        }
+        inv_s[r] = ok ? 1.0f / l : 0.0f;
+        lp_warp_arrive(&c_full[n_tiles & 1]);             // (one phase more than tiles: the sums are there)
+    } else {
+        // ---- accumulators of row r
+        const int r = threadIdx.x - 128, token = r >> 4;
+        const uint32_t o_addr = tmem_o + ((uint32_t)((warp - 4) * 32) << 16);
+        bool ok = !*abort_flag;
+        for (int i = 0; i < n_tiles && ok; ++i) {
+            const int b = i & 1;
+            ok = lp_warp_wait(&c_full[b], (uint32_t)(i >> 1) & 1u, abort_flag);
+            if (!ok) break;
+            const float corr = corr_s[b * 128 + r];
+            if (i > 0 && __any_sync(0xffffffffu, corr != 1.0f)) {
+                ok = lp_warp_wait(o_done, (uint32_t)(i - 1) & 1u, abort_flag);
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll 2
+                for (int c = 0; c < LP_VC; c += 32) {
+                    uint32_t v[32];
+                    tmem_ld16(o_addr + (uint32_t)c, v);
+                    tmem_ld16(o_addr + (uint32_t)c + 16u, v + 16);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * corr);
+                    tmem_st16(o_addr + (uint32_t)c, v);
+                    tmem_st16(o_addr + (uint32_t)c + 16u, v + 16);
+                }
+                tmem_st_wait();
+                tc_fence_before();
+            }
+            lp_warp_arrive(&p_full[b]);
+        }
+        if (ok) ok = lp_warp_wait(&c_full[n_tiles & 1], (uint32_t)(n_tiles >> 1) & 1u, abort_flag);
+        if (ok) ok = lp_warp_wait(o_done, (uint32_t)(n_tiles - 1) & 1u, abort_flag);
+        if (!ok && lane == 0) give_up();
+        ok = __all_sync(0xffffffffu, ok) && !*abort_flag;
+        ok = __all_sync(0xffffffffu, ok);
+        tc_fence_after();
+        if (ok) {
+            const float inv = inv_s[r];
+            TO* dst = out + (long)(tok0 + token) * out_ld + (long)(head0 + (r & 15)) * LAT_RANK + half * LP_VC;
+#pragma unroll 1
+            for (int c = 0; c < LP_VC; c += 32) {
+                uint32_t v[32];
+                tmem_ld16(o_addr + (uint32_t)c, v);       // all lanes of the warp take part
+                tmem_ld16(o_addr + (uint32_t)c + 16u, v + 16);
+                tmem_ld_wait();
+                if (token >= tokens) continue;
+                __align__(16) TO o[32];
+#pragma unroll
+                for (int j = 0; j < 32; ++j) o[j] = from_f32<TO>(__uint_as_float(v[j]) * inv);
+#pragma unroll
+                for (int j = 0; j < 32 * (int)sizeof(TO) / 16; ++j)
+                    reinterpret_cast<uint4*>(dst + c)[j] = reinterpret_cast<const uint4*>(o)[j];
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 9) {
+        tc_fence_after();
+        tmem_dealloc(tmem_o, 512u);
+    }
+}
+
+// What the prompt kernel takes beyond what latent_attention_tc_kernel does: whole groups of 16 heads, 16-byte aligned rows
+// of the output, and pages that tiles of 32 keys consist of or lie in, in whole groups of eight rows (the swizzle's unit).
+FL_API int fl_latent_prompt_takes(int heads, int page_size) {
+    return heads % 16 == 0 && (page_size % 32 == 0 || page_size == 8 || page_size == 16);
+}
+
+// As fl_latent_attention_tc without splits, for steps of prompts; cache: [cache_rows][rank + rot], cache_rows = pages x page_size.
+FL_API int fl_latent_prompt(const void* q, long q_ld, void* out, int out_dtype, long out_ld, const void* cache, long cache_rows,
+                            int page_size, const int* block_table, int bt_stride, const int* req_start, const int* req_ctx,
+                            const int* req_qlen, int n_requests, int n_tokens, int heads, int window, float scale,
+                            const float* sink, int* status, cudaStream_t stream) {
+    if (n_tokens <= 0 || n_requests <= 0) return 0;
+    if (!fl_latent_prompt_takes(heads, page_size) || cache_rows >= (1l << 31) || heads / 16 * LP_HALVES > 65535)
+        return (int)cudaErrorInvalidValue;
+    if (((uintptr_t)q % 16) || (q_ld % 8) || ((uintptr_t)cache % 16) || ((uintptr_t)out % 16) || out_ld % 8)
+        return (int)cudaErrorMisalignedAddress;
+    EncodeTiledFn encode = encode_tiled_fn();
+    if (!encode) return (int)cudaErrorNotSupported;
+    CUtensorMap map_q, map_k;
+    {
+        // the queries as [tokens][heads][width]: a box is 8 tokens x 16 heads x 64 columns, 128 rows in that order
+        cuuint64_t dims[3] = {LT_WIDTH, (cuuint64_t)heads, (cuuint64_t)n_tokens};
+        cuuint64_t strides[2] = {LT_WIDTH * 2, (cuuint64_t)q_ld * 2};
+        cuuint32_t box[3] = {64, 16, LP_TOKENS}, elem[3] = {1, 1, 1};
+        if (encode(&map_q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(q), dims, strides, box, elem,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return (int)cudaErrorInvalidValue;
+    }
+    int rc = make_map(&map_k, cache, cache_rows, LT_WIDTH, LT_WIDTH, page_size < LT_KEYS ? page_size : LT_KEYS);
+    if (rc) return rc;
+    // plain stream order (no programmatic overlap): this kernel takes all of an SM's tensor memory
+    const dim3 grid(n_tokens / LP_TOKENS + n_requests, heads / 16 * LP_HALVES);
+    FL_DISPATCH(out_dtype, TO, {
+        rc = (int)cudaFuncSetAttribute(latent_prompt_kernel<TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, LP_SMEM);
+        if (rc) return rc;
+        latent_prompt_kernel<TO><<<grid, LP_THREADS, LP_SMEM, stream>>>(map_q, map_k, (TO*)out, out_ld, page_size, (int)cache_rows,
+                                                                        block_table, bt_stride, req_start, req_ctx, req_qlen,
+                                                                        n_requests, window, scale, sink, status);
+        return fl_launch_status();
+    });
+    return 0;
+}
+#else
+FL_API int fl_latent_prompt_takes(int heads, int page_size) { (void)heads; (void)page_size; return 0; }
+#endif

@@ -627,6 +627,35 @@ def latent_attention_tc(q, out, cache, block_table, tok_req, positions, heads, r
               int(n_splits), _ptr(partial), _ptr(sink), _stream()), "latent_attention_tc", 2 if split_keys else 1)
 
 
+def latent_prompt_takes(dtype, rank: int, rot: int, heads: int, page_size: int) -> bool:
+    """Whether the tcgen05 kernel for prompts serves this number format and these sizes."""
+    if not latent_tc_takes(dtype, rank, rot):
+        return False
+    key = ("latent_prompt", rank, rot, heads, page_size)
+    if key not in _fns:
+        fn = load_library(*latent_tc_library(rank, rot)).fl_latent_prompt_takes
+        fn.argtypes, fn.restype = [c_int, c_int], c_int
+        _fns[key] = bool(fn(heads, page_size))
+    return _fns[key]
+
+
+def latent_prompt(q, out, cache, block_table, req_start, req_ctx, req_qlen, heads, rank, rot, window, scale, page_size, sink=None):
+    """`latent_attention_tc` without splits, for steps of prompts: the same results, eight tokens of a request at a time
+    (sizes: `latent_prompt_takes`)."""
+    _require_cuda(q, out, cache, block_table, req_start, req_ctx, req_qlen, sink)
+    if q.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or not cache.is_contiguous():
+        raise KernelError("latent_prompt: q and cache must be bfloat16, the cache contiguous")
+    name, defines = latent_tc_library(rank, rot)
+    from .gemm_tc import status_word
+    fn = _fn(name, "fl_latent_prompt", [c_void_p, c_long, c_void_p, c_int, c_long, c_void_p, c_long, c_int, c_void_p, c_int, c_void_p,
+                                        c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p],
+             defines)
+    _check(fn(_ptr(q), _ld(q), _ptr(out), dtype_code(out), _ld(out), _ptr(cache), cache.shape[0] * page_size, page_size,
+              _ptr(block_table), block_table.stride(0), _ptr(req_start), _ptr(req_ctx), _ptr(req_qlen), req_qlen.numel(),
+              q.shape[0], heads, int(window or 0), float(scale), _ptr(sink), _ptr(status_word(q.device)), _stream()),
+           "latent_prompt")
+
+
 def gemm_simt_batched(a, a_batch, w, out, out_batch):
     """out[:, b * out_batch : b * out_batch + N] = a[:, b * a_batch : b * a_batch + K] @ w[b]^T for every b:
     w is [batch, N, K]; a and out are 2-D buffers whose column blocks are the batch."""

@@ -462,6 +462,42 @@ def test_tensor_core_latent_attention_against_the_cuda_core_kernel(rank, rot, he
         assert float((result - want).abs().mean()) <= 2e-3
 
 
+@pytest.mark.parametrize("rank,rot,heads,page,window,sink", [(512, 64, 16, 16, 100, False), (512, 64, 16, 64, None, True),
+                                                             (512, 64, 32, 32, 1000, False), (256, 64, 16, 8, 33, True)])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_latent_prompt_kernel_is_the_other_kernel_bit_for_bit(rank, rot, heads, page, window, sink, out_dtype):
+    """Whole prompts, portions behind cached rows, lengths around the groups of eight tokens and the tiles of 32 keys,
+    single tokens among them; places that no request has written are NaN.  Some keys stand out, so that maxima move late."""
+    from fastllm_py_b200.native import ops
+
+    torch.manual_seed(heads + page)
+    width = rank + rot
+    lens = [(0, 70), (150, 1), (33, 9), (0, 8), (96, 33), (515, 130), (7, 1)]      # (cached before the step, tokens in it)
+    per = -(-700 // page)
+    table = torch.randperm(per * len(lens) + 3, device="cuda").to(torch.int32)[:per * len(lens)].view(len(lens), -1).contiguous()
+    cache = torch.full((per * len(lens) + 3, page, width), float("nan"), device="cuda", dtype=torch.bfloat16)
+    for r, (c, n) in enumerate(lens):
+        rows = torch.randn(c + n, width, device="cuda")
+        rows[::41] *= 3.0
+        for a in range(0, c + n, page):
+            cache[table[r, a // page].long(), :min(page, c + n - a)] = rows[a:a + page].to(torch.bfloat16)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    tok_req = i32([r for r, (_, n) in enumerate(lens) for _ in range(n)])
+    positions = i32([c + i for c, n in lens for i in range(n)])
+    starts = [sum(n for _, n in lens[:r]) for r in range(len(lens) + 1)]
+    n = starts[-1]
+    q = (0.3 * torch.randn(n, heads * width + 8, device="cuda")).to(torch.bfloat16)[:, :heads * width]
+    sinks = torch.randn(heads, device="cuda") if sink else None
+    want = torch.empty(n, heads * rank, device="cuda", dtype=out_dtype)
+    got = torch.full((n + 1, heads * rank), 7.0, device="cuda", dtype=out_dtype)
+    assert ops.latent_prompt_takes(torch.bfloat16, rank, rot, heads, page)
+    ops.latent_attention_tc(q, want, cache, table, tok_req, positions, heads, rank, rot, window, 0.1, page, sink=sinks)
+    ops.latent_prompt(q, got[:n], cache, table, i32(starts), i32([c for c, _ in lens]), i32([m for _, m in lens]), heads, rank, rot,
+                      window, 0.1, page, sinks)
+    assert bool(torch.isfinite(want).all()) and bool((got[n:] == 7.0).all())
+    assert torch.equal(got[:n], want)
+
+
 def test_gated_product_with_relu_and_gelu_in_its_epilogue():
     """The tensor-core product that applies the gate's activation itself, for the activations beside silu,
     in its one-tile form (a decode-sized step) and its CTA-pair form (a prompt-sized step)."""
