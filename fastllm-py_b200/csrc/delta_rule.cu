@@ -104,12 +104,16 @@ __global__ void delta_tail_kernel(const T* __restrict__ proj, long ld, float* __
     }
 }
 
-// One block: one request, one head, DELTA_COLS value columns.  Thread (col, part) keeps the DPT elements
+// One block: one request, one head, COLS value columns.  Thread (col, part) keeps the DPT elements
 // d = part * DPT + i of column `col` of S.  The tokens' inputs (k, q of the head, the block's v columns,
-// beta, decay) come through shared memory in chunks of DELTA_CHUNK tokens, the next chunk in flight
-// (cp.async) while this one is consumed: the recurrence never waits for global memory.  In shared memory
+// beta, decay, and q . k, which no state enters) come through shared memory in chunks of DELTA_CHUNK tokens, the next
+// chunk fetched (cp.async) and its q . k summed by a warp of its own while this one is consumed: the threads that walk
+// the recurrence do nothing else, a warp of them being alone on its scheduler.  In shared memory
 // a part's k (and q) elements are contiguous and parts are DPT + 4 floats apart, so a thread fetches them
 // four at a time without bank conflicts.
+// What bounds a long prompt: the chain from one token's u to the next one's.  2048 tokens, 16 heads of 128 x 128: 326 us,
+// 160 ns a token; 679 us with the fetches and q . k on the same threads (156 instructions a token and warp, a fifth of the
+// time at the barrier behind the two warps that fetched) and one multiply-add an element.
 #define DELTA_CHUNK 16
 
 __device__ __forceinline__ void delta_cp16(float* smem, const float* gmem) {
@@ -122,24 +126,42 @@ __device__ __forceinline__ void delta_cp4(float* smem, const float* gmem) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s), "l"(gmem));
 }
 
-template <int DPT, int COLS, bool VEC>
-__global__ void __launch_bounds__(COLS * DELTA_PARTS) delta_scan_kernel(
+__device__ __forceinline__ float2 delta_fma2(const float2 a, const float2 b, const float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)),
+          "l"(reinterpret_cast<const unsigned long long&>(c)));
+    return d;
+}
+__device__ __forceinline__ float2 delta_mul2(const float2 a, const float2 b) {
+    float2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+    return d;
+}
+
+template <int DPT, int COLS>
+__global__ void __launch_bounds__(COLS * DELTA_PARTS + 32) delta_scan_kernel(
     float* __restrict__ work, long work_ld, float* __restrict__ state, long state_stride,
     const int* __restrict__ req_start, const int* __restrict__ req_ctx, const int* __restrict__ req_qlen,
     const int* __restrict__ req_slot, int heads, int kv_heads, int dim, int vdim) {
     static_assert(DPT % 4 == 0, "a thread's elements are fetched four at a time");
     pdl_wait();
     pdl_trigger();
+    constexpr int THREADS = COLS * DELTA_PARTS;              // ... that walk the recurrence; 32 more fetch
     constexpr int PART = DPT + 4;                            // floats between parts
     constexpr int KQ = DELTA_PARTS * PART;                   // k (and q) of one token
-    constexpr int PER_TOKEN = 2 * KQ + COLS + 4;       // k | q | v COLS | beta | decay | pad
+    constexpr int PER_TOKEN = 2 * KQ + COLS + 4;             // k | q | v COLS | beta | decay | q . k | pad
     extern __shared__ __align__(16) float delta_in[];        // [2][DELTA_CHUNK][PER_TOKEN]
     const int r = blockIdx.x / heads, h = blockIdx.x % heads;
     const int g = h / (heads / kv_heads);
-    const int part = threadIdx.x & (DELTA_PARTS - 1), col = threadIdx.x / DELTA_PARTS;
+    const bool fetches = threadIdx.x >= THREADS;
+    const int part = threadIdx.x & (DELTA_PARTS - 1), col = fetches ? 0 : threadIdx.x / DELTA_PARTS;
     const int j = blockIdx.y * COLS + col;
-    const bool live = j < vdim;
-    const int jj = live ? j : vdim - 1;                      // idle columns shadow the last one and store nothing
+    const bool live = j < vdim && !fetches;
+    const int jj = j < vdim ? j : vdim - 1;                  // idle columns shadow the last one and store nothing
     const int start = req_start[r], qlen = req_qlen[r];
     float* s_col = state + (long)req_slot[r] * state_stride + ((long)h * vdim + jj) * dim;
     const int qk_cols = kv_heads * dim, hv = heads * vdim;
@@ -149,62 +171,185 @@ __global__ void __launch_bounds__(COLS * DELTA_PARTS) delta_scan_kernel(
         for (int idx = threadIdx.x; idx < used; idx += blockDim.x) delta_in[idx] = 0.0f;
         __syncthreads();
     }
-    // rows whose pieces are all 16-byte aligned are copied four floats at a time, 128 slots a token
-    const bool wide = dim % 4 == 0 && vdim % 4 == 0 && v0 + COLS <= vdim && dim / 2 + COLS / 4 + 2 <= 128 && work_ld % 4 == 0;
+    // rows whose pieces are all 16-byte aligned are copied four floats at a time
+    const bool wide = dim % 4 == 0 && vdim % 4 == 0 && v0 + COLS <= vdim && work_ld % 4 == 0;
     auto fetch = [&](int buf, int first) {                   // tokens first .. first + DELTA_CHUNK - 1 of the portion
         float* dst = delta_in + (long)buf * DELTA_CHUNK * PER_TOKEN;
         const int n_tok = min(DELTA_CHUNK, qlen - first);
+        const float* row = work + (long)(start + first) * work_ld;
+        const int lane = threadIdx.x & 31;
         if (wide) {
-            const int c = threadIdx.x & 127, quarter = dim / 4;
-            for (int n = threadIdx.x >> 7; n < n_tok; n += (COLS * DELTA_PARTS) >> 7) {
-                const float* row = work + (long)(start + first + n) * work_ld;
-                float* to = dst + (long)n * PER_TOKEN;
-                if (c < 2 * quarter) {                                            // k, then q
-                    const int d = (c < quarter ? c : c - quarter) * 4;
-                    delta_cp16(to + (c < quarter ? 0 : KQ) + (d / DPT) * PART + d % DPT,
-                               row + (c < quarter ? qk_cols : 0) + g * dim + d);
-                } else if (c < 2 * quarter + COLS / 4) {
-                    const int e = (c - 2 * quarter) * 4;
-                    delta_cp16(to + 2 * KQ + e, row + 2 * qk_cols + h * vdim + v0 + e);
-                } else if (c < 2 * quarter + COLS / 4 + 2) {                      // beta, decay
-                    const int e = c - 2 * quarter - COLS / 4;
-                    delta_cp4(to + 2 * KQ + COLS + e, row + 2 * qk_cols + hv + e * heads + h);
+            for (int d = lane * 4; d < dim; d += 128) {                           // k and q, four elements a lane
+                const int at = (d / DPT) * PART + d % DPT;
+                const float* src = row + g * dim + d;
+                float* to = dst + at;
+                for (int n = 0; n < n_tok; ++n, src += work_ld, to += PER_TOKEN) {
+                    delta_cp16(to, src + qk_cols);
+                    delta_cp16(to + KQ, src);
                 }
             }
-            asm volatile("cp.async.commit_group;");
-            return;
-        }
-        const int wanted = 2 * dim + COLS + 2;
-        for (int idx = threadIdx.x; idx < n_tok * wanted; idx += blockDim.x) {
-            const int n = idx / wanted, e = idx % wanted;
-            const float* row = work + (long)(start + first + n) * work_ld;
-            const float* src;
-            int at;
-            if (e < 2 * dim) {                                                    // k, then q
-                const int d = e < dim ? e : e - dim;
-                src = row + (e < dim ? qk_cols : 0) + g * dim + d;
-                at = (e < dim ? 0 : KQ) + (d / DPT) * PART + d % DPT;
-            } else if (e < 2 * dim + COLS) {
-                src = row + 2 * qk_cols + h * vdim + min(v0 + e - 2 * dim, vdim - 1);
-                at = 2 * KQ + (e - 2 * dim);
-            } else {                                                              // beta, decay
-                src = row + 2 * qk_cols + hv + (e - 2 * dim - COLS) * heads + h;
-                at = 2 * KQ + COLS + (e - 2 * dim - COLS);
+            if (lane < COLS / 4 + 2) {                                            // v, beta, decay
+                const bool is_v = lane < COLS / 4;
+                const int e = lane - COLS / 4;
+                const float* src = row + 2 * qk_cols + (is_v ? h * vdim + v0 + lane * 4 : hv + e * heads + h);
+                float* to = dst + 2 * KQ + (is_v ? lane * 4 : COLS + e);
+                for (int n = 0; n < n_tok; ++n, src += work_ld, to += PER_TOKEN) {
+                    if (is_v) delta_cp16(to, src);
+                    else delta_cp4(to, src);
+                }
             }
-            delta_cp4(dst + (long)n * PER_TOKEN + at, src);
+        } else {
+            const int wanted = 2 * dim + COLS + 2;
+            for (int idx = lane; idx < n_tok * wanted; idx += 32) {
+                const int n = idx / wanted, e = idx % wanted;
+                const float* from = row + (long)n * work_ld;
+                int at;
+                if (e < 2 * dim) {                                                // k, then q
+                    const int d = e < dim ? e : e - dim;
+                    from += (e < dim ? qk_cols : 0) + g * dim + d;
+                    at = (e < dim ? 0 : KQ) + (d / DPT) * PART + d % DPT;
+                } else if (e < 2 * dim + COLS) {
+                    from += 2 * qk_cols + h * vdim + min(v0 + e - 2 * dim, vdim - 1);
+                    at = 2 * KQ + (e - 2 * dim);
+                } else {                                                          // beta, decay
+                    from += 2 * qk_cols + hv + (e - 2 * dim - COLS) * heads + h;
+                    at = 2 * KQ + COLS + (e - 2 * dim - COLS);
+                }
+                delta_cp4(dst + (long)n * PER_TOKEN + at, from);
+            }
         }
-        asm volatile("cp.async.commit_group;");
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float S[DPT];
+    // q . k of the chunk's tokens, a token's eight parts side by side
+    auto products = [&](int buf, int first) {
+        const int n_tok = min(DELTA_CHUNK, qlen - first);
+        for (int n0 = 0; n0 < n_tok; n0 += 4) {
+            const int n = n0 + ((threadIdx.x & 31) >> 3);
+            float* tok = delta_in + ((long)buf * DELTA_CHUNK + min(n, n_tok - 1)) * PER_TOKEN;
+            float c[2] = {0.0f, 0.0f};
+#pragma unroll
+            for (int i = 0; i < DPT; i += 4) {
+                const float4 kv = *reinterpret_cast<const float4*>(tok + part * PART + i);
+                const float4 qv = *reinterpret_cast<const float4*>(tok + KQ + part * PART + i);
+                c[0] = fmaf(qv.x, kv.x, c[0]);
+                c[1] = fmaf(qv.y, kv.y, c[1]);
+                c[0] = fmaf(qv.z, kv.z, c[0]);
+                c[1] = fmaf(qv.w, kv.w, c[1]);
+            }
+            float qk = c[0] + c[1];
+#pragma unroll
+            for (int o = 1; o < DELTA_PARTS; o <<= 1) qk += __shfl_xor_sync(0xffffffffu, qk, o);
+            if (part == 0 && n < n_tok) tok[2 * KQ + COLS + 2] = qk;
+        }
+    };
+    if (fetches) {
+        fetch(0, 0);
+        for (int first = 0, buf = 0; first < qlen; first += DELTA_CHUNK, buf ^= 1) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncwarp();
+            products(buf, first);
+            __syncthreads();                                 // chunk `first` is there, the one before has been consumed
+            if (first + DELTA_CHUNK < qlen) fetch(buf ^ 1, first + DELTA_CHUNK);
+        }
+        return;
+    }
+    float2 S[DPT / 2];
     const bool fresh = req_ctx[r] == 0;
-    fetch(0, 0);
-    // VEC (steps of single tokens, where reading and writing the state is all the work): every thread's elements
-    // exist and every column starts on 16 bytes, so the state moves four floats at a time
-    const bool whole = VEC && dim == DELTA_PARTS * DPT && state_stride % 4 == 0;
-    if (whole && !fresh) {
+#pragma unroll
+    for (int i = 0; i < DPT; ++i) {
+        const int d = part * DPT + i;
+        const float v = (!fresh && d < dim) ? s_col[d] : 0.0f;
+        if (i & 1) S[i / 2].y = v;
+        else S[i / 2].x = v;
+    }
+    float* o_tok = work + (long)start * work_ld + 2 * qk_cols + hv + 2 * heads + h * vdim + j;
+    for (int first = 0, buf = 0; first < qlen; first += DELTA_CHUNK, buf ^= 1) {
+        __syncthreads();
+        const float* in = delta_in + (long)buf * DELTA_CHUNK * PER_TOKEN;
+        const int n_tok = min(DELTA_CHUNK, qlen - first);
+        // With a = S^T k, b = S^T q (S before the token) and c = q . k:  u = beta (v - g a) and the read-out of the updated
+        // state is g b + c u.  Only u stands between this token's sums and the next token's: the next token's inputs are
+        // fetched, and the state is multiplied by its decay, while the sums cross the column's lanes.
+        float4 kn[DPT / 4], qn[DPT / 4], sn;
+        float vn;
+        auto ask = [&](const float* tok) {
+#pragma unroll
+            for (int i = 0; i < DPT / 4; ++i) {
+                kn[i] = *reinterpret_cast<const float4*>(tok + part * PART + 4 * i);
+                qn[i] = *reinterpret_cast<const float4*>(tok + KQ + part * PART + 4 * i);
+            }
+            vn = tok[2 * KQ + col];
+            sn = *reinterpret_cast<const float4*>(tok + 2 * KQ + COLS);           // beta, decay, q . k
+        };
+        ask(in);
+#pragma unroll 2
+        for (int n = 0; n < n_tok; ++n) {
+            float2 k[DPT / 2], a = make_float2(0.0f, 0.0f), b = make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int i = 0; i < DPT / 4; ++i) {
+                k[2 * i] = make_float2(kn[i].x, kn[i].y);
+                k[2 * i + 1] = make_float2(kn[i].z, kn[i].w);
+                a = delta_fma2(S[2 * i], k[2 * i], a);
+                b = delta_fma2(S[2 * i], make_float2(qn[i].x, qn[i].y), b);
+                a = delta_fma2(S[2 * i + 1], k[2 * i + 1], a);
+                b = delta_fma2(S[2 * i + 1], make_float2(qn[i].z, qn[i].w), b);
+            }
+            float dot = a.x + a.y, read = b.x + b.y;
+            const float v = vn;
+            const float4 sc = sn;
+            if (n + 1 < n_tok) in += PER_TOKEN;
+            ask(in);
+#pragma unroll
+            for (int o = 1; o < DELTA_PARTS; o <<= 1) {
+                dot += __shfl_xor_sync(0xffffffffu, dot, o);
+                read += __shfl_xor_sync(0xffffffffu, read, o);
+            }
+            const float2 decay2 = make_float2(sc.y, sc.y);
+#pragma unroll
+            for (int i = 0; i < DPT / 2; ++i) S[i] = delta_mul2(decay2, S[i]);
+            const float u = __fmul_rn(sc.x, fmaf(-sc.y, dot, v));
+            const float2 u2 = make_float2(u, u);
+#pragma unroll
+            for (int i = 0; i < DPT / 2; ++i) S[i] = delta_fma2(k[i], u2, S[i]);
+            if (live && part == 0) *o_tok = fmaf(sc.y, read, sc.z * u);
+            o_tok += work_ld;
+        }
+    }
+    if (live) {
+#pragma unroll
+        for (int i = 0; i < DPT; ++i) {
+            const int d = part * DPT + i;
+            if (d < dim) s_col[d] = i & 1 ? S[i / 2].y : S[i / 2].x;
+        }
+    }
+}
+
+// The same for steps in which every request brings one token, where reading and writing the state is all the work: a
+// thread asks for its elements of S first (16 bytes at a time where every column starts on 16 bytes), k and q come
+// through shared memory meanwhile.  (8 and 16 requests, 16 heads of 128 x 128: 6.5 and 9.8 us, through the scan's chunk
+// stages 7.0 and 11.3.)
+template <int DPT>
+__global__ void __launch_bounds__(DELTA_COLS * DELTA_PARTS) delta_step_kernel(
+    float* __restrict__ work, long work_ld, float* __restrict__ state, long state_stride,
+    const int* __restrict__ req_start, const int* __restrict__ req_ctx, const int* __restrict__ req_slot, int heads,
+    int kv_heads, int dim, int vdim) {
+    pdl_wait();
+    pdl_trigger();
+    constexpr int PART = DPT + 4, KQ = DELTA_PARTS * PART;   // as in the scan
+    __shared__ __align__(16) float kq_s[2 * KQ];
+    const int r = blockIdx.x / heads, h = blockIdx.x % heads;
+    const int part = threadIdx.x & (DELTA_PARTS - 1), j = blockIdx.y * DELTA_COLS + threadIdx.x / DELTA_PARTS;
+    const int jj = min(j, vdim - 1);                         // idle columns shadow the last one and store nothing
+    const int qk_cols = kv_heads * dim, hv = heads * vdim, g = h / (heads / kv_heads);
+    float* row = work + (long)req_start[r] * work_ld;
+    float* s_col = state + (long)req_slot[r] * state_stride + ((long)h * vdim + jj) * dim;
+    const bool fresh = req_ctx[r] == 0;
+    const bool whole = dim == DELTA_PARTS * DPT && state_stride % 4 == 0 && ((uintptr_t)state & 15) == 0;
+    float S[DPT];
+    if (whole) {
 #pragma unroll
         for (int i = 0; i < DPT; i += 4) {
-            const float4 v = *reinterpret_cast<const float4*>(s_col + part * DPT + i);
+            const float4 v = fresh ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : *reinterpret_cast<const float4*>(s_col + part * DPT + i);
             S[i] = v.x; S[i + 1] = v.y; S[i + 2] = v.z; S[i + 3] = v.w;
         }
     } else {
@@ -214,58 +359,46 @@ __global__ void __launch_bounds__(COLS * DELTA_PARTS) delta_scan_kernel(
             S[i] = (!fresh && d < dim) ? s_col[d] : 0.0f;
         }
     }
-    float* o_base = work + (long)start * work_ld + 2 * qk_cols + hv + 2 * heads + h * vdim + j;
-    for (int first = 0, buf = 0; first < qlen; first += DELTA_CHUNK, buf ^= 1) {
-        if (first + DELTA_CHUNK < qlen) {
-            fetch(buf ^ 1, first + DELTA_CHUNK);
-            asm volatile("cp.async.wait_group 1;");
-        } else {
-            asm volatile("cp.async.wait_group 0;");
-        }
-        __syncthreads();
-        const float* in = delta_in + (long)buf * DELTA_CHUNK * PER_TOKEN;
-        const int n_tok = min(DELTA_CHUNK, qlen - first);
-        for (int n = 0; n < n_tok; ++n, in += PER_TOKEN) {
-            // With a = S^T k, b = S^T q (S before the token) and c = q . k:  u = beta (v - g a) and the
-            // read-out of the updated state is g b + c u.  The three sums are independent, so their chains
-            // and their reductions over the column's lanes overlap; only u stands between this token's
-            // sums and the next token's.
-            float k[DPT], a[2] = {0.0f, 0.0f}, bq[2] = {0.0f, 0.0f}, c[2] = {0.0f, 0.0f};
-#pragma unroll
-            for (int i = 0; i < DPT; i += 4) {
-                const float4 kv = *reinterpret_cast<const float4*>(in + part * PART + i);
-                const float4 qv = *reinterpret_cast<const float4*>(in + KQ + part * PART + i);
-                k[i] = kv.x; k[i + 1] = kv.y; k[i + 2] = kv.z; k[i + 3] = kv.w;
-                a[0] += S[i] * kv.x;      bq[0] += S[i] * qv.x;      c[0] += qv.x * kv.x;
-                a[1] += S[i + 1] * kv.y;  bq[1] += S[i + 1] * qv.y;  c[1] += qv.y * kv.y;
-                a[0] += S[i + 2] * kv.z;  bq[0] += S[i + 2] * qv.z;  c[0] += qv.z * kv.z;
-                a[1] += S[i + 3] * kv.w;  bq[1] += S[i + 3] * qv.w;  c[1] += qv.w * kv.w;
-            }
-            float dot = a[0] + a[1], read = bq[0] + bq[1], qk = c[0] + c[1];
-#pragma unroll
-            for (int o = 1; o < DELTA_PARTS; o <<= 1) {
-                dot += __shfl_xor_sync(0xffffffffu, dot, o);
-                read += __shfl_xor_sync(0xffffffffu, read, o);
-                qk += __shfl_xor_sync(0xffffffffu, qk, o);
-            }
-            const float decay = in[2 * KQ + COLS + 1];
-            const float u = in[2 * KQ + COLS] * (in[2 * KQ + col] - decay * dot);
-#pragma unroll
-            for (int i = 0; i < DPT; ++i) S[i] = fmaf(k[i], u, decay * S[i]);
-            if (live && part == 0) o_base[(long)(first + n) * work_ld] = decay * read + qk * u;
-        }
-        __syncthreads();                                     // the chunk is overwritten by the fetch after next
+    for (int i = threadIdx.x; i < 2 * DELTA_PARTS * DPT; i += DELTA_COLS * DELTA_PARTS) {       // k, then q
+        const int side = i / (DELTA_PARTS * DPT), d = i - side * (DELTA_PARTS * DPT);
+        kq_s[side * KQ + (d / DPT) * PART + d % DPT] = d < dim ? row[(side == 0 ? qk_cols : 0) + g * dim + d] : 0.0f;
     }
-    if (live && whole) {
+    const float v = row[2 * qk_cols + h * vdim + jj], beta = row[2 * qk_cols + hv + h], decay = row[2 * qk_cols + hv + heads + h];
+    __syncthreads();
+    float k[DPT], a[2] = {0.0f, 0.0f}, b[2] = {0.0f, 0.0f}, c[2] = {0.0f, 0.0f};
+#pragma unroll
+    for (int i = 0; i < DPT; i += 4) {
+        const float4 kv = *reinterpret_cast<const float4*>(kq_s + part * PART + i);
+        const float4 qv = *reinterpret_cast<const float4*>(kq_s + KQ + part * PART + i);
+        k[i] = kv.x; k[i + 1] = kv.y; k[i + 2] = kv.z; k[i + 3] = kv.w;
+        const float q[4] = {qv.x, qv.y, qv.z, qv.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            a[e & 1] = fmaf(S[i + e], k[i + e], a[e & 1]);
+            b[e & 1] = fmaf(S[i + e], q[e], b[e & 1]);
+            c[e & 1] = fmaf(q[e], k[i + e], c[e & 1]);
+        }
+    }
+    float dot = a[0] + a[1], read = b[0] + b[1], qk = c[0] + c[1];
+#pragma unroll
+    for (int o = 1; o < DELTA_PARTS; o <<= 1) {
+        dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        read += __shfl_xor_sync(0xffffffffu, read, o);
+        qk += __shfl_xor_sync(0xffffffffu, qk, o);
+    }
+    const float u = __fmul_rn(beta, fmaf(-decay, dot, v));
+    if (j >= vdim) return;
+    if (part == 0) row[2 * qk_cols + hv + 2 * heads + h * vdim + j] = fmaf(decay, read, qk * u);
+#pragma unroll
+    for (int i = 0; i < DPT; ++i) S[i] = fmaf(k[i], u, __fmul_rn(decay, S[i]));
+    if (whole) {
 #pragma unroll
         for (int i = 0; i < DPT; i += 4)
             *reinterpret_cast<float4*>(s_col + part * DPT + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
-    } else if (live) {
+    } else {
 #pragma unroll
-        for (int i = 0; i < DPT; ++i) {
-            const int d = part * DPT + i;
-            if (d < dim) s_col[d] = S[i];
-        }
+        for (int i = 0; i < DPT; ++i)
+            if (part * DPT + i < dim) s_col[part * DPT + i] = S[i];
     }
 }
 
@@ -318,7 +451,7 @@ FL_API int fl_delta_prep(const void* proj, int dtype, long ld, const void* conv_
     return 0;
 }
 
-// single_tokens: every request of the step brings one token (the state then moves in 16-byte pieces).
+// single_tokens: every request of the step brings one token (a kernel of its own).
 // work: [n_tokens, work_ld] floats, a row = q | k (kv_heads x dim each) | v (heads x vdim) | beta | decay (heads
 // each) | o (heads x vdim): fl_delta_prep fills all but o, fl_delta_scan reads them and fills o.
 FL_API int fl_delta_scan(float* work, long work_ld, float* state, long state_stride,
@@ -333,22 +466,24 @@ FL_API int fl_delta_scan(float* work, long work_ld, float* state, long state_str
     const int cols = narrow ? 16 : DELTA_COLS;
     dim3 grid(n_requests * heads, (vdim + cols - 1) / cols);
     if (grid.y > 65535) return (int)cudaErrorInvalidValue;
-#define FL_DELTA_SCAN_COLS(DPT, COLS, VEC)                                                                          \
+#define FL_DELTA_SCAN_COLS(DPT, COLS)                                                                               \
     {                                                                                                               \
         const size_t smem = (size_t)2 * DELTA_CHUNK * (2 * DELTA_PARTS * (DPT + 4) + COLS + 4) * sizeof(float);     \
         static bool raised = false;                                                                                 \
         if (smem > 48 * 1024 && !raised) {                                                                          \
-            const cudaError_t rc = cudaFuncSetAttribute(delta_scan_kernel<DPT, COLS, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            const cudaError_t rc = cudaFuncSetAttribute(delta_scan_kernel<DPT, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
             if (rc != cudaSuccess) return (int)rc;                                                                  \
             raised = true;                                                                                          \
         }                                                                                                           \
-        return fl_launch(delta_scan_kernel<DPT, COLS, VEC>, grid, dim3(COLS * DELTA_PARTS), smem, stream, work, work_ld, state, \
+        return fl_launch(delta_scan_kernel<DPT, COLS>, grid, dim3(COLS * DELTA_PARTS + 32), smem, stream, work, work_ld, state, \
                          state_stride, req_start, req_ctx, req_qlen, req_slot, heads, kv_heads, dim, vdim);         \
     }
 #define FL_DELTA_SCAN(DPT)                                                                                          \
     if (per_thread <= DPT) {                                                                                        \
-        if (single_tokens) { if (narrow) FL_DELTA_SCAN_COLS(DPT, 16, true) else FL_DELTA_SCAN_COLS(DPT, 32, true) }  \
-        else { if (narrow) FL_DELTA_SCAN_COLS(DPT, 16, false) else FL_DELTA_SCAN_COLS(DPT, 32, false) }             \
+        if (single_tokens)                                                                                          \
+            return fl_launch(delta_step_kernel<DPT>, dim3(grid.x, (vdim + DELTA_COLS - 1) / DELTA_COLS), dim3(DELTA_COLS * DELTA_PARTS), 0, \
+                             stream, work, work_ld, state, state_stride, req_start, req_ctx, req_slot, heads, kv_heads, dim, vdim); \
+        if (narrow) FL_DELTA_SCAN_COLS(DPT, 16) else FL_DELTA_SCAN_COLS(DPT, 32)                                    \
     }
     FL_DELTA_SCAN(4);
     FL_DELTA_SCAN(8);
