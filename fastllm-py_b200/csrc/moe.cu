@@ -9,7 +9,7 @@
 //                 equal groups of neighbours, a group's score is the sum of the `group_top` largest
 //                 s + bias in it (1: the largest), and only experts of the `keep` best groups (ties to
 //                 the lower index) can be chosen
-//   moe_gate_up   per (token, choice): act(W_gate[e] h) * (W_up[e] h), one warp per feature; experts
+//   moe_gate_up   per (token, choice): act(W_gate[e] h) * (W_up[e] h), a warp a feature or several; experts
 //                 without a gate: act(W_up[e] h), the unit's f(x, 1)
 //   moe_down      per token: sum over its choices, in order of choice, of weight * W_down[e] a (with
 //                 `accumulate` added to what `out` holds: a shared unit's result)
@@ -107,8 +107,124 @@ __global__ void __launch_bounds__(128) moe_pick_kernel(const float* __restrict__
         }
 }
 
+// The order of a row's sum x . w, whichever kernel makes it: 32 chains, chain c adding up the elements c, c + 32, ... with
+// fused multiply-adds, and the chains added in a tree (neighbours 16 apart first).  The kernels for any size give a warp a
+// row and a lane a chain, which fetches 2 bytes a lane: 8 tokens x 4 of 32 experts of 2048 x 1408 took 85 + 62 us a layer,
+// bound by the number of loads (59 + 53 by rows).  Where rows are whole blocks of 32 elements and 16-byte aligned, a lane takes the MOE_V
+// neighbouring chains that 16 bytes hold, 32 / MOE_V lanes a row, and a warp several rows at once.
+template <typename TW> struct MoeRows {
+    static constexpr int V = 16 / (int)sizeof(TW);       // chains a lane
+    static constexpr int LPR = 32 / V;                   // lanes a row
+    static constexpr int ROWS = 32 / LPR;                // rows a warp
+};
+
+// acc[r][v] += x . w of this lane's chains for `ROWS` rows `second` elements apart; x and w begin at the lane's first chain
+template <int ROWS, int U, typename TW>
+__device__ __forceinline__ void moe_rows_dot(const float* __restrict__ x, const TW* __restrict__ w, long second, int n,
+                                             float (&acc)[ROWS][MoeRows<TW>::V]) {
+    constexpr int V = MoeRows<TW>::V;
+    for (int i = 0; i < n; i += U * 32) {
+        uint4 raw[ROWS][U];
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r)
+                if (i + j * 32 < n) raw[r][j] = *reinterpret_cast<const uint4*>(w + r * second + i + j * 32);
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            if (i + j * 32 >= n) break;
+#pragma unroll
+            for (int v = 0; v < V; v += 4) {
+                const float4 xv = *reinterpret_cast<const float4*>(x + i + j * 32 + v);
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r) {
+                    const TW* e = reinterpret_cast<const TW*>(&raw[r][j]) + v;
+                    acc[r][v] = fmaf(xv.x, to_f32<TW>(e[0]), acc[r][v]);
+                    acc[r][v + 1] = fmaf(xv.y, to_f32<TW>(e[1]), acc[r][v + 1]);
+                    acc[r][v + 2] = fmaf(xv.z, to_f32<TW>(e[2]), acc[r][v + 2]);
+                    acc[r][v + 3] = fmaf(xv.w, to_f32<TW>(e[3]), acc[r][v + 3]);
+                }
+            }
+        }
+    }
+}
+// the sum of a row's 32 chains, in every lane of the row
+template <int V> __device__ __forceinline__ float moe_rows_sum(float (&acc)[V]) {
+#pragma unroll
+    for (int o = 16; o >= V; o >>= 1)
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[v] += __shfl_xor_sync(0xffffffffu, acc[v], o / V);
+#pragma unroll
+    for (int o = V / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int v = 0; v < o; ++v) acc[v] += acc[v + o];
+    return acc[0];
+}
+
 // w_gu: [experts][2 ff][width] (gate rows, then up rows), or [experts][ff][width] without a gate;
 // a: [tokens x top][ff] float
+#define MOE_GU_WARPS 4
+template <typename T, typename TW>
+__global__ void __launch_bounds__(MOE_GU_WARPS * 32) moe_gate_up_rows_kernel(
+    const T* __restrict__ h, long h_ld, const TW* __restrict__ w_gu, const int* __restrict__ chosen, float* __restrict__ a,
+    int width, int ff, int top, FlGate act, int gated, const float* __restrict__ in_weights) {
+    pdl_wait();
+    pdl_trigger();
+    using L = MoeRows<TW>;
+    extern __shared__ __align__(16) float moe_x[];      // [width]
+    const int pair = blockIdx.x, t = pair / top;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < width; i += blockDim.x) moe_x[i] = to_f32<T>(h[(long)t * h_ld + i]);
+    __syncthreads();
+    const int f = (blockIdx.y * MOE_GU_WARPS + warp) * L::ROWS + lane / L::LPR, c0 = (lane % L::LPR) * L::V;
+    const int fr = min(f, ff - 1);                       // lanes beyond the last feature repeat it and store nothing
+    const float win = in_weights != nullptr ? in_weights[pair] : 1.0f;      // what multiplies the expert's input
+    if (!gated) {
+        float acc[1][L::V] = {};
+        moe_rows_dot<1, 8>(moe_x + c0, w_gu + ((long)chosen[pair] * ff + fr) * width + c0, 0, width, acc);
+        const float x = moe_rows_sum(acc[0]);
+        if (c0 == 0 && f < ff) a[(long)pair * ff + f] = fl_gated(x * win, 1.0f, act);
+        return;
+    }
+    float acc[2][L::V] = {};
+    moe_rows_dot<2, 8>(moe_x + c0, w_gu + ((long)chosen[pair] * 2 * ff + fr) * width + c0, (long)ff * width, width, acc);
+    const float g = moe_rows_sum(acc[0]), u = moe_rows_sum(acc[1]);
+    if (c0 == 0 && f < ff) a[(long)pair * ff + f] = fl_gated(g * win, u * win, act);
+}
+
+// w_down: [experts][width][ff]; a warp takes every eighth choice of the token, the choices are added in order
+#define MOE_DOWN_WARPS 8
+template <typename T, typename TW>
+__global__ void __launch_bounds__(MOE_DOWN_WARPS * 32) moe_down_rows_kernel(
+    const float* __restrict__ a, const TW* __restrict__ w_down, const int* __restrict__ chosen, const float* __restrict__ weights,
+    T* __restrict__ out, long out_ld, int width, int ff, int top, int accumulate) {
+    pdl_wait();
+    pdl_trigger();
+    using L = MoeRows<TW>;
+    __shared__ float y_s[MOE_DOWN_WARPS][L::ROWS];
+    const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int row = lane / L::LPR, c = blockIdx.y * L::ROWS + row, c0 = (lane % L::LPR) * L::V;
+    const int cr = min(c, width - 1);
+    float sum = 0.0f;
+    for (int k0 = 0; k0 < top; k0 += warps) {
+        if (k0 + warp < top) {
+            const long pair = (long)t * top + k0 + warp;
+            float acc[1][L::V] = {};
+            moe_rows_dot<1, 11>(a + pair * ff + c0, w_down + ((long)chosen[pair] * width + cr) * ff + c0, 0, ff, acc);
+            const float y = moe_rows_sum(acc[0]);
+            if (c0 == 0) y_s[warp][row] = y;
+        }
+        __syncthreads();
+        if (warp == 0)
+            for (int k = 0; k < warps && k0 + k < top; ++k)
+                sum += (weights != nullptr ? weights[(long)t * top + k0 + k] : 1.0f) * y_s[k][row];
+        __syncthreads();
+    }
+    if (warp == 0 && c0 == 0 && c < width)
+        out[(long)t * out_ld + c] = from_f32<T>(accumulate ? to_f32<T>(out[(long)t * out_ld + c]) + sum : sum);
+}
+
+// the same for any sizes
 template <typename T, typename TW>
 __global__ void __launch_bounds__(256) moe_gate_up_kernel(const T* __restrict__ h, long h_ld, const TW* __restrict__ w_gu,
                                                           const int* __restrict__ chosen, float* __restrict__ a,
@@ -116,7 +232,7 @@ __global__ void __launch_bounds__(256) moe_gate_up_kernel(const T* __restrict__ 
                                                           const float* __restrict__ in_weights) {
     pdl_wait();
     pdl_trigger();
-    extern __shared__ float moe_x[];                    // [width]
+    extern __shared__ __align__(16) float moe_x[];      // [width]
     const int pair = blockIdx.x, t = pair / top;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < width; i += blockDim.x) moe_x[i] = to_f32<T>(h[(long)t * h_ld + i]);
@@ -127,7 +243,7 @@ __global__ void __launch_bounds__(256) moe_gate_up_kernel(const T* __restrict__ 
     if (!gated) {
         const TW* wx = w_gu + ((long)chosen[pair] * ff + f) * width;
         float x = 0.0f;
-        for (int i = lane; i < width; i += 32) x += moe_x[i] * to_f32<TW>(wx[i]);
+        for (int i = lane; i < width; i += 32) x = fmaf(moe_x[i], to_f32<TW>(wx[i]), x);
         x = warp_sum(x);
         if (lane == 0) a[(long)pair * ff + f] = fl_gated(x * win, 1.0f, act);
         return;
@@ -136,15 +252,14 @@ __global__ void __launch_bounds__(256) moe_gate_up_kernel(const T* __restrict__ 
     const TW* wu = wg + (long)ff * width;
     float g = 0.0f, u = 0.0f;
     for (int i = lane; i < width; i += 32) {
-        g += moe_x[i] * to_f32<TW>(wg[i]);
-        u += moe_x[i] * to_f32<TW>(wu[i]);
+        g = fmaf(moe_x[i], to_f32<TW>(wg[i]), g);
+        u = fmaf(moe_x[i], to_f32<TW>(wu[i]), u);
     }
     g = warp_sum(g);
     u = warp_sum(u);
     if (lane == 0) a[(long)pair * ff + f] = fl_gated(g * win, u * win, act);
 }
 
-// w_down: [experts][width][ff]
 template <typename T, typename TW>
 __global__ void __launch_bounds__(256) moe_down_kernel(const float* __restrict__ a, const TW* __restrict__ w_down,
                                                        const int* __restrict__ chosen, const float* __restrict__ weights,
@@ -161,7 +276,7 @@ __global__ void __launch_bounds__(256) moe_down_kernel(const float* __restrict__
         const TW* wd = w_down + ((long)chosen[pair] * width + c) * ff;
         const float* ar = a + pair * ff;
         float y = 0.0f;
-        for (int i = lane; i < ff; i += 32) y += ar[i] * to_f32<TW>(wd[i]);
+        for (int i = lane; i < ff; i += 32) y = fmaf(ar[i], to_f32<TW>(wd[i]), y);
         sum += (weights != nullptr ? weights[pair] : 1.0f) * warp_sum(y);
     }
     if (lane == 0) out[(long)t * out_ld + c] = from_f32<T>(accumulate ? to_f32<T>(out[(long)t * out_ld + c]) + sum : sum);
@@ -191,14 +306,29 @@ FL_API int fl_moe_experts(const void* h, int dtype, long h_ld, const void* w_gu,
     if ((size_t)width * sizeof(float) > 48 * 1024 || (ff + 7) / 8 > 65535 || (width + 7) / 8 > 65535 || act < 0 || act >= FL_ACT_COUNT)
         return (int)cudaErrorInvalidValue;
     int rc = 0;
-    FL_DISPATCH(dtype, T, FL_DISPATCH(w_dtype, TW,
-        rc = fl_launch(moe_gate_up_kernel<T, TW>, dim3(n_tokens * top, (ff + 7) / 8), dim3(256),
-                       (size_t)width * sizeof(float), stream, (const T*)h, h_ld, (const TW*)w_gu, chosen, a, width, ff,
-                       top, FlGate{act, act_p0, act_p1}, gated, weight_on_input ? weights : nullptr)));
+    const FlGate unit{act, act_p0, act_p1};
+    const float *in_weights = weight_on_input ? weights : nullptr, *out_weights = weight_on_input ? nullptr : weights;
+    const bool rows = width % 32 == 0 && ff % 32 == 0 && (((uintptr_t)w_gu | (uintptr_t)w_down | (uintptr_t)a) % 16) == 0;
+    FL_DISPATCH(dtype, T, FL_DISPATCH(w_dtype, TW, {
+        constexpr int PER = MOE_GU_WARPS * MoeRows<TW>::ROWS;
+        if (rows)
+            rc = fl_launch(moe_gate_up_rows_kernel<T, TW>, dim3(n_tokens * top, (ff + PER - 1) / PER), dim3(MOE_GU_WARPS * 32),
+                           (size_t)width * sizeof(float), stream, (const T*)h, h_ld, (const TW*)w_gu, chosen, a, width, ff, top,
+                           unit, gated, in_weights);
+        else
+            rc = fl_launch(moe_gate_up_kernel<T, TW>, dim3(n_tokens * top, (ff + 7) / 8), dim3(256), (size_t)width * sizeof(float),
+                           stream, (const T*)h, h_ld, (const TW*)w_gu, chosen, a, width, ff, top, unit, gated, in_weights);
+    }));
     if (rc) return rc;
-    FL_DISPATCH(dtype, T, FL_DISPATCH(w_dtype, TW,
+    FL_DISPATCH(dtype, T, FL_DISPATCH(w_dtype, TW, {
+        constexpr int PER = MoeRows<TW>::ROWS;
+        if (rows)
+            return fl_launch(moe_down_rows_kernel<T, TW>, dim3(n_tokens, (width + PER - 1) / PER),
+                             dim3(32 * (top < MOE_DOWN_WARPS ? top : MOE_DOWN_WARPS)), 0, stream, (const float*)a,
+                             (const TW*)w_down, chosen, out_weights, (T*)out, out_ld, width, ff, top, accumulate);
         return fl_launch(moe_down_kernel<T, TW>, dim3(n_tokens, (width + 7) / 8), dim3(256), 0, stream, (const float*)a,
-                         (const TW*)w_down, chosen, weight_on_input ? nullptr : weights, (T*)out, out_ld, width, ff, top, accumulate)));
+                         (const TW*)w_down, chosen, out_weights, (T*)out, out_ld, width, ff, top, accumulate);
+    }));
     return 0;
 }
 
