@@ -720,12 +720,27 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_pair_kernel(
     cluster_sync_all();
 }
 
-// Width in tokens of the pair kernel's tiles for M tokens and room for `bnt`: as many tiles as whole ones
-// would take, equally wide, a multiple of 32 (the epilogue's round).  Each CTA's box of token rows is half of it.
-static int tc_pair_tile_tokens(int M, int bnt) {
-    const int tiles = (M + bnt - 1) / bnt;
-    const int wt = ((M + tiles - 1) / tiles + 31) / 32 * 32;
-    return wt < bnt ? wt : bnt;
+// Width in tokens of the pair kernel's tiles for M tokens and room for `bnt`, a multiple of 32 (the epilogue's round); each
+// CTA's box of token rows is half of it.  As many tiles as whole ones would take, equally wide, or up to three more where
+// that fills the pairs' rounds better: a round takes about 256 + width cycles a K step (what the operands take on their way
+// from L2: 16 KB of weights and 64 bytes a token for each CTA).  512 tokens, 43 feature tiles, 74 pairs: two tiles of 256
+// are 86 units, a round and a sixth, three of 192 are two rounds of 7/8 the length.
+static int tc_pair_tile_tokens(int M, int bnt, int tiles_n, int splits, int num_sms) {
+    const int fewest = (M + bnt - 1) / bnt, pairs = num_sms / 2;
+    int best = 0;
+    long best_cost = 0;
+    for (int tiles = fewest; tiles <= fewest + 3; ++tiles) {
+        int wt = ((M + tiles - 1) / tiles + 31) / 32 * 32;
+        if (wt > bnt) wt = bnt;
+        if (best && wt < 128) break;
+        const long units = (long)tiles_n * ((M + wt - 1) / wt) * splits;
+        const long cost = (units + pairs - 1) / pairs * (256 + wt);
+        if (best == 0 || cost * 20 < best_cost * 19) {
+            best = wt;
+            best_cost = cost;
+        }
+    }
+    return best;
 }
 
 template <int BNT, typename OutT, bool GATED = false, bool ROPE = false>
@@ -745,7 +760,7 @@ static int launch_tc_pair(const CUtensorMap& map_w, const CUtensorMap& map_a, vo
         configured = true;
     }
     const int tiles_n = GATED ? (N + 127) / 128 : (N + 255) / 256;
-    const int wt = tc_pair_tile_tokens(M, BNT);
+    const int wt = tc_pair_tile_tokens(M, BNT, tiles_n, splits, num_sms);
     const int num_tiles = tiles_n * ((M + wt - 1) / wt);
     const long num_units = (long)num_tiles * splits;
     const int pairs = num_units < num_sms / 2 ? (int)num_units : num_sms / 2;
@@ -1031,7 +1046,7 @@ static int gemm_tc_impl(const void* A, long lda, const void* W, long ldw, void* 
     const bool paired = bn >= 512;                           // 512, 640, 576: pair kernel, 256 / 128 / 64 tokens wide
     const int bnt = bn == 512 ? 256 : bn - 512;
     if (paired && (num_sms < 2 || (bnt != 64 && bnt != 128 && bnt != 256))) return (int)cudaErrorInvalidValue;
-    rc = make_map(&map_a, A, M, K, lda, paired ? tc_pair_tile_tokens(M, bnt) / 2 : bn);
+    rc = make_map(&map_a, A, M, K, lda, paired ? tc_pair_tile_tokens(M, bnt, (N + 255) / 256, splits, num_sms) / 2 : bn);
     if (rc) return rc;
     if (paired) {                                            // each CTA of a pair loads half of the token rows
         float* part = splits > 1 ? workspace : nullptr;
@@ -1110,7 +1125,7 @@ FL_API int fl_gemm_tc_glu(const void* A, long lda, const void* W, long ldw, void
     int rc = make_w_map(&map_w, W, 2L * I, K, ldw, feat);           // boxes of `feat` weight rows
     if (rc) return rc;
     const int wp = ldw == 0 ? 2 * I : 0;
-    rc = make_map(&map_a, A, M, K, lda, bn > 256 ? tc_pair_tile_tokens(M, 256) / 2 : bn);
+    rc = make_map(&map_a, A, M, K, lda, bn > 256 ? tc_pair_tile_tokens(M, 256, (I + 127) / 128, 1, num_sms) / 2 : bn);
     if (rc) return rc;
     if (bn == 512)
         return launch_tc_pair<256, bf16, true>(map_w, map_a, C, ldc, M, I, K, num_sms, status, stream, I, 1, 0, nullptr, 0, nullptr, wp, act);
@@ -1155,7 +1170,7 @@ FL_API int fl_gemm_tc_qkv_rope(const void* A, long lda, const void* W, long ldw,
     int rc = make_w_map(&map_w, W, N, K, ldw, TC_BM);
     if (rc) return rc;
     const int wp = ldw == 0 ? N : 0;
-    rc = make_map(&map_a, A, M, K, lda, tc_pair_tile_tokens(M, bnt) / 2);
+    rc = make_map(&map_a, A, M, K, lda, tc_pair_tile_tokens(M, bnt, (N + 255) / 256, 1, num_sms) / 2);
     if (rc) return rc;
     TcRope rope = {positions, slots, cos_table, sin_table, (bf16*)k_cache, (bf16*)v_cache, page_stride, page_size,
                    n_heads, n_kv_heads};
