@@ -163,8 +163,11 @@ template <int V> __device__ __forceinline__ float moe_rows_sum(float (&acc)[V]) 
 
 // w_gu: [experts][2 ff][width] (gate rows, then up rows), or [experts][ff][width] without a gate;
 // a: [tokens x top][ff] float
+// U: blocks of 32 elements on their way at once, of each row.  With more warps than the SMs hold at a time, fewer of them
+// and more warps resident are faster (8 tokens x 4, both products out of a cold cache: 106 us with 4 and 8, 127 with 8 and
+// 11); with fewer warps than that, more (one token: 42 us with 8 and 11, 48 with 4 and 8).
 #define MOE_GU_WARPS 4
-template <typename T, typename TW>
+template <typename T, typename TW, int U>
 __global__ void __launch_bounds__(MOE_GU_WARPS * 32) moe_gate_up_rows_kernel(
     const T* __restrict__ h, long h_ld, const TW* __restrict__ w_gu, const int* __restrict__ chosen, float* __restrict__ a,
     int width, int ff, int top, FlGate act, int gated, const float* __restrict__ in_weights) {
@@ -181,20 +184,20 @@ __global__ void __launch_bounds__(MOE_GU_WARPS * 32) moe_gate_up_rows_kernel(
     const float win = in_weights != nullptr ? in_weights[pair] : 1.0f;      // what multiplies the expert's input
     if (!gated) {
         float acc[1][L::V] = {};
-        moe_rows_dot<1, 8>(moe_x + c0, w_gu + ((long)chosen[pair] * ff + fr) * width + c0, 0, width, acc);
+        moe_rows_dot<1, U>(moe_x + c0, w_gu + ((long)chosen[pair] * ff + fr) * width + c0, 0, width, acc);
         const float x = moe_rows_sum(acc[0]);
         if (c0 == 0 && f < ff) a[(long)pair * ff + f] = fl_gated(x * win, 1.0f, act);
         return;
     }
     float acc[2][L::V] = {};
-    moe_rows_dot<2, 8>(moe_x + c0, w_gu + ((long)chosen[pair] * 2 * ff + fr) * width + c0, (long)ff * width, width, acc);
+    moe_rows_dot<2, U>(moe_x + c0, w_gu + ((long)chosen[pair] * 2 * ff + fr) * width + c0, (long)ff * width, width, acc);
     const float g = moe_rows_sum(acc[0]), u = moe_rows_sum(acc[1]);
     if (c0 == 0 && f < ff) a[(long)pair * ff + f] = fl_gated(g * win, u * win, act);
 }
 
 // w_down: [experts][width][ff]; a warp takes every eighth choice of the token, the choices are added in order
 #define MOE_DOWN_WARPS 8
-template <typename T, typename TW>
+template <typename T, typename TW, int U>
 __global__ void __launch_bounds__(MOE_DOWN_WARPS * 32) moe_down_rows_kernel(
     const float* __restrict__ a, const TW* __restrict__ w_down, const int* __restrict__ chosen, const float* __restrict__ weights,
     T* __restrict__ out, long out_ld, int width, int ff, int top, int accumulate) {
@@ -210,7 +213,7 @@ __global__ void __launch_bounds__(MOE_DOWN_WARPS * 32) moe_down_rows_kernel(
         if (k0 + warp < top) {
             const long pair = (long)t * top + k0 + warp;
             float acc[1][L::V] = {};
-            moe_rows_dot<1, 11>(a + pair * ff + c0, w_down + ((long)chosen[pair] * width + cr) * ff + c0, 0, ff, acc);
+            moe_rows_dot<1, U>(a + pair * ff + c0, w_down + ((long)chosen[pair] * width + cr) * ff + c0, 0, ff, acc);
             const float y = moe_rows_sum(acc[0]);
             if (c0 == 0) y_s[warp][row] = y;
         }
@@ -308,11 +311,12 @@ FL_API int fl_moe_experts(const void* h, int dtype, long h_ld, const void* w_gu,
     int rc = 0;
     const FlGate unit{act, act_p0, act_p1};
     const float *in_weights = weight_on_input ? weights : nullptr, *out_weights = weight_on_input ? nullptr : weights;
+    const bool few = (long)n_tokens * top * ((ff + 31) / 32) * MOE_GU_WARPS <= 148 * 16;    // 16 warps an SM with U = 8
     const bool rows = width % 32 == 0 && ff % 32 == 0 && (((uintptr_t)w_gu | (uintptr_t)w_down | (uintptr_t)a) % 16) == 0;
     FL_DISPATCH(dtype, T, FL_DISPATCH(w_dtype, TW, {
         constexpr int PER = MOE_GU_WARPS * MoeRows<TW>::ROWS;
         if (rows)
-            rc = fl_launch(moe_gate_up_rows_kernel<T, TW>, dim3(n_tokens * top, (ff + PER - 1) / PER), dim3(MOE_GU_WARPS * 32),
+            rc = fl_launch(few ? moe_gate_up_rows_kernel<T, TW, 8> : moe_gate_up_rows_kernel<T, TW, 4>, dim3(n_tokens * top, (ff + PER - 1) / PER), dim3(MOE_GU_WARPS * 32),
                            (size_t)width * sizeof(float), stream, (const T*)h, h_ld, (const TW*)w_gu, chosen, a, width, ff, top,
                            unit, gated, in_weights);
         else
@@ -323,7 +327,7 @@ FL_API int fl_moe_experts(const void* h, int dtype, long h_ld, const void* w_gu,
     FL_DISPATCH(dtype, T, FL_DISPATCH(w_dtype, TW, {
         constexpr int PER = MoeRows<TW>::ROWS;
         if (rows)
-            return fl_launch(moe_down_rows_kernel<T, TW>, dim3(n_tokens, (width + PER - 1) / PER),
+            return fl_launch(few ? moe_down_rows_kernel<T, TW, 11> : moe_down_rows_kernel<T, TW, 8>, dim3(n_tokens, (width + PER - 1) / PER),
                              dim3(32 * (top < MOE_DOWN_WARPS ? top : MOE_DOWN_WARPS)), 0, stream, (const float*)a,
                              (const TW*)w_down, chosen, out_weights, (T*)out, out_ld, width, ff, top, accumulate);
         return fl_launch(moe_down_kernel<T, TW>, dim3(n_tokens, (width + 7) / 8), dim3(256), 0, stream, (const float*)a,
