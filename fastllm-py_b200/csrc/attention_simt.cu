@@ -4,7 +4,7 @@
 // The keys of a token are taken in tiles of 64 that start at multiples of 64 of
 // the absolute key position.  A tile has a result of its own (its maximum, the
 // sum of exp(score - maximum) and the weighted values, softmax in float with the
-// exact expf; a score is summed over the head's columns in order, the weighted
+// exact expf; a score is summed in four chains over the head's columns, the weighted
 // values over the tile's keys in order), and the tiles' results are folded from
 // the first to the last.  So the order of every sum depends only on the token's
 // own position: the result is the same bit for bit however the sequence was cut
@@ -21,8 +21,7 @@
 // (tile t to CTA t mod CL), which hand their results over through distributed
 // shared memory.  One block a (token, head) pair, each thread walking a key row
 // in global memory, took 196 us a layer for 4 tokens over 700 keys and 16 heads
-// of 128 in 32 bits, and 450 us for a prompt of 300 tokens; this takes 50 and 146
-// (profiled inside a step, with the wait for the product before it).
+// of 128 in 32 bits, and 450 us for a prompt of 300 tokens; this takes 31 and 91.
 //
 // fastllm-py's counterparts: `_sdpa` (fastllm_py/model.py:341-353: scores scaled
 // by head_dim^-1/2, keys beyond the query masked, softmax and the weighted sum in
@@ -49,13 +48,14 @@ __device__ __forceinline__ void att_cp16(float* smem, const float* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
 }
 
-template <typename T, int QT, int CL>
+// NV: value columns a thread (1: heads of up to 128)
+template <typename T, int QT, int CL, int NV>
 __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
     const T* __restrict__ q, long q_ld, T* __restrict__ out, long out_ld,
     const T* __restrict__ k_cache, const T* __restrict__ v_cache, long page_stride, int page_size,
     const int* __restrict__ block_table, int bt_stride, const int* __restrict__ tok_req,
     const int* __restrict__ positions, int n_tokens, int n_heads, int n_kv_heads, int head_dim, int window,
-    float scale, int vec) {
+    float scale, int vec, int page_shift) {
     pdl_wait();
     pdl_trigger();
     namespace cg = cooperative_groups;
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rank = CL == 1 ? 0 : (int)(blockIdx.x % CL), h = blockIdx.y;
-    const int t_begin = (int)(blockIdx.x / CL) * QT, t_end = min(n_tokens, t_begin + QT);
+    const int t_begin = (int)((gridDim.x - 1 - blockIdx.x) / CL) * QT, t_end = min(n_tokens, t_begin + QT);
     const int kvh = h / (n_heads / n_kv_heads);
     const long head_off = (long)kvh * page_size * head_dim;
 
@@ -94,38 +94,38 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
             const int r = i / dp, d = i - r * dp;
             q_s[i] = d < head_dim ? to_f32<T>(q[(long)(t0 + r) * q_ld + (long)h * head_dim + d]) : 0.0f;
         }
-        float acc[QT][2] = {}, m[QT], l[QT];
+        float acc[QT][NV] = {}, m[QT], l[QT];
         bool begun[QT];
 #pragma unroll
         for (int i = 0; i < QT; ++i) m[i] = -CUDART_INF_F, l[i] = 0.0f, begun[i] = false;
-        const int d0 = tid, d1 = tid + ATT_THREADS;
+        const int d0 = tid, d1 = tid + ATT_THREADS;                 // (d1: NV 2 only)
 
         auto lowest = [&](int i) { return window > 0 ? max(0, pos[i] - window + 1) : 0; };
         auto sees = [&](int i, int tile) { return i < nq && pos[i] >= tile * ATT_TILE && lowest(i) < (tile + 1) * ATT_TILE; };
 
         // The result of one tile: maximum and sum of query i in ml[2 i], ml[2 i + 1], the weighted values in `a`.
-        auto do_tile = [&](int tile, float* ml, float (&a)[QT][2]) {
+        auto do_tile = [&](int tile, float* ml, float (&a)[QT][NV]) {
             const int base = tile * ATT_TILE, keys = min(ATT_TILE, last + 1 - base);
             // keys and values of the tile, rows past the last visible key left as zeros (their pages may hold anything)
             if (sizeof(T) == 4 && vec) {
-                const int per = head_dim / 4;
-#pragma unroll 1
-                for (int side = 0; side < 2; ++side) {
-                    float* dst = side == 0 ? k_s : v_s;
-                    const int pitch = side == 0 ? kp : dp;
-                    const float* src = reinterpret_cast<const float*>(side == 0 ? k_cache : v_cache);
-                    for (int i = tid; i < ATT_TILE * per; i += ATT_THREADS) {
-                        const int r = i / per, c = (i - r * per) * 4, j = base + r;
-                        if (r < keys) {
-                            const long off = (long)bt[j / page_size] * page_stride + head_off + (long)(j % page_size) * head_dim;
-                            att_cp16(dst + r * pitch + c, src + off + c);
-                        } else {
-                            *reinterpret_cast<float4*>(dst + r * pitch + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        }
+                // a thread copies one 16-byte column of every `step`-th row
+                const int per = head_dim / 4, step = ATT_THREADS / per, c = (tid % per) * 4;
+                const float *kc = reinterpret_cast<const float*>(k_cache) + head_off + c, *vc = reinterpret_cast<const float*>(v_cache) + head_off + c;
+#pragma unroll 4
+                for (int r = tid / per; r < ATT_TILE; r += step) {
+                    const int j = base + r;
+                    if (r < keys) {
+                        const int page = page_shift >= 0 ? j >> page_shift : j / page_size;
+                        const long off = (long)bt[page] * page_stride + (long)(j - page * page_size) * head_dim;
+                        att_cp16(k_s + r * kp + c, kc + off);
+                        att_cp16(v_s + r * dp + c, vc + off);
+                    } else {
+                        *reinterpret_cast<float4*>(k_s + r * kp + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        *reinterpret_cast<float4*>(v_s + r * dp + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
-                    asm volatile("cp.async.commit_group;" ::: "memory");
                 }
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
             } else {
                 for (int i = tid; i < ATT_TILE * dp; i += ATT_THREADS) {
                     const int r = i / dp, c = i - r * dp, j = base + r;
@@ -144,21 +144,22 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
             constexpr int HALF = QT > 1 ? QT / 2 : 1;
             const int key = tid & (ATT_TILE - 1), i0 = (tid / ATT_TILE) * HALF;
             if (QT > 1 || tid < ATT_TILE) {
-                float dot[HALF] = {};
+                float dot[HALF][4] = {};
 #pragma unroll 4
                 for (int d = 0; d < dp; d += 4) {
                     const float4 k4 = *reinterpret_cast<const float4*>(k_s + key * kp + d);
 #pragma unroll
                     for (int i = 0; i < HALF; ++i) {
                         const float4 q4 = *reinterpret_cast<const float4*>(q_s + (i0 + i) * dp + d);
-                        dot[i] = fmaf(q4.x, k4.x, dot[i]);
-                        dot[i] = fmaf(q4.y, k4.y, dot[i]);
-                        dot[i] = fmaf(q4.z, k4.z, dot[i]);
-                        dot[i] = fmaf(q4.w, k4.w, dot[i]);
+                        dot[i][0] = fmaf(q4.x, k4.x, dot[i][0]);
+                        dot[i][1] = fmaf(q4.y, k4.y, dot[i][1]);
+                        dot[i][2] = fmaf(q4.z, k4.z, dot[i][2]);
+                        dot[i][3] = fmaf(q4.w, k4.w, dot[i][3]);
                     }
                 }
 #pragma unroll
-                for (int i = 0; i < HALF; ++i) s_s[(i0 + i) * ATT_TILE + key] = dot[i] * scale;
+                for (int i = 0; i < HALF; ++i)
+                    s_s[(i0 + i) * ATT_TILE + key] = ((dot[i][0] + dot[i][1]) + (dot[i][2] + dot[i][3])) * scale;
             }
             __syncthreads();
 #pragma unroll
@@ -174,61 +175,67 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
                 const float lt = warp_sum(pa + pb);
                 if (lane == 0) ml[2 * i] = mt, ml[2 * i + 1] = lt;
             }
-            if (sizeof(T) == 4 && vec) asm volatile("cp.async.wait_group 0;" ::: "memory");
             __syncthreads();
             // keys outside a query's range are left out rather than weighted by zero: they may hold infinities
+            int from[QT], count[QT];                     // the keys of the tile that query i sees
+            int common = nq == QT ? ATT_TILE : 0;        // as many first keys are seen by all
 #pragma unroll
-            for (int i = 0; i < QT; ++i) a[i][0] = a[i][1] = 0.0f;
-            bool all = true;
+            for (int i = 0; i < QT; ++i) {
+                from[i] = max(0, lowest(i) - base);
+                count[i] = i < nq ? max(0, min(ATT_TILE - 1, pos[i] - base) - from[i] + 1) : 0;
+                common = from[i] > 0 ? 0 : min(common, count[i]);
 #pragma unroll
-            for (int i = 0; i < QT; ++i)
-                if (i < nq) all = all && lowest(i) <= base && pos[i] >= base + ATT_TILE - 1;
-            if (all && nq == QT) {
+                for (int v = 0; v < NV; ++v) a[i][v] = 0.0f;
+            }
 #pragma unroll 4
-                for (int j = 0; j < ATT_TILE; ++j) {
-                    const float v0 = d0 < head_dim ? v_s[j * dp + d0] : 0.0f, v1 = d1 < head_dim ? v_s[j * dp + d1] : 0.0f;
+            for (int j = 0; j < common; ++j) {
+                float v[NV];
+                v[0] = d0 < head_dim ? v_s[j * dp + d0] : 0.0f;
+                if (NV > 1) v[NV - 1] = d1 < head_dim ? v_s[j * dp + d1] : 0.0f;
 #pragma unroll
-                    for (int i = 0; i < QT; ++i) {
-                        const float p = p_s[j * QT + i];
-                        a[i][0] = fmaf(p, v0, a[i][0]);
-                        if (d1 < head_dim) a[i][1] = fmaf(p, v1, a[i][1]);
-                    }
+                for (int i = 0; i < QT; ++i) {
+                    const float p = p_s[j * QT + i];
+#pragma unroll
+                    for (int e = 0; e < NV; ++e) a[i][e] = fmaf(p, v[e], a[i][e]);
                 }
-            } else {
-                for (int j = 0; j < keys; ++j) {
-                    const float v0 = d0 < head_dim ? v_s[j * dp + d0] : 0.0f, v1 = d1 < head_dim ? v_s[j * dp + d1] : 0.0f;
+            }
+            for (int j = common; j < keys; ++j) {
+                float v[NV];
+                v[0] = d0 < head_dim ? v_s[j * dp + d0] : 0.0f;
+                if (NV > 1) v[NV - 1] = d1 < head_dim ? v_s[j * dp + d1] : 0.0f;
 #pragma unroll
-                    for (int i = 0; i < QT; ++i) {
-                        if (i >= nq || base + j < lowest(i) || base + j > pos[i]) continue;
-                        const float p = p_s[j * QT + i];
-                        a[i][0] = fmaf(p, v0, a[i][0]);
-                        if (d1 < head_dim) a[i][1] = fmaf(p, v1, a[i][1]);
-                    }
+                for (int i = 0; i < QT; ++i) {
+                    if ((unsigned)(j - from[i]) >= (unsigned)count[i]) continue;
+                    const float p = p_s[j * QT + i];
+#pragma unroll
+                    for (int e = 0; e < NV; ++e) a[i][e] = fmaf(p, v[e], a[i][e]);
                 }
             }
         };
-        auto fold = [&](int i, float mt, float lt, float a0, float a1) {
+        auto fold = [&](int i, float mt, float lt, const float (&at)[NV]) {
             if (!begun[i]) {
                 begun[i] = true;
-                m[i] = mt, l[i] = lt, acc[i][0] = a0, acc[i][1] = a1;
+                m[i] = mt, l[i] = lt;
+#pragma unroll
+                for (int e = 0; e < NV; ++e) acc[i][e] = at[e];
                 return;
             }
             const float m_new = fmaxf(m[i], mt), c = expf(m[i] - m_new), ct = expf(mt - m_new);
             m[i] = m_new;
             l[i] = l[i] * c + lt * ct;
-            acc[i][0] = acc[i][0] * c + a0 * ct;
-            acc[i][1] = acc[i][1] * c + a1 * ct;
+#pragma unroll
+            for (int e = 0; e < NV; ++e) acc[i][e] = acc[i][e] * c + at[e] * ct;
         };
 
         const int tile0 = first / ATT_TILE, tile1 = last / ATT_TILE + 1;
         __syncthreads();                                 // the queries are there
         if constexpr (CL == 1) {
             for (int tile = tile0; tile < tile1; ++tile) {
-                float a[QT][2];
+                float a[QT][NV];
                 do_tile(tile, hold_ml, a);
 #pragma unroll
                 for (int i = 0; i < QT; ++i)
-                    if (sees(i, tile)) fold(i, hold_ml[2 * i], hold_ml[2 * i + 1], a[i][0], a[i][1]);
+                    if (sees(i, tile)) fold(i, hold_ml[2 * i], hold_ml[2 * i + 1], a[i]);
                 __syncthreads();                         // the tile's shared memory is read, the next one may come
             }
         } else {
@@ -238,27 +245,38 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
                 for (int slot = 0; slot < HOLD; ++slot) {
                     const int tile = round + slot * CL + rank;
                     if (tile >= tile1) break;
-                    float a[QT][2];
+                    float a[QT][NV];
                     do_tile(tile, hold_ml + slot * 2 * QT, a);
 #pragma unroll
                     for (int i = 0; i < QT; ++i) {
                         if (d0 < head_dim) hold_acc[(slot * QT + i) * dp + d0] = a[i][0];
-                        if (d1 < head_dim) hold_acc[(slot * QT + i) * dp + d1] = a[i][1];
+                        if (NV > 1 && d1 < head_dim) hold_acc[(slot * QT + i) * dp + d1] = a[i][NV - 1];
                     }
                     __syncthreads();
                 }
                 cluster.sync();
                 // query i is folded by CTA i mod CL
                 const int stop = min(tile1, round + CL * HOLD);
-                for (int tile = round; tile < stop; ++tile) {
-                    const int slot = (tile - round) / CL, from = (tile - round) % CL;
-                    const float* ml = cluster.map_shared_rank(hold_ml, from) + slot * 2 * QT;
-                    const float* ha = cluster.map_shared_rank(hold_acc, from) + slot * QT * dp;
 #pragma unroll
-                    for (int i = 0; i < QT; ++i)
-                        if (i % CL == rank && sees(i, tile))
-                            fold(i, ml[2 * i], ml[2 * i + 1], d0 < head_dim ? ha[i * dp + d0] : 0.0f,
-                                 d1 < head_dim ? ha[i * dp + d1] : 0.0f);
+                for (int i = 0; i < QT; ++i) {
+                    if (i % CL != rank || i >= nq) continue;
+                    constexpr int BATCH = 8;             // results on their way at once
+                    for (int t = round; t < stop; t += BATCH) {
+                        float mt[BATCH], lt[BATCH], at[BATCH][NV];
+#pragma unroll
+                        for (int e = 0; e < BATCH; ++e) {
+                            const int n = min(t + e, stop - 1) - round, slot = n / CL;
+                            const float* ml = cluster.map_shared_rank(hold_ml, n % CL) + slot * 2 * QT;
+                            const float* ha = cluster.map_shared_rank(hold_acc, n % CL) + (slot * QT + i) * dp;
+                            mt[e] = ml[2 * i];
+                            lt[e] = ml[2 * i + 1];
+                            at[e][0] = d0 < head_dim ? ha[d0] : 0.0f;
+                            if (NV > 1) at[e][NV - 1] = d1 < head_dim ? ha[d1] : 0.0f;
+                        }
+#pragma unroll
+                        for (int e = 0; e < BATCH; ++e)
+                            if (t + e < stop && sees(i, t + e)) fold(i, mt[e], lt[e], at[e]);
+                    }
                 }
                 cluster.sync();
             }
@@ -268,21 +286,24 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
             if (i >= nq || (CL > 1 && i % CL != rank)) continue;
             T* o = out + (long)(t0 + i) * out_ld + (long)h * head_dim;
             if (d0 < head_dim) o[d0] = from_f32<T>(acc[i][0] / l[i]);
-            if (d1 < head_dim) o[d1] = from_f32<T>(acc[i][1] / l[i]);
+            if (NV > 1 && d1 < head_dim) o[d1] = from_f32<T>(acc[i][NV - 1] / l[i]);
         }
         __syncthreads();                                 // the queries are read, the next request's may come
     }
 }
 
-template <typename T, int QT, int CL>
+template <typename T, int QT, int CL, int NV>
 static int att_launch(const T* q, long q_ld, T* out, long out_ld, const T* k_cache, const T* v_cache, long page_stride,
                       int page_size, const int* block_table, int bt_stride, const int* tok_req, const int* positions,
                       int n_tokens, int n_heads, int n_kv_heads, int head_dim, int window, float scale, cudaStream_t stream) {
-    auto kernel = paged_attention_simt_kernel<T, QT, CL>;
+    auto kernel = paged_attention_simt_kernel<T, QT, CL, NV>;
     const size_t smem = 4 * (size_t)att_floats(QT, AttHold<QT>::TILES, att_pad(head_dim));
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return (int)err;
-    const int vec = head_dim % 4 == 0 && page_stride % 4 == 0 && (((uintptr_t)k_cache | (uintptr_t)v_cache) % 16) == 0;
+    const int vec = head_dim % 4 == 0 && ATT_THREADS % (head_dim / 4) == 0 && page_stride % 4 == 0 && (((uintptr_t)k_cache | (uintptr_t)v_cache) % 16) == 0;
+    int page_shift = -1;
+    if ((page_size & (page_size - 1)) == 0)
+        for (page_shift = 0; (1 << page_shift) < page_size;) ++page_shift;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((n_tokens + QT - 1) / QT) * CL, n_heads);
     cfg.blockDim = dim3(ATT_THREADS);
@@ -298,7 +319,7 @@ static int att_launch(const T* q, long q_ld, T* out, long out_ld, const T* k_cac
     cfg.attrs = attr;
     cfg.numAttrs = fl_pdl_enabled() ? 2 : 1;
     return (int)cudaLaunchKernelEx(&cfg, kernel, q, q_ld, out, out_ld, k_cache, v_cache, page_stride, page_size, block_table,
-                                   bt_stride, tok_req, positions, n_tokens, n_heads, n_kv_heads, head_dim, window, scale, vec);
+                                   bt_stride, tok_req, positions, n_tokens, n_heads, n_kv_heads, head_dim, window, scale, vec, page_shift);
 }
 
 // q: [n_tokens, q_ld] with head h at columns [h*head_dim, (h+1)*head_dim);
@@ -318,20 +339,28 @@ FL_API int fl_paged_attention_simt(const void* q, int dtype, long q_ld, void* ou
     // As many CTAs a cluster as keep the launch within two CTAs an SM or so: more only wait for one another.
     const long units = (long)((n_tokens + (single ? 0 : 7)) / (single ? 1 : 8)) * n_heads;
     const int cl = units * 4 <= 2L * sms ? 8 : units <= sms ? 4 : units <= 2L * sms ? 2 : 1;
-#define ATT_GO(QT, CL)                                                                                                    \
-    FL_DISPATCH(dtype, T, return (att_launch<T, QT, CL>((const T*)q, q_ld, (T*)out, out_ld, (const T*)k_cache,            \
-                                                        (const T*)v_cache, page_stride, page_size, block_table, bt_stride, \
-                                                        tok_req, positions, n_tokens, n_heads, n_kv_heads, head_dim,      \
-                                                        window, scale, stream)))
-    if (single) {
-        if (cl == 8) ATT_GO(1, 8);
-        if (cl == 4) ATT_GO(1, 4);
-        if (cl == 2) ATT_GO(1, 2);
-        ATT_GO(1, 1);
+#define ATT_GO(QT, CL, NV)                                                                                                \
+    FL_DISPATCH(dtype, T, return (att_launch<T, QT, CL, NV>((const T*)q, q_ld, (T*)out, out_ld, (const T*)k_cache,        \
+                                                            (const T*)v_cache, page_stride, page_size, block_table,      \
+                                                            bt_stride, tok_req, positions, n_tokens, n_heads, n_kv_heads, \
+                                                            head_dim, window, scale, stream)))
+    if (head_dim > ATT_THREADS) {
+        if (single) {
+            if (cl >= 4) ATT_GO(1, 4, 2);
+            ATT_GO(1, 1, 2);
+        }
+        if (cl >= 4) ATT_GO(8, 4, 2);
+        ATT_GO(8, 1, 2);
     }
-    if (cl == 8) ATT_GO(8, 8);
-    if (cl == 4) ATT_GO(8, 4);
-    if (cl == 2) ATT_GO(8, 2);
-    ATT_GO(8, 1);
+    if (single) {
+        if (cl == 8) ATT_GO(1, 8, 1);
+        if (cl == 4) ATT_GO(1, 4, 1);
+        if (cl == 2) ATT_GO(1, 2, 1);
+        ATT_GO(1, 1, 1);
+    }
+    if (cl == 8) ATT_GO(8, 8, 1);
+    if (cl == 4) ATT_GO(8, 4, 1);
+    if (cl == 2) ATT_GO(8, 2, 1);
+    ATT_GO(8, 1, 1);
 #undef ATT_GO
 }
