@@ -1115,6 +1115,15 @@ FL_API int fl_gemm_tc_glu(const void* A, long lda, const void* W, long ldw, void
         while (bn < M) bn *= 2;
         feat = 16;
         while (feat < 64 && (I + feat - 1) / feat > 2 * num_sms) feat += 8;
+        // An MMA takes the time to read 128 rows of weights from shared memory, however few of them are features, so an SM
+        // with two CTAs is twice as long at its K steps.  Where CTAs of at most 64 features fill nearly all SMs one by one,
+        // that is faster (5504 features, K = 2048, 1 token: 230 CTAs of 24 took 13.0 us, 138 of 40 take 11.5).
+        for (int one = 16; one <= 64; one += 8) {
+            const int ctas = (I + one - 1) / one;
+            if (ctas > num_sms) continue;
+            if (ctas * 8 >= num_sms * 7 && one > feat) feat = one;
+            break;
+        }
         if ((I + feat - 1) / feat < (num_sms + 1) / 2) return -1;
     } else {
         int splits = 0;
