@@ -81,6 +81,72 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(
     }
 }
 
+// The same for prompts with heads of 128 channels on both sides and up to four taps: a warp takes PREP_TOKENS neighbouring
+// tokens of one unit, four channels a lane, so the taps are read once, a unit's sum of squares stays in the warp and 16
+// tokens' decays (double precision, a thread each) are formed side by side.  A block a (token, unit) took 101 us for 2048
+// tokens of 32 units, most of it blocks coming and going; a layer takes 45 us less so.  Sums in the order of the block's: the four
+// groups of 32 channels by themselves, then (0 + 2) + (1 + 3).
+#define PREP_TOKENS 16
+template <typename T, typename TW>
+__global__ void __launch_bounds__(128) delta_prep_rows_kernel(
+    const T* __restrict__ proj, long ld, const TW* __restrict__ conv_w, const TW* __restrict__ a_log,
+    const TW* __restrict__ dt_bias, const float* __restrict__ state, long state_stride, long tail_off,
+    const int* __restrict__ tok_req, const int* __restrict__ positions, const int* __restrict__ req_ctx,
+    const int* __restrict__ req_slot, float* __restrict__ work, long work_ld, int n_tokens,
+    int heads, int kv_heads, int taps, float unit_eps, float q_scale) {
+    pdl_wait();
+    pdl_trigger();
+    constexpr int D = 128;
+    const int lane = threadIdx.x & 31, unit = blockIdx.y * 4 + (threadIdx.x >> 5);
+    if (unit >= 2 * kv_heads + heads) return;
+    const int t0 = blockIdx.x * PREP_TOKENS, t1 = min(n_tokens, t0 + PREP_TOKENS);
+    const int qk_cols = kv_heads * D, hv = heads * D, channels = 2 * qk_cols + hv, first = unit * D + lane;
+    const bool is_v = unit >= 2 * kv_heads;
+    float w[4][4];                                           // [channel group][tap, oldest first; from 4 - taps on]
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) w[e][k] = k >= 4 - taps ? to_f32<TW>(conv_w[(long)(first + 32 * e) * taps + k - (4 - taps)]) : 0.0f;
+#pragma unroll 2
+    for (int t = t0; t < t1; ++t) {
+        const int r = tok_req[t], pos = positions[t], ctx = req_ctx[r];
+        const float* tail = state + (long)req_slot[r] * state_stride + tail_off;
+        const T* row = proj + (long)t * ld;
+        float y[4], ss[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int c = first + 32 * e;
+            float acc = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int back = 3 - k, p = pos - back;
+                if (back >= taps || p < 0) continue;
+                const float x = p >= ctx ? to_f32<T>(row[c - (long)back * ld]) : tail[(long)(p - ctx + taps - 1) * channels + c];
+                acc = fmaf(w[e][k], x, acc);
+            }
+            y[e] = acc / (1.0f + expf(-acc));
+            ss[e] = y[e] * y[e];
+        }
+        float f = 1.0f;
+        if (!is_v) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) ss[e] = warp_sum(ss[e]);
+            f = (unit < kv_heads ? q_scale : 1.0f) / sqrtf((ss[0] + ss[2]) + (ss[1] + ss[3]) + unit_eps);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) work[(long)t * work_ld + first + 32 * e] = is_v ? y[e] : y[e] * f;
+    }
+    if (is_v && t0 + lane < t1) {
+        const int t = t0 + lane, h = unit - 2 * kv_heads;
+        const T* row = proj + (long)t * ld;
+        const double b = (double)to_f32<T>(row[channels + hv + h]);
+        const double a = (double)to_f32<T>(row[channels + hv + heads + h]) + (double)to_f32<TW>(dt_bias[h]);
+        const double softplus = a > 30.0 ? a : log1p(exp(a));
+        work[(long)t * work_ld + channels + h] = (float)(1.0 / (1.0 + exp(-b)));
+        work[(long)t * work_ld + channels + heads + h] = (float)exp(-exp((double)to_f32<TW>(a_log[h])) * softplus);
+    }
+}
+
 template <typename T>
 __global__ void delta_tail_kernel(const T* __restrict__ proj, long ld, float* __restrict__ state, long state_stride,
                                   long tail_off, const int* __restrict__ req_start, const int* __restrict__ req_ctx,
@@ -438,11 +504,19 @@ FL_API int fl_delta_prep(const void* proj, int dtype, long ld, const void* conv_
     if (taps < 1 || heads % kv_heads || n_requests > 65535 || units > 65535 || (size_t)widest * sizeof(float) > 48 * 1024)
         return (int)cudaErrorInvalidValue;
     int rc = 0;
-    FL_DISPATCH(dtype, T, FL_DISPATCH(w_dtype, TW,
-        rc = fl_launch(delta_prep_kernel<T, TW>, dim3(n_tokens, units), dim3(128), (size_t)widest * sizeof(float), stream,
+    // (from 256 tokens on: 32 units are then 512 warps, about one for every scheduler)
+    if (dim == 128 && vdim == 128 && taps <= 4 && n_tokens >= 256)
+        FL_DISPATCH(dtype, T, FL_DISPATCH(w_dtype, TW,
+            rc = fl_launch(delta_prep_rows_kernel<T, TW>, dim3((n_tokens + PREP_TOKENS - 1) / PREP_TOKENS, (units + 3) / 4), dim3(128), 0,
+                           stream, (const T*)proj, ld, (const TW*)conv_w, (const TW*)a_log, (const TW*)dt_bias, (const float*)state,
+                           state_stride, tail_off, tok_req, positions, req_ctx, req_slot, work, work_ld, n_tokens, heads, kv_heads,
+                           taps, unit_eps, q_scale)))
+    else
+        FL_DISPATCH(dtype, T, FL_DISPATCH(w_dtype, TW,
+            rc = fl_launch(delta_prep_kernel<T, TW>, dim3(n_tokens, units), dim3(128), (size_t)widest * sizeof(float), stream,
                        (const T*)proj, ld, (const TW*)conv_w, (const TW*)a_log, (const TW*)dt_bias, (const float*)state,
                        state_stride, tail_off, tok_req, positions, req_ctx, req_slot, work, work_ld, heads, kv_heads,
-                       dim, vdim, taps, unit_eps, q_scale)));
+                       dim, vdim, taps, unit_eps, q_scale)))
     if (rc || taps == 1) return rc;
     FL_DISPATCH(dtype, T,
         return fl_launch(delta_tail_kernel<T>, dim3((channels + 255) / 256, n_requests), dim3(256), 0, stream,

@@ -262,6 +262,40 @@ def test_command_line_on_a_random_weights_folder(tmp_path):
 
 # ------------------------------------------------------------------ kernels alone
 
+@pytest.mark.parametrize("taps", [1, 2, 4])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_delta_preparation_of_prompts_is_that_of_few_tokens(taps, dtype):
+    """From 256 tokens on, with heads of 128, a kernel of its own prepares them: the same bits as in slices of fewer tokens,
+    over requests that meet inside its groups of 16, at their start, behind a saved tail and shorter than the taps."""
+    from types import SimpleNamespace
+
+    from fastllm_py_b200.native import ops
+
+    torch.manual_seed(taps)
+    heads, kv_heads, dim = 6, 3, 128
+    lens = [(0, 133), (7, 1), (0, 2), (1, 5), (90, 178)]                       # (tokens before the step, tokens in it)
+    n, qk, hv = sum(m for _, m in lens), kv_heads * dim, heads * dim
+    channels, tail_off = 2 * qk + hv, hv * dim
+    proj = torch.randn(n, channels + hv + 2 * heads, device="cuda").to(dtype)
+    conv = (0.5 * torch.randn(channels, taps, device="cuda")).to(dtype)
+    a_log, dt_bias = torch.randn(heads, device="cuda").to(dtype), torch.randn(heads, device="cuda").to(dtype)
+    state = torch.randn(len(lens), tail_off + 3 * channels, device="cuda")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    starts = i32([sum(m for _, m in lens[:r]) for r in range(len(lens) + 1)])
+    tok_req, positions = i32([r for r, (_, m) in enumerate(lens) for _ in range(m)]), i32([c + i for c, m in lens for i in range(m)])
+    works = []
+    for cuts in ([(0, n)], [(0, 100), (100, 255), (255, n)]):
+        work = torch.zeros(n, 2 * qk + hv + 2 * heads + hv, device="cuda")
+        for a, b in cuts:
+            step = SimpleNamespace(tok_req=tok_req[a:b], positions=positions[a:b], req_start=starts - a, req_ctx=i32([c for c, _ in lens]),
+                                   req_qlen=i32([m for _, m in lens]), req_slot=i32(list(range(len(lens)))), n_requests=len(lens), n_tokens=b - a)
+            ops.delta_prep(proj[a:b], conv, a_log, dt_bias, state.clone(), tail_off, step, work[a:b], heads, kv_heads, dim, dim, taps, 1e-6,
+                           dim ** -0.5)
+        works.append(work)
+    assert n >= 256 and bool(torch.isfinite(works[0]).all()) and float(works[0].abs().sum()) > 0
+    assert torch.equal(works[0], works[1])
+
+
 @pytest.mark.parametrize("width, ff, counts, top, gated, on_input", [
     (32, 32, [1], 1, True, False), (96, 160, [255, 0, 257, 1], 1, True, True), (256, 224, [64, 65, 256, 600], 2, True, False),
     (544, 416, [300, 31, 513], 3, False, True), (128, 96, [3] * 70, 2, False, False), (2048, 1408, [250, 270, 8], 1, True, False)])
