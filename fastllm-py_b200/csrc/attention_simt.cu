@@ -106,7 +106,8 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
         // The result of one tile: maximum and sum of query i in ml[2 i], ml[2 i + 1], the weighted values in `a`.
         auto do_tile = [&](int tile, float* ml, float (&a)[QT][NV]) {
             const int base = tile * ATT_TILE, keys = min(ATT_TILE, last + 1 - base);
-            // keys and values of the tile, rows past the last visible key left as zeros (their pages may hold anything)
+            // keys and values of the tile, rows outside first .. last left as zeros: what lies past the last visible key may
+            // hold anything, and the table has -1 for pages that every window in the step has passed
             if (sizeof(T) == 4 && vec) {
                 // a thread copies one 16-byte column of every `step`-th row
                 const int per = head_dim / 4, step = ATT_THREADS / per, c = (tid % per) * 4;
@@ -114,7 +115,7 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
 #pragma unroll 4
                 for (int r = tid / per; r < ATT_TILE; r += step) {
                     const int j = base + r;
-                    if (r < keys) {
+                    if (j >= first && r < keys) {
                         const int page = page_shift >= 0 ? j >> page_shift : j / page_size;
                         const long off = (long)bt[page] * page_stride + (long)(j - page * page_size) * head_dim;
                         att_cp16(k_s + r * kp + c, kc + off);
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
                 for (int i = tid; i < ATT_TILE * dp; i += ATT_THREADS) {
                     const int r = i / dp, c = i - r * dp, j = base + r;
                     float kv = 0.0f, vv = 0.0f;
-                    if (r < keys && c < head_dim) {
+                    if (j >= first && r < keys && c < head_dim) {
                         const long off = (long)bt[j / page_size] * page_stride + head_off + (long)(j % page_size) * head_dim + c;
                         kv = to_f32<T>(k_cache[off]);
                         vv = to_f32<T>(v_cache[off]);

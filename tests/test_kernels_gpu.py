@@ -413,6 +413,31 @@ def test_cuda_core_attention_order(head_dim, window, dtype):
             assert torch.equal(run(a, a + n, single), base[a:a + n]), (a, n, single)
 
 
+@pytest.mark.parametrize("head_dim, page_size, dtype", [(128, 16, torch.float32), (48, 8, torch.float32), (64, 16, torch.bfloat16)])
+@pytest.mark.parametrize("q_lens", [[1], [1, 1, 1], [9, 8, 40]])
+def test_cuda_core_attention_behind_pages_given_back(q_lens, head_dim, page_size, dtype):
+    """The table has -1 for the pages that every window has passed, in the middle of a tile of keys too.  The cache lies
+    inside a larger allocation, so that a page of -1 would be memory of this test."""
+    window = 37
+    case = AttentionCase(q_lens, [310, 140, 131][:len(q_lens)], 4, 2, head_dim, page_size, dtype, seed=5)
+    room = torch.full((case.cache.shape[0] + 4, *case.cache.shape[1:]), float("nan"), dtype=dtype, device=DEV)
+    room[2:-2] = case.cache
+    case.cache = room[2:-2]
+    for r, ctx in enumerate(case.ctx_lens):
+        gone = (ctx - window + 1) // page_size
+        assert gone * page_size % 64, "the first tile holds keys of pages that are gone"
+        case.cache[case.block_table[r, :gone].long()] = float("nan")
+        case.block_table[r, :gone] = -1
+    want = case.reference(window)
+    assert float((run_simt(case, window) - want).abs().max()) <= case.tolerance()
+    from fastllm_py_b200.native import ops
+
+    alone = torch.zeros_like(case.q)
+    ops.paged_attention_simt(case.q, alone, case.cache, case.block_table, case.tok_req, case.positions, case.heads,
+                             case.kv_heads, head_dim, window, head_dim ** -0.5, page_size, True)
+    assert float((alone.float().cpu() - want).abs().max()) <= case.tolerance()
+
+
 @pytest.mark.parametrize("runner", [run_simt, run_fast, run_fast_tcgen05, run_fast_cuda_core_decode])
 def test_a_far_key_among_hundreds_is_found(runner):
     """One key far back (and one right at a page edge, one at a split edge) gets
