@@ -169,8 +169,8 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
                 const int ja = base + lane, jb = ja + 32;
                 const bool va = ja >= lowest(i) && ja <= pos[i], vb = jb >= lowest(i) && jb <= pos[i];
                 const float sa = va ? s_s[i * ATT_TILE + lane] : -CUDART_INF_F, sb = vb ? s_s[i * ATT_TILE + lane + 32] : -CUDART_INF_F;
-                const float mt = warp_max(fmaxf(sa, sb));
-                const float pa = va ? expf(sa - mt) : 0.0f, pb = vb ? expf(sb - mt) : 0.0f;
+                const float mt = warp_max(fmaxf(sa, sb)), at = mt == -CUDART_INF_F ? 0.0f : mt;     // (scores of -inf: no weight)
+                const float pa = va ? expf(sa - at) : 0.0f, pb = vb ? expf(sb - at) : 0.0f;
                 p_s[lane * QT + i] = pa;
                 p_s[(lane + 32) * QT + i] = pb;
                 const float lt = warp_sum(pa + pb);
@@ -221,7 +221,8 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
                 for (int e = 0; e < NV; ++e) acc[i][e] = at[e];
                 return;
             }
-            const float m_new = fmaxf(m[i], mt), c = expf(m[i] - m_new), ct = expf(mt - m_new);
+            const float m_new = fmaxf(m[i], mt), at_new = m_new == -CUDART_INF_F ? 0.0f : m_new;
+            const float c = expf(m[i] - at_new), ct = expf(mt - at_new);
             m[i] = m_new;
             l[i] = l[i] * c + lt * ct;
 #pragma unroll

@@ -438,6 +438,25 @@ def test_cuda_core_attention_behind_pages_given_back(q_lens, head_dim, page_size
     assert float((alone.float().cpu() - want).abs().max()) <= case.tolerance()
 
 
+@pytest.mark.parametrize("low", [(0, 64), (64, 128), (128, 210), (0, 210)])
+@pytest.mark.parametrize("q_lens", [[1], [10]])
+def test_cuda_core_attention_with_scores_of_minus_infinity(low, q_lens):
+    """Tiles whose keys all score -infinity, the first, a middle and the last one, weigh nothing beside the others; where
+    there are no others the result is 0 / 0."""
+    case = AttentionCase(q_lens, [200], 2, 1, 32, 16, torch.float32, seed=6)
+    case.q[:, ::32] = 1.0
+    for q in case.q_rows:
+        q[:, :, 0] = 1.0
+    case.k_full[0][low[0]:low[1], :, 0] = -math.inf
+    for j in range(low[0], min(low[1], case.k_full[0].shape[0])):
+        case.cache[case.block_table[0, j // 16].long(), 0, :, j % 16, 0] = -math.inf
+    got, want = run_simt(case), case.reference()
+    if low == (0, 210):
+        assert bool(got.isnan().all()) and bool(want.isnan().all())
+    else:
+        assert bool(want.isfinite().all()) and float((got - want).abs().max()) <= case.tolerance()
+
+
 @pytest.mark.parametrize("runner", [run_simt, run_fast, run_fast_tcgen05, run_fast_cuda_core_decode])
 def test_a_far_key_among_hundreds_is_found(runner):
     """One key far back (and one right at a page edge, one at a split edge) gets
