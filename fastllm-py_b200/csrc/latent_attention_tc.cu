@@ -387,8 +387,8 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
     uint64_t* s_full = k_empty + LP_STAGES;               // [2]
     uint64_t* c_full = s_full + 2;                        // [2] the rows' rescaling factors are there
     uint64_t* p_full = c_full + 2;                        // [2] weights written and accumulators rescaled
-    uint64_t* o_done = p_full + 2;
-    uint32_t* tmem_slot = (uint32_t*)(o_done + 1);
+    uint64_t* o_done = p_full + 2;                        // [2] values of tile i are added up: barrier i & 1, phase i >> 1
+    uint32_t* tmem_slot = (uint32_t*)(o_done + 2);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     volatile int* never = abort_flag + 1;                 // stays 0: for waits that must not be cut short
     float* corr_s = reinterpret_cast<float*>((unsigned char*)bars + 256);                // [2][128]
@@ -423,8 +423,8 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
             mbar_init(&s_full[b], 1);
             mbar_init(&c_full[b], 4);
             mbar_init(&p_full[b], 8);
+            mbar_init(&o_done[b], 1);
         }
-        mbar_init(o_done, 1);
         *abort_flag = (*(volatile int*)status != 0) ? 1 : 0;
         *never = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
                     umma_bf16_ts(tmem_o, tmem_s + (uint32_t)(b * LT_KEYS + k * 8), lp_desc_values(va + (uint32_t)(k * 16 * 128)), idesc_o,
                                  (i > 0 || k > 0) ? 1u : 0u);
                 umma_commit(&k_empty[s]);
-                umma_commit(o_done);                      // phase i: the accumulators hold the tiles up to i
+                umma_commit(&o_done[b]);                  // the accumulators hold the tiles up to i
             }
             __syncwarp();
         }
@@ -586,7 +586,9 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
         inv_s[r] = ok ? 1.0f / l : 0.0f;
         lp_warp_arrive(&c_full[n_tiles & 1]);             // (one phase more than tiles: the sums are there)
     } else {
-        // ---- accumulators of row r
+        // ---- accumulators of row r.  A wait on o_done tells a phase from the one before it only, so no barrier of the two
+        // may get two phases ahead of these warps: they wait for the values of tile i - 2 before they let those of tile i
+        // go (the scores of tile i came after them: this wait is over at once), and for tile i - 1 where they rescale.
         const int r = threadIdx.x - 128, token = r >> 4;
         const uint32_t o_addr = tmem_o + ((uint32_t)((warp - 4) * 32) << 16);
         bool ok = !*abort_flag;
@@ -594,9 +596,11 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
             const int b = i & 1;
             ok = lp_warp_wait(&c_full[b], (uint32_t)(i >> 1) & 1u, abort_flag);
             if (!ok) break;
+            if (i > 1) ok = lp_warp_wait(&o_done[i & 1], (uint32_t)((i - 2) >> 1) & 1u, abort_flag);
+            if (!ok) break;
             const float corr = corr_s[b * 128 + r];
             if (i > 0 && __any_sync(0xffffffffu, corr != 1.0f)) {
-                ok = lp_warp_wait(o_done, (uint32_t)(i - 1) & 1u, abort_flag);
+                ok = lp_warp_wait(&o_done[(i - 1) & 1], (uint32_t)((i - 1) >> 1) & 1u, abort_flag);
                 if (!ok) break;
                 tc_fence_after();
 #pragma unroll 2
@@ -616,7 +620,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
             lp_warp_arrive(&p_full[b]);
         }
         if (ok) ok = lp_warp_wait(&c_full[n_tiles & 1], (uint32_t)(n_tiles >> 1) & 1u, abort_flag);
-        if (ok) ok = lp_warp_wait(o_done, (uint32_t)(n_tiles - 1) & 1u, abort_flag);
+        if (ok) ok = lp_warp_wait(&o_done[(n_tiles - 1) & 1], (uint32_t)((n_tiles - 1) >> 1) & 1u, abort_flag);
         if (!ok && lane == 0) give_up();
         ok = __all_sync(0xffffffffu, ok) && !*abort_flag;
         ok = __all_sync(0xffffffffu, ok);

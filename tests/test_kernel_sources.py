@@ -3,6 +3,8 @@ kernels' sources, since no run may provoke them."""
 import re
 from pathlib import Path
 
+import pytest
+
 CSRC = Path(__file__).resolve().parent.parent / "fastllm-py_b200" / "csrc"
 
 
@@ -15,3 +17,46 @@ def test_cuda_core_attention_looks_up_only_pages_in_sight():
     for at in lookups:
         guard = text[text.rindex("if (", 0, at):at].split("{")[0]
         assert "j >= first" in guard and "r < keys" in guard, guard
+
+
+def waits_on_values(name):
+    """The o_done protocol of an attention kernel on the tensor cores, from its source: how many barriers, which one a
+    block's value product arrives on, and the waits (barrier, parity) of the warps that rescale and read the accumulators:
+    [one in every block, if there is one], where they rescale, at the end; functions of the block i, or of their number n."""
+    text = (CSRC / name).read_text()
+    expr = lambda c: re.sub(r"(\d)u\b", r"\1", c.replace("(uint32_t)", "").replace("n_tiles", "n").replace("n_blocks", "n"))
+    index = lambda c: expr(c[len("&o_done["):-1]) if "[" in c else "0"
+    commit = re.search(r"commit\((&o_done\[[^\]]*\]|o_done)\)", text).group(1)
+    commit = index(commit).replace("b", "(i & 1)")
+    waits = [(index(m.group(1)), expr(m.group(2))) for m in
+             re.finditer(r"warp_wait\((&o_done\[[^\]]*\]|o_done), (.*?), abort_flag\)", text)]
+    return commit, waits
+
+
+@pytest.mark.parametrize("name", ["latent_attention_tc.cu"])
+def test_waits_for_the_value_products_cannot_pass_early(name):
+    """A wait on a barrier's parity is over when the phase of that parity is the one completed last: also while the barrier
+    still is two phases behind.  Every state that the value products can be in at each wait, going only by what the warp
+    itself has waited for, with every choice of the blocks that rescale: a wait is over exactly when its product is done."""
+    commit, waits = waits_on_values(name)
+    assert 2 <= len(waits) <= 3
+    every, rescale, final = ([None] + waits)[-3:]
+    at = lambda e, **v: eval(e, {}, v)                                    # the source's own expressions
+    barrier_of = lambda t: at(commit, i=t)
+
+    def wait(known, most, target, barrier, parity):
+        """`known` .. `most` products may be done, in order; waits for product `target`."""
+        for done in range(known, most + 1):
+            phase = sum(barrier_of(t) == barrier for t in range(done))    # phases of this barrier that are complete
+            assert ((phase - 1) & 1 == parity) == (done > target), (done, target)
+        return max(known, target + 1)
+
+    for n in range(1, 9):
+        for choice in range(1 << n):
+            known = 0                                                     # so many products are known to be done
+            for i in range(n):                                            # product i waits for this warp: at most i are done
+                if every is not None and i > 1:
+                    known = wait(known, i, i - 2, at(every[0], i=i), at(every[1], i=i))
+                if i > 0 and choice >> i & 1:
+                    known = wait(known, i, i - 1, at(rescale[0], i=i), at(rescale[1], i=i))
+            wait(known, n, n - 1, at(final[0], n=n), at(final[1], n=n))
