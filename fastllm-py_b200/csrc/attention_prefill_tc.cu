@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
     uint64_t* k_empty = k_full + FT_STAGES;
     uint64_t* s_full = bars + 5;                                       // [2]
     uint64_t* p_full = bars + 9;                                       // [2]
-    uint64_t* o_done = bars + 11;
+    uint64_t* o_done = bars + 11;                                      // [2] P V of block i is done: barrier i & 1, phase i >> 1
     uint32_t* tmem_slot = (uint32_t*)(bars + 13);
     uint64_t* x_bar = bars + 14;                                       // the softmax threads' exchange point
     uint64_t* v_full = k_empty + FT_STAGES;
@@ -322,8 +322,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
         for (int s = 0; s < 2; ++s) {
             ft_bar_init(&s_full[s], 1);
             ft_bar_init(&p_full[s], FT_SOFTMAX_WARPS);
+            ft_bar_init(&o_done[s], 1);
         }
-        ft_bar_init(o_done, 1);
         ft_bar_init(x_bar, FT_SOFTMAX_WARPS);
         *abort_flag = (*(volatile int*)status != 0) ? 1 : 0;
         *never = 0;
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
                     ft_mma_ts(tmem_o, pa + (uint32_t)(k * 8), ft_desc_mnmajor(va + (uint32_t)(k * 16 * 128)), idesc_o,
                               (i > 0 || k > 0) ? 1u : 0u);
                 ft_commit(&v_empty[vs]);
-                ft_commit(o_done);                  // phase i: O holds the blocks up to i
+                ft_commit(&o_done[b]);              // O holds the blocks up to i
             }
             if (!ok && !*abort_flag) { *abort_flag = 1; atomicCAS(status, 0, FT_ERR_WAIT); }
         }
@@ -428,6 +428,10 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
         bool ok = !*abort_flag;
         for (int i = 0; i < n_blocks && ok; ++i) {
             const int sb = i & 1;
+            // A wait on o_done tells a phase from the one before it only, so neither of the two barriers may get two phases
+            // ahead of this warp: P(i), which it sends below, lets P V of block i go, so that of block i - 2 is waited for
+            // here (S(i) came after it: where S(i) is there, this wait is over at once).
+            if (i > 1 && !ft_warp_wait(&o_done[i & 1], (uint32_t)((i - 2) >> 1) & 1u, abort_flag)) FT_GIVE_UP();
             if (!ft_warp_wait(&s_full[sb], (uint32_t)(i >> 1) & 1u, abort_flag)) FT_GIVE_UP();
             ft_fence_after();
             const int key0 = (kb_begin + i) * FT_BN + part * FT_KP;      // first key of this thread's part
@@ -474,7 +478,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
                 // O holds blocks 0 .. i - 1 once P V of block i - 1 is complete.  The whole warp reads,
                 // scales and writes its rows back (rows that keep their scale by 1): the loads and
                 // stores of tensor memory are warp-wide instructions.
-                if (!ft_warp_wait(o_done, (uint32_t)(i - 1) & 1u, abort_flag)) FT_GIVE_UP();
+                if (!ft_warp_wait(&o_done[(i - 1) & 1], (uint32_t)((i - 1) >> 1) & 1u, abort_flag)) FT_GIVE_UP();
                 ft_fence_after();
 #pragma unroll
                 for (int c = 0; c < FT_OD; c += 32) {
@@ -509,7 +513,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
         }
         // the whole of O, then the row's sum: the parts' sums (all relative to the same maximum)
         if (ok && n_blocks > 0) {
-            ok = ft_warp_wait(o_done, (uint32_t)(n_blocks - 1) & 1u, abort_flag);
+            ok = ft_warp_wait(&o_done[(n_blocks - 1) & 1], (uint32_t)((n_blocks - 1) >> 1) & 1u, abort_flag);
             if (!ok && !*abort_flag) { *abort_flag = 1; atomicCAS(status, 0, FT_ERR_WAIT); }
             ft_fence_after();
         }

@@ -33,7 +33,7 @@ def waits_on_values(name):
     return commit, waits
 
 
-@pytest.mark.parametrize("name", ["latent_attention_tc.cu"])
+@pytest.mark.parametrize("name", ["latent_attention_tc.cu", "attention_prefill_tc.cu"])
 def test_waits_for_the_value_products_cannot_pass_early(name):
     """A wait on a barrier's parity is over when the phase of that parity is the one completed last: also while the barrier
     still is two phases behind.  Every state that the value products can be in at each wait, going only by what the warp
