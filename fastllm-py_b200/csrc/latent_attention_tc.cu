@@ -31,24 +31,28 @@ __device__ __forceinline__ void lt_cp16(void* smem, const void* gmem, int bytes)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes));
 }
 
-template <typename TO>
-__global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
-    const bf16* __restrict__ q, long q_ld, TO* __restrict__ out, long out_ld, const bf16* __restrict__ cache,
-    int page_size, const int* __restrict__ block_table, int bt_stride, const int* __restrict__ tok_req,
-    const int* __restrict__ positions, int heads, int window, float scale, int split_keys, float* __restrict__ partial, const float* __restrict__ sink) {
-    pdl_wait();
-    pdl_trigger();
-    extern __shared__ __align__(16) unsigned char lt_smem[];
+#define LT_SMEM ((16 * LT_PITCH + 2 * LT_KEYS * LT_PITCH + 16 * LT_PPITCH) * 2 + 2 * LT_WARPS * 16 * 4)
+
+// Among the threads of `latent_token`: the whole block, or the first four warps of a larger one.
+template <bool WHOLE> __device__ __forceinline__ void lt_sync() {
+    if (WHOLE) __syncthreads();
+    else asm volatile("bar.sync 1, %0;" ::"n"(LT_WARPS * 32) : "memory");
+}
+
+// One token and 16 heads, by threads 0 .. LT_WARPS * 32 - 1 of the block (WHOLE: it has no others) with LT_SMEM bytes at
+// lt_smem.  q, out: the token's rows; bt: its request's row of the block table; partial: where the token's splits go.
+template <typename TO, bool WHOLE>
+__device__ __forceinline__ void latent_token(unsigned char* lt_smem, const bf16* __restrict__ q, TO* __restrict__ out,
+                                             const bf16* __restrict__ cache, int page_size, const int* __restrict__ bt, int pos,
+                                             int heads, int head0, int window, float scale, int split_keys, int split, int n_splits,
+                                             float* __restrict__ partial, const float* __restrict__ sink) {
     bf16* q_s = reinterpret_cast<bf16*>(lt_smem);                         // [16][LT_PITCH]
     bf16* k_s = q_s + 16 * LT_PITCH;                                      // [2][LT_KEYS][LT_PITCH]
     bf16* p_s = k_s + 2 * LT_KEYS * LT_PITCH;                             // [16][LT_PPITCH]
     float* red_max = reinterpret_cast<float*>(p_s + 16 * LT_PPITCH);      // [LT_WARPS][16]
     float* red_sum = red_max + LT_WARPS * 16;                             // [LT_WARPS][16]
-    const int t = blockIdx.x, head0 = blockIdx.y * 16;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int pos = positions[t];
     const int lo = window > 0 ? max(0, pos - window + 1) : 0;
-    const int* bt = block_table + (long)tok_req[t] * bt_stride;
 
     auto stage = [&](int buf, int tile) {
         bf16* dst = k_s + (long)buf * LT_KEYS * LT_PITCH;
@@ -63,21 +67,21 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
         }
         asm volatile("cp.async.commit_group;");
     };
-    // with split_keys (a multiple of LT_KEYS) the block takes only the keys of split blockIdx.z, counted from
+    // with split_keys (a multiple of LT_KEYS) the block takes only the keys of split `split`, counted from
     // the multiple of split_keys at or below the first visible key, and leaves (accumulator, maximum, sum)
     // in `partial` for the merge kernel; the splits' borders depend on the token's own position only
     int first_tile = (lo / LT_KEYS) * LT_KEYS, last = pos;
     if (split_keys > 0) {
-        first_tile = (lo / split_keys + (int)blockIdx.z) * split_keys;
+        first_tile = (lo / split_keys + split) * split_keys;
         last = min(pos, first_tile + split_keys - 1);
         first_tile = max(first_tile, (lo / LT_KEYS) * LT_KEYS);      // (no tile wholly out of sight: its maximum would be -inf)
     }
     float* part_row = nullptr;
     if (split_keys > 0) {
-        part_row = partial + (((long)t * heads) * gridDim.z + blockIdx.z) * (LAT_RANK + 2);     // + head * gridDim.z * (rank + 2)
+        part_row = partial + (long)split * (LAT_RANK + 2);   // + head * n_splits * (rank + 2)
         if (first_tile > pos) {                              // nothing of this split is in sight
             for (int r = tid; r < 16 && head0 + r < heads; r += LT_WARPS * 32) {
-                float* pr = part_row + (long)(head0 + r) * gridDim.z * (LAT_RANK + 2);
+                float* pr = part_row + (long)(head0 + r) * n_splits * (LAT_RANK + 2);
                 pr[LAT_RANK] = -CUDART_INF_F;
                 pr[LAT_RANK + 1] = 0.0f;
             }
@@ -88,7 +92,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
     for (int c = tid; c < 16 * (LT_WIDTH / 8); c += LT_WARPS * 32) {     // the 16 heads' q~
         const int r = c / (LT_WIDTH / 8), piece = c % (LT_WIDTH / 8);
         uint4 v = make_uint4(0, 0, 0, 0);
-        if (head0 + r < heads) v = *reinterpret_cast<const uint4*>(q + (long)t * q_ld + (long)(head0 + r) * LT_WIDTH + piece * 8);
+        if (head0 + r < heads) v = *reinterpret_cast<const uint4*>(q + (long)(head0 + r) * LT_WIDTH + piece * 8);
         *reinterpret_cast<uint4*>(q_s + r * LT_PITCH + piece * 8) = v;
     }
     float acc[LT_NT][4];
@@ -112,7 +116,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
         } else {
             asm volatile("cp.async.wait_group 0;");
         }
-        __syncthreads();
+        lt_sync<WHOLE>();
         const bf16* ks = k_s + (long)buf * LT_KEYS * LT_PITCH;
         // ---- scores of this warp's 8 keys
         float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -145,7 +149,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
             red_max[warp * 16 + row0] = mx[0];
             red_max[warp * 16 + row0 + 8] = mx[1];
         }
-        __syncthreads();
+        lt_sync<WHOLE>();
         float corr[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -162,7 +166,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
             if ((lane & 3) == 0) red_sum[warp * 16 + r] = sum;
             *reinterpret_cast<__nv_bfloat162*>(p_s + r * LT_PPITCH + warp * 8 + (lane & 3) * 2) = __floats2bfloat162_rn(p0, p1);
         }
-        __syncthreads();
+        lt_sync<WHOLE>();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             float sum = 0.0f;
@@ -192,14 +196,14 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
                              : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
             }
         }
-        __syncthreads();                                     // the tile, p_s and the reductions are rewritten next
+        lt_sync<WHOLE>();                                     // the tile, p_s and the reductions are rewritten next
     }
     if (split_keys > 0) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int head = head0 + row0 + h * 8;
             if (head >= heads) continue;
-            float* pr = part_row + (long)head * gridDim.z * (LAT_RANK + 2);
+            float* pr = part_row + (long)head * n_splits * (LAT_RANK + 2);
             float* o = pr + warp * LT_VCOLS + (lane & 3) * 2;
 #pragma unroll
             for (int n = 0; n < LT_NT; ++n) {
@@ -217,7 +221,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
     for (int h = 0; h < 2; ++h) {
         const int head = head0 + row0 + h * 8;
         if (head >= heads) continue;
-        TO* o = out + (long)t * out_ld + (long)head * LAT_RANK + warp * LT_VCOLS + (lane & 3) * 2;
+        TO* o = out + (long)head * LAT_RANK + warp * LT_VCOLS + (lane & 3) * 2;
         const float inv = 1.0f / l_run[h];
 #pragma unroll
         for (int n = 0; n < LT_NT; ++n) {
@@ -225,6 +229,21 @@ __global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
             o[n * 8 + 1] = from_f32<TO>(acc[n][h * 2 + 1] * inv);
         }
     }
+}
+
+template <typename TO>
+__global__ void __launch_bounds__(LT_WARPS * 32) latent_attention_tc_kernel(
+    const bf16* __restrict__ q, long q_ld, TO* __restrict__ out, long out_ld, const bf16* __restrict__ cache,
+    int page_size, const int* __restrict__ block_table, int bt_stride, const int* __restrict__ tok_req,
+    const int* __restrict__ positions, int heads, int window, float scale, int split_keys, float* __restrict__ partial, const float* __restrict__ sink) {
+    pdl_wait();
+    pdl_trigger();
+    extern __shared__ __align__(16) unsigned char lt_smem[];
+    const int t = blockIdx.x;
+    latent_token<TO, true>(lt_smem, q + (long)t * q_ld, out + (long)t * out_ld, cache, page_size,
+                           block_table + (long)tok_req[t] * bt_stride, positions[t], heads, blockIdx.y * 16, window, scale,
+                           split_keys, blockIdx.z, gridDim.z,
+                           split_keys > 0 ? partial + (long)t * heads * gridDim.z * (LAT_RANK + 2) : nullptr, sink);
 }
 
 // out[t, head] = sum_z acc_z e^(m_z - M) / ([e^(sink - M) +] sum_z l_z e^(m_z - M)), splits in order; one block per (token, head).
@@ -271,8 +290,7 @@ FL_API int fl_latent_attention_tc(const void* q, long q_ld, void* out, int out_d
         return (int)cudaErrorInvalidValue;
     if (((uintptr_t)q % 16) || (q_ld % 8) || ((uintptr_t)cache % 16) || (heads + 15) / 16 > 65535)
         return (int)cudaErrorInvalidValue;
-    const size_t smem = (size_t)(16 * LT_PITCH + 2 * LT_KEYS * LT_PITCH + 16 * LT_PPITCH) * sizeof(bf16) +
-                        2 * LT_WARPS * 16 * sizeof(float);
+    const size_t smem = LT_SMEM;
     static bool raised = false;
     if (!raised && smem > 48 * 1024) {
         cudaError_t rc = cudaFuncSetAttribute(latent_attention_tc_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -301,6 +319,11 @@ FL_API int fl_latent_attention_tc(const void* q, long q_ld, void* out, int out_d
 // weights' sums in the same tree, a rescaling at every tile where the maximum moved (where it did not, the other kernel
 // multiplies by one), so results are the same bit for bit.
 //
+// A tile serves tokens that do not see all of its keys, with weights of zero, and zero times a value that is not finite is
+// NaN, where the other kernel never reads keys out of a token's sight.  Such a key shows in its scores (a sum with a term
+// that is not finite is not finite): where a score out of a token's sight is not finite, the CTA's tokens are done again
+// token by token, by the other kernel's code.  Only tiles at a border of what the tokens see are looked at.
+//
 // Tensor memory holds 512 columns, so a CTA accumulates LP_VC = 256 value columns at most, and the CTAs of a tile's two
 // halves both compute its scores.  Roles in a CTA of 320 threads:
 //   warps 0-3  a row's weights: scores from tensor memory, maximum, exponentials, the weights as bfloat16 back into tensor
@@ -327,6 +350,7 @@ FL_API int fl_latent_attention_tc(const void* q, long q_ld, void* out, int out_d
 #define LP_SMEM (LP_ATOMS * LP_Q_ATOM + LP_STAGES * LP_STAGE_BYTES + 256 + 3 * 128 * 4 + 1024)
 enum { LP_ERR_WAIT = 141 };
 static_assert(LP_SMEM <= 232448, "more shared memory than a CTA can have");
+static_assert(LT_SMEM <= LP_ATOMS * LP_Q_ATOM + LP_STAGES * LP_STAGE_BYTES, "tokens done again find room in the tiles' place");
 
 __device__ __forceinline__ void lp_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -371,12 +395,23 @@ __device__ __forceinline__ uint64_t lp_desc_values(uint32_t saddr) {
            ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
+// The tokens of a CTA one by one (a function of its own, so that the kernel's warps keep their registers).
+template <typename TO>
+__device__ __noinline__ void lp_again(unsigned char* smem, const bf16* q, long q_ld, TO* out, long out_ld, const bf16* cache,
+                                      int page_size, const int* bt, int pos, int tokens, int heads, int head0, int window,
+                                      float scale, const float* sink) {
+    for (int k = 0; k < tokens; ++k)
+        latent_token<TO, false>(smem, q + k * q_ld, out + k * out_ld, cache, page_size, bt, pos + k, heads, head0, window, scale, 0,
+                                0, 1, nullptr, sink);
+}
+
 template <typename TO>
 __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
-    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, TO* __restrict__ out, long out_ld,
-    int page_size, int cache_rows, const int* __restrict__ block_table, int bt_stride, const int* __restrict__ req_start,
-    const int* __restrict__ req_ctx, const int* __restrict__ req_qlen, int n_requests, int window, float scale,
-    const float* __restrict__ sink, int* __restrict__ status) {
+    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const bf16* __restrict__ q, long q_ld,
+    TO* __restrict__ out, long out_ld, const bf16* __restrict__ cache, int heads, int page_size, int cache_rows,
+    const int* __restrict__ block_table, int bt_stride, const int* __restrict__ req_start, const int* __restrict__ req_ctx,
+    const int* __restrict__ req_qlen, int n_requests, int window, float scale, const float* __restrict__ sink,
+    int* __restrict__ status) {
     extern __shared__ unsigned char lp_raw[];
     unsigned char* q_s = (unsigned char*)(((uintptr_t)lp_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* k_s = q_s + LP_ATOMS * LP_Q_ATOM;
@@ -391,6 +426,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
     uint32_t* tmem_slot = (uint32_t*)(o_done + 2);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     volatile int* never = abort_flag + 1;                 // stays 0: for waits that must not be cut short
+    volatile int* again = never + 1;                      // the tokens are done again
     float* corr_s = reinterpret_cast<float*>((unsigned char*)bars + 256);                // [2][128]
     float* inv_s = corr_s + 2 * 128;                                                     // [128]
 
@@ -427,6 +463,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
         }
         *abort_flag = (*(volatile int*)status != 0) ? 1 : 0;
         *never = 0;
+        *again = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -527,6 +564,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
         const uint32_t lanes = (uint32_t)(warp * 32) << 16;
         const int pos = token < tokens ? pos_first + token : -1;
         const int lo = window > 0 ? max(0, pos - window + 1) : 0;
+        const int lo_last = window > 0 ? max(0, pos_last - window + 1) : 0;
         float m = -CUDART_INF_F, l = 0.0f;
         if (sink != nullptr) {
             m = sink[head0 + (r & 15)];
@@ -546,6 +584,13 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
             tmem_ld16(tmem_s + (uint32_t)(b * LT_KEYS) + 16u + lanes, v + 16);
             tmem_ld_wait();
             const int key0 = (t_begin + i) * LT_KEYS;
+            if (key0 + LT_KEYS - 1 > pos_first || key0 < lo_last) {       // some token does not see all of the tile
+                bool odd = false;
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    odd |= (key0 + j < lo || key0 + j > pos) && !(fabsf(__uint_as_float(v[j])) < CUDART_INF_F);
+                if (odd && token < tokens) *again = 1;
+            }
             float p[32], mx[4];
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
@@ -625,7 +670,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
         ok = __all_sync(0xffffffffu, ok) && !*abort_flag;
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
-        if (ok) {
+        if (ok && !*again) {
             const float inv = inv_s[r];
             TO* dst = out + (long)(tok0 + token) * out_ld + (long)(head0 + (r & 15)) * LAT_RANK + half * LP_VC;
 #pragma unroll 1
@@ -650,6 +695,9 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
         tc_fence_after();
         tmem_dealloc(tmem_o, 512u);
     }
+    if (*again && !*abort_flag && half == 0 && warp < LT_WARPS)           // (all columns: the halves agree, their scores are the same)
+        lp_again<TO>(q_s, q + (long)tok0 * q_ld, q_ld, out + (long)tok0 * out_ld, out_ld, cache, page_size, block_table + (long)req * bt_stride,
+                     pos_first, tokens, heads, head0, window, scale, sink);
 }
 
 // What the prompt kernel takes beyond what latent_attention_tc_kernel does: whole groups of 16 heads, 16-byte aligned rows
@@ -688,7 +736,8 @@ FL_API int fl_latent_prompt(const void* q, long q_ld, void* out, int out_dtype, 
     FL_DISPATCH(out_dtype, TO, {
         rc = (int)cudaFuncSetAttribute(latent_prompt_kernel<TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, LP_SMEM);
         if (rc) return rc;
-        latent_prompt_kernel<TO><<<grid, LP_THREADS, LP_SMEM, stream>>>(map_q, map_k, (TO*)out, out_ld, page_size, (int)cache_rows,
+        latent_prompt_kernel<TO><<<grid, LP_THREADS, LP_SMEM, stream>>>(map_q, map_k, (const bf16*)q, q_ld, (TO*)out, out_ld,
+                                                                        (const bf16*)cache, heads, page_size, (int)cache_rows,
                                                                         block_table, bt_stride, req_start, req_ctx, req_qlen,
                                                                         n_requests, window, scale, sink, status);
         return fl_launch_status();

@@ -532,6 +532,35 @@ def test_latent_prompt_kernel_is_the_other_kernel_bit_for_bit(rank, rot, heads, 
     assert torch.equal(got[:n], want)
 
 
+@pytest.mark.parametrize("rank,heads,page,window", [(512, 16, 16, None), (512, 32, 64, 40), (256, 16, 8, 33)])
+def test_latent_prompt_kernel_with_rows_that_are_not_finite(rank, heads, page, window):
+    """An infinite or NaN cache row is the concern of the tokens that see it: not of the earlier ones of its group of eight,
+    not of those whose window has passed it, and the result does not depend on how the prompt is cut."""
+    from fastllm_py_b200.native import ops
+
+    torch.manual_seed(rank + page)
+    rot, n = 64, 150
+    width = rank + rot
+    odd = {13: float("inf"), 64: float("-inf"), 101: float("nan")}                # row -> what it holds in one column
+    table = torch.randperm(-(-n // page) + 2, device="cuda").to(torch.int32)[:-(-n // page)].view(1, -1).contiguous()
+    cache = torch.zeros(table.numel() + 2, page, width, device="cuda", dtype=torch.bfloat16)
+    for j, row in enumerate(torch.randn(n, width, device="cuda")):
+        cache[table[0, j // page].long(), j % page] = row.to(torch.bfloat16)
+        if j in odd:
+            cache[table[0, j // page].long(), j % page, 7 * j % rank] = odd[j]
+    q = (0.3 * torch.randn(n, heads * width, device="cuda")).to(torch.bfloat16)
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    want = torch.empty(n, heads * rank, device="cuda", dtype=torch.bfloat16)
+    ops.latent_attention_tc(q, want, cache, table, i32(*[0] * n), i32(*range(n)), heads, rank, rot, window, 0.1, page)
+    seen = torch.tensor([any(j <= t and (window is None or j > t - window) for j in odd) for t in range(n)], device="cuda")
+    assert bool(want[~seen].isfinite().all()) and not bool(want[seen].isfinite().all(dim=1).any())
+    for cuts in ((0, n), (0, 11, 100, n)):
+        got = torch.empty_like(want)
+        for a, b in zip(cuts, cuts[1:]):
+            ops.latent_prompt(q[a:b], got[a:b], cache, table, i32(0, b - a), i32(a), i32(b - a), heads, rank, rot, window, 0.1, page)
+        assert bool(((got == want) | (got.isnan() & want.isnan())).all()), cuts
+
+
 def test_gated_product_with_relu_and_gelu_in_its_epilogue():
     """The tensor-core product that applies the gate's activation itself, for the activations beside silu,
     in its one-tile form (a decode-sized step) and its CTA-pair form (a prompt-sized step)."""
