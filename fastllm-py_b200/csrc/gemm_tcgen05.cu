@@ -187,9 +187,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(
             // is complete; two halves in turn, one barrier a round), and the threads share out the
             // 16 x feat results, a token's features side by side.
             // All four warps take the same decisions, so that the barrier below is always met.
-            if (!ok) *abort_flag = 1;
-            epilogue_sync();
-            ok = !*abort_flag;
+            ok = !epilogue_any(!ok || *abort_flag != 0);
             const int row = quarter * 32 + lane;
             const int f0 = tile_n * feat;
             const uint32_t t_base = tmem_acc + ((uint32_t)(quarter * 32) << 16);
@@ -243,9 +241,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(
             // 16 tokens x 128 features at a time go through shared memory (the ring is idle once the
             // accumulator is complete; two halves in turn, one barrier a round) and leave as whole rows.
             // All four warps take the same decisions, so that the barrier below is always met.
-            if (!ok) *abort_flag = 1;
-            epilogue_sync();
-            ok = !*abort_flag;
+            ok = !epilogue_any(!ok || *abort_flag != 0);
             const uint32_t t_base = tmem_acc + ((uint32_t)(quarter * 32) << 16);
             const int t0 = tile_m * BN;
             const int e = quarter * 32 + lane;                        // this thread's feature among the CTA's 128
@@ -584,11 +580,9 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_pair_kernel(
         for (int i = 0; i < my_units && ok; ++i) {
             const int buf = i & 1;
             const uint32_t use = (uint32_t)(i >> 1);
-            bool got = mbar_wait(&acc_full[buf], use & 1u, abort_flag);
+            const bool got = mbar_wait(&acc_full[buf], use & 1u, abort_flag);
             if (!got && !*abort_flag) { *abort_flag = 1; atomicCAS(status, 0, TC_ERR_ACC_WAIT); }
-            epilogue_sync();                                // the four warps decide together (they share barriers below)
-            got = !*abort_flag;
-            if (!got) {
+            if (epilogue_any(!got || *abort_flag != 0)) {   // the four warps decide together (they share barriers below)
                 ok = false;
                 break;
             }

@@ -569,8 +569,7 @@ __global__ void __launch_bounds__(TC_THREADS) moe_group_kernel(
             const int buf = i & 1;
             const uint32_t use = (uint32_t)(i >> 1);
             if (!mbar_wait(&acc_full[buf], use & 1u, abort_flag)) give_up();
-            epilogue_sync();                                // the four warps decide together (they share barriers below)
-            if (*abort_flag) break;
+            if (epilogue_any(*abort_flag != 0)) break;      // the four warps decide together (they share barriers below)
             tc_fence_after();
             const int4 t = tiles[u / tiles_n];
             const int f0 = (u % tiles_n) * FEATURES + (int)rank * (FEATURES / 2), cols = n_out - f0;

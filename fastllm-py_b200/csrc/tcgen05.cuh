@@ -157,6 +157,22 @@ template <int N> __device__ __forceinline__ void unary_act(uint32_t (&r)[N], con
 
 // A barrier among the four epilogue warps only (hardware barrier 1; barrier 0 is __syncthreads).
 __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// The same, and whether any of the 128 threads came with `flag`: how they decide to give up.  After a plain barrier each
+// would read the abort flag for itself, and one that another role sets between two of these reads would leave some warps at
+// a barrier that the others never come to.
+__device__ __forceinline__ bool epilogue_any(bool flag) {
+    uint32_t any;
+    __syncwarp();
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, 1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(any)
+        : "r"((uint32_t)flag)
+        : "memory");
+    return any != 0;
+}
 
 // Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes
 // (64 bfloat16) in the 128-byte swizzle: 8-row groups are 1024 bytes apart.

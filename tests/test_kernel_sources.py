@@ -60,3 +60,14 @@ def test_waits_for_the_value_products_cannot_pass_early(name):
                 if i > 0 and choice >> i & 1:
                     known = wait(known, i, i - 1, at(rescale[0], i=i), at(rescale[1], i=i))
             wait(known, n, n - 1, at(final[0], n=n), at(final[1], n=n))
+
+
+def test_epilogue_warps_give_up_together():
+    """The epilogue's four warps meet at barriers of their own, so they must leave a unit of work together.  The abort flag can
+    change between two warps' looks at it: no decision to leave may be a look after a barrier, only the barrier's own vote."""
+    for path in sorted(CSRC.glob("*.cu")):
+        text = path.read_text()
+        assert not re.search(r"epilogue_sync\(\);[^\n]*\n[^\n]*abort_flag", text), path.name
+        voted = re.findall(r"epilogue_any\([^;]*abort_flag", text)
+        assert len(voted) == {"gemm_tcgen05.cu": 3, "moe.cu": 1}.get(path.name, 0), path.name
+    assert re.search(r"epilogue_any\(bool flag\).*?red\.or\.pred", (CSRC / "tcgen05.cuh").read_text(), re.S)

@@ -94,6 +94,31 @@ def test_tensor_core_gemm_in_cta_pairs_every_tile_and_split(bn, splits, m, out_d
         assert float((slabs.sum(0).cpu() - ref).abs().max()) <= 1e-3 * math.sqrt(k)
 
 
+def test_products_after_a_recorded_fault_leave_at_once():
+    """With a fault in the status word every role of every kernel gives up at its first look, whatever it waits for then:
+    the launches return and write nothing."""
+    from fastllm_py_b200.native import gemm_tc
+
+    g = torch.Generator().manual_seed(9)
+    a, w = (torch.randn(600, 520, generator=g).to(torch.bfloat16).to(DEV), torch.randn(2 * 1500, 520, generator=g).to(torch.bfloat16).to(DEV))
+    word = gemm_tc.status_word(torch.device(DEV))
+    outs = []
+    try:
+        word.fill_(101)
+        for m, bn in ((5, 16), (60, 64), (200, 256), (90, 576), (150, 640), (600, 512)):
+            outs.append(torch.full((m, 3000), 7.0, dtype=torch.bfloat16, device=DEV))
+            gemm_tc.gemm(a[:m], w, outs[-1], bn=bn, splits=1)
+        for m in (5, 600):
+            outs.append(torch.full((m, 1500), 7.0, dtype=torch.bfloat16, device=DEV))
+            gemm_tc.gemm_swiglu(a[:m], w, outs[-1])
+        torch.cuda.synchronize()
+        assert int(word.item()) == 101 and all(bool((o == 7.0).all()) for o in outs)
+    finally:
+        word.zero_()
+    gemm_tc.gemm(a, w, outs[5], bn=512, splits=1)                         # and the next launch works again
+    assert float((outs[5].float() - a.float() @ w.float().t()).abs().max()) <= 1.0
+
+
 @pytest.mark.parametrize("m, n, k", [(3, 300, 728), (40, 130, 72), (70, 515, 200), (300, 700, 1000), (600, 257, 520)])
 def test_packed_weights_give_the_row_major_result(m, n, k):
     """A weight packed by k-block ([ceil(K / 64)][N][64], what a model's matrices become at load) and
