@@ -98,7 +98,8 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const TA* __restrict__ A
 // A CTA of 64 threads serves 8 x RT features: thread (slice s, row r) sums slice s of features r, r + 8, ... for all MT
 // rows of A.  W and A pass through a ring of shared-memory stages, 32 inputs of every slice each, filled by 16-byte
 // cp.async: what bounds the product is the stream of W, so the ring keeps 3 of 4 stages (24 KB a CTA, several CTAs an
-// SM) in flight and W's first stages are asked for before the preceding kernel has ended.  A staged row of W is padded
+// SM) in flight, and where the caller says that no kernel writes W (constant_w) its first stages are asked for before the
+// preceding kernel has ended.  A staged row of W is padded
 // to 36 floats: the eight lanes of a quarter warp, on eight rows, then read all 32 banks.  MT rows of A are read
 // (rows past M repeat the last one and are not written).  RT = 2 above four rows of A, so that a value of A that has
 // been read from shared memory serves two features.
@@ -123,7 +124,8 @@ __device__ __forceinline__ void sk_cp16(float* smem, const float* gmem, bool val
 template <typename TC, int MT>
 __global__ void __launch_bounds__(64) gemm_f32_skinny_kernel(const float* __restrict__ A, long lda,
                                                              const float* __restrict__ W, long ldw,
-                                                             TC* __restrict__ C, long ldc, int M, int N, int K, int slice) {
+                                                             TC* __restrict__ C, long ldc, int M, int N, int K, int slice,
+                                                             int constant_w) {
     using L = Skinny<MT>;
     constexpr int RT = L::RT, R = L::R, STAGES = L::STAGES;
     extern __shared__ __align__(16) float sk_smem[];
@@ -143,10 +145,12 @@ __global__ void __launch_bounds__(64) gemm_f32_skinny_kernel(const float* __rest
 #pragma unroll
         for (int m = 0; m < MT; ++m) sk_cp16(dst + m * SK_BK, k < K ? A + (long)min(m, M - 1) * lda + k : A, k < K);
     };
-    for (int t = 0; t < STAGES - 1 && t < n_st; ++t) load_w(t);
+    if (constant_w)
+        for (int t = 0; t < STAGES - 1 && t < n_st; ++t) load_w(t);
     pdl_wait();
     pdl_trigger();
     for (int t = 0; t < STAGES - 1; ++t) {
+        if (t < n_st && !constant_w) load_w(t);
         if (t < n_st) load_a(t);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
@@ -363,12 +367,12 @@ __global__ void __cluster_dims__(1, 1, GS_SLICES) __launch_bounds__(TL_THREADS, 
 
 // ------------------------------------------------------------ host side
 template <typename TC, int MT>
-static int gs_skinny(const float* A, long lda, const float* W, long ldw, TC* C, long ldc, int M, int N, int K, cudaStream_t stream) {
+static int gs_skinny(const float* A, long lda, const float* W, long ldw, TC* C, long ldc, int M, int N, int K, int constant_w, cudaStream_t stream) {
     using L = Skinny<MT>;
     auto kernel = gemm_f32_skinny_kernel<TC, MT>;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
     if (err != cudaSuccess) return (int)err;
-    return fl_launch(kernel, dim3((N + L::R - 1) / L::R), dim3(64), L::SMEM, stream, A, lda, W, ldw, C, ldc, M, N, K, gs_slice(K));
+    return fl_launch(kernel, dim3((N + L::R - 1) / L::R), dim3(64), L::SMEM, stream, A, lda, W, ldw, C, ldc, M, N, K, gs_slice(K), constant_w);
 }
 
 // Float operands that 16-byte loads can read.  Up to 16 rows W's bytes decide and the skinny kernel streams them; above,
@@ -376,12 +380,12 @@ static int gs_skinny(const float* A, long lda, const float* W, long ldw, TC* C, 
 // CTAs (two an SM) times the inputs that a CTA goes through, a split CTA paying about 40 inputs' time for the exchange.
 template <typename TC>
 static int gs_f32(const float* A, long lda, const float* W, long ldw, TC* C, long ldc, int M, int N, int K, int sms,
-                  cudaStream_t stream) {
-    if (M <= 1) return gs_skinny<TC, 1>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-    if (M <= 2) return gs_skinny<TC, 2>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-    if (M <= 4) return gs_skinny<TC, 4>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-    if (M <= 8) return gs_skinny<TC, 8>(A, lda, W, ldw, C, ldc, M, N, K, stream);
-    if (M <= 16) return gs_skinny<TC, 16>(A, lda, W, ldw, C, ldc, M, N, K, stream);
+                  int constant_w, cudaStream_t stream) {
+    if (M <= 1) return gs_skinny<TC, 1>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
+    if (M <= 2) return gs_skinny<TC, 2>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
+    if (M <= 4) return gs_skinny<TC, 4>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
+    if (M <= 8) return gs_skinny<TC, 8>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
+    if (M <= 16) return gs_skinny<TC, 16>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
     const int slice = gs_slice(K);
     dim3 grid((N + TL_BN - 1) / TL_BN, (M + TL_BM - 1) / TL_BM);
     if (grid.y > 65535) return (int)cudaErrorInvalidValue;
@@ -395,12 +399,13 @@ static int gs_f32(const float* A, long lda, const float* W, long ldw, TC* C, lon
     return fl_launch(gemm_f32_tile_kernel<TC>, grid, dim3(TL_THREADS), 0, stream, A, lda, W, ldw, C, ldc, M, N, K, slice);
 }
 
+// constant_w: no kernel that may still run when this one is launched writes W (which is then read ahead of it).
 FL_API int fl_gemm_simt(const void* A, int a_dtype, long lda, const void* W, int w_dtype, long ldw,
-                        void* C, int c_dtype, long ldc, int M, int N, int K, int sms, cudaStream_t stream) {
+                        void* C, int c_dtype, long ldc, int M, int N, int K, int sms, int constant_w, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (a_dtype == FL_F32 && w_dtype == FL_F32 && K > 0 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
         ((uintptr_t)A | (uintptr_t)W) % 16 == 0) {
-        FL_DISPATCH(c_dtype, TC, return gs_f32<TC>((const float*)A, lda, (const float*)W, ldw, (TC*)C, ldc, M, N, K, sms, stream));
+        FL_DISPATCH(c_dtype, TC, return gs_f32<TC>((const float*)A, lda, (const float*)W, ldw, (TC*)C, ldc, M, N, K, sms, constant_w, stream));
     }
     dim3 grid((N + GS_BN - 1) / GS_BN, (M + GS_BM - 1) / GS_BM);
     if (grid.y > 65535) return (int)cudaErrorInvalidValue;

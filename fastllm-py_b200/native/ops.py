@@ -1364,15 +1364,16 @@ def paged_attention_simt(q, out, cache, block_table, tok_req, positions, n_heads
 
 # ----------------------------------------------------------------------- GEMM
 
-def gemm_simt(a, w, out):
-    """out[M, N] = a[M, K] @ w[N, K]^T, float accumulation on CUDA cores, any dtypes."""
+def gemm_simt(a, w, out, constant_w=False):
+    """out[M, N] = a[M, K] @ w[N, K]^T, float accumulation on CUDA cores, any dtypes.  `constant_w`: no kernel that may still
+    be running writes `w`, as is so for a model's matrices (it is then read before the kernel in front has ended)."""
     _require_cuda(a, w, out)
     if a.shape[1] != w.shape[1] or out.shape[0] != a.shape[0] or out.shape[1] != w.shape[0]:
         raise KernelError(f"gemm: shapes {tuple(a.shape)} x {tuple(w.shape)}^T -> {tuple(out.shape)}")
     fn = _fn("gemm_simt", "fl_gemm_simt", [c_void_p, c_int, c_long, c_void_p, c_int, c_long, c_void_p,
-                                           c_int, c_long, c_int, c_int, c_int, c_int, c_void_p])
+                                           c_int, c_long, c_int, c_int, c_int, c_int, c_int, c_void_p])
     _check(fn(_ptr(a), dtype_code(a), _ld(a), _ptr(w), dtype_code(w), _ld(w), _ptr(out), dtype_code(out), _ld(out),
-              a.shape[0], w.shape[0], a.shape[1], _sms(a.device), _stream()), "gemm_simt")
+              a.shape[0], w.shape[0], a.shape[1], _sms(a.device), int(constant_w), _stream()), "gemm_simt")
 
 
 # ------------------------------------------------------------------- sampling

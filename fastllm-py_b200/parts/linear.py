@@ -67,7 +67,7 @@ class Linear:
         if self.weight is None:
             raise ops.KernelError("this Linear's matrix was packed for bfloat16 activations; it cannot "
                                   "serve 32-bit activations as well")
-        ops.gemm_simt(a, self.weight, out)
+        ops.gemm_simt(a, self.weight, out, constant_w=True)      # (a model's matrix: no kernel of a step writes it)
         return None
 
     def forward_activated(self, a: torch.Tensor, out: torch.Tensor, activation: str, params=(0.0, 0.0)) -> None:

@@ -226,6 +226,25 @@ def test_float_gemm_kernels(n, k):
         assert torch.equal(half, general[:m].to(torch.bfloat16)), m
 
 
+@pytest.mark.parametrize("m", [1, 3, 16])
+def test_float_gemm_of_a_matrix_that_the_kernel_before_wrote(m):
+    """The product for few rows reads its matrix ahead of the kernel before only where the caller says it may: here that
+    kernel writes the matrix, and lets the product start before it has."""
+    from fastllm_py_b200.native import ops
+
+    g = torch.Generator().manual_seed(m)
+    a, x, y = torch.randn(m, 1024, generator=g).to(DEV), torch.randn(2048, 512, generator=g).to(DEV), torch.randn(1024, 512, generator=g).to(DEV)
+    w, out, settled = torch.empty(2048, 1024, device=DEV), torch.empty(m, 2048, device=DEV), torch.empty(m, 2048, device=DEV)
+    ops.gemm_simt(x, y, w)
+    torch.cuda.synchronize()
+    ops.gemm_simt(a, w, settled, constant_w=True)
+    for _ in range(20):
+        w.fill_(float("nan"))
+        ops.gemm_simt(x, y, w)
+        ops.gemm_simt(a, w, out)
+        assert torch.equal(out, settled)
+
+
 # ------------------------------------------------------------------ attention
 
 class AttentionCase:
