@@ -390,15 +390,16 @@ __global__ void __launch_bounds__(COLS * DELTA_PARTS + 32) delta_scan_kernel(
     }
 }
 
-// The same for steps in which every request brings one token, where reading and writing the state is all the work: a
+// The same for steps of as many tokens as requests, all of which bring one token as a rule: reading and writing the state is
+// all the work then.  (Requests that bring none and others that bring several are walked token by token.)  A
 // thread asks for its elements of S first (16 bytes at a time where every column starts on 16 bytes), k and q come
 // through shared memory meanwhile.  (8 and 16 requests, 16 heads of 128 x 128: 6.5 and 9.8 us, through the scan's chunk
 // stages 7.0 and 11.3.)
 template <int DPT>
 __global__ void __launch_bounds__(DELTA_COLS * DELTA_PARTS) delta_step_kernel(
     float* __restrict__ work, long work_ld, float* __restrict__ state, long state_stride,
-    const int* __restrict__ req_start, const int* __restrict__ req_ctx, const int* __restrict__ req_slot, int heads,
-    int kv_heads, int dim, int vdim) {
+    const int* __restrict__ req_start, const int* __restrict__ req_ctx, const int* __restrict__ req_qlen,
+    const int* __restrict__ req_slot, int heads, int kv_heads, int dim, int vdim) {
     pdl_wait();
     pdl_trigger();
     constexpr int PART = DPT + 4, KQ = DELTA_PARTS * PART;   // as in the scan
@@ -425,38 +426,42 @@ __global__ void __launch_bounds__(DELTA_COLS * DELTA_PARTS) delta_step_kernel(
             S[i] = (!fresh && d < dim) ? s_col[d] : 0.0f;
         }
     }
-    for (int i = threadIdx.x; i < 2 * DELTA_PARTS * DPT; i += DELTA_COLS * DELTA_PARTS) {       // k, then q
-        const int side = i / (DELTA_PARTS * DPT), d = i - side * (DELTA_PARTS * DPT);
-        kq_s[side * KQ + (d / DPT) * PART + d % DPT] = d < dim ? row[(side == 0 ? qk_cols : 0) + g * dim + d] : 0.0f;
-    }
-    const float v = row[2 * qk_cols + h * vdim + jj], beta = row[2 * qk_cols + hv + h], decay = row[2 * qk_cols + hv + heads + h];
-    __syncthreads();
-    float k[DPT], a[2] = {0.0f, 0.0f}, b[2] = {0.0f, 0.0f}, c[2] = {0.0f, 0.0f};
-#pragma unroll
-    for (int i = 0; i < DPT; i += 4) {
-        const float4 kv = *reinterpret_cast<const float4*>(kq_s + part * PART + i);
-        const float4 qv = *reinterpret_cast<const float4*>(kq_s + KQ + part * PART + i);
-        k[i] = kv.x; k[i + 1] = kv.y; k[i + 2] = kv.z; k[i + 3] = kv.w;
-        const float q[4] = {qv.x, qv.y, qv.z, qv.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            a[e & 1] = fmaf(S[i + e], k[i + e], a[e & 1]);
-            b[e & 1] = fmaf(S[i + e], q[e], b[e & 1]);
-            c[e & 1] = fmaf(q[e], k[i + e], c[e & 1]);
+    const int qlen = req_qlen[r];
+    for (int n = 0; n < qlen; ++n, row += work_ld) {
+        if (n > 0) __syncthreads();                          // the token before has been read
+        for (int i = threadIdx.x; i < 2 * DELTA_PARTS * DPT; i += DELTA_COLS * DELTA_PARTS) {       // k, then q
+            const int side = i / (DELTA_PARTS * DPT), d = i - side * (DELTA_PARTS * DPT);
+            kq_s[side * KQ + (d / DPT) * PART + d % DPT] = d < dim ? row[(side == 0 ? qk_cols : 0) + g * dim + d] : 0.0f;
         }
-    }
-    float dot = a[0] + a[1], read = b[0] + b[1], qk = c[0] + c[1];
+        const float v = row[2 * qk_cols + h * vdim + jj], beta = row[2 * qk_cols + hv + h], decay = row[2 * qk_cols + hv + heads + h];
+        __syncthreads();
+        float k[DPT], a[2] = {0.0f, 0.0f}, b[2] = {0.0f, 0.0f}, c[2] = {0.0f, 0.0f};
 #pragma unroll
-    for (int o = 1; o < DELTA_PARTS; o <<= 1) {
-        dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        read += __shfl_xor_sync(0xffffffffu, read, o);
-        qk += __shfl_xor_sync(0xffffffffu, qk, o);
+        for (int i = 0; i < DPT; i += 4) {
+            const float4 kv = *reinterpret_cast<const float4*>(kq_s + part * PART + i);
+            const float4 qv = *reinterpret_cast<const float4*>(kq_s + KQ + part * PART + i);
+            k[i] = kv.x; k[i + 1] = kv.y; k[i + 2] = kv.z; k[i + 3] = kv.w;
+            const float q[4] = {qv.x, qv.y, qv.z, qv.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                a[e & 1] = fmaf(S[i + e], k[i + e], a[e & 1]);
+                b[e & 1] = fmaf(S[i + e], q[e], b[e & 1]);
+                c[e & 1] = fmaf(q[e], k[i + e], c[e & 1]);
+            }
+        }
+        float dot = a[0] + a[1], read = b[0] + b[1], qk = c[0] + c[1];
+#pragma unroll
+        for (int o = 1; o < DELTA_PARTS; o <<= 1) {
+            dot += __shfl_xor_sync(0xffffffffu, dot, o);
+            read += __shfl_xor_sync(0xffffffffu, read, o);
+            qk += __shfl_xor_sync(0xffffffffu, qk, o);
+        }
+        const float u = __fmul_rn(beta, fmaf(-decay, dot, v));
+        if (part == 0 && j < vdim) row[2 * qk_cols + hv + 2 * heads + h * vdim + j] = fmaf(decay, read, qk * u);
+#pragma unroll
+        for (int i = 0; i < DPT; ++i) S[i] = fmaf(k[i], u, __fmul_rn(decay, S[i]));
     }
-    const float u = __fmul_rn(beta, fmaf(-decay, dot, v));
     if (j >= vdim) return;
-    if (part == 0) row[2 * qk_cols + hv + 2 * heads + h * vdim + j] = fmaf(decay, read, qk * u);
-#pragma unroll
-    for (int i = 0; i < DPT; ++i) S[i] = fmaf(k[i], u, __fmul_rn(decay, S[i]));
     if (whole) {
 #pragma unroll
         for (int i = 0; i < DPT; i += 4)
@@ -525,7 +530,7 @@ FL_API int fl_delta_prep(const void* proj, int dtype, long ld, const void* conv_
     return 0;
 }
 
-// single_tokens: every request of the step brings one token (a kernel of its own).
+// single_tokens: the step has as many tokens as requests, one each as a rule (a kernel of its own).
 // work: [n_tokens, work_ld] floats, a row = q | k (kv_heads x dim each) | v (heads x vdim) | beta | decay (heads
 // each) | o (heads x vdim): fl_delta_prep fills all but o, fl_delta_scan reads them and fills o.
 FL_API int fl_delta_scan(float* work, long work_ld, float* state, long state_stride,
@@ -556,7 +561,7 @@ FL_API int fl_delta_scan(float* work, long work_ld, float* state, long state_str
     if (per_thread <= DPT) {                                                                                        \
         if (single_tokens)                                                                                          \
             return fl_launch(delta_step_kernel<DPT>, dim3(grid.x, (vdim + DELTA_COLS - 1) / DELTA_COLS), dim3(DELTA_COLS * DELTA_PARTS), 0, \
-                             stream, work, work_ld, state, state_stride, req_start, req_ctx, req_slot, heads, kv_heads, dim, vdim); \
+                             stream, work, work_ld, state, state_stride, req_start, req_ctx, req_qlen, req_slot, heads, kv_heads, dim, vdim); \
         if (narrow) FL_DELTA_SCAN_COLS(DPT, 16) else FL_DELTA_SCAN_COLS(DPT, 32)                                    \
     }
     FL_DELTA_SCAN(4);

@@ -296,6 +296,33 @@ def test_delta_preparation_of_prompts_is_that_of_few_tokens(taps, dtype):
     assert torch.equal(works[0], works[1])
 
 
+@pytest.mark.parametrize("dim, vdim", [(128, 128), (32, 48), (20, 7)])
+@pytest.mark.parametrize("lens", [[2, 0], [0, 3, 0], [1, 1, 0, 2], [4, 0, 0, 0]])
+def test_delta_scan_of_as_many_tokens_as_requests(lens, dim, vdim):
+    """Not every such step brings a token of each request: the requests' results and states are those of a step each."""
+    from types import SimpleNamespace
+
+    from fastllm_py_b200.native import ops
+
+    torch.manual_seed(dim + len(lens))
+    heads, kv_heads, n = 4, 2, sum(lens)
+    qk, hv = kv_heads * dim, heads * vdim
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    work = 0.3 * torch.randn(n, 2 * qk + hv + 2 * heads + hv, device="cuda")
+    state = torch.randn(len(lens) + 1, hv * dim, device="cuda")
+    starts = [sum(lens[:r]) for r in range(len(lens) + 1)]
+    ctx, slots = [5 * (r % 2) for r in range(len(lens))], [(r + 1) % (len(lens) + 1) for r in range(len(lens))]
+    want, want_state = work.clone(), state.clone()
+    for r, m in enumerate(lens):
+        # (the whole step's rows beside it, so that the step has more tokens than requests and takes the other kernel)
+        step = SimpleNamespace(req_start=i32(starts[r], n), req_ctx=i32(ctx[r]), req_qlen=i32(m), req_slot=i32(slots[r]), n_requests=1)
+        ops.delta_scan(want, want_state, step, heads, kv_heads, dim, vdim)
+    step = SimpleNamespace(req_start=i32(*starts), req_ctx=i32(*ctx), req_qlen=i32(*lens), req_slot=i32(*slots), n_requests=len(lens))
+    assert n == len(lens) and n > 1
+    ops.delta_scan(work, state, step, heads, kv_heads, dim, vdim)
+    assert torch.equal(work, want) and torch.equal(state, want_state)
+
+
 @pytest.mark.parametrize("width, ff, counts, top, gated, on_input", [
     (32, 32, [1], 1, True, False), (96, 160, [255, 0, 257, 1], 1, True, True), (256, 224, [64, 65, 256, 600], 2, True, False),
     (544, 416, [300, 31, 513], 3, False, True), (128, 96, [3] * 70, 2, False, False), (2048, 1408, [250, 270, 8], 1, True, False)])
