@@ -735,8 +735,9 @@ static int moe_group_launch(const void* a, const void* w, long w_rows, int n_pai
 }
 
 // ints: rows + n_tokens * top + rows / 64 + 1 of them, rows = fl_moe_group_rows: row -> pair, pair -> row, the list of tiles
-// (from a multiple of four) and its length, 2 pairs + pairs / 64 + 4 experts + 4 at most;
-// act: bfloat16 [rows, ff]; y: float [rows, width], which holds the gathered tokens before it holds the results.
+// (from a 16-byte boundary on) and its length, 2 pairs + pairs / 64 + 4 experts + 4 at most;
+// act: bfloat16 [rows, ff], 16-byte aligned; y: float [rows, width], of which the first 16-byte boundary on holds the
+// gathered tokens and then the results, a row a pair.
 FL_API int fl_moe_experts_grouped(const void* h, long h_ld, const void* w_gu, const void* w_down, const int* chosen,
                                   const float* weights, int* ints, void* act, float* y, void* out, long out_ld,
                                   int n_tokens, int width, int ff, int top, int experts, int act_code, float act_p0, float act_p1,
@@ -748,11 +749,12 @@ FL_API int fl_moe_experts_grouped(const void* h, long h_ld, const void* w_gu, co
     const int n_pairs = n_tokens * top;
     int* row_pair = ints;
     int* pair_row = ints + n_pairs;
-    int4* tiles = reinterpret_cast<int4*>(ints + (2L * n_pairs + 3) / 4 * 4);
+    int4* tiles = reinterpret_cast<int4*>(((uintptr_t)(ints + 2L * n_pairs) + 15) & ~(uintptr_t)15);
+    y = reinterpret_cast<float*>(((uintptr_t)y + 15) & ~(uintptr_t)15);
     const int max_tiles = n_pairs / MOE_TN + (experts < n_pairs ? experts : n_pairs);
     int* n_tiles = reinterpret_cast<int*>(tiles + max_tiles);
     if ((size_t)experts * sizeof(int) > 48 * 1024 || width % 32 || ff % 32 || num_sms < 2 ||
-        (((uintptr_t)h | (uintptr_t)ints | (uintptr_t)act | (uintptr_t)y) % 16) || (h_ld % 8))
+        (((uintptr_t)h | (uintptr_t)act) % 16) || (h_ld % 8))
         return (int)cudaErrorInvalidValue;
     int rc = fl_launch(moe_sort_kernel, dim3(1), dim3(1024), (size_t)experts * sizeof(int), stream, chosen, n_pairs, experts,
                        row_pair, pair_row, tiles, n_tiles);

@@ -362,6 +362,30 @@ def test_grouped_expert_products_against_64_bits(width, ff, counts, top, gated, 
     assert bool((off <= 2.0 ** -8 * want.abs() + 1.1 * 2.0 ** -9 * size + 1e-5 * size.max()).all()), float((off / size).max())
 
 
+def test_grouped_expert_products_in_buffers_at_any_element():
+    """The lists and the float rows may begin at any element of a larger buffer, with no more room than was asked for."""
+    from fastllm_py_b200.native import ops
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    experts, n, top, width, ff = 3, 131, 2, 96, 64
+    h = torch.randn(n, width, device="cuda", generator=g).to(torch.bfloat16)
+    up = (0.1 * torch.randn(experts, 2 * ff, width, device="cuda", generator=g)).to(torch.bfloat16)
+    down = (0.1 * torch.randn(experts, width, ff, device="cuda", generator=g)).to(torch.bfloat16)
+    chosen = torch.stack([torch.randperm(experts, device="cuda", generator=g)[:top] for _ in range(n)]).to(torch.int32)
+    weights = torch.rand(n, top, device="cuda", generator=g)
+    rows = ops.moe_group_rows(n, top, experts)
+    n_ints, outs = rows + n * top + rows // 64 + 1, []
+    act = torch.empty(rows, ff, device="cuda", dtype=torch.bfloat16)
+    for shift in range(4):
+        ints, y = torch.full((n_ints + 8,), -7, dtype=torch.int32, device="cuda"), torch.full((rows * width + 8,), 7.0, device="cuda")
+        outs.append(torch.empty(n, width, device="cuda", dtype=torch.bfloat16))
+        ops.moe_experts_grouped(h, up, down, chosen, weights, ints[shift:shift + n_ints], act, y[shift:shift + rows * width].view(rows, width),
+                                outs[-1])
+        assert bool((ints[:shift] == -7).all()) and bool((ints[shift + n_ints:] == -7).all())
+        assert bool((y[:shift] == 7.0).all()) and bool((y[shift + rows * width:] == 7.0).all())
+        assert torch.equal(outs[-1], outs[0])
+
+
 def test_grouped_expert_products_against_the_per_token_kernels():
     from fastllm_py_b200.native import ops
 
