@@ -737,8 +737,10 @@ static int tc_pair_tile_tokens(int M, int bnt, int tiles_n, int splits, int num_
     return best;
 }
 
+// (The tensor map of A is made here: its boxes are half as many rows as the tiles are wide, and a width of its own anywhere
+// else would leave a stage waiting for bytes that do not come.)
 template <int BNT, typename OutT, bool GATED = false, bool ROPE = false>
-static int launch_tc_pair(const CUtensorMap& map_w, const CUtensorMap& map_a, void* C, long ldc, int M, int N,
+static int launch_tc_pair(const CUtensorMap& map_w, const void* A, long lda, void* C, long ldc, int M, int N,
                           int K, int num_sms, int* status, cudaStream_t stream, int gate_rows = 0, int splits = 1,
                           int kb_per_split = 0, float* partial = nullptr, long ld_partial = 0,
                           const TcRope* rope_args = nullptr, int wp = 0, FlGate act = FlGate{FL_ACT_NONE, 0.0f, 0.0f}) {
@@ -755,6 +757,9 @@ static int launch_tc_pair(const CUtensorMap& map_w, const CUtensorMap& map_a, vo
     }
     const int tiles_n = GATED ? (N + 127) / 128 : (N + 255) / 256;
     const int wt = tc_pair_tile_tokens(M, BNT, tiles_n, splits, num_sms);
+    CUtensorMap map_a;
+    const int rc = make_map(&map_a, A, M, K, lda, wt / 2);
+    if (rc) return rc;
     const int num_tiles = tiles_n * ((M + wt - 1) / wt);
     const long num_units = (long)num_tiles * splits;
     const int pairs = num_units < num_sms / 2 ? (int)num_units : num_sms / 2;
@@ -777,13 +782,13 @@ static int launch_tc_pair(const CUtensorMap& map_w, const CUtensorMap& map_a, vo
 }
 
 template <typename OutT>
-static int dispatch_tc_pair(int bnt, const CUtensorMap& map_w, const CUtensorMap& map_a, void* C, long ldc, int M,
+static int dispatch_tc_pair(int bnt, const CUtensorMap& map_w, const void* A, long lda, void* C, long ldc, int M,
                             int N, int K, int num_sms, int* status, cudaStream_t stream, int splits,
                             int kb_per_split, float* partial, long ld_partial, int wp, FlGate act) {
     switch (bnt) {
-        case 64: return launch_tc_pair<64, OutT>(map_w, map_a, C, ldc, M, N, K, num_sms, status, stream, 0, splits, kb_per_split, partial, ld_partial, nullptr, wp, act);
-        case 128: return launch_tc_pair<128, OutT>(map_w, map_a, C, ldc, M, N, K, num_sms, status, stream, 0, splits, kb_per_split, partial, ld_partial, nullptr, wp, act);
-        case 256: return launch_tc_pair<256, OutT>(map_w, map_a, C, ldc, M, N, K, num_sms, status, stream, 0, splits, kb_per_split, partial, ld_partial, nullptr, wp, act);
+        case 64: return launch_tc_pair<64, OutT>(map_w, A, lda, C, ldc, M, N, K, num_sms, status, stream, 0, splits, kb_per_split, partial, ld_partial, nullptr, wp, act);
+        case 128: return launch_tc_pair<128, OutT>(map_w, A, lda, C, ldc, M, N, K, num_sms, status, stream, 0, splits, kb_per_split, partial, ld_partial, nullptr, wp, act);
+        case 256: return launch_tc_pair<256, OutT>(map_w, A, lda, C, ldc, M, N, K, num_sms, status, stream, 0, splits, kb_per_split, partial, ld_partial, nullptr, wp, act);
     }
     return (int)cudaErrorInvalidValue;
 }
@@ -1040,14 +1045,14 @@ static int gemm_tc_impl(const void* A, long lda, const void* W, long ldw, void* 
     const bool paired = bn >= 512;                           // 512, 640, 576: pair kernel, 256 / 128 / 64 tokens wide
     const int bnt = bn == 512 ? 256 : bn - 512;
     if (paired && (num_sms < 2 || (bnt != 64 && bnt != 128 && bnt != 256))) return (int)cudaErrorInvalidValue;
-    rc = make_map(&map_a, A, M, K, lda, paired ? tc_pair_tile_tokens(M, bnt, (N + 255) / 256, splits, num_sms) / 2 : bn);
+    if (!paired) rc = make_map(&map_a, A, M, K, lda, bn);
     if (rc) return rc;
-    if (paired) {                                            // each CTA of a pair loads half of the token rows
+    if (paired) {
         float* part = splits > 1 ? workspace : nullptr;
         if (c_dtype == FL_BF16)
-            rc = dispatch_tc_pair<bf16>(bnt, map_w, map_a, C, ldc, M, N, K, num_sms, status, stream, splits, kb_per_split, part, ld_partial, wp, act);
+            rc = dispatch_tc_pair<bf16>(bnt, map_w, A, lda, C, ldc, M, N, K, num_sms, status, stream, splits, kb_per_split, part, ld_partial, wp, act);
         else if (c_dtype == FL_F32)
-            rc = dispatch_tc_pair<float>(bnt, map_w, map_a, C, ldc, M, N, K, num_sms, status, stream, splits, kb_per_split, part, ld_partial, wp, act);
+            rc = dispatch_tc_pair<float>(bnt, map_w, A, lda, C, ldc, M, N, K, num_sms, status, stream, splits, kb_per_split, part, ld_partial, wp, act);
         else
             return (int)cudaErrorInvalidValue;
     } else if (c_dtype == FL_BF16) {
@@ -1128,10 +1133,10 @@ FL_API int fl_gemm_tc_glu(const void* A, long lda, const void* W, long ldw, void
     int rc = make_w_map(&map_w, W, 2L * I, K, ldw, feat);           // boxes of `feat` weight rows
     if (rc) return rc;
     const int wp = ldw == 0 ? 2 * I : 0;
-    rc = make_map(&map_a, A, M, K, lda, bn > 256 ? tc_pair_tile_tokens(M, 256, (I + 127) / 128, 1, num_sms) / 2 : bn);
-    if (rc) return rc;
     if (bn == 512)
-        return launch_tc_pair<256, bf16, true>(map_w, map_a, C, ldc, M, I, K, num_sms, status, stream, I, 1, 0, nullptr, 0, nullptr, wp, act);
+        return launch_tc_pair<256, bf16, true>(map_w, A, lda, C, ldc, M, I, K, num_sms, status, stream, I, 1, 0, nullptr, 0, nullptr, wp, act);
+    rc = make_map(&map_a, A, M, K, lda, bn);
+    if (rc) return rc;
     const int kb = (K + TC_BK - 1) / TC_BK;
     switch (bn) {
         case 16: return launch_tc<16, 6, bf16, true>(map_w, map_a, C, ldc, nullptr, 0, M, I, K, 1, kb, status, stream, I, feat, wp, act);
@@ -1169,18 +1174,16 @@ FL_API int fl_gemm_tc_qkv_rope(const void* A, long lda, const void* W, long ldw,
     int bn = 0, splits = 0;
     fl_gemm_tc_plan_for(M, N, K, num_sms, 1, &bn, &splits);
     if (tc_cost(M, N, K, num_sms, bnt == 256 ? 512 : 640, 1, 1) > tc_cost(M, N, K, num_sms, bn, splits, 1) + 3.0) return -1;
-    CUtensorMap map_w, map_a;
+    CUtensorMap map_w;
     int rc = make_w_map(&map_w, W, N, K, ldw, TC_BM);
     if (rc) return rc;
     const int wp = ldw == 0 ? N : 0;
-    rc = make_map(&map_a, A, M, K, lda, tc_pair_tile_tokens(M, bnt, (N + 255) / 256, 1, num_sms) / 2);
-    if (rc) return rc;
     TcRope rope = {positions, slots, cos_table, sin_table, (bf16*)k_cache, (bf16*)v_cache, page_stride, page_size,
                    n_heads, n_kv_heads};
     switch (bnt) {
-        case 64: return launch_tc_pair<64, bf16, false, true>(map_w, map_a, C, ldc, M, N, K, num_sms, status, stream, 0, 1, 0, nullptr, 0, &rope, wp);
-        case 128: return launch_tc_pair<128, bf16, false, true>(map_w, map_a, C, ldc, M, N, K, num_sms, status, stream, 0, 1, 0, nullptr, 0, &rope, wp);
-        case 256: return launch_tc_pair<256, bf16, false, true>(map_w, map_a, C, ldc, M, N, K, num_sms, status, stream, 0, 1, 0, nullptr, 0, &rope, wp);
+        case 64: return launch_tc_pair<64, bf16, false, true>(map_w, A, lda, C, ldc, M, N, K, num_sms, status, stream, 0, 1, 0, nullptr, 0, &rope, wp);
+        case 128: return launch_tc_pair<128, bf16, false, true>(map_w, A, lda, C, ldc, M, N, K, num_sms, status, stream, 0, 1, 0, nullptr, 0, &rope, wp);
+        case 256: return launch_tc_pair<256, bf16, false, true>(map_w, A, lda, C, ldc, M, N, K, num_sms, status, stream, 0, 1, 0, nullptr, 0, &rope, wp);
     }
     return -1;
 }

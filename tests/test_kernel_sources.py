@@ -71,3 +71,13 @@ def test_epilogue_warps_give_up_together():
         voted = re.findall(r"epilogue_any\([^;]*abort_flag", text)
         assert len(voted) == {"gemm_tcgen05.cu": 3, "moe.cu": 1}.get(path.name, 0), path.name
     assert re.search(r"epilogue_any\(bool flag\).*?red\.or\.pred", (CSRC / "tcgen05.cuh").read_text(), re.S)
+
+
+def test_a_pair_tile_has_one_width():
+    """The box of the token rows, the bytes that a stage expects and the MMA's N all follow the width of a CTA pair's tiles: it
+    is worked out in one place, which also makes the map."""
+    text = (CSRC / "gemm_tcgen05.cu").read_text()
+    assert len(re.findall(r"\btc_pair_tile_tokens\(", text)) == 2                     # the function and its one call
+    launch = text[text.index("static int launch_tc_pair("):]
+    launch = launch[:launch.index("\n}\n")]
+    assert "tc_pair_tile_tokens(" in launch and "make_map(&map_a, A, M, K, lda, wt / 2)" in launch
