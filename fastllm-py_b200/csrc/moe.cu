@@ -304,14 +304,14 @@ FL_API int fl_moe_pick(const float* z, long z_ld, const void* bias, int bias_dty
 FL_API int fl_moe_experts(const void* h, int dtype, long h_ld, const void* w_gu, const void* w_down, int w_dtype,
                           const int* chosen, const float* weights, float* a, void* out, long out_ld, int n_tokens,
                           int width, int ff, int top, int act, float act_p0, float act_p1, int gated,
-                          int accumulate, int weight_on_input, cudaStream_t stream) {
+                          int accumulate, int weight_on_input, int num_sms, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if ((size_t)width * sizeof(float) > 48 * 1024 || (ff + 7) / 8 > 65535 || (width + 7) / 8 > 65535 || act < 0 || act >= FL_ACT_COUNT)
         return (int)cudaErrorInvalidValue;
     int rc = 0;
     const FlGate unit{act, act_p0, act_p1};
     const float *in_weights = weight_on_input ? weights : nullptr, *out_weights = weight_on_input ? nullptr : weights;
-    const bool few = (long)n_tokens * top * ((ff + 31) / 32) * MOE_GU_WARPS <= 148 * 16;    // 16 warps an SM with U = 8
+    const bool few = (long)n_tokens * top * ((ff + 31) / 32) * MOE_GU_WARPS <= 16L * num_sms;    // 16 warps an SM with U = 8
     const bool rows = width % 32 == 0 && ff % 32 == 0 && (((uintptr_t)w_gu | (uintptr_t)w_down | (uintptr_t)a) % 16) == 0;
     FL_DISPATCH(dtype, T, FL_DISPATCH(w_dtype, TW, {
         constexpr int PER = MOE_GU_WARPS * MoeRows<TW>::ROWS;

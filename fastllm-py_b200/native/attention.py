@@ -218,10 +218,7 @@ def prefill_attention(q, out, cache_tensor, block_table, req_start, req_ctx, req
 
 
 def num_sms(device) -> int:
-    key = ("sms", device)
-    if key not in _state:
-        _state[key] = torch.cuda.get_device_properties(device).multi_processor_count
-    return _state[key]
+    return ops.sm_count(device)
 
 
 def paged_attention(q, out, cache, step, heads, kv_heads, head_dim, window, scale, split_keys, n_splits):

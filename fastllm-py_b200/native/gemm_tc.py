@@ -61,10 +61,7 @@ def status_word(device) -> torch.Tensor:
 
 
 def _num_sms(device) -> int:
-    key = ("sms", device)
-    if key not in _state:
-        _state[key] = torch.cuda.get_device_properties(device).multi_processor_count
-    return _state[key]
+    return ops.sm_count(device)
 
 
 _plans: dict = {}

@@ -54,7 +54,7 @@ def _stream():
 _sm_counts: dict = {}
 
 
-def _sms(device) -> int:
+def sm_count(device) -> int:
     n = _sm_counts.get(device)
     if n is None:
         n = _sm_counts[device] = torch.cuda.get_device_properties(device).multi_processor_count
@@ -478,9 +478,6 @@ def retention_prep(proj, work, heads, dim, vdim, rot, cos, sin, positions, k_sca
               _ptr(cos), _ptr(sin), _ptr(positions), float(k_scale), _stream()), "retention_prep")
 
 
-_sm_counts: dict = {}
-
-
 def retention_scan(work, o, state, decay, step, heads, dim, vdim, fixed_order=False):
     """Per request and head S <- decay S + k v^T, o = S^T q over the step's tokens; q | k | v are the float32 columns
     of `work`, `o` float32 [N, heads * vdim]; state rows [heads, vdim, dim] float32 are read (unless the request
@@ -490,14 +487,11 @@ def retention_scan(work, o, state, decay, step, heads, dim, vdim, fixed_order=Fa
     if work.dtype != torch.float32 or o.dtype != torch.float32 or state.dtype != torch.float32 or \
             decay.dtype != torch.float32:
         raise KernelError("retention_scan: work, o, state and decay must be float32")
-    sms = _sm_counts.get(work.device)
-    if sms is None:
-        sms = _sm_counts[work.device] = torch.cuda.get_device_properties(work.device).multi_processor_count
     fn = _fn("retention", "fl_retention_scan", [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p,
                                                 c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                                 c_int, c_void_p])
     _check(fn(_ptr(work), _ld(work), _ptr(o), _ld(o), _ptr(state), state.stride(0), _ptr(decay), _ptr(step.req_start),
-              _ptr(step.req_ctx), _ptr(step.req_qlen), _ptr(step.req_slot), step.n_requests, heads, dim, vdim, sms,
+              _ptr(step.req_ctx), _ptr(step.req_qlen), _ptr(step.req_slot), step.n_requests, heads, dim, vdim, sm_count(work.device),
               int(fixed_order), _stream()), "retention_scan")
 
 
@@ -1271,12 +1265,12 @@ def moe_experts(h, w_gate_up, w_down, chosen, weights, act_buf, out, activation=
     if not gated:
         ff2 *= 2
     fn = _fn("moe", "fl_moe_experts", [c_void_p, c_int, c_long, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
-                                       c_void_p, c_long, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_int, c_int,
+                                       c_void_p, c_long, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_int, c_int, c_int,
                                        c_void_p])
     _check(fn(_ptr(h), dtype_code(h), _ld(h), _ptr(w_gate_up), _ptr(w_down), dtype_code(w_gate_up), _ptr(chosen),
               _ptr(weights), _ptr(act_buf), _ptr(out), _ld(out), h.shape[0], width, ff2 // 2, chosen.shape[1],
               activation_code(activation), float(params[0]), float(params[1]), int(gated), int(accumulate),
-              int(weight_on_input), _stream()), "moe_experts", 2)
+              int(weight_on_input), sm_count(h.device), _stream()), "moe_experts", 2)
 
 
 def moe_group_rows(n_tokens: int, top: int, experts: int) -> int:
@@ -1313,7 +1307,7 @@ def moe_experts_grouped(h, w_gate_up, w_down, chosen, weights, ints, act, y, out
     _check(fn(_ptr(h), _ld(h), _ptr(w_gate_up), _ptr(w_down), _ptr(chosen), _ptr(weights), _ptr(ints), _ptr(act),
               _ptr(y), _ptr(out), _ld(out), h.shape[0], width, ff2 // 2, chosen.shape[1], experts,
               activation_code(activation), float(params[0]), float(params[1]), int(gated), int(accumulate),
-              int(weight_on_input), _sms(h.device), _ptr(status_word(h.device)), _stream()), "moe_experts_grouped", 5)
+              int(weight_on_input), sm_count(h.device), _ptr(status_word(h.device)), _stream()), "moe_experts_grouped", 5)
 
 
 # -------------------------------------------------------------- rope + cache
@@ -1358,7 +1352,7 @@ def paged_attention_simt(q, out, cache, block_table, tok_req, positions, n_heads
     v_ptr = c_void_p(cache.data_ptr() + cache.stride(1) * cache.element_size())
     _check(fn(_ptr(q), dtype_code(q), _ld(q), _ptr(out), _ld(out), k_ptr, v_ptr, cache.stride(0),
               page_size, _ptr(block_table), block_table.stride(0), _ptr(tok_req), _ptr(positions),
-              q.shape[0], n_heads, n_kv_heads, head_dim, int(window or 0), float(scale), int(single), _sms(q.device),
+              q.shape[0], n_heads, n_kv_heads, head_dim, int(window or 0), float(scale), int(single), sm_count(q.device),
               _stream()), "paged_attention_simt")
 
 
@@ -1373,7 +1367,7 @@ def gemm_simt(a, w, out, constant_w=False):
     fn = _fn("gemm_simt", "fl_gemm_simt", [c_void_p, c_int, c_long, c_void_p, c_int, c_long, c_void_p,
                                            c_int, c_long, c_int, c_int, c_int, c_int, c_int, c_void_p])
     _check(fn(_ptr(a), dtype_code(a), _ld(a), _ptr(w), dtype_code(w), _ld(w), _ptr(out), dtype_code(out), _ld(out),
-              a.shape[0], w.shape[0], a.shape[1], _sms(a.device), int(constant_w), _stream()), "gemm_simt")
+              a.shape[0], w.shape[0], a.shape[1], sm_count(a.device), int(constant_w), _stream()), "gemm_simt")
 
 
 # ------------------------------------------------------------------- sampling

@@ -323,6 +323,35 @@ def test_delta_scan_of_as_many_tokens_as_requests(lens, dim, vdim):
     assert torch.equal(work, want) and torch.equal(state, want_state)
 
 
+@pytest.mark.parametrize("n, top, width, ff", [(1, 1, 32, 32), (3, 4, 96, 160), (2, 9, 416, 96), (5, 17, 64, 416), (16, 4, 288, 704)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("gated, on_input", [(True, False), (False, True)])
+def test_expert_rows_are_those_of_the_kernels_for_any_size(n, top, width, ff, dtype, gated, on_input):
+    """Matrices whose rows begin on 16 bytes go to kernels that take several rows a warp (few and many loads in flight: the
+    last two sizes have more warps than the GPU holds); copies one element further go to the others: the same bits, in both
+    formats of the weights, with more choices than a block has warps, and added to what is there."""
+    from fastllm_py_b200.native import ops
+
+    g = torch.Generator(device="cuda").manual_seed(n + top)
+    experts = 20
+    h = torch.randn(n, width, device="cuda", generator=g).to(dtype)
+    mats = [torch.randn(experts, (2 if gated else 1) * ff, width, device="cuda", generator=g).to(dtype) * width ** -0.5,
+            torch.randn(experts, width, ff, device="cuda", generator=g).to(dtype) * ff ** -0.5]
+    off = []
+    for m in mats:
+        off.append(torch.empty(m.numel() + 1, device="cuda", dtype=dtype)[1:].view(m.shape))
+        off[-1].copy_(m)
+    chosen = torch.stack([torch.randperm(experts, device="cuda", generator=g)[:top] for _ in range(n)]).to(torch.int32)
+    weights = torch.rand(n, top, device="cuda", generator=g)
+    outs = []
+    for up, down in (mats, off):
+        act, out = torch.empty(n * top, ff, device="cuda"), torch.ones(n, width, device="cuda", dtype=dtype)
+        ops.moe_experts(h, up, down, chosen, weights, act, out, "silu" if gated else "relu_squared", gated=gated, accumulate=True,
+                        weight_on_input=on_input)
+        outs.append(out)
+    assert bool(outs[0].isfinite().all()) and bool((outs[0] != 1.0).any()) and torch.equal(outs[0], outs[1])
+
+
 @pytest.mark.parametrize("width, ff, counts, top, gated, on_input", [
     (32, 32, [1], 1, True, False), (96, 160, [255, 0, 257, 1], 1, True, True), (256, 224, [64, 65, 256, 600], 2, True, False),
     (544, 416, [300, 31, 513], 3, False, True), (128, 96, [3] * 70, 2, False, False), (2048, 1408, [250, 270, 8], 1, True, False)])
