@@ -75,6 +75,8 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
     const int t_begin = (int)((gridDim.x - 1 - blockIdx.x) / CL) * QT, t_end = min(n_tokens, t_begin + QT);
     const int kvh = h / (n_heads / n_kv_heads);
     const long head_off = (long)kvh * page_size * head_dim;
+    const int pieces = vec ? head_dim / (16 / (int)sizeof(T)) : 1;          // 16-byte pieces of a row
+    const int row0 = tid / pieces, piece0 = tid - row0 * pieces;            // this thread's first one of a tile
 
     for (int t0 = t_begin, nq; t0 < t_end; t0 += nq) {  // tokens of one request at a time
         const int req = tok_req[t0];
@@ -90,10 +92,10 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
                 last = max(last, pos[i]);
             }
         }
-        for (int i = tid; i < nq * dp; i += ATT_THREADS) {
-            const int r = i / dp, d = i - r * dp;
-            q_s[i] = d < head_dim ? to_f32<T>(q[(long)(t0 + r) * q_ld + (long)h * head_dim + d]) : 0.0f;
-        }
+        for (int r = QT == 1 ? 0 : warp; r < nq; r += ATT_THREADS / 32)
+#pragma unroll 4
+            for (int d = QT == 1 ? tid : lane; d < dp; d += QT == 1 ? ATT_THREADS : 32)
+                q_s[r * dp + d] = d < head_dim ? to_f32<T>(q[(long)(t0 + r) * q_ld + (long)h * head_dim + d]) : 0.0f;
         float acc[QT][NV] = {}, m[QT], l[QT];
         bool begun[QT];
 #pragma unroll
@@ -108,36 +110,68 @@ __global__ void __launch_bounds__(ATT_THREADS) paged_attention_simt_kernel(
             const int base = tile * ATT_TILE, keys = min(ATT_TILE, last + 1 - base);
             // keys and values of the tile, rows outside first .. last left as zeros: what lies past the last visible key may
             // hold anything, and the table has -1 for pages that every window in the step has passed
-            if (sizeof(T) == 4 && vec) {
-                // a thread copies one 16-byte column of every `step`-th row
-                const int per = head_dim / 4, step = ATT_THREADS / per, c = (tid % per) * 4;
-                const float *kc = reinterpret_cast<const float*>(k_cache) + head_off + c, *vc = reinterpret_cast<const float*>(v_cache) + head_off + c;
-#pragma unroll 4
-                for (int r = tid / per; r < ATT_TILE; r += step) {
-                    const int j = base + r;
-                    if (j >= first && r < keys) {
-                        const int page = page_shift >= 0 ? j >> page_shift : j / page_size;
-                        const long off = (long)bt[page] * page_stride + (long)(j - page * page_size) * head_dim;
-                        att_cp16(k_s + r * kp + c, kc + off);
-                        att_cp16(v_s + r * dp + c, vc + off);
-                    } else {
-                        *reinterpret_cast<float4*>(k_s + r * kp + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        *reinterpret_cast<float4*>(v_s + r * dp + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            auto in_sight = [&](int r, long& off) {
+                const int j = base + r;
+                if (j >= first && r < keys) {
+                    const int page = page_shift >= 0 ? j >> page_shift : j / page_size;
+                    off = (long)bt[page] * page_stride + head_off + (long)(j - page * page_size) * head_dim;
+                    return true;
+                }
+                return false;
+            };
+            if (vec) {
+                // 16 bytes a thread and step; the next step's piece lies ATT_THREADS pieces on: `rows` rows and `rest` pieces
+                constexpr int V = 16 / (int)sizeof(T), BATCH = sizeof(T) == 4 ? 1 : 4;
+                const int rows = ATT_THREADS / pieces, rest = ATT_THREADS - rows * pieces;
+                int r = row0, c = piece0;
+#pragma unroll(sizeof(T) == 4 ? 4 : 1)
+                while (r < ATT_TILE) {
+                    uint4 kr[BATCH], vr[BATCH];
+                    int at_k[BATCH], at_v[BATCH];
+#pragma unroll
+                    for (int b = 0; b < BATCH; ++b) {
+                        long off;
+                        at_k[b] = r < ATT_TILE ? r * kp + c * V : -1;
+                        at_v[b] = r * dp + c * V;
+                        kr[b] = vr[b] = make_uint4(0u, 0u, 0u, 0u);
+                        if (r < ATT_TILE && in_sight(r, off)) {
+                            if constexpr (sizeof(T) == 4) {
+                                att_cp16(k_s + at_k[b], reinterpret_cast<const float*>(k_cache) + off + c * V);
+                                att_cp16(v_s + at_v[b], reinterpret_cast<const float*>(v_cache) + off + c * V);
+                                at_k[b] = -1;
+                            } else {
+                                kr[b] = *reinterpret_cast<const uint4*>(k_cache + off + c * V);
+                                vr[b] = *reinterpret_cast<const uint4*>(v_cache + off + c * V);
+                            }
+                        }
+                        r += rows;
+                        c += rest;
+                        if (c >= pieces) c -= pieces, ++r;
+                    }
+#pragma unroll
+                    for (int b = 0; b < BATCH; ++b) {
+                        if (at_k[b] < 0) continue;
+                        const T *ke = reinterpret_cast<const T*>(&kr[b]), *ve = reinterpret_cast<const T*>(&vr[b]);
+#pragma unroll
+                        for (int e = 0; e < V; e += 4) {
+                            *reinterpret_cast<float4*>(k_s + at_k[b] + e) =
+                                make_float4(to_f32<T>(ke[e]), to_f32<T>(ke[e + 1]), to_f32<T>(ke[e + 2]), to_f32<T>(ke[e + 3]));
+                            *reinterpret_cast<float4*>(v_s + at_v[b] + e) =
+                                make_float4(to_f32<T>(ve[e]), to_f32<T>(ve[e + 1]), to_f32<T>(ve[e + 2]), to_f32<T>(ve[e + 3]));
+                        }
                     }
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
                 asm volatile("cp.async.wait_group 0;" ::: "memory");
             } else {
-                for (int i = tid; i < ATT_TILE * dp; i += ATT_THREADS) {
-                    const int r = i / dp, c = i - r * dp, j = base + r;
-                    float kv = 0.0f, vv = 0.0f;
-                    if (j >= first && r < keys && c < head_dim) {
-                        const long off = (long)bt[j / page_size] * page_stride + head_off + (long)(j % page_size) * head_dim + c;
-                        kv = to_f32<T>(k_cache[off]);
-                        vv = to_f32<T>(v_cache[off]);
+#pragma unroll 4
+                for (int r = warp; r < ATT_TILE; r += ATT_THREADS / 32) {
+                    long off = 0;
+                    const bool in = in_sight(r, off);
+                    for (int c = lane; c < dp; c += 32) {
+                        k_s[r * kp + c] = in && c < head_dim ? to_f32<T>(k_cache[off + c]) : 0.0f;
+                        v_s[r * dp + c] = in && c < head_dim ? to_f32<T>(v_cache[off + c]) : 0.0f;
                     }
-                    k_s[r * kp + c] = kv;
-                    v_s[i] = vv;
                 }
             }
             __syncthreads();
@@ -302,7 +336,8 @@ static int att_launch(const T* q, long q_ld, T* out, long out_ld, const T* k_cac
     const size_t smem = 4 * (size_t)att_floats(QT, AttHold<QT>::TILES, att_pad(head_dim));
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return (int)err;
-    const int vec = head_dim % 4 == 0 && ATT_THREADS % (head_dim / 4) == 0 && page_stride % 4 == 0 && (((uintptr_t)k_cache | (uintptr_t)v_cache) % 16) == 0;
+    constexpr int V = 16 / (int)sizeof(T);
+    const int vec = head_dim % V == 0 && page_stride % V == 0 && (((uintptr_t)k_cache | (uintptr_t)v_cache) % 16) == 0;
     int page_shift = -1;
     if ((page_size & (page_size - 1)) == 0)
         for (page_shift = 0; (1 << page_shift) < page_size;) ++page_shift;
@@ -324,23 +359,55 @@ static int att_launch(const T* q, long q_ld, T* out, long out_ld, const T* k_cac
                                    bt_stride, tok_req, positions, n_tokens, n_heads, n_kv_heads, head_dim, window, scale, vec, page_shift);
 }
 
+// What a launch of groups of `qt` tokens on clusters of `cl` CTAs takes, in microseconds, fitted (on the logarithm, 24 %
+// root-mean-square error) to runs of both group sizes over heads of 16 to 256, prompts of 8 to 1024 tokens and portions
+// behind up to 2000: rounds of as many CTAs as the SMs hold, in each of which a CTA begins and goes through its share of the
+// tiles, one tile taking as long as a CTA alone takes for it or as the SM takes for those of all its CTAs.
+static double att_cost(long units, int tiles, int qt, int cl, int head_dim, int sms) {
+    const size_t smem = 4 * (size_t)att_floats(qt, qt == 1 ? AttHold<1>::TILES : AttHold<8>::TILES, att_pad(head_dim)) + 1024;
+    int places = (int)(228 * 1024 / smem);
+    if (places > (qt == 1 ? 4 : 3)) places = qt == 1 ? 4 : 3;
+    const double wide = head_dim / 128.0, waves = (double)units * cl / ((double)places * sms);
+    const double beside = waves >= 1.0 ? places : ceil(waves * places);
+    const double alone = qt == 1 ? 2.7 + 2.3 * wide : 6.8 + 3.1 * wide, shared = (qt == 1 ? 2.0 * wide : 1.0 + 3.0 * wide) * beside;
+    const double share = (tiles + cl - 1) / cl;                          // (of the last tokens: earlier ones see fewer tiles)
+    return (waves <= 2.0 ? ceil(waves) : waves + 0.5) *
+           ((qt == 1 ? 0.0 : 5.4) + (waves <= 1.0 ? share : 0.5 * share + 0.5) * (alone > shared ? alone : shared));
+}
+
 // q: [n_tokens, q_ld] with head h at columns [h*head_dim, (h+1)*head_dim);
 // out likewise.  tok_req[t] is the row of `block_table` that token t's request
 // uses; positions[t] is the token's absolute position, whose key (already in
-// the cache) is the last one it sees.  window <= 0 means all keys.  `single`: neighbouring tokens belong to
-// different requests (a hint, results do not depend on it).
+// the cache) is the last one it sees.  window <= 0 means all keys.  Two hints, on which results do not depend: `single`:
+// neighbouring tokens belong to different requests; `longest`: the most keys that a token of the step has (0: not known).
 FL_API int fl_paged_attention_simt(const void* q, int dtype, long q_ld, void* out, long out_ld,
                                    const void* k_cache, const void* v_cache, long page_stride,
                                    int page_size, const int* block_table, int bt_stride,
                                    const int* tok_req, const int* positions, int n_tokens,
-                                   int n_heads, int n_kv_heads, int head_dim, int window, float scale, int single, int sms,
-                                   cudaStream_t stream) {
+                                   int n_heads, int n_kv_heads, int head_dim, int window, float scale, int single, int longest,
+                                   int sms, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (head_dim < 1 || head_dim > 2 * ATT_THREADS || n_heads > 65535 || n_heads % n_kv_heads)
         return (int)cudaErrorInvalidValue;
     // As many CTAs a cluster as keep the launch within two CTAs an SM or so: more only wait for one another.
     const long units = (long)((n_tokens + (single ? 0 : 7)) / (single ? 1 : 8)) * n_heads;
-    const int cl = units * 4 <= 2L * sms ? 8 : units <= sms ? 4 : units <= 2L * sms ? 2 : 1;
+    int cl = units * 4 <= 2L * sms ? 8 : units <= sms ? 4 : units <= 2L * sms ? 2 : 1;
+    if (longest > 0 && !single) {
+        // Where the number of keys is known: groups of eight tokens, or one token a CTA if some cluster makes that cheaper.
+        // (Few tokens over few keys wait for one tile, which eight tokens take twice as long for: a prompt of 8 tokens, 16
+        // heads of 128, took 12.9 us in groups of eight and takes 5.)  Picks are 3.5 % off the better one on average.
+        auto tiles = [&](int qt) {
+            int keys = longest;
+            if (window > 0 && keys > window + qt + ATT_TILE - 2) keys = window + qt + ATT_TILE - 2;
+            return (keys + ATT_TILE - 1) / ATT_TILE;
+        };
+        const bool two = head_dim > ATT_THREADS;                          // (kernels for clusters of 4 and 1 only)
+        double best = att_cost(units, tiles(8), 8, two ? (cl >= 4 ? 4 : 1) : cl, head_dim, sms);
+        for (int c = 1; c <= (two ? 4 : 8); c *= two ? 4 : 2) {
+            const double t = att_cost((long)n_tokens * n_heads, tiles(1), 1, c, head_dim, sms);
+            if (t < best) best = t, single = 1, cl = c;
+        }
+    }
 #define ATT_GO(QT, CL, NV)                                                                                                \
     FL_DISPATCH(dtype, T, return (att_launch<T, QT, CL, NV>((const T*)q, q_ld, (T*)out, out_ld, (const T*)k_cache,        \
                                                             (const T*)v_cache, page_stride, page_size, block_table,      \

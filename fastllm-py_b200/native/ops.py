@@ -1339,21 +1339,22 @@ def rope_kv_write(qkv, n_heads, n_kv_heads, head_dim, rot_dim, cos, sin, positio
 # ------------------------------------------------------------------ attention
 
 def paged_attention_simt(q, out, cache, block_table, tok_req, positions, n_heads, n_kv_heads,
-                         head_dim, window, scale, page_size, single=False):
+                         head_dim, window, scale, page_size, single=False, longest=0):
     """Causal attention of every token in q over its request's cached keys (CUDA cores).  `single`: every token is of
-    another request, so neighbours share no keys (how the work is dealt out; the results are the same)."""
+    another request, so neighbours share no keys; `longest`: the most keys that a token has, where that is known (how the
+    work is dealt out; the results are the same)."""
     _require_cuda(q, out, cache, block_table, tok_req, positions)
     if head_dim > 256:
         raise KernelError(f"attention: head_dim {head_dim} is beyond the kernel's limit of 256")
     fn = _fn("attention_simt", "fl_paged_attention_simt",
              [c_void_p, c_int, c_long, c_void_p, c_long, c_void_p, c_void_p, c_long, c_int, c_void_p,
-              c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p])
+              c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int, c_void_p])
     k_ptr = c_void_p(cache.data_ptr())
     v_ptr = c_void_p(cache.data_ptr() + cache.stride(1) * cache.element_size())
     _check(fn(_ptr(q), dtype_code(q), _ld(q), _ptr(out), _ld(out), k_ptr, v_ptr, cache.stride(0),
               page_size, _ptr(block_table), block_table.stride(0), _ptr(tok_req), _ptr(positions),
-              q.shape[0], n_heads, n_kv_heads, head_dim, int(window or 0), float(scale), int(single), sm_count(q.device),
-              _stream()), "paged_attention_simt")
+              q.shape[0], n_heads, n_kv_heads, head_dim, int(window or 0), float(scale), int(single), int(longest),
+              sm_count(q.device), _stream()), "paged_attention_simt")
 
 
 # ----------------------------------------------------------------------- GEMM

@@ -157,4 +157,6 @@ class Attention(Part):
         else:
             ops.paged_attention_simt(q, ctx, cache.tensor, cache.block_table, step.tok_req,
                                      step.positions, self.heads, self.kv_heads, self.head_dim,
-                                     self.window, self.scale, cache.page_size, single=step.max_q_len == 1)
+                                     self.window, self.scale, cache.page_size, single=step.max_q_len == 1,
+                                     # (a decode step may be captured and serve longer requests later)
+                                     longest=0 if step.max_q_len == 1 else step.max_seq_len)

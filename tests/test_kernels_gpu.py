@@ -457,6 +457,24 @@ def test_cuda_core_attention_order(head_dim, window, dtype):
             assert torch.equal(run(a, a + n, single), base[a:a + n]), (a, n, single)
 
 
+@pytest.mark.parametrize("heads, kv_heads, head_dim", [(2, 1, 128), (6, 2, 96), (8, 8, 48), (4, 2, 80), (3, 3, 20), (2, 2, 7), (4, 1, 256)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_cuda_core_attention_hints_and_copies(heads, kv_heads, head_dim, dtype):
+    """Heads that a tile's copy takes in 16-byte pieces, whole threads' shares of a row or not, and one value at a time; and
+    how many keys the caller says there are changes who does the work, not a bit of the result."""
+    from fastllm_py_b200.native import ops
+
+    for q_lens, ctx in (([3], [0]), ([9, 1, 30], [0, 90, 200]), ([70], [700])):
+        case = AttentionCase(q_lens, ctx, heads, kv_heads, head_dim, 16, dtype, seed=7)
+        outs = []
+        for longest in (0, 1, max(a + b for a, b in zip(q_lens, ctx)), 100000):
+            outs.append(torch.zeros_like(case.q))
+            ops.paged_attention_simt(case.q, outs[-1], case.cache, case.block_table, case.tok_req, case.positions, heads, kv_heads,
+                                     head_dim, None, head_dim ** -0.5, 16, longest=longest)
+            assert torch.equal(outs[-1], outs[0]), (q_lens, longest)
+        assert float((outs[0].float().cpu() - case.reference()).abs().max()) <= case.tolerance()
+
+
 @pytest.mark.parametrize("head_dim, page_size, dtype", [(128, 16, torch.float32), (48, 8, torch.float32), (64, 16, torch.bfloat16)])
 @pytest.mark.parametrize("q_lens", [[1], [1, 1, 1], [9, 8, 40]])
 def test_cuda_core_attention_behind_pages_given_back(q_lens, head_dim, page_size, dtype):
