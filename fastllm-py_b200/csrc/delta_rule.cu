@@ -509,8 +509,9 @@ FL_API int fl_delta_prep(const void* proj, int dtype, long ld, const void* conv_
     if (taps < 1 || heads % kv_heads || n_requests > 65535 || units > 65535 || (size_t)widest * sizeof(float) > 48 * 1024)
         return (int)cudaErrorInvalidValue;
     int rc = 0;
-    // (from 256 tokens on: 32 units are then 512 warps, about one for every scheduler)
-    if (dim == 128 && vdim == 128 && taps <= 4 && n_tokens >= 256)
+    // A warp takes some 37 us for its 16 tokens however few warps there are; a block a (token, unit) takes 3 us and 1.4 ns for
+    // each: with 32 units 16 us for 256 tokens, 27 for 512, 50 for 1024 and 96 for 2048 (the warps 37, 38, 38 and 42).
+    if (dim == 128 && vdim == 128 && taps <= 4 && (long)n_tokens * units >= 24000)
         FL_DISPATCH(dtype, T, FL_DISPATCH(w_dtype, TW,
             rc = fl_launch(delta_prep_rows_kernel<T, TW>, dim3((n_tokens + PREP_TOKENS - 1) / PREP_TOKENS, (units + 3) / 4), dim3(128), 0,
                            stream, (const T*)proj, ld, (const TW*)conv_w, (const TW*)a_log, (const TW*)dt_bias, (const float*)state,

@@ -265,15 +265,15 @@ def test_command_line_on_a_random_weights_folder(tmp_path):
 @pytest.mark.parametrize("taps", [1, 2, 4])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_delta_preparation_of_prompts_is_that_of_few_tokens(taps, dtype):
-    """From 256 tokens on, with heads of 128, a kernel of its own prepares them: the same bits as in slices of fewer tokens,
-    over requests that meet inside its groups of 16, at their start, behind a saved tail and shorter than the taps."""
+    """From 24000 (token, unit) pairs on, with heads of 128, a kernel of its own prepares them: the same bits as in slices of
+    fewer tokens, over requests that meet inside its groups of 16, at their start, behind a saved tail and shorter than the taps."""
     from types import SimpleNamespace
 
     from fastllm_py_b200.native import ops
 
     torch.manual_seed(taps)
     heads, kv_heads, dim = 6, 3, 128
-    lens = [(0, 133), (7, 1), (0, 2), (1, 5), (90, 178)]                       # (tokens before the step, tokens in it)
+    lens = [(0, 133), (7, 1), (0, 2), (1, 5), (90, 178), (3, 1801)]            # (tokens before the step, tokens in it)
     n, qk, hv = sum(m for _, m in lens), kv_heads * dim, heads * dim
     channels, tail_off = 2 * qk + hv, hv * dim
     proj = torch.randn(n, channels + hv + 2 * heads, device="cuda").to(dtype)
@@ -292,7 +292,7 @@ def test_delta_preparation_of_prompts_is_that_of_few_tokens(taps, dtype):
             ops.delta_prep(proj[a:b], conv, a_log, dt_bias, state.clone(), tail_off, step, work[a:b], heads, kv_heads, dim, dim, taps, 1e-6,
                            dim ** -0.5)
         works.append(work)
-    assert n >= 256 and bool(torch.isfinite(works[0]).all()) and float(works[0].abs().sum()) > 0
+    assert n * (heads + 2 * kv_heads) >= 24000 and bool(torch.isfinite(works[0]).all()) and float(works[0].abs().sum()) > 0
     assert torch.equal(works[0], works[1])
 
 
