@@ -180,6 +180,8 @@ __global__ void delta_tail_kernel(const T* __restrict__ proj, long ld, float* __
 // What bounds a long prompt: the chain from one token's u to the next one's.  2048 tokens, 16 heads of 128 x 128: 326 us,
 // 160 ns a token; 679 us with the fetches and q . k on the same threads (156 instructions a token and warp, a fifth of the
 // time at the barrier behind the two warps that fetched) and one multiply-add an element.
+// Registers are kept to what lets two blocks of 32 columns share an SM: several requests' prompts bring more blocks than SMs
+// (8 x 100 tokens, 16 heads of 128 x 128: 121 us with one block an SM, 96 with two).
 #define DELTA_CHUNK 16
 
 __device__ __forceinline__ void delta_cp16(float* smem, const float* gmem) {
@@ -209,7 +211,7 @@ __device__ __forceinline__ float2 delta_mul2(const float2 a, const float2 b) {
 }
 
 template <int DPT, int COLS>
-__global__ void __launch_bounds__(COLS * DELTA_PARTS + 32) delta_scan_kernel(
+__global__ void __launch_bounds__(COLS * DELTA_PARTS + 32, COLS == 32 && DPT <= 16 ? 2 : 1) delta_scan_kernel(
     float* __restrict__ work, long work_ld, float* __restrict__ state, long state_stride,
     const int* __restrict__ req_start, const int* __restrict__ req_ctx, const int* __restrict__ req_qlen,
     const int* __restrict__ req_slot, int heads, int kv_heads, int dim, int vdim) {
@@ -237,8 +239,11 @@ __global__ void __launch_bounds__(COLS * DELTA_PARTS + 32) delta_scan_kernel(
         for (int idx = threadIdx.x; idx < used; idx += blockDim.x) delta_in[idx] = 0.0f;
         __syncthreads();
     }
-    // rows whose pieces are all 16-byte aligned are copied four floats at a time
-    const bool wide = dim % 4 == 0 && vdim % 4 == 0 && v0 + COLS <= vdim && work_ld % 4 == 0;
+    // k and q, and the block's v, are copied four floats at a time where their pieces are all 16-byte aligned, else one at a
+    // time; either way a lane keeps its place in the row and walks the tokens (a place worked out per element left the
+    // recurrence waiting for this warp: 2048 tokens of a head in rows of 514 floats took 2264 us and take 384)
+    const bool wide = dim % 4 == 0 && vdim % 4 == 0 && work_ld % 4 == 0 && ((uintptr_t)work & 15) == 0;
+    const bool wide_v = wide && v0 + COLS <= vdim;
     auto fetch = [&](int buf, int first) {                   // tokens first .. first + DELTA_CHUNK - 1 of the portion
         float* dst = delta_in + (long)buf * DELTA_CHUNK * PER_TOKEN;
         const int n_tok = min(DELTA_CHUNK, qlen - first);
@@ -246,42 +251,34 @@ __global__ void __launch_bounds__(COLS * DELTA_PARTS + 32) delta_scan_kernel(
         const int lane = threadIdx.x & 31;
         if (wide) {
             for (int d = lane * 4; d < dim; d += 128) {                           // k and q, four elements a lane
-                const int at = (d / DPT) * PART + d % DPT;
                 const float* src = row + g * dim + d;
-                float* to = dst + at;
+                float* to = dst + (d / DPT) * PART + d % DPT;
                 for (int n = 0; n < n_tok; ++n, src += work_ld, to += PER_TOKEN) {
                     delta_cp16(to, src + qk_cols);
                     delta_cp16(to + KQ, src);
                 }
             }
-            if (lane < COLS / 4 + 2) {                                            // v, beta, decay
-                const bool is_v = lane < COLS / 4;
-                const int e = lane - COLS / 4;
-                const float* src = row + 2 * qk_cols + (is_v ? h * vdim + v0 + lane * 4 : hv + e * heads + h);
-                float* to = dst + 2 * KQ + (is_v ? lane * 4 : COLS + e);
+        } else {
+            for (int d = lane; d < dim; d += 32) {
+                const float* src = row + g * dim + d;
+                float* to = dst + (d / DPT) * PART + d % DPT;
+#pragma unroll 2
                 for (int n = 0; n < n_tok; ++n, src += work_ld, to += PER_TOKEN) {
-                    if (is_v) delta_cp16(to, src);
-                    else delta_cp4(to, src);
+                    delta_cp4(to, src + qk_cols);
+                    delta_cp4(to + KQ, src);
                 }
             }
-        } else {
-            const int wanted = 2 * dim + COLS + 2;
-            for (int idx = lane; idx < n_tok * wanted; idx += 32) {
-                const int n = idx / wanted, e = idx % wanted;
-                const float* from = row + (long)n * work_ld;
-                int at;
-                if (e < 2 * dim) {                                                // k, then q
-                    const int d = e < dim ? e : e - dim;
-                    from += (e < dim ? qk_cols : 0) + g * dim + d;
-                    at = (e < dim ? 0 : KQ) + (d / DPT) * PART + d % DPT;
-                } else if (e < 2 * dim + COLS) {
-                    from += 2 * qk_cols + h * vdim + min(v0 + e - 2 * dim, vdim - 1);
-                    at = 2 * KQ + (e - 2 * dim);
-                } else {                                                          // beta, decay
-                    from += 2 * qk_cols + hv + (e - 2 * dim - COLS) * heads + h;
-                    at = 2 * KQ + COLS + (e - 2 * dim - COLS);
-                }
-                delta_cp4(dst + (long)n * PER_TOKEN + at, from);
+        }
+        const int v_lanes = wide_v ? COLS / 4 : COLS;        // lanes with a piece of v each, then beta, decay
+        for (int p = lane; p < v_lanes + 2; p += 32) {
+            const bool is_v = p < v_lanes;
+            const int e = p - v_lanes, c = wide_v ? p * 4 : p;
+            const float* src = row + 2 * qk_cols + (is_v ? h * vdim + min(v0 + c, vdim - 1) : hv + e * heads + h);
+            float* to = dst + 2 * KQ + (is_v ? c : COLS + e);
+#pragma unroll 2
+            for (int n = 0; n < n_tok; ++n, src += work_ld, to += PER_TOKEN) {
+                if (is_v && wide_v) delta_cp16(to, src);
+                else delta_cp4(to, src);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
