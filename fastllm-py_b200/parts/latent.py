@@ -168,9 +168,15 @@ class LatentAttention(Part):
 
     def _prompts(self, step, n_tokens: int, page_size: int) -> bool:
         """Whether a step without splits goes to the prompt kernel: it takes eight neighbouring tokens of a request at a
-        time at the price of 3.4 single tokens in the other kernel (2048 tokens: 416 us against 971), so it is the faster
-        one until half of its rows stay empty.  The results are the same."""
+        time at the price of 3.4 single tokens in the other kernel where both fill the GPU (2048 tokens: 416 us against
+        971), so it is the faster one until half of its rows stay empty.  A tile of keys alone takes it as long as the other
+        (4.6 us with a latent of 512), or longer (3.6 against 2.9 with 256, which leaves the other room for more blocks an
+        SM): with few blocks the other kernel is as fast (128 tokens of 16 heads behind 1000: 153 us both) or faster (256:
+        128 us against 103; level at 384 tokens).  The results are the same."""
         if not step.q_lens or not ops.latent_prompt_takes(self.ctx.dtype, self.rank, self.rot, self.heads, page_size):
+            return False
+        blocks = n_tokens * -(-self.heads // 16)                          # the other kernel's
+        if 2 * blocks <= (2 if self.rank > 256 else 5) * ops.sm_count(self.ctx.device):
             return False
         return 4 * sum(-(-q // 8) for q in step.q_lens) <= n_tokens       # four of eight rows at least
 
