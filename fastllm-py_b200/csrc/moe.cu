@@ -312,10 +312,16 @@ FL_API int fl_moe_experts(const void* h, int dtype, long h_ld, const void* w_gu,
     const FlGate unit{act, act_p0, act_p1};
     const float *in_weights = weight_on_input ? weights : nullptr, *out_weights = weight_on_input ? nullptr : weights;
     const bool few = (long)n_tokens * top * ((ff + 31) / 32) * MOE_GU_WARPS <= 16L * num_sms;    // 16 warps an SM with U = 8
-    const bool rows = width % 32 == 0 && ff % 32 == 0 && (((uintptr_t)w_gu | (uintptr_t)w_down | (uintptr_t)a) % 16) == 0;
+    // Several rows a warp pay once that still leaves warps enough: for the first product eight of them an SM (1 token x 4
+    // choices, 1408 features: 704 warps, 3 us slower than a row a warp; 8 pairs, 1408 warps, 5 us faster); for the second,
+    // whose warps take a choice each, with two choices or more, or with 8192 rows' worth of bfloat16 outputs (1 choice of 2048
+    // outputs: 1 token 14.6 us a row a warp and 22.7 eight rows a warp, 8 tokens 49 and 36).
+    const bool aligned = width % 32 == 0 && ff % 32 == 0 && (((uintptr_t)w_gu | (uintptr_t)w_down | (uintptr_t)a) % 16) == 0;
+    const bool rows_up = aligned && (long)n_tokens * top * ((ff + 31) / 32) * MOE_GU_WARPS > 8L * num_sms;
+    const bool rows_down = aligned && (top > 1 || (long)n_tokens * width * 2 >= 8192L * (w_dtype == FL_F32 ? 4 : 2));
     FL_DISPATCH(dtype, T, FL_DISPATCH(w_dtype, TW, {
         constexpr int PER = MOE_GU_WARPS * MoeRows<TW>::ROWS;
-        if (rows)
+        if (rows_up)
             rc = fl_launch(few ? moe_gate_up_rows_kernel<T, TW, 8> : moe_gate_up_rows_kernel<T, TW, 4>, dim3(n_tokens * top, (ff + PER - 1) / PER), dim3(MOE_GU_WARPS * 32),
                            (size_t)width * sizeof(float), stream, (const T*)h, h_ld, (const TW*)w_gu, chosen, a, width, ff, top,
                            unit, gated, in_weights);
@@ -326,7 +332,7 @@ FL_API int fl_moe_experts(const void* h, int dtype, long h_ld, const void* w_gu,
     if (rc) return rc;
     FL_DISPATCH(dtype, T, FL_DISPATCH(w_dtype, TW, {
         constexpr int PER = MoeRows<TW>::ROWS;
-        if (rows)
+        if (rows_down)
             return fl_launch(few ? moe_down_rows_kernel<T, TW, 11> : moe_down_rows_kernel<T, TW, 8>, dim3(n_tokens, (width + PER - 1) / PER),
                              dim3(32 * (top < MOE_DOWN_WARPS ? top : MOE_DOWN_WARPS)), 0, stream, (const float*)a,
                              (const TW*)w_down, chosen, out_weights, (T*)out, out_ld, width, ff, top, accumulate);

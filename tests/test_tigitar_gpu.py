@@ -323,13 +323,15 @@ def test_delta_scan_of_as_many_tokens_as_requests(lens, dim, vdim):
     assert torch.equal(work, want) and torch.equal(state, want_state)
 
 
-@pytest.mark.parametrize("n, top, width, ff", [(1, 1, 32, 32), (3, 4, 96, 160), (2, 9, 416, 96), (5, 17, 64, 416), (16, 4, 288, 704)])
+@pytest.mark.parametrize("n, top, width, ff", [(1, 1, 32, 32), (3, 4, 96, 160), (2, 9, 416, 96), (8, 4, 160, 320), (64, 1, 288, 64),
+                                                (5, 17, 64, 416), (16, 4, 288, 704)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("gated, on_input", [(True, False), (False, True)])
 def test_expert_rows_are_those_of_the_kernels_for_any_size(n, top, width, ff, dtype, gated, on_input):
-    """Matrices whose rows begin on 16 bytes go to kernels that take several rows a warp (few and many loads in flight: the
-    last two sizes have more warps than the GPU holds); copies one element further go to the others: the same bits, in both
-    formats of the weights, with more choices than a block has warps, and added to what is there."""
+    """Matrices whose rows begin on 16 bytes go to kernels that take several rows a warp where that leaves warps enough (the
+    second product from the second size on, the first from the fourth on but the fifth; with fewer loads in flight in the last
+    two); copies one element further go to the others: the same bits, in both formats of the weights, with more choices than a
+    block has warps, and added to what is there."""
     from fastllm_py_b200.native import ops
 
     g = torch.Generator(device="cuda").manual_seed(n + top)
