@@ -1116,8 +1116,10 @@ FL_API int fl_gemm_tc_glu(const void* A, long lda, const void* W, long ldw, void
         while (feat < 64 && (I + feat - 1) / feat > 2 * num_sms) feat += 8;
         // An MMA takes the time to read 128 rows of weights from shared memory, however few of them are features, so an SM
         // with two CTAs is twice as long at its K steps.  Where CTAs of at most 64 features fill nearly all SMs one by one,
-        // that is faster (5504 features, K = 2048, 1 token: 230 CTAs of 24 took 13.0 us, 138 of 40 take 11.5).
-        for (int one = 16; one <= 64; one += 8) {
+        // that is faster: K = 2048, 1 token, 5504 features 12.2 us (138 CTAs of 40) instead of 13.3 (230 of 24), 9472 13.4
+        // instead of 14.5; 128 tokens, 9472 features 20.1 instead of 21.5.  With 33 to 64 tokens it is not (48 tokens, 8192
+        // features: 14.5 us, two CTAs an SM 13.8; 9472: 15.4 and 14.9; 5504: 13.7 and 14.0).
+        for (int one = 16; one <= 64 && bn != 64; one += 8) {
             const int ctas = (I + one - 1) / one;
             if (ctas > num_sms) continue;
             if (ctas * 8 >= num_sms * 7 && one > feat) feat = one;
