@@ -164,8 +164,8 @@ template <int V> __device__ __forceinline__ float moe_rows_sum(float (&acc)[V]) 
 // w_gu: [experts][2 ff][width] (gate rows, then up rows), or [experts][ff][width] without a gate;
 // a: [tokens x top][ff] float
 // U: blocks of 32 elements on their way at once, of each row.  With more warps than the SMs hold at a time, fewer of them
-// and more warps resident are faster (8 tokens x 4, both products out of a cold cache: 106 us with 4 and 8, 127 with 8 and
-// 11); with fewer warps than that, more (one token: 42 us with 8 and 11, 48 with 4 and 8).
+// and more warps resident are faster (8 tokens x 4, both products out of a cold cache: 101 us with 4 and 8, 114 with 8 and
+// 11); with fewer warps than that, more (one token: 24.4 us with 8 and 11, 30.7 with 4 and 8).
 #define MOE_GU_WARPS 4
 template <typename T, typename TW, int U>
 __global__ void __launch_bounds__(MOE_GU_WARPS * 32) moe_gate_up_rows_kernel(
@@ -312,13 +312,13 @@ FL_API int fl_moe_experts(const void* h, int dtype, long h_ld, const void* w_gu,
     const FlGate unit{act, act_p0, act_p1};
     const float *in_weights = weight_on_input ? weights : nullptr, *out_weights = weight_on_input ? nullptr : weights;
     const bool few = (long)n_tokens * top * ((ff + 31) / 32) * MOE_GU_WARPS <= 16L * num_sms;    // 16 warps an SM with U = 8
-    // Several rows a warp pay once that still leaves warps enough: for the first product eight of them an SM (1 token x 4
-    // choices, 1408 features: 704 warps, 3 us slower than a row a warp; 8 pairs, 1408 warps, 5 us faster); for the second,
-    // whose warps take a choice each, with two choices or more, or with 8192 rows' worth of bfloat16 outputs (1 choice of 2048
-    // outputs: 1 token 14.6 us a row a warp and 22.7 eight rows a warp, 8 tokens 49 and 36).
+    // Several rows a warp pay once that leaves warps enough.  For the second product, whose warps take a choice each: two
+    // choices or more, or 8192 rows' worth of bfloat16 outputs (both products, 1 choice of 32 experts of 2048 x 1408: 1 token
+    // 14.6 us a row a warp and 22.7 eight rows a warp, 8 tokens 49 and 36).  For the first: beside such a second one, with a
+    // warp an SM (1 token x 4: 24.6 us, 30.6 with a row a warp in the first product, 36.8 in both).
     const bool aligned = width % 32 == 0 && ff % 32 == 0 && (((uintptr_t)w_gu | (uintptr_t)w_down | (uintptr_t)a) % 16) == 0;
-    const bool rows_up = aligned && (long)n_tokens * top * ((ff + 31) / 32) * MOE_GU_WARPS > 8L * num_sms;
     const bool rows_down = aligned && (top > 1 || (long)n_tokens * width * 2 >= 8192L * (w_dtype == FL_F32 ? 4 : 2));
+    const bool rows_up = rows_down && (long)n_tokens * top * ((ff + 31) / 32) * MOE_GU_WARPS >= num_sms;
     FL_DISPATCH(dtype, T, FL_DISPATCH(w_dtype, TW, {
         constexpr int PER = MOE_GU_WARPS * MoeRows<TW>::ROWS;
         if (rows_up)

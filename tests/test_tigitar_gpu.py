@@ -328,9 +328,8 @@ def test_delta_scan_of_as_many_tokens_as_requests(lens, dim, vdim):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("gated, on_input", [(True, False), (False, True)])
 def test_expert_rows_are_those_of_the_kernels_for_any_size(n, top, width, ff, dtype, gated, on_input):
-    """Matrices whose rows begin on 16 bytes go to kernels that take several rows a warp where that leaves warps enough (the
-    second product from the second size on, the first from the fourth on but the fifth; with fewer loads in flight in the last
-    two); copies one element further go to the others: the same bits, in both formats of the weights, with more choices than a
+    """Matrices whose rows begin on 16 bytes go to kernels that take several rows a warp where that leaves warps enough (both
+    products from the second size on; with fewer loads in flight in the last two); copies one element further go to the others: the same bits, in both formats of the weights, with more choices than a
     block has warps, and added to what is there."""
     from fastllm_py_b200.native import ops
 
