@@ -348,7 +348,8 @@ FL_API int fl_moe_experts(const void* h, int dtype, long h_ld, const void* w_gu,
 // that share an expert's matrix.
 //
 //   moe_sort        one block: counts per expert, row -> pair, pair -> row, and the list of tiles: an expert's rows are
-//                   cut into as few tiles of at most 256 as will do, equally wide (a multiple of 64)
+//                   cut into as few tiles of at most 256 (of small matrices 128 or 64) as will do, equally wide (a multiple
+//                   of 64)
 //   moe_gather      the tokens' rows in the order of the pairs
 //   moe_group       tcgen05.mma over CTA pairs.  GATED: a pair's 256 weight rows are 128 gate rows and the 128 up rows of
 //                   the same features, the epilogue writes f(g, u) (bfloat16, in row order); UP: experts without a gate,
@@ -366,7 +367,7 @@ struct MoeTile {
 
 __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ chosen, int n_pairs, int experts,
                                                        int* __restrict__ row_pair, int* __restrict__ pair_row,
-                                                       int4* __restrict__ tiles, int* __restrict__ n_tiles_out) {
+                                                       int4* __restrict__ tiles, int* __restrict__ n_tiles_out, int tile_rows) {
     pdl_wait();
     pdl_trigger();
     extern __shared__ int count[];                       // [experts] counts, then cursors
@@ -378,7 +379,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
         const int lane = threadIdx.x;
         int rows_before = 0, tiles_before = 0;
         for (int e0 = 0; e0 < experts; e0 += 32) {
-            const int c = e0 + lane < experts ? count[e0 + lane] : 0, nt = (c + MOE_TN - 1) / MOE_TN;
+            const int c = e0 + lane < experts ? count[e0 + lane] : 0, nt = (c + tile_rows - 1) / tile_rows;
             int row = c, tile = nt;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -741,7 +742,7 @@ static int moe_group_launch(const void* a, const void* w, long w_rows, int n_pai
 }
 
 // ints: rows + n_tokens * top + rows / 64 + 1 of them, rows = fl_moe_group_rows: row -> pair, pair -> row, the list of tiles
-// (from a 16-byte boundary on) and its length, 2 pairs + pairs / 64 + 4 experts + 4 at most;
+// (from a 16-byte boundary on) and its length, 2 pairs + pairs / 64 + 4 experts + 4 at most with tiles of 256;
 // act: bfloat16 [rows, ff], 16-byte aligned; y: float [rows, width], of which the first 16-byte boundary on holds the
 // gathered tokens and then the results, a row a pair.
 FL_API int fl_moe_experts_grouped(const void* h, long h_ld, const void* w_gu, const void* w_down, const int* chosen,
@@ -757,13 +758,22 @@ FL_API int fl_moe_experts_grouped(const void* h, long h_ld, const void* w_gu, co
     int* pair_row = ints + n_pairs;
     int4* tiles = reinterpret_cast<int4*>(((uintptr_t)(ints + 2L * n_pairs) + 15) & ~(uintptr_t)15);
     y = reinterpret_cast<float*>(((uintptr_t)y + 15) & ~(uintptr_t)15);
-    const int max_tiles = n_pairs / MOE_TN + (experts < n_pairs ? experts : n_pairs);
+    // Tiles of 256 rows, or narrower ones where matrices of few rows would leave most CTA pairs idle (and where the list has
+    // room for them): 2048 pairs, 8 experts of 256 x 128, are 8 units of 256 rows.
+    const int some = experts < n_pairs ? experts : n_pairs;
+    const int n_up = gated ? (ff + 127) / 128 : (ff + 255) / 256, n_down = (width + 255) / 256, n_few = n_up < n_down ? n_up : n_down;
+    const long rows = fl_moe_group_rows(n_tokens, top, experts), room = rows + n_pairs + rows / 64 + 1 - (2L * n_pairs + 3) - 1;
+    int tile_rows = MOE_TN;
+    while (tile_rows > 64 && (long)(n_pairs / tile_rows > some ? n_pairs / tile_rows : some) * n_few < num_sms / 2 &&
+           4L * (2 * n_pairs / tile_rows + some) <= room)
+        tile_rows /= 2;
+    const int max_tiles = n_pairs / tile_rows + some;
     int* n_tiles = reinterpret_cast<int*>(tiles + max_tiles);
     if ((size_t)experts * sizeof(int) > 48 * 1024 || width % 32 || ff % 32 || num_sms < 2 ||
         (((uintptr_t)h | (uintptr_t)act) % 16) || (h_ld % 8))
         return (int)cudaErrorInvalidValue;
     int rc = fl_launch(moe_sort_kernel, dim3(1), dim3(1024), (size_t)experts * sizeof(int), stream, chosen, n_pairs, experts,
-                       row_pair, pair_row, tiles, n_tiles);
+                       row_pair, pair_row, tiles, n_tiles, tile_rows);
     if (rc) return rc;
     const long pieces = (long)n_pairs * (width / 8);
     rc = fl_launch(moe_gather_kernel, dim3((unsigned)((pieces + 255) / 256)), dim3(256), 0, stream, (const bf16*)h, h_ld,
