@@ -355,7 +355,9 @@ def test_expert_rows_are_those_of_the_kernels_for_any_size(n, top, width, ff, dt
 
 @pytest.mark.parametrize("width, ff, counts, top, gated, on_input", [
     (32, 32, [1], 1, True, False), (96, 160, [255, 0, 257, 1], 1, True, True), (256, 224, [64, 65, 256, 600], 2, True, False),
-    (544, 416, [300, 31, 513], 3, False, True), (128, 96, [3] * 70, 2, False, False), (2048, 1408, [250, 270, 8], 1, True, False)])
+    (544, 416, [300, 31, 513], 3, False, True), (128, 96, [3] * 70, 2, False, False), (2048, 1408, [250, 270, 8], 1, True, False),
+    # (tiles of 64 pairs above; of 128, and of 256)
+    (2048, 1408, [300, 257, 129, 600], 1, True, False), (2048, 1408, [255, 257, 256, 513, 1, 64, 65, 300, 31, 600], 1, True, False)])
 def test_grouped_expert_products_against_64_bits(width, ff, counts, top, gated, on_input):
     """Experts with one, few, many and no rows, at and beside the tiles' edges, in the order of the pairs or not.  What may
     differ from 64 bits: the unit's result is rounded to bfloat16 (2^-9 of each term of the second product), the output
