@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
         // and O stays in tensor memory, where P V accumulates; it is rescaled (read, multiplied,
         // written back by these threads) only when a row's maximum has grown by more than 2^8
         // since the scale in use was set: until then the exponentials simply use the older maximum
-        // (they stay below 2^8, well inside bfloat16 and float), and no thread waits for P V.
+        // (they stay below 2^8, well inside bfloat16 and float), and no thread waits for the last P V.
         const int r = threadIdx.x & 127;
         const int part = threadIdx.x >> 7;
         const int pos_r = ctx + row0 + r;

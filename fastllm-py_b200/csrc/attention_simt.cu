@@ -20,8 +20,9 @@
 // (token, head) pairs in the step the tiles are dealt out to the cluster's CTAs
 // (tile t to CTA t mod CL), which hand their results over through distributed
 // shared memory.  One block a (token, head) pair, each thread walking a key row
-// in global memory, took 196 us a layer for 4 tokens over 700 keys and 16 heads
-// of 128 in 32 bits, and 450 us for a prompt of 300 tokens; this takes 31 and 91.
+// in global memory, took 91 us for 4 tokens over 700 keys and 16 heads of 128 in
+// 32 bits, and 437 us for a prompt of 300 tokens; this takes 25 and 82 (in
+// bfloat16 93, 430, 29 and 83; 32 tokens over 700 keys 280 and 178).
 //
 // fastllm-py's counterparts: `_sdpa` (fastllm_py/model.py:341-353: scores scaled
 // by head_dim^-1/2, keys beyond the query masked, softmax and the weighted sum in

@@ -6,13 +6,15 @@
 // causal convolution over time and silu; beta = sigmoid(b) and g = exp(-exp(A_log) softplus(a + dt_bias))
 // are per head and token.  The read-out sees the token's own write.
 //
-// Four kernels, all float inside:
+// Kernels, all float inside:
 //   delta_prep        per token and head: convolution over the last `taps` inputs (from the step's rows or, before
-//                     the portion's start, from the request's saved tail), silu, unit norms, beta, decay
+//                     the portion's start, from the request's saved tail), silu, unit norms, beta, decay;
+//                     delta_prep_rows the same for long steps, 16 tokens a warp
 //   delta_tail        per request: the last taps - 1 raw inputs of the portion become the saved tail
-//   delta_scan        per (request, head, 32 value columns): the recurrence over the portion's tokens,
+//   delta_scan        per (request, head, 32 or 16 value columns): the recurrence over the portion's tokens,
 //                     one value column's state spread over eight lanes' registers, inputs staged
-//                     through shared memory a chunk of tokens ahead
+//                     through shared memory a chunk of tokens ahead by a warp of its own; delta_step the
+//                     same for steps of as many tokens as requests
 //   delta_gated_norm  per (token, head): o / rms(o) * w * silu(gate)
 //
 // A request's state row is [heads][vdim][dim] floats (a column of S is contiguous) followed by the
@@ -83,8 +85,8 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(
 
 // The same for prompts with heads of 128 channels on both sides and up to four taps: a warp takes PREP_TOKENS neighbouring
 // tokens of one unit, four channels a lane, so the taps are read once, a unit's sum of squares stays in the warp and 16
-// tokens' decays (double precision, a thread each) are formed side by side.  A block a (token, unit) took 101 us for 2048
-// tokens of 32 units, most of it blocks coming and going; a layer takes 45 us less so.  Sums in the order of the block's: the four
+// tokens' decays (double precision, a thread each) are formed side by side.  A block a (token, unit) takes 96 us for 2048
+// tokens of 32 units, most of it blocks coming and going; this takes 42.  Sums in the order of the block's: the four
 // groups of 32 channels by themselves, then (0 + 2) + (1 + 3).
 #define PREP_TOKENS 16
 template <typename T, typename TW>
@@ -177,8 +179,8 @@ __global__ void delta_tail_kernel(const T* __restrict__ proj, long ld, float* __
 // the recurrence do nothing else, a warp of them being alone on its scheduler.  In shared memory
 // a part's k (and q) elements are contiguous and parts are DPT + 4 floats apart, so a thread fetches them
 // four at a time without bank conflicts.
-// What bounds a long prompt: the chain from one token's u to the next one's.  2048 tokens, 16 heads of 128 x 128: 326 us,
-// 160 ns a token; 679 us with the fetches and q . k on the same threads (156 instructions a token and warp, a fifth of the
+// What bounds a long prompt: the chain from one token's u to the next one's.  2048 tokens, 16 heads of 128 x 128: 310 us,
+// 151 ns a token; 676 us with the fetches and q . k on the same threads (156 instructions a token and warp, a fifth of the
 // time at the barrier behind the two warps that fetched) and one multiply-add an element.
 // Registers are kept to what lets two blocks of 32 columns share an SM: several requests' prompts bring more blocks than SMs
 // (8 x 100 tokens, 16 heads of 128 x 128: 121 us with one block an SM, 96 with two).

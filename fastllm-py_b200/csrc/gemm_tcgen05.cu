@@ -941,9 +941,9 @@ static void plan_one_tile(int M, int N, int K, int num_sms, int* bn_out, int* sp
 // kernel with that token tile; 512, 640: the CTA-pair kernel, 256 or 128 tokens wide.  `deferred`: the
 // partial sums of a split K are left to the consumer kernel, which adds them as it reads them; else a reduce
 // kernel follows.  The constants were fitted (least squares on the logarithm) to event-timed runs of every
-// candidate on B200 for 12 weight shapes of 2048 to 102400 features and 2048 to 22016 inputs at 80 to 768
-// tokens: 8 % root-mean-square error, and the candidate the model picks is within 1.6 % of the best one on
-// average (15 % at worst).  One-tile CTAs cost a fixed start plus a time per 64-deep K step that is a fifth
+// candidate on B200 for 12 weight shapes of 2048 to 102400 features and 2048 to 22016 inputs at 80 to 1024
+// tokens, with tiles of whole widths; against runs of the tiles that tc_pair_tile_tokens cuts now the candidate that the
+// model picks is 1.6 % off the best one on average (19 % at worst).  One-tile CTAs cost a fixed start plus a time per 64-deep K step that is a fifth
 // shorter when a CTA has its SM to itself; a pair costs a fixed 7.3 us a launch and 0.28 to 0.31 us a K step;
 // no product is faster than its operands stream from memory; partial sums cost their bytes.
 static double tc_cost(int M, int N, int K, int num_sms, int bn, int splits, int deferred) {

@@ -110,8 +110,8 @@ __global__ void __launch_bounds__(128) moe_pick_kernel(const float* __restrict__
 // The order of a row's sum x . w, whichever kernel makes it: 32 chains, chain c adding up the elements c, c + 32, ... with
 // fused multiply-adds, and the chains added in a tree (neighbours 16 apart first).  The kernels for any size give a warp a
 // row and a lane a chain, which fetches 2 bytes a lane: 8 tokens x 4 of 32 experts of 2048 x 1408 took 85 + 62 us a layer,
-// bound by the number of loads (59 + 53 by rows).  Where rows are whole blocks of 32 elements and 16-byte aligned, a lane takes the MOE_V
-// neighbouring chains that 16 bytes hold, 32 / MOE_V lanes a row, and a warp several rows at once.
+// bound by the number of loads (57 + 44 by rows).  Where rows are whole blocks of 32 elements and 16-byte aligned, a lane takes
+// the MoeRows::V neighbouring chains that 16 bytes hold, 32 / V lanes a row, and a warp several rows at once.
 template <typename TW> struct MoeRows {
     static constexpr int V = 16 / (int)sizeof(TW);       // chains a lane
     static constexpr int LPR = 32 / V;                   // lanes a row
@@ -360,10 +360,7 @@ FL_API int fl_moe_experts(const void* h, int dtype, long h_ld, const void* w_gu,
 // A row's sums do not depend on the other rows of its tile, so the order of rows within an expert (it
 // comes from atomics) does not show in the results.
 #define MOE_TN 256               // rows (pairs) of a tile at most
-
-struct MoeTile {
-    int expert, row0, rows, n;   // n: rows in the MMA, a multiple of 64
-};
+// a tile of the list, an int4: expert, first row, rows, rows in the MMA (a multiple of 64)
 
 __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ chosen, int n_pairs, int experts,
                                                        int* __restrict__ row_pair, int* __restrict__ pair_row,

@@ -1,5 +1,6 @@
-// Shared by the products on the Blackwell tensor cores (gemm_tcgen05.cu, moe_tc.cu): tile sizes, the PTX that TMA loads,
-// mbarriers, tensor memory and tcgen05.mma take, the gated units of their epilogues, and the tensor maps.
+// Shared by the products on the Blackwell tensor cores (gemm_tcgen05.cu, moe.cu) and the latent attention of prompts
+// (latent_attention_tc.cu): tile sizes, the PTX that TMA loads, mbarriers, tensor memory and tcgen05.mma take, the gated units
+// of the products' epilogues and how their warps give up, and the tensor maps.
 #pragma once
 
 #include <cuda.h>

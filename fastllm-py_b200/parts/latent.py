@@ -168,7 +168,7 @@ class LatentAttention(Part):
 
     def _prompts(self, step, n_tokens: int, page_size: int) -> bool:
         """Whether a step without splits goes to the prompt kernel: it takes eight neighbouring tokens of a request at a
-        time at the price of 3.4 single tokens in the other kernel where both fill the GPU (2048 tokens: 416 us against
+        time at the price of 3.4 single tokens in the other kernel where both fill the GPU (2048 tokens: 413 us against
         971), so it is the faster one until half of its rows stay empty.  A tile of keys alone takes it as long as the other
         (4.6 us with a latent of 512), or longer (3.6 against 2.9 with 256, which leaves the other room for more blocks an
         SM): with few blocks the other kernel is as fast (128 tokens of 16 heads behind 1000: 153 us both) or faster (256:

@@ -8,8 +8,9 @@ of the weights (larger than L2 together).
     python tests/data/measure_gemm_candidates.py --planned     # the planned products against cuBLAS, as a table
 
 gemm_candidates_b200.jsonl beside this file is its output on one B200 for the token counts 80, 128, 192, 256,
-384, 512, 768 and 96, 160, 320, 448, 640, 1024; tests/test_bench_and_loading.py holds the plan against it, and
-the constants of the plan's cost model (tc_cost in csrc/gemm_tcgen05.cu) were fitted to it.
+384, 512, 768 and 96, 160, 320, 448, 640, 1024; tests/test_bench_and_loading.py holds the plan against it (the
+constants of the plan's cost model, tc_cost in csrc/gemm_tcgen05.cu, were fitted to an earlier output, before
+the CTA pairs' tiles were cut to fill their last round).
 """
 import json
 import sys
