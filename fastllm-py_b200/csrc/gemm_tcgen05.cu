@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(
     const uint32_t tmem_acc = *tmem_slot;
 
     pdl_trigger();
+    int issued = 0;                                          // (thread 0: fills of the ring)
     if (warp == 0) {
         if (lane == 0) {
             // ---- producer: TMA loads of the weight tile and the token tile.
@@ -126,6 +127,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(
                 unsigned char* b_dst = tiles + it * stage_bytes + w_bytes;
                 tma_load_2d(b_dst, &map_a, &full_bar[it], (kb_begin + it) * TC_BK, tile_m * BN);
             }
+            issued = ahead;
             int s = ahead % n_stages;
             uint32_t ph = (uint32_t)(ahead / n_stages) & 1u;
             for (int it = ahead; it < n_iters && !*abort_flag; ++it) {
@@ -138,6 +140,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(
                 const int k0 = (kb_begin + it) * TC_BK;
                 load_weights(a_dst, &full_bar[s], k0);
                 tma_load_2d(a_dst + w_bytes, &map_a, &full_bar[s], k0, tile_m * BN);
+                ++issued;
                 if (++s == n_stages) { s = 0; ph ^= 1u; }
             }
         }
@@ -285,6 +288,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(
     }
     tc_fence_before();
     __syncthreads();
+    if (threadIdx.x == 0 && *abort_flag) tma_drain(full_bar, n_stages, issued);
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_acc, TMEM_COLS);
@@ -506,6 +510,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_pair_kernel(
         }
     };
 
+    int issued = 0;                                         // (thread 0: fills of the ring)
     if (warp == 0) {
         if (lane == 0 && !*abort_flag) {
             // ---- producer (both CTAs): this CTA's 128 weight rows and BNT/2 token rows of each stage,
@@ -528,6 +533,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_pair_kernel(
                     load_weights(dst, &full_bar[s], kb, tn);
                     tma_load_2d_pair(dst + L::W_BYTES, &map_a, &full_bar[s], kb * TC_BK,
                                      tm * wt + (int)rank * (wt / 2));
+                    ++issued;
                     if (++s == L::STAGES) { s = 0; ph ^= 1u; }
                 }
             }
@@ -703,6 +709,8 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_pair_kernel(
     }
     tc_fence_before();
     __syncthreads();
+    if (threadIdx.x == 0 && *abort_flag) tma_drain(full_bar, rank == 0 ? L::STAGES : 0, issued);
+    __syncwarp();
     cluster_sync_all();                                     // the peer is done with this CTA's barriers and memory
     if (warp == 1) {
         tc_fence_after();

@@ -496,6 +496,7 @@ __global__ void __launch_bounds__(TC_THREADS) moe_group_kernel(
     auto give_up = [&]() {
         if (!*abort_flag) { *abort_flag = 1; atomicCAS(status, 0, MOE_ERR_WAIT); }
     };
+    int issued = 0;                                         // (thread 0: fills of the ring)
     if (warp == 0) {
         if (lane == 0 && !*abort_flag) {
             // ---- producer (both CTAs): this CTA's 128 weight rows and half of the tile's rows, k-block after k-block
@@ -523,6 +524,7 @@ __global__ void __launch_bounds__(TC_THREADS) moe_group_kernel(
                     for (int r = 0; r < half; r += 32)
                         tma_load_2d_pair(dst + L::W_BYTES + r * TC_BK * 2, &map_a, &full_bar[s], kb * TC_BK,
                                          t.y + (int)rank * half + r);
+                    ++issued;
                     if (++s == L::STAGES) { s = 0; ph ^= 1u; }
                 }
             }
@@ -653,6 +655,8 @@ __global__ void __launch_bounds__(TC_THREADS) moe_group_kernel(
     }
     tc_fence_before();
     __syncthreads();
+    if (threadIdx.x == 0 && *abort_flag) tma_drain(full_bar, rank == 0 ? L::STAGES : 0, issued);
+    __syncwarp();
     cluster_sync_all();                                     // the peer is done with this CTA's barriers and memory
     if (warp == 1) {
         tc_fence_after();

@@ -56,6 +56,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
     return true;
 }
+// For a CTA that gives up: the copies on their way must land before its shared memory goes to another CTA.  Called by the
+// thread that issued `issued` fills of a ring of `stages`: waits for the last of them, up to the first that does not land
+// within the limit, and a millisecond more (the fills of a pair's other CTA signal the leader's barriers only, which take no
+// notice of them before the leader's own).
+__device__ __forceinline__ void tma_drain(uint64_t* full_bar, int stages, int issued) {
+    bool landed = true;
+    for (int k = issued > stages ? issued - stages : 0; k < issued && landed; ++k) {
+        const uint64_t t0 = global_ns();
+        while (landed && !mbar_try_wait(&full_bar[k % stages], (uint32_t)(k / stages) & 1u)) landed = global_ns() - t0 <= TC_WAIT_LIMIT_NS;
+    }
+    const uint64_t t0 = global_ns();
+    while (issued > 0 && global_ns() - t0 < 1000000ull) {}
+}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x,
                                             int y) {
     asm volatile(

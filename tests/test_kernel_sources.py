@@ -81,3 +81,18 @@ def test_a_pair_tile_has_one_width():
     launch = text[text.index("static int launch_tc_pair("):]
     launch = launch[:launch.index("\n}\n")]
     assert "tc_pair_tile_tokens(" in launch and "make_map(&map_a, A, M, K, lda, wt / 2)" in launch
+
+
+@pytest.mark.parametrize("name, kernels", [("gemm_tcgen05.cu", ["gemm_tc_kernel", "gemm_tc_pair_kernel"]), ("moe.cu", ["moe_group_kernel"])])
+def test_products_that_give_up_wait_for_their_copies(name, kernels):
+    """A CTA that leaves with copies on their way would have them land in the next CTA's shared memory: after all roles have
+    met, the thread that issued every fill waits for them, where the abort flag is set, before the CTA (or the pair) may go."""
+    text = (CSRC / name).read_text()
+    for kernel in kernels:
+        body = text[text.index(f" {kernel}("):]
+        body = body[:body.index("\n}\n")]
+        met = body.rindex("tc_fence_before();\n    __syncthreads();")
+        drain = body.index("if (threadIdx.x == 0 && *abort_flag) tma_drain(full_bar, ", met)
+        assert drain < body.index("dealloc", met) and ("cluster_sync_all" not in body or drain < body.index("cluster_sync_all", met))
+        ring = body[body.index("int issued = 0;"):met]
+        assert ring.count("++issued;\n") == 1 and ring.index("++issued;") < ring.index("if (++s ==")
