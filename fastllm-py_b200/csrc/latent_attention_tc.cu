@@ -334,8 +334,10 @@ FL_API int fl_latent_attention_tc(const void* q, long q_ld, void* out, int out_d
 //   warp 8     TMA: queries once, then the keys' pages, LP_STAGES tiles ahead; a page that no row sees is fetched from
 //              beyond the tensor, which gives zeros
 //   warp 9     the MMAs: scores of tile i + 1, then values of tile i
-// What bounds it: the keys' way through L2, two tiles being all that fits beside the queries (without the copies 243 us),
-// and the 36 narrow MMAs of a tile's scores (110 us); exponentials and rescaling cost 25 us together.
+// Two thirds of the queries are kept in tensor memory (written there once by warps 0-7): the score MMAs that take them from
+// there do not read 4 KB of shared memory each, and four tiles of keys find room instead of two, so that a tile's way through
+// L2 is hidden.  (With all of the queries in shared memory that way showed between any two tiles: a tile's stage is free only
+// after its values, which come after the next tile's scores.  413 us, 243 without the copies.)
 #if LT_WIDTH % 64 == 0 && LAT_RANK % 64 == 0 && LT_WIDTH <= 576 && (LAT_RANK <= 256 || LAT_RANK == 512)
 #define LP_BUILT 1
 #include "tcgen05.cuh"
@@ -343,16 +345,20 @@ FL_API int fl_latent_attention_tc(const void* q, long q_ld, void* out, int out_d
 #define LP_VC (LAT_RANK <= 256 ? LAT_RANK : 256)         // value columns of a CTA
 #define LP_HALVES (LAT_RANK / LP_VC)
 #define LP_ATOMS (LT_WIDTH / 64)                          // 64-column swizzle atoms of a row
-#define LP_STAGES 2
 #define LP_Q_ATOM (128 * 128)                             // bytes of an atom of the 128 query rows
 #define LP_K_ATOM (LT_KEYS * 128)
 #define LP_STAGE_BYTES (LP_ATOMS * LP_K_ATOM)
+// Queries in tensor memory, beside 256 columns of accumulators and two score buffers: the first six atoms (192 columns); the
+// other atoms' rows are in shared memory.
+#define LP_TQ (LP_ATOMS < 6 ? LP_ATOMS : 6)
+#define LP_SQ (LP_ATOMS - LP_TQ)
+#define LP_STAGES 4
 #define LP_TOKENS 8
 #define LP_THREADS 320
-#define LP_SMEM (LP_ATOMS * LP_Q_ATOM + LP_STAGES * LP_STAGE_BYTES + 256 + 3 * 128 * 4 + 1024)
+#define LP_SMEM (LP_SQ * LP_Q_ATOM + LP_STAGES * LP_STAGE_BYTES + 256 + 3 * 128 * 4 + 1024)
 enum { LP_ERR_WAIT = 141 };
 static_assert(LP_SMEM <= 232448, "more shared memory than a CTA can have");
-static_assert(LT_SMEM <= LP_ATOMS * LP_Q_ATOM + LP_STAGES * LP_STAGE_BYTES, "tokens done again find room in the tiles' place");
+static_assert(LT_SMEM <= LP_SQ * LP_Q_ATOM + LP_STAGES * LP_STAGE_BYTES, "tokens done again find room in the tiles' place");
 
 __device__ __forceinline__ void lp_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -416,7 +422,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
     int* __restrict__ status) {
     extern __shared__ unsigned char lp_raw[];
     unsigned char* q_s = (unsigned char*)(((uintptr_t)lp_raw + 1023) & ~(uintptr_t)1023);
-    unsigned char* k_s = q_s + LP_ATOMS * LP_Q_ATOM;
+    unsigned char* k_s = q_s + LP_SQ * LP_Q_ATOM;
     uint64_t* bars = (uint64_t*)(k_s + LP_STAGES * LP_STAGE_BYTES);
     uint64_t* q_full = bars;
     uint64_t* k_full = bars + 1;                          // [LP_STAGES]
@@ -425,7 +431,8 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
     uint64_t* c_full = s_full + 2;                        // [2] the rows' rescaling factors are there
     uint64_t* p_full = c_full + 2;                        // [2] weights written and accumulators rescaled
     uint64_t* o_done = p_full + 2;                        // [2] values of tile i are added up: barrier i & 1, phase i >> 1
-    uint32_t* tmem_slot = (uint32_t*)(o_done + 2);
+    uint64_t* t_full = o_done + 2;                        // the queries in tensor memory are there
+    uint32_t* tmem_slot = (uint32_t*)(t_full + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     volatile int* never = abort_flag + 1;                 // stays 0: for waits that must not be cut short
     volatile int* again = never + 1;                      // the tokens are done again
@@ -453,6 +460,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
+        mbar_init(t_full, 8);
         for (int s = 0; s < LP_STAGES; ++s) {
             mbar_init(&k_full[s], 1);
             mbar_init(&k_empty[s], 1);
@@ -477,17 +485,36 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_o = *tmem_slot, tmem_s = tmem_o + 256;          // two score buffers of 32 columns
+    const uint32_t tmem_q = tmem_s + 2 * LT_KEYS;                       // 32 columns an atom
     auto give_up = [&]() {
         if (!*abort_flag) { *abort_flag = 1; atomicCAS(status, 0, LP_ERR_WAIT); }
     };
+    if (warp < 8) {
+        // a row's queries for tensor memory, pairs of elements a column, every other atom by warps 4-7
+        const int r = threadIdx.x & 127;
+        const bf16* src = q + (long)(tok0 + (r >> 4)) * q_ld + (long)(head0 + (r & 15)) * LT_WIDTH;
+        const uint32_t dst = tmem_q + ((uint32_t)((warp & 3) * 32) << 16);
+#pragma unroll 1
+        for (int a = warp >> 2; a < LP_TQ; a += 2) {
+            uint4 w[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                w[j] = (r >> 4) < tokens ? reinterpret_cast<const uint4*>(src + a * 64)[j] : make_uint4(0u, 0u, 0u, 0u);
+            tmem_st16(dst + (uint32_t)(a * 32), reinterpret_cast<const uint32_t*>(w));
+            tmem_st16(dst + (uint32_t)(a * 32 + 16), reinterpret_cast<const uint32_t*>(w + 4));
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        lp_warp_arrive(t_full);
+    }
 
     if (warp == 8) {
         // ---- producer: a lane issues one box, the part of a page that lies in the tile x 64 columns
         const int* bt = block_table + (long)req * bt_stride;
         const int box = min(page_size, LT_KEYS), boxes = LT_KEYS / box;
         if (lane == 0 && !*abort_flag) {
-            mbar_expect_tx(q_full, LP_ATOMS * LP_Q_ATOM);
-            for (int a = 0; a < LP_ATOMS; ++a) lp_tma_3d(q_s + a * LP_Q_ATOM, &map_q, q_full, a * 64, head0, tok0);
+            mbar_expect_tx(q_full, LP_SQ * LP_Q_ATOM);
+            for (int a = 0; a < LP_SQ; ++a) lp_tma_3d(q_s + a * LP_Q_ATOM, &map_q, q_full, (LP_TQ + a) * 64, head0, tok0);
         }
         __syncwarp();
         int i = 0;
@@ -529,17 +556,22 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
             }
             tc_fence_after();
             if (lane == 0) {
-                const uint32_t qa = smem_u32(q_s), ka = smem_u32(k_s + s * LP_STAGE_BYTES);
-#pragma unroll 4
-                for (int k = 0; k < LT_WIDTH / 16; ++k)
-                    umma_bf16(tmem_s + (uint32_t)(b * LT_KEYS), smem_desc_sw128(qa + (uint32_t)((k >> 2) * LP_Q_ATOM + (k & 3) * 32)),
-                              smem_desc_sw128(ka + (uint32_t)((k >> 2) * LP_K_ATOM + (k & 3) * 32)), idesc_s, k > 0 ? 1u : 0u);
+                // (a descriptor's address counts 16 bytes)
+                const uint64_t qd = smem_desc_sw128(smem_u32(q_s)), kd = smem_desc_sw128(smem_u32(k_s + s * LP_STAGE_BYTES));
+                const uint32_t d = tmem_s + (uint32_t)(b * LT_KEYS);
+#pragma unroll
+                for (int k = 0; k < LP_TQ * 4; ++k)
+                    umma_bf16_ts(d, tmem_q + (uint32_t)(k * 8), kd + (uint64_t)(((k >> 2) * LP_K_ATOM + (k & 3) * 32) >> 4), idesc_s, k > 0 ? 1u : 0u);
+#pragma unroll
+                for (int k = LP_TQ * 4; k < LP_ATOMS * 4; ++k)
+                    umma_bf16(d, qd + (uint64_t)((((k >> 2) - LP_TQ) * LP_Q_ATOM + (k & 3) * 32) >> 4),
+                              kd + (uint64_t)(((k >> 2) * LP_K_ATOM + (k & 3) * 32) >> 4), idesc_s, 1u);
                 umma_commit(&s_full[b]);
             }
             __syncwarp();
             return true;
         };
-        if (ok) ok = lp_warp_wait(q_full, 0, abort_flag);
+        if (ok) ok = lp_warp_wait(t_full, 0, abort_flag) && lp_warp_wait(q_full, 0, abort_flag);
         if (ok) ok = scores(0);
         for (int i = 0; i < n_tiles && ok; ++i) {
             // the scores of tile i + 1 go where those of tile i - 1 and then its weights were: the values of tile i - 1 were
