@@ -207,12 +207,17 @@ struct FtSmem {
     static constexpr int TOTAL = TILES + BARS + SLACK;
 };
 
+// ROWS: a cache row holds a token's key and its value (k | v, pages [n_kv_heads][page_size][2 HEAD_DIM]); `sink` ([heads], or
+// null) is a term exp(sink) of each head's denominator, and `gate` (or null) multiplies a row's result by the sigmoid of its
+// gate, `gate_cols` numbers a head (one, or one a channel), before it is rounded.
+template <bool ROWS>
 __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
     bf16* __restrict__ out, long out_ld, int page_size, int kv_rows_total, const int* __restrict__ block_table,
     int bt_stride, const int* __restrict__ req_start, const int* __restrict__ req_ctx,
     const int* __restrict__ req_qlen, int n_requests, int include_single, int n_heads, int n_kv_heads,
-    int window, float scale_log2e, int* __restrict__ status) {
+    int window, float scale_log2e, int* __restrict__ status, const float* __restrict__ sink, const bf16* __restrict__ gate,
+    long gate_ld, int gate_cols) {
     extern __shared__ __align__(1024) unsigned char ft_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)ft_raw + 1023) & ~(uintptr_t)1023);
     if (base + FtSmem::TILES + FtSmem::BARS > ft_raw + FtSmem::TOTAL) {       // uniform over the CTA
@@ -287,10 +292,10 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
             int row = kv_rows_total;
             if (first_key <= pos_last && last_key >= lo_tile) {
                 const long pg = bt[first_key / page_size];
-                row = (int)(((pg * 2 + is_v) * n_kv_heads + kvh) * page_size);
+                row = (int)((ROWS ? pg * n_kv_heads + kvh : (pg * 2 + is_v) * n_kv_heads + kvh) * page_size);
             }
             const int off = s * FtSmem::KV_BYTES + a * FT_ATOM_BYTES + p * page_size * 128;
-            ft_tma_2d(ring + off, &map_kv, &full[s], a * 64, row);
+            ft_tma_2d(ring + off, &map_kv, &full[s], a * 64 + (ROWS ? is_v * HEAD_DIM : 0), row);
         }
     };
     // The producer warps set up their own barriers and send for the queries and the first block (the rings are
@@ -396,6 +401,15 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
                 if (i + 1 < n_blocks && !issue_s(i + 1)) { ok = false; break; }
                 const int b = i & 1, vs = i % FT_STAGES;
                 if (!ft_wait(&v_full[vs], (uint32_t)(i / FT_STAGES) & 1u, abort_flag)) { ok = false; break; }
+                if (ROWS && i == n_blocks - 1) {
+                    // what the last page holds behind the tile's last key may be anything, and a weight of zero does not
+                    // make a value that is not finite vanish: those rows become zeros
+                    const int from = pos_last + 1 - (kb_begin + i) * FT_BN, to = (from + page_size - 1) / page_size * page_size;
+                    for (int a = 0; a < FT_ATOMS; ++a)
+                        for (int o = from * 128; o < to * 128; o += 16)
+                            *reinterpret_cast<uint4*>(v_s + vs * FtSmem::KV_BYTES + a * FT_ATOM_BYTES + o) = make_uint4(0u, 0u, 0u, 0u);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                }
                 if (!ft_wait(&p_full[b], (uint32_t)(i >> 1) & 1u, abort_flag)) { ok = false; break; }
                 ft_fence_after();
                 // O (+)= P(i) V(i): A = P from tensor memory (rows in the lanes, 16 keys = 8 columns of
@@ -425,6 +439,10 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
         // [round parity][part][row]: a round's values stay untouched while the next round's are written
         float* part_max_all = reinterpret_cast<float*>(bars + FtSmem::BAR_SLOTS);
         float m_run = -CUDART_INF_F, l_run = 0.0f;           // m_run: the maximum the scale in use is based on
+        if (ROWS && sink != nullptr) {                       // the running maximum and sum start from the sink's term
+            m_run = sink[h] * 1.4426950408889634f;
+            l_run = part == 0 ? 1.0f : 0.0f;
+        }
         bool ok = !*abort_flag;
         for (int i = 0; i < n_blocks && ok; ++i) {
             const int sb = i & 1;
@@ -525,7 +543,15 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
 #pragma unroll
         for (int q = 1; q < FT_PARTS; ++q) l_row += part_sum[q * 128 + r];
         if (met && ok && !*abort_flag && n_blocks > 0) {
-            const float inv = 1.0f / l_row;
+            float inv = 1.0f / l_row;
+            const bf16* gate_row = nullptr;
+            if (ROWS && gate != nullptr && r < rows_here) {
+                gate_row = gate + (long)(tok0 + r) * gate_ld;
+                if (gate_cols == 1) {
+                    inv *= 1.0f / (1.0f + expf(-__bfloat162float(gate_row[h])));
+                    gate_row = nullptr;
+                }
+            }
             bf16* dst = out + (long)(tok0 + r) * out_ld + (long)h * HEAD_DIM + part * FT_OD;
 #pragma unroll
             for (int c = 0; c < FT_OD; c += 32) {
@@ -538,9 +564,15 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
                         uint4 o4;
                         __nv_bfloat162* wp = reinterpret_cast<__nv_bfloat162*>(&o4);
 #pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            wp[e] = __floats2bfloat162_rn(__uint_as_float(w[d + 2 * e]) * inv,
-                                                          __uint_as_float(w[d + 2 * e + 1]) * inv);
+                        for (int e = 0; e < 4; ++e) {
+                            float f0 = __uint_as_float(w[d + 2 * e]) * inv, f1 = __uint_as_float(w[d + 2 * e + 1]) * inv;
+                            if (ROWS && gate_row != nullptr) {
+                                const bf16* gc = gate_row + h * HEAD_DIM + part * FT_OD + c + d + 2 * e;
+                                f0 *= 1.0f / (1.0f + expf(-__bfloat162float(gc[0])));
+                                f1 *= 1.0f / (1.0f + expf(-__bfloat162float(gc[1])));
+                            }
+                            wp[e] = __floats2bfloat162_rn(f0, f1);
+                        }
                         *reinterpret_cast<uint4*>(dst + c + d) = o4;
                     }
                 }
@@ -590,27 +622,25 @@ FL_API int fl_attention_prefill_tc_takes(int page_size) {
     return page_size >= 8 && page_size <= FT_BN && page_size % 8 == 0 && FT_BN % page_size == 0;
 }
 
-// The arguments of fl_attention_prefill (attention_prefill.cu) with the cache given
-// as one tensor [n_pages, 2, n_kv_heads, page_size, HEAD_DIM] and a status word.
-FL_API int fl_attention_prefill_tc(const void* q, long q_ld, void* out, long out_ld, const void* cache,
-                                   long n_pages, int page_size, const int* block_table, int bt_stride,
-                                   const int* req_start, const int* req_ctx, const int* req_qlen,
-                                   int n_requests, int n_tokens, int include_single, int n_heads,
-                                   int n_kv_heads, int window, float scale, int* status, cudaStream_t stream) {
+template <bool ROWS>
+static int ft_launch(const void* q, long q_ld, void* out, long out_ld, const void* cache, long n_pages, int page_size,
+                     const int* block_table, int bt_stride, const int* req_start, const int* req_ctx, const int* req_qlen,
+                     int n_requests, int n_tokens, int include_single, int n_heads, int n_kv_heads, int window, float scale,
+                     const float* sink, const void* gate, long gate_ld, int gate_cols, int* status, cudaStream_t stream) {
     if (n_requests <= 0 || n_tokens <= 0) return 0;
     if (!fl_attention_prefill_tc_takes(page_size) || n_heads > 65535 || n_heads % n_kv_heads)
         return (int)cudaErrorInvalidValue;
     if ((q_ld % 8) || (out_ld % 8)) return (int)cudaErrorMisalignedAddress;
-    const long kv_rows = n_pages * 2 * n_kv_heads * page_size;
+    const long kv_rows = n_pages * (ROWS ? 1 : 2) * n_kv_heads * page_size;
     if (kv_rows >= (1l << 31)) return (int)cudaErrorInvalidValue;
     CUtensorMap map_q, map_kv;
     int rc = ft_make_map(&map_q, q, n_tokens, (long)n_heads * HEAD_DIM, q_ld, FT_BM);
     if (rc) return rc;
-    rc = ft_make_map(&map_kv, cache, kv_rows, HEAD_DIM, HEAD_DIM, page_size);
+    rc = ft_make_map(&map_kv, cache, kv_rows, ROWS ? 2 * HEAD_DIM : HEAD_DIM, ROWS ? 2 * HEAD_DIM : HEAD_DIM, page_size);
     if (rc) return rc;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              FtSmem::TOTAL);
         if (e != cudaSuccess) return (int)e;
         configured = true;
@@ -619,8 +649,33 @@ FL_API int fl_attention_prefill_tc(const void* q, long q_ld, void* out, long out
     if (max_tiles > 65535) return (int)cudaErrorInvalidValue;
     dim3 grid(n_heads, max_tiles);                 // heads fastest: every head's late (long) tiles start first
     // plain stream order (no programmatic overlap): this kernel takes all of an SM's tensor memory
-    attention_prefill_tc_kernel<<<grid, FT_THREADS, FtSmem::TOTAL, stream>>>(
+    attention_prefill_tc_kernel<ROWS><<<grid, FT_THREADS, FtSmem::TOTAL, stream>>>(
         map_q, map_kv, (bf16*)out, out_ld, page_size, (int)kv_rows, block_table, bt_stride, req_start, req_ctx,
-        req_qlen, n_requests, include_single, n_heads, n_kv_heads, window, scale * 1.4426950408889634f, status);
+        req_qlen, n_requests, include_single, n_heads, n_kv_heads, window, scale * 1.4426950408889634f, status, sink,
+        (const bf16*)gate, gate_ld, gate_cols);
     return fl_launch_status();
+}
+
+// The arguments of fl_attention_prefill (attention_prefill.cu) with the cache given
+// as one tensor [n_pages, 2, n_kv_heads, page_size, HEAD_DIM] and a status word.
+FL_API int fl_attention_prefill_tc(const void* q, long q_ld, void* out, long out_ld, const void* cache,
+                                   long n_pages, int page_size, const int* block_table, int bt_stride,
+                                   const int* req_start, const int* req_ctx, const int* req_qlen,
+                                   int n_requests, int n_tokens, int include_single, int n_heads,
+                                   int n_kv_heads, int window, float scale, int* status, cudaStream_t stream) {
+    return ft_launch<false>(q, q_ld, out, out_ld, cache, n_pages, page_size, block_table, bt_stride, req_start, req_ctx,
+                            req_qlen, n_requests, n_tokens, include_single, n_heads, n_kv_heads, window, scale, nullptr,
+                            nullptr, 0, 0, status, stream);
+}
+
+// The same over a cache of rows k | v, [n_pages, n_kv_heads, page_size, 2 HEAD_DIM], every earlier token seen, with a sink
+// and a gate (see the kernel; either may be null).
+FL_API int fl_attention_prefill_rows(const void* q, long q_ld, void* out, long out_ld, const void* cache, long n_pages,
+                                     int page_size, const int* block_table, int bt_stride, const int* req_start,
+                                     const int* req_ctx, const int* req_qlen, int n_requests, int n_tokens,
+                                     int include_single, int n_heads, int n_kv_heads, float scale, const float* sink,
+                                     const void* gate, long gate_ld, int gate_cols, int* status, cudaStream_t stream) {
+    return ft_launch<true>(q, q_ld, out, out_ld, cache, n_pages, page_size, block_table, bt_stride, req_start, req_ctx,
+                           req_qlen, n_requests, n_tokens, include_single, n_heads, n_kv_heads, 0, scale, sink, gate,
+                           gate_ld, gate_cols, status, stream);
 }

@@ -834,13 +834,44 @@ def sink_tc_library(dim: int, vdim: int):
     return "sink_attention_tc", {"SINK_DIM": dim, "SINK_VDIM": vdim}
 
 
+def _sink_rows_pay(step, include_single: bool) -> bool:
+    return True
+
+
+def sink_rows_takes(dim: int, vdim: int, window, keep_first, cap, rel, chunk, page_size: int) -> bool:
+    """Whether the prompt attention on tcgen05 serves such a layer: keys and values of 64 or 128, every earlier token seen,
+    scores as they are."""
+    from .attention import tc_prefill_takes
+    return dim == vdim and tc_prefill_takes(dim, page_size) and not window and not keep_first and not cap and rel is None and not chunk
+
+
+def sink_attention_rows(q, out, cache, block_table, step, heads, kv_heads, size, scale, sink, page_size, include_single, gate):
+    """`sink_attention_tc` for layers that `sink_rows_takes`, on tcgen05 in tiles of 128 rows."""
+    from .gemm_tc import status_word
+
+    fn = _fn("attention_prefill_tc", "fl_attention_prefill_rows",
+             [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
+              c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_long, c_int, c_void_p, c_void_p],
+             {"HEAD_DIM": size})
+    _check(fn(_ptr(q), _ld(q), _ptr(out), _ld(out), _ptr(cache), cache.shape[0], page_size, _ptr(block_table),
+              block_table.stride(0), _ptr(step.req_start), _ptr(step.req_ctx), _ptr(step.req_qlen), step.n_requests,
+              q.shape[0], int(include_single), heads, kv_heads, float(scale), _ptr(sink),
+              *_gate_args(gate, out, heads, size), _ptr(status_word(q.device)), _stream()), "attention_prefill_rows")
+
+
 def sink_attention_tc(q, out, cache, block_table, step, heads, kv_heads, dim, vdim, window, keep_first, scale, cap,
                       bucket_of, rel, sink, page_size, include_single=True, chunk=None, gate=None):
     """`sink_attention_simt` on tensor cores: q, cache and out bfloat16; one build per (dim, vdim); 64 rows of a
-    request and one head per block, single tokens as tiles of one row (left out with include_single=False)."""
+    request and one head per block, single tokens as tiles of one row (left out with include_single=False).  Prompts of
+    layers that `sink_rows_takes` go to tcgen05 in tiles of 128 rows."""
     _require_cuda(q, out, cache, block_table, bucket_of, rel, sink, gate)
     if q.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
         raise KernelError("sink_attention_tc: q, cache and out must be bfloat16")
+    if sink_rows_takes(dim, vdim, window, keep_first, cap, rel, chunk, page_size) and _sink_rows_pay(step, include_single) \
+            and cache.is_contiguous() and _ld(q) % 8 == 0 and _ld(out) % 8 == 0 \
+            and (q.data_ptr() | out.data_ptr() | cache.data_ptr()) % 16 == 0:
+        sink_attention_rows(q, out, cache, block_table, step, heads, kv_heads, dim, scale, sink, page_size, include_single, gate)
+        return
     name, defines = sink_tc_library(dim, vdim)
     fn = _fn(name, "fl_sink_attention_tc", [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_int, c_void_p, c_int,
                                             c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,

@@ -172,13 +172,17 @@ class NormedAttention(ProjectedMixer):
     def native_builds(self):
         """(library, defines) pairs compiled for this part's sizes, so that a model's first load builds them beside
         its other libraries."""
-        return [ops.sink_tc_library(self.dim, self.vdim)] if self._tc() else []
+        if not self._tc():
+            return []
+        rows = ops.sink_rows_takes(self.dim, self.vdim, self.window, 0, None, None, self.chunk, self.ctx.page_size)
+        return [ops.sink_tc_library(self.dim, self.vdim)] + ([("attention_prefill_tc", {"HEAD_DIM": self.dim})] if rows else [])
 
     def reserve(self, limits):
         super().reserve(limits)
         if self._tc():
             from ..native.build import load_library
-            load_library(*ops.sink_tc_library(self.dim, self.vdim))        # built now, not inside the first step
+            for library in self.native_builds():
+                load_library(*library)                        # built now, not inside the first step
         if self.ctx.device.type == "cuda" and self._splits_single_tokens():
             longest = -(-limits.max_model_len // 1024) * 1024
             self._partials(min(limits.max_tokens, limits.max_requests),

@@ -70,3 +70,40 @@ def test_delta_scan_that_looks_ahead(lens, dim, vdim):
         errors.append((float((got.double() - want).abs().max()), float((state.double() - want_state).abs().max())))
     assert errors[1][0] <= 2 * errors[0][0] + 1e-6 and errors[1][1] <= 2 * errors[0][1] + 1e-6, errors
     assert errors[1][0] < 1e-4 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("size,heads,kv_heads,page", [(128, 4, 1, 16), (64, 6, 3, 8), (128, 2, 2, 128)])
+@pytest.mark.parametrize("gate,sink", [(None, False), ("head", True), ("channel", False)])
+def test_prompt_attention_over_rows_of_keys_and_values(size, heads, kv_heads, page, gate, sink):
+    """tcgen05 tiles against the CUDA-core kernel (both round a row's result to bfloat16 once, tcgen05 the weights too: 2^-8 of
+    the values' size each); what the last page holds behind a prompt's last token is not finite."""
+    torch.manual_seed(size + heads)
+    ctx, lens = [0, 130, 5, 1, 0], [300, 129, 1, 64, 2]
+    per = [-(-(c + m) // page) for c, m in zip(ctx, lens)]
+    cache = torch.randn(sum(per), kv_heads, page, 2 * size, device="cuda").to(torch.bfloat16)
+    bt = torch.zeros(len(lens), max(per), dtype=torch.int32, device="cuda")
+    for r, n in enumerate(per):
+        bt[r, :n] = torch.arange(sum(per[:r]), sum(per[:r]) + n)
+        rest = n * page - ctx[r] - lens[r]
+        if rest:
+            cache[int(bt[r, n - 1]), :, page - rest:, size:] = float("inf")
+            cache[int(bt[r, n - 1]), :, page - rest:, :size] = float("nan")
+    starts = [sum(lens[:r]) for r in range(len(lens) + 1)]
+    n = starts[-1]
+    step = SimpleNamespace(req_start=i32(starts), req_ctx=i32(ctx), req_qlen=i32(lens), n_requests=len(lens), q_lens=lens)
+    tok_req = i32([r for r, m in enumerate(lens) for _ in range(m)])
+    positions = i32([c + i for c, m in zip(ctx, lens) for i in range(m)])
+    q = torch.randn(n, heads * size, device="cuda").to(torch.bfloat16)
+    g = None if gate is None else torch.randn(n, heads if gate == "head" else heads * size, device="cuda").to(torch.bfloat16)
+    s = torch.randn(heads, device="cuda") if sink else None
+    want, got = torch.empty_like(q), torch.zeros_like(q)
+    ops.sink_attention_simt(q, want, cache, bt, tok_req, positions, heads, kv_heads, size, size, None, 0, size ** -0.5, None, None,
+                            None, s, page, gate=g)
+    assert ops.sink_rows_takes(size, size, None, 0, None, None, None, page)
+    ops.sink_attention_rows(q, got, cache, bt, step, heads, kv_heads, size, size ** -0.5, s, page, True, g)
+    assert bool(got.isfinite().all())
+    assert float((got.float() - want.float()).abs().max()) <= 2 ** -6 * float(want.float().abs().max())
+    alone = torch.zeros_like(q)
+    ops.sink_attention_rows(q, alone, cache, bt, step, heads, kv_heads, size, size ** -0.5, s, page, False, g)
+    single = starts[2]
+    assert not bool(alone[single].any()) and torch.equal(alone[:single], got[:single]) and torch.equal(alone[single + 1:], got[single + 1:])
