@@ -184,13 +184,7 @@ __global__ void delta_tail_kernel(const T* __restrict__ proj, long ld, float* __
 // time at the barrier behind the two warps that fetched) and one multiply-add an element.
 // Registers are kept to what lets two blocks of 32 columns share an SM: several requests' prompts bring more blocks than SMs
 // (8 x 100 tokens, 16 heads of 128 x 128: 121 us with one block an SM, 96 with two).
-//
-// AHEAD (16-bit models; a 32-bit one wants the same bits however a prompt is cut, and a portion's first token has nothing to
-// look ahead from): with S the state before token t, the next token's sum is S_(t+1)^T k_(t+1) = g_t S^T k_(t+1) +
-// (k_t . k_(t+1)) u_t, so the sum over S can be made while u_t is not known yet.  A token's iteration makes the sums of the
-// token after the next one, whose way across the lanes is then over long before they are wanted, and between u_t and u_(t+1)
-// lie two multiply-adds.  What bounds it then are the reads of k and q from shared memory (8 x 512 bytes a warp and token).
-template <bool AHEAD> struct DeltaChunk { static constexpr int TOKENS = AHEAD ? 18 : 16; };     // (six tokens a turn of the unrolled loop)
+#define DELTA_CHUNK 16
 
 __device__ __forceinline__ void delta_cp16(float* smem, const float* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -218,19 +212,18 @@ __device__ __forceinline__ float2 delta_mul2(const float2 a, const float2 b) {
     return d;
 }
 
-template <int DPT, int COLS, bool AHEAD>
-__global__ void __launch_bounds__(COLS * DELTA_PARTS + 32, COLS == 32 && DPT <= 16 && !AHEAD ? 2 : 1) delta_scan_kernel(
+template <int DPT, int COLS>
+__global__ void __launch_bounds__(COLS * DELTA_PARTS + 32, COLS == 32 && DPT <= 16 ? 2 : 1) delta_scan_kernel(
     float* __restrict__ work, long work_ld, float* __restrict__ state, long state_stride,
     const int* __restrict__ req_start, const int* __restrict__ req_ctx, const int* __restrict__ req_qlen,
     const int* __restrict__ req_slot, int heads, int kv_heads, int dim, int vdim) {
     static_assert(DPT % 4 == 0, "a thread's elements are fetched four at a time");
     pdl_wait();
     pdl_trigger();
-    constexpr int DELTA_CHUNK = DeltaChunk<AHEAD>::TOKENS;
     constexpr int THREADS = COLS * DELTA_PARTS;              // ... that walk the recurrence; 32 more fetch
     constexpr int PART = DPT + 4;                            // floats between parts
     constexpr int KQ = DELTA_PARTS * PART;                   // k (and q) of one token
-    constexpr int PER_TOKEN = 2 * KQ + COLS + 4;             // k | q | v COLS | beta | decay | q . k | k . k before it
+    constexpr int PER_TOKEN = 2 * KQ + COLS + 4;             // k | q | v COLS | beta | decay | q . k | pad
     extern __shared__ __align__(16) float delta_in[];        // [2][DELTA_CHUNK][PER_TOKEN]
     const int r = blockIdx.x / heads, h = blockIdx.x % heads;
     const int g = h / (heads / kv_heads);
@@ -312,26 +305,6 @@ __global__ void __launch_bounds__(COLS * DELTA_PARTS + 32, COLS == 32 && DPT <= 
 #pragma unroll
             for (int o = 1; o < DELTA_PARTS; o <<= 1) qk += __shfl_xor_sync(0xffffffffu, qk, o);
             if (part == 0 && n < n_tok) tok[2 * KQ + COLS + 2] = qk;
-            if constexpr (AHEAD) {                           // (the chunk before is being consumed, and not yet overwritten)
-                const int m = min(n, n_tok - 1);
-                const float* before = m > 0 ? tok - PER_TOKEN : delta_in + ((long)(buf ^ 1) * DELTA_CHUNK + DELTA_CHUNK - 1) * PER_TOKEN;
-                float d[2] = {0.0f, 0.0f};
-                if (m > 0 || first > 0) {
-#pragma unroll
-                    for (int i = 0; i < DPT; i += 4) {
-                        const float4 kv = *reinterpret_cast<const float4*>(tok + part * PART + i);
-                        const float4 bv = *reinterpret_cast<const float4*>(before + part * PART + i);
-                        d[0] = fmaf(bv.x, kv.x, d[0]);
-                        d[1] = fmaf(bv.y, kv.y, d[1]);
-                        d[0] = fmaf(bv.z, kv.z, d[0]);
-                        d[1] = fmaf(bv.w, kv.w, d[1]);
-                    }
-                }
-                float kk = d[0] + d[1];
-#pragma unroll
-                for (int o = 1; o < DELTA_PARTS; o <<= 1) kk += __shfl_xor_sync(0xffffffffu, kk, o);
-                if (part == 0 && n < n_tok) tok[2 * KQ + COLS + 3] = kk;
-            }
         }
     };
     if (fetches) {
@@ -355,68 +328,6 @@ __global__ void __launch_bounds__(COLS * DELTA_PARTS + 32, COLS == 32 && DPT <= 
         else S[i / 2].x = v;
     }
     float* o_tok = work + (long)start * work_ld + 2 * qk_cols + hv + 2 * heads + h * vdim + j;
-    if constexpr (AHEAD) {
-        // Of the token whose turn it is (0), the next (1) and the one that is looked at (2, just read): k, v, and beta, decay,
-        // q . k and k . k; p: S^T k with the state before the token before it; b: S^T q with the state before the token itself.
-        // Two tokens before the first leave the state as it is (beta 0, decay 1).
-        float2 k0[DPT / 2], k1[DPT / 2], q1[DPT / 2];
-#pragma unroll
-        for (int i = 0; i < DPT / 2; ++i) k0[i] = k1[i] = q1[i] = make_float2(0.0f, 0.0f);
-        float4 s0 = make_float4(0.0f, 1.0f, 0.0f, 0.0f), s1 = s0;
-        float v0 = 0.0f, v1 = 0.0f, p0 = 0.0f, p1 = 0.0f, b = 0.0f, u = 0.0f, decay = 1.0f;
-        int t = -2;                                          // the token whose turn it is
-        auto turn = [&](const float2 (&k2)[DPT / 2], const float2 (&q2)[DPT / 2], float v2, const float4 s2) {
-            u = s0.x * fmaf(-s0.y, fmaf(decay, p0, s0.w * u), v0);
-            decay = s0.y;
-            const float2 decay2 = make_float2(decay, decay), u2 = make_float2(u, u);
-            float2 x = make_float2(0.0f, 0.0f), y = make_float2(0.0f, 0.0f);
-#pragma unroll
-            for (int i = 0; i < DPT / 2; ++i) {
-                S[i] = delta_fma2(k0[i], u2, delta_mul2(decay2, S[i]));
-                x = delta_fma2(S[i], k2[i], x);
-                y = delta_fma2(S[i], q1[i], y);
-            }
-            float p2 = x.x + x.y, b1 = y.x + y.y;
-#pragma unroll
-            for (int o = 1; o < DELTA_PARTS; o <<= 1) {
-                p2 += __shfl_xor_sync(0xffffffffu, p2, o);
-                b1 += __shfl_xor_sync(0xffffffffu, b1, o);
-            }
-            if (t >= 0) {
-                if (live && part == 0) *o_tok = fmaf(decay, b, s0.z * u);
-                o_tok += work_ld;
-            }
-            ++t;
-#pragma unroll
-            for (int i = 0; i < DPT / 2; ++i) k0[i] = k1[i], k1[i] = k2[i], q1[i] = q2[i];
-            s0 = s1, s1 = s2, v0 = v1, v1 = v2, p0 = p1, p1 = p2, b = b1;
-        };
-        for (int first = 0, buf = 0; first < qlen; first += DELTA_CHUNK, buf ^= 1) {
-            __syncthreads();
-            const float* in = delta_in + (long)buf * DELTA_CHUNK * PER_TOKEN;
-            const int n_tok = min(DELTA_CHUNK, qlen - first);
-#pragma unroll 6
-            for (int n = 0; n < n_tok; ++n, in += PER_TOKEN) {
-                float2 k2[DPT / 2], q2[DPT / 2];
-#pragma unroll
-                for (int i = 0; i < DPT / 4; ++i) {
-                    const float4 kv = *reinterpret_cast<const float4*>(in + part * PART + 4 * i);
-                    const float4 qv = *reinterpret_cast<const float4*>(in + KQ + part * PART + 4 * i);
-                    k2[2 * i] = make_float2(kv.x, kv.y), k2[2 * i + 1] = make_float2(kv.z, kv.w);
-                    q2[2 * i] = make_float2(qv.x, qv.y), q2[2 * i + 1] = make_float2(qv.z, qv.w);
-                }
-                turn(k2, q2, in[2 * KQ + col], *reinterpret_cast<const float4*>(in + 2 * KQ + COLS));
-            }
-        }
-        float2 none[DPT / 2];
-#pragma unroll
-        for (int i = 0; i < DPT / 2; ++i) none[i] = make_float2(0.0f, 0.0f);
-        const float4 still = make_float4(0.0f, 1.0f, 0.0f, 0.0f);
-        if (qlen > 0) {
-            turn(none, none, 0.0f, still);
-            turn(none, none, 0.0f, still);
-        }
-    } else
     for (int first = 0, buf = 0; first < qlen; first += DELTA_CHUNK, buf ^= 1) {
         __syncthreads();
         const float* in = delta_in + (long)buf * DELTA_CHUNK * PER_TOKEN;
@@ -619,33 +530,31 @@ FL_API int fl_delta_prep(const void* proj, int dtype, long ld, const void* conv_
     return 0;
 }
 
-// ahead: the form that looks ahead of the token whose turn it is (results depend in their last bits on where a prompt is cut).
 // single_tokens: the step has as many tokens as requests, one each as a rule (a kernel of its own).
 // work: [n_tokens, work_ld] floats, a row = q | k (kv_heads x dim each) | v (heads x vdim) | beta | decay (heads
 // each) | o (heads x vdim): fl_delta_prep fills all but o, fl_delta_scan reads them and fills o.
 FL_API int fl_delta_scan(float* work, long work_ld, float* state, long state_stride,
                          const int* req_start, const int* req_ctx, const int* req_qlen, const int* req_slot,
-                         int n_requests, int heads, int kv_heads, int dim, int vdim, int single_tokens, int ahead,
-                         cudaStream_t stream) {
+                         int n_requests, int heads, int kv_heads, int dim, int vdim, int single_tokens, cudaStream_t stream) {
     if (n_requests <= 0) return 0;
     if (heads % kv_heads || dim < 1 || dim > 32 * DELTA_PARTS) return (int)cudaErrorInvalidValue;
     const int per_thread = (dim + DELTA_PARTS - 1) / DELTA_PARTS;
     // a block takes 32 value columns, or 16 when blocks of 32 would leave most of the GPU idle (a lone
     // request's prompt): the recurrence is a chain per token, so what counts is how many SMs walk it
-    const bool narrow = ahead || ((long)n_requests * heads * ((vdim + 31) / 32) < 96 && vdim > 16);
+    const bool narrow = (long)n_requests * heads * ((vdim + 31) / 32) < 96 && vdim > 16;
     const int cols = narrow ? 16 : DELTA_COLS;
     dim3 grid(n_requests * heads, (vdim + cols - 1) / cols);
     if (grid.y > 65535) return (int)cudaErrorInvalidValue;
-#define FL_DELTA_SCAN_COLS(DPT, COLS, AHEAD)                                                                        \
+#define FL_DELTA_SCAN_COLS(DPT, COLS)                                                                               \
     {                                                                                                               \
-        const size_t smem = (size_t)2 * DeltaChunk<AHEAD>::TOKENS * (2 * DELTA_PARTS * (DPT + 4) + COLS + 4) * sizeof(float); \
+        const size_t smem = (size_t)2 * DELTA_CHUNK * (2 * DELTA_PARTS * (DPT + 4) + COLS + 4) * sizeof(float);     \
         static bool raised = false;                                                                                 \
         if (smem > 48 * 1024 && !raised) {                                                                          \
-            const cudaError_t rc = cudaFuncSetAttribute(delta_scan_kernel<DPT, COLS, AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            const cudaError_t rc = cudaFuncSetAttribute(delta_scan_kernel<DPT, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
             if (rc != cudaSuccess) return (int)rc;                                                                  \
             raised = true;                                                                                          \
         }                                                                                                           \
-        return fl_launch(delta_scan_kernel<DPT, COLS, AHEAD>, grid, dim3(COLS * DELTA_PARTS + 32), smem, stream, work, work_ld, state, \
+        return fl_launch(delta_scan_kernel<DPT, COLS>, grid, dim3(COLS * DELTA_PARTS + 32), smem, stream, work, work_ld, state, \
                          state_stride, req_start, req_ctx, req_qlen, req_slot, heads, kv_heads, dim, vdim);         \
     }
 #define FL_DELTA_SCAN(DPT)                                                                                          \
@@ -653,8 +562,7 @@ FL_API int fl_delta_scan(float* work, long work_ld, float* state, long state_str
         if (single_tokens)                                                                                          \
             return fl_launch(delta_step_kernel<DPT>, dim3(grid.x, (vdim + DELTA_COLS - 1) / DELTA_COLS), dim3(DELTA_COLS * DELTA_PARTS), 0, \
                              stream, work, work_ld, state, state_stride, req_start, req_ctx, req_qlen, req_slot, heads, kv_heads, dim, vdim); \
-        if (ahead) FL_DELTA_SCAN_COLS(DPT, 16, true)                                                                \
-        if (narrow) FL_DELTA_SCAN_COLS(DPT, 16, false) else FL_DELTA_SCAN_COLS(DPT, 32, false)                      \
+        if (narrow) FL_DELTA_SCAN_COLS(DPT, 16) else FL_DELTA_SCAN_COLS(DPT, 32)                                    \
     }
     FL_DELTA_SCAN(4);
     FL_DELTA_SCAN(8);

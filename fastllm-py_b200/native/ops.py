@@ -529,17 +529,15 @@ def delta_prep(proj, conv_w, a_log, dt_bias, state, tail_off, step, work, heads,
               _stream()), "delta_prep", 1 if taps == 1 else 2)
 
 
-def delta_scan(work, state, step, heads, kv_heads, dim, vdim, ahead=False):
+def delta_scan(work, state, step, heads, kv_heads, dim, vdim):
     """The recurrence over each request's tokens of the step; state rows are read (unless the request
-    starts) and written; the o columns of `work` are filled.  `ahead`: by the faster kernel for prompts, whose results depend
-    in their last bits on where a prompt was cut into steps."""
+    starts) and written; the o columns of `work` are filled."""
     _require_cuda(work, state)
     fn = _fn("delta_rule", "fl_delta_scan", [c_void_p, c_long, c_void_p, c_long, c_void_p, c_void_p,
-                                             c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                                             c_void_p])
+                                             c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p])
     _check(fn(_ptr(work), _ld(work), _ptr(state), state.stride(0), _ptr(step.req_start), _ptr(step.req_ctx),
               _ptr(step.req_qlen), _ptr(step.req_slot), step.n_requests, heads, kv_heads, dim, vdim,
-              int(work.shape[0] == step.n_requests), int(ahead), _stream()), "delta_scan")
+              int(work.shape[0] == step.n_requests), _stream()), "delta_scan")
 
 
 def delta_gated_norm(work, o_col, proj, gate_col, weight, out, heads, vdim, eps):

@@ -93,7 +93,7 @@ class GatedDelta(Part):
         work = ws.rows("delta_work", n, self.work_cols, torch.float32)
         ops.delta_prep(proj, self.conv, self.a_log, self.dt_bias, cache.tensor, self.state_floats, step, work,
                        self.heads, self.kv_heads, self.dim, self.vdim, self.taps, self.unit_eps, self.q_scale)
-        ops.delta_scan(work, cache.tensor, step, self.heads, self.kv_heads, self.dim, self.vdim, ahead=dt == torch.bfloat16)
+        ops.delta_scan(work, cache.tensor, step, self.heads, self.kv_heads, self.dim, self.vdim)
         y = ws.rows("delta_y", n, self.hv, dt)
         ops.delta_gated_norm(work, self.work_cols - self.hv, proj, self.channels, self.norm, y, self.heads,
                              self.vdim, self.norm_eps)
