@@ -6,7 +6,10 @@
 // rows x 128 columns (32 where there are no more than 64 rows: a step of few tokens is bound by the way of W's rows through
 // a few blocks, and the more blocks share it the better) of one batch entry, K in steps of 32 through a cp.async ring of 3
 // (6) stages with one barrier a step.  The tile leaves by way of shared memory, 16 bytes a thread and whole rows of it side by
-// side where C's rows allow: element by element the stores of 2048 rows x 16 x 512 columns took most of the time.
+// side where C's rows allow: element by element the stores of 2048 rows x 16 x 512 columns took most of the time.  Bound by its stores (33 MB), else by
+// one block's serial way through K: 16 products of K = 128 and N = 512 took 3.5 us for 4 rows, 17.2 for 300 and 55.7 for 2048
+// in blocks of 64 x 64 and a ring of 3 stages, and take 2.5, 6.0 and 23.7; of K = 512 and N = 128 8.1, 11.6 and 33.6, now 4.2,
+// 7.7 and 22.2.
 // With `gate` (laid out like C: gate + b * g_batch, ldg between rows) the epilogue writes C * sigmoid(gate): the
 // product is rounded to C's type first, as a gate applied by a kernel of its own would have read it.
 // K must be a multiple of 32 and every A row 16-byte aligned; other shapes go to gemm_simt's batched form.
@@ -24,9 +27,11 @@ template <int BN> struct GmTile {
     static constexpr int BYTES = STAGES * STAGE * 2 > GM_BM * OUT_PITCH * 4 ? STAGES * STAGE * 2 : GM_BM * OUT_PITCH * 4;
 };
 
-__device__ __forceinline__ void gm_cp16(void* smem, const void* gmem) {
+// `there` false: zeroes, and nothing is read.  (Rows past M that all read the last row again meet in the same few sectors of
+// L2: 8 rows x 16 heads x 512 columns took 7.1 us, 2.5 with zeroes.)
+__device__ __forceinline__ void gm_cp16(void* smem, const void* gmem, bool there) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(there ? 16 : 0));
 }
 
 // wide: C's rows (and the gate's) are whole and aligned pieces of 16 bytes
@@ -53,10 +58,10 @@ __global__ void __launch_bounds__(256) gemm_mma_batched_kernel(const bf16* __res
     auto stage = [&](int kb) {                                  // (also past the last one: the ring counts groups of copies)
         if (kb < n_k) {
             bf16* dst = ring + kb % L::STAGES * L::STAGE + ar * GM_PITCH + ac;
-            gm_cp16(dst, a_src + kb * GM_BK);
+            gm_cp16(dst, a_src + kb * GM_BK, m0 + ar < M);
 #pragma unroll
             for (int i = 0; i < W_PIECES; ++i)
-                if (BN >= 64 || ar < BN) gm_cp16(dst + (GM_BM + i * 64) * GM_PITCH, w_src[i] + kb * GM_BK);
+                if (BN >= 64 || ar < BN) gm_cp16(dst + (GM_BM + i * 64) * GM_PITCH, w_src[i] + kb * GM_BK, n0 + ar + i * 64 < N);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
