@@ -832,8 +832,24 @@ def sink_tc_library(dim: int, vdim: int):
     return "sink_attention_tc", {"SINK_DIM": dim, "SINK_VDIM": vdim}
 
 
-def _sink_rows_pay(step, include_single: bool) -> bool:
-    return True
+def _sink_rows_pay(step, heads: int, include_single: bool, sms: int) -> bool:
+    """Which of the two prompt kernels is the faster one: tcgen05 takes tiles of 128 tokens, one an SM, at about 7.5 us and 1.5
+    for every 128 keys, the other takes 64 tokens, three an SM, at 5.3 us and 3.4 for every 64 keys.  Many prompts (or
+    portions) of a few tokens go to the other one, as they fill no tile: 20 of 8 tokens with 16 heads take it 16.5 us against
+    28, one of 4 tokens 7.9 against 9.6; the 2048 tokens of one prompt 217 against 38, 64 tokens behind 1500 93 against 27."""
+    tiles = small_tiles = 0
+    keys = small_keys = 0.0                                   # that the tiles go through, in blocks of 128 (of 64)
+    for q, ctx in zip(getattr(step, "q_lens", ()), getattr(step, "ctx_lens", ())):
+        if q == 1 and not include_single:
+            continue
+        n, m = -(-q // 128), -(-q // 64)
+        tiles, small_tiles = tiles + n, small_tiles + m
+        keys += n * (ctx / 128 + (n + 1) / 2)
+        small_keys += m * (ctx / 64 + (m + 1) / 2)
+    if not tiles:
+        return True                                           # (a step built by hand, without its lengths)
+    return -(-tiles * heads // sms) * (7.5 + 1.5 * keys / tiles) < \
+        -(-small_tiles * heads // (3 * sms)) * (5.3 + 3.4 * small_keys / small_tiles)
 
 
 def sink_rows_takes(dim: int, vdim: int, window, keep_first, cap, rel, chunk, page_size: int) -> bool:
@@ -865,9 +881,9 @@ def sink_attention_tc(q, out, cache, block_table, step, heads, kv_heads, dim, vd
     _require_cuda(q, out, cache, block_table, bucket_of, rel, sink, gate)
     if q.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
         raise KernelError("sink_attention_tc: q, cache and out must be bfloat16")
-    if sink_rows_takes(dim, vdim, window, keep_first, cap, rel, chunk, page_size) and _sink_rows_pay(step, include_single) \
-            and cache.is_contiguous() and _ld(q) % 8 == 0 and _ld(out) % 8 == 0 \
-            and (q.data_ptr() | out.data_ptr() | cache.data_ptr()) % 16 == 0:
+    if sink_rows_takes(dim, vdim, window, keep_first, cap, rel, chunk, page_size) and cache.is_contiguous() \
+            and _ld(q) % 8 == 0 and _ld(out) % 8 == 0 and (q.data_ptr() | out.data_ptr() | cache.data_ptr()) % 16 == 0 \
+            and _sink_rows_pay(step, heads, include_single, sm_count(q.device)):
         sink_attention_rows(q, out, cache, block_table, step, heads, kv_heads, dim, scale, sink, page_size, include_single, gate)
         return
     name, defines = sink_tc_library(dim, vdim)
