@@ -543,20 +543,64 @@ FL_API int fl_glu(const void* gu, int dtype, long gu_ld, void* out, long out_ld,
 //
 // One CTA a row; a thread's KEEP chunks of four neighbouring elements stay in registers, and all their loads (the slabs or
 // y, x, both weights) are issued before the first reduction, so a row costs one round trip to memory and two reductions, and
-// nothing is read twice.  Threads and chunks follow from the row's length alone, and a chunk that 16-byte loads cannot read
-// (VEC false) is taken an element at a time, so equal rows give equal sums in every form.  (2048 rows of 2048: 18.4 us an
-// element at a time with the row in shared memory, 9.0 so, of 6.4 us of bytes out of memory; 8 rows of 9 slabs 6.2 and 3.5.)
-template <bool PARTIAL, typename TD, typename TW, typename TO, int KEEP, bool VEC>
-__global__ void __launch_bounds__(1024) sandwich_norm_kernel(
+// nothing is read twice.  A chunk that 16-byte loads cannot read (VEC false) is taken an element at a time; every form sums
+// the squares in one order: element i belongs to chain i mod 512 of up to 512, a chain goes from its first element to its
+// last, and the chains are added as a block's threads are (32 by 32, then the groups).  A thread holds four chains, 128 of
+// them all; of a row that is too long for one thread's registers (over 4096), blocks of 128 threads take 2048 elements each and
+// hand the chains on (WIDE).  2048 rows of 2048 take 9.0 us (6.4 us of bytes out of
+// memory; an element at a time with the row in shared memory 18.4), 8 rows of 9 slabs 3.8 (6.1).
+#define SAND_CHAINS 512
+#define SAND_LONGEST 12256               // elements of a row
+template <bool PARTIAL, typename TD, typename TW, typename TO, int KEEP, bool VEC, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? 768 : SAND_CHAINS / 4) sandwich_norm_kernel(
     float* __restrict__ x, long x_ld, const void* __restrict__ y, long y_ld, int splits, long split_stride,
     const TW* __restrict__ w_post, float eps_post, const TW* __restrict__ w_pre, float eps_pre, TO* __restrict__ out,
     long out_ld, int dim, const int* __restrict__ rows, int write_back) {
     pdl_wait();
     pdl_trigger();
-    __shared__ float scratch[32];
-    const int r = blockIdx.x;
+    __shared__ float scratch[SAND_CHAINS / 32];
+    __shared__ float4 carry[WIDE ? SAND_CHAINS / 4 : 1];
+    const int r = blockIdx.x, lane = threadIdx.x & 31, part = WIDE ? threadIdx.x / (SAND_CHAINS / 4) : 0;
+    const int own = threadIdx.x % (SAND_CHAINS / 4), i0 = own * 4 + part * KEEP * SAND_CHAINS;
     const long src = rows ? (long)rows[r] : (long)r;
     float* xr = x + src * x_ld;
+    auto squares = [&](const float4 (&v)[KEEP]) {
+        float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        auto chain = [&] {
+#pragma unroll
+            for (int c = 0; c < KEEP; ++c)
+                if (i0 + c * SAND_CHAINS < dim) {
+                    s.x = fmaf(v[c].x, v[c].x, s.x);
+                    s.y = fmaf(v[c].y, v[c].y, s.y);
+                    s.z = fmaf(v[c].z, v[c].z, s.z);
+                    s.w = fmaf(v[c].w, v[c].w, s.w);
+                }
+        };
+        if constexpr (WIDE) {
+            for (int p = 0; p < (int)blockDim.x / (SAND_CHAINS / 4); ++p) {
+                if (p == part) {
+                    if (p > 0) s = carry[own];
+                    chain();
+                    carry[own] = s;
+                }
+                __syncthreads();
+            }
+            s = carry[own];
+        } else {
+            chain();
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+            s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+            s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+            s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
+            s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
+        }
+        __syncthreads();                                // scratch may still be read from the call before
+        if ((lane & 7) == 0 && part == 0) scratch[own / 8] = (s.x + s.z) + (s.y + s.w);
+        __syncthreads();
+        return warp_sum(lane < min((int)blockDim.x, SAND_CHAINS / 4) / 8 ? scratch[lane] : 0.0f);
+    };
     auto get = [&](const auto* p, int i, float4& v) {
         if constexpr (VEC) {
             load4(p + i, v);
@@ -579,39 +623,44 @@ __global__ void __launch_bounds__(1024) sandwich_norm_kernel(
             if (i + 3 < dim) p[i + 3] = from_f32<T>(v.w);
         }
     };
-    const int step = blockDim.x * 4;
     float4 sub[KEEP], sum[KEEP], post[KEEP], pre[KEEP];
-    float ss = 0.0f;
 #pragma unroll
     for (int c = 0; c < KEEP; ++c) {
-        const int i = threadIdx.x * 4 + c * step;
+        const int i = i0 + c * SAND_CHAINS;
+        sub[c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (i < dim) {
             get(xr, i, sum[c]);
             get(w_post, i, post[c]);
             if (out != nullptr) get(w_pre, i, pre[c]);
-            if constexpr (PARTIAL) {
-                const float* pr = static_cast<const float*>(y) + src * y_ld;
-                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll 8
-                for (int z = 0; z < splits; ++z) {
-                    float4 q;
-                    get(pr + (long)z * split_stride, i, q);
-                    v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
-                }
-                sub[c] = make_float4(to_f32<TO>(from_f32<TO>(v.x)), to_f32<TO>(from_f32<TO>(v.y)), to_f32<TO>(from_f32<TO>(v.z)),
-                                     to_f32<TO>(from_f32<TO>(v.w)));
-            } else {
-                get(static_cast<const TD*>(y) + src * y_ld, i, sub[c]);
-            }
-            ss += sub[c].x * sub[c].x + sub[c].y * sub[c].y + sub[c].z * sub[c].z + sub[c].w * sub[c].w;
+            if constexpr (!PARTIAL) get(static_cast<const TD*>(y) + src * y_ld, i, sub[c]);
         }
     }
-    ss = block_sum(ss, scratch);
-    const float inv_post = 1.0f / sqrtf(ss / (float)dim + eps_post);
-    ss = 0.0f;
+    if constexpr (PARTIAL) {
+        const float* pr = static_cast<const float*>(y) + src * y_ld;
+        constexpr int BATCH = WIDE ? 1 : KEEP >= 8 ? 2 : KEEP == 4 ? 5 : 10;      // slabs on their way at once
+        for (int z0 = 0; z0 < splits; z0 += BATCH) {
+            float4 q[BATCH][KEEP];
+#pragma unroll
+            for (int b = 0; b < BATCH; ++b)
+#pragma unroll
+                for (int c = 0; c < KEEP; ++c)
+                    if (z0 + b < splits && i0 + c * SAND_CHAINS < dim) get(pr + (long)(z0 + b) * split_stride, i0 + c * SAND_CHAINS, q[b][c]);
+#pragma unroll
+            for (int b = 0; b < BATCH; ++b)
+#pragma unroll
+                for (int c = 0; c < KEEP; ++c)
+                    if (z0 + b < splits && i0 + c * SAND_CHAINS < dim)
+                        sub[c].x += q[b][c].x, sub[c].y += q[b][c].y, sub[c].z += q[b][c].z, sub[c].w += q[b][c].w;
+        }
+#pragma unroll
+        for (int c = 0; c < KEEP; ++c)
+            sub[c] = make_float4(to_f32<TO>(from_f32<TO>(sub[c].x)), to_f32<TO>(from_f32<TO>(sub[c].y)),
+                                 to_f32<TO>(from_f32<TO>(sub[c].z)), to_f32<TO>(from_f32<TO>(sub[c].w)));
+    }
+    const float inv_post = 1.0f / sqrtf(squares(sub) / (float)dim + eps_post);
 #pragma unroll
     for (int c = 0; c < KEEP; ++c) {
-        const int i = threadIdx.x * 4 + c * step;
+        const int i = i0 + c * SAND_CHAINS;
         if (i < dim) {
             float4& v = sum[c];
             v.x += sub[c].x * inv_post * post[c].x;
@@ -619,23 +668,20 @@ __global__ void __launch_bounds__(1024) sandwich_norm_kernel(
             v.z += sub[c].z * inv_post * post[c].z;
             v.w += sub[c].w * inv_post * post[c].w;
             if (write_back) put(xr, i, v);
-            ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
         }
     }
     if (out == nullptr) return;
-    ss = block_sum(ss, scratch);
-    const float inv_pre = 1.0f / sqrtf(ss / (float)dim + eps_pre);
+    const float inv_pre = 1.0f / sqrtf(squares(sum) / (float)dim + eps_pre);
     TO* o = out + (long)r * out_ld;
 #pragma unroll
     for (int c = 0; c < KEEP; ++c) {
-        const int i = threadIdx.x * 4 + c * step;
+        const int i = i0 + c * SAND_CHAINS;
         if (i < dim)
             put(o, i, make_float4(sum[c].x * inv_pre * pre[c].x, sum[c].y * inv_pre * pre[c].y, sum[c].z * inv_pre * pre[c].z,
                                   sum[c].w * inv_pre * pre[c].w));
     }
 }
 
-// 256 threads a row (many rows share an SM) up to 4096 elements, then as many as four chunks a thread need.
 template <bool PARTIAL, typename TD, typename TW, typename TO>
 static int sandwich_launch(float* x, long x_ld, const void* y, long y_ld, int splits, long split_stride, const void* w_post,
                            float eps_post, const void* w_pre, float eps_pre, void* out, long out_ld, int n_rows, int dim,
@@ -643,22 +689,30 @@ static int sandwich_launch(float* x, long x_ld, const void* y, long y_ld, int sp
     const bool vec = vec4_ok(dim, x, x_ld, 4) && vec4_ok(dim, y, y_ld, PARTIAL ? 4 : sizeof(TD)) && split_stride % 4 == 0 &&
                      vec4_ok(dim, w_post, 4, sizeof(TW)) &&
                      (out == nullptr || (vec4_ok(dim, w_pre, 4, sizeof(TW)) && vec4_ok(dim, out, out_ld, sizeof(TO))));
-    const int chunks = (dim + 3) / 4;
-    const int threads = chunks <= 256 ? (chunks + 31) / 32 * 32 : chunks <= 1024 ? 256 : chunks <= 2048 ? 512 : 1024;
-#define FL_SANDWICH(KEEP, VEC)                                                                                                       \
-    return fl_launch(sandwich_norm_kernel<PARTIAL, TD, TW, TO, KEEP, VEC>, dim3(n_rows), dim3(threads), 0, stream, x, x_ld, y, y_ld, \
-                     splits, split_stride, (const TW*)w_post, eps_post, (const TW*)w_pre, eps_pre, (TO*)out, out_ld, dim, rows,      \
-                     rows ? 0 : 1)
-    if (chunks <= threads) {
-        if (vec) FL_SANDWICH(1, true);
-        FL_SANDWICH(1, false);
+    const int chunks = (dim + SAND_CHAINS - 1) / SAND_CHAINS;           // a thread's
+    const int threads = chunks > 8 ? SAND_CHAINS / 4 * ((chunks + 3) / 4) : chunks > 1 ? SAND_CHAINS / 4 : (dim + 127) / 128 * 32;
+#define FL_SANDWICH(KEEP, VEC, WIDE)                                                                                                \
+    return fl_launch(sandwich_norm_kernel<PARTIAL, TD, TW, TO, KEEP, VEC, WIDE>, dim3(n_rows), dim3(threads), 0, stream, x, x_ld, y, \
+                     y_ld, splits, split_stride, (const TW*)w_post, eps_post, (const TW*)w_pre, eps_pre, (TO*)out, out_ld, dim,     \
+                     rows, rows ? 0 : 1)
+    if (chunks <= 1) {
+        if (vec) FL_SANDWICH(1, true, false);
+        FL_SANDWICH(1, false, false);
     }
-    if (chunks <= 2 * threads) {
-        if (vec) FL_SANDWICH(2, true);
-        FL_SANDWICH(2, false);
+    if (chunks <= 2) {
+        if (vec) FL_SANDWICH(2, true, false);
+        FL_SANDWICH(2, false, false);
     }
-    if (vec) FL_SANDWICH(4, true);
-    FL_SANDWICH(4, false);
+    if (chunks <= 4) {
+        if (vec) FL_SANDWICH(4, true, false);
+        FL_SANDWICH(4, false, false);
+    }
+    if (chunks <= 8) {
+        if (vec) FL_SANDWICH(8, true, false);
+        FL_SANDWICH(8, false, false);
+    }
+    if (vec) FL_SANDWICH(4, true, true);
+    FL_SANDWICH(4, false, true);
 #undef FL_SANDWICH
 }
 
@@ -667,7 +721,7 @@ FL_API int fl_sandwich_norm(float* x, long x_ld, const void* y, int y_dtype, lon
                             float eps_post, const void* w_pre, float eps_pre, int w_dtype, void* out, int out_dtype,
                             long out_ld, int n_rows, int dim, const int* rows, cudaStream_t stream) {
     if (n_rows <= 0) return 0;
-    if ((size_t)dim * sizeof(float) > 48 * 1024) return (int)cudaErrorInvalidValue;
+    if (dim > SAND_LONGEST) return (int)cudaErrorInvalidValue;
     FL_DISPATCH(y_dtype, TD, FL_DISPATCH(w_dtype, TW, FL_DISPATCH(out_dtype, TO,
         return (sandwich_launch<false, TD, TW, TO>(x, x_ld, y, y_ld, 0, 0, w_post, eps_post, w_pre, eps_pre, out, out_ld,
                                                    n_rows, dim, rows, stream)))));
@@ -678,7 +732,7 @@ FL_API int fl_sandwich_norm_partial(float* x, long x_ld, const float* partial, i
                                     const void* w_post, float eps_post, const void* w_pre, float eps_pre, int w_dtype,
                                     void* out, int out_dtype, long out_ld, int n_rows, int dim, cudaStream_t stream) {
     if (n_rows <= 0) return 0;
-    if ((size_t)dim * sizeof(float) > 48 * 1024 || out == nullptr) return (int)cudaErrorInvalidValue;
+    if (dim > SAND_LONGEST || out == nullptr) return (int)cudaErrorInvalidValue;
     FL_DISPATCH(w_dtype, TW, FL_DISPATCH(out_dtype, TO,
         return (sandwich_launch<true, float, TW, TO>(x, x_ld, partial, ld, splits, split_stride, w_post, eps_post, w_pre,
                                                      eps_pre, out, out_ld, n_rows, dim, nullptr, stream))));
