@@ -17,8 +17,8 @@
 //   gemm_f32_tile_kernel    float operands, more rows: bound by the multiply-adds
 //   gemm_simt_kernel        any operand types, alignments and batches
 // The last one served everything before: 350 us a product for 4 rows and 590 us for 300 rows of a layer with 2048 and
-// 5504 columns (10 TFLOP/s); the others take 12 to 37 us (1.4 to 3.4 TB/s of W, out of a cold cache) and 88 to 416 us (29
-// to 32 TFLOP/s, 38 with 32256 features).
+// 5504 columns (10 TFLOP/s); the others take 7 to 25 us (2.3 to 3.7 TB/s of W, out of a cold cache) and 67 to 305 us (37
+// to 44 TFLOP/s).
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -207,17 +207,22 @@ __global__ void __launch_bounds__(64) gemm_f32_skinny_kernel(const float* __rest
 }
 
 // ------------------------------------------------------------ more rows
-// 64 rows x 128 features per CTA of 128 threads, 8 x 8 results a thread (four 16-byte reads of shared memory per 64
-// multiply-adds: with 4 x 8 a thread the reads took longer than the multiply-adds), two CTAs an SM; both operands are
-// turned to [input][row] on their way into shared memory (columns exchanged by a pattern of the input's index, so that
-// neither the turned stores nor the 16-byte reads meet in a bank), the next 16 inputs wait in registers meanwhile.  Bound
-// by the multiply-adds: they are issued in pairs (fma.rn.f32x2, the same rounding), which leaves issue slots for the reads.
-// SPLIT: a cluster of GS_SLICES CTAs shares a tile, each sums one slice, and each adds up an eighth of the rows from the
-// others' shared memory, in the order of the slices; no partial sum goes to global memory.
+// A cluster of GS_SLICES CTAs shares a tile of 64 rows x TL_BN features; each sums one slice, and each adds up an eighth of
+// the rows from the others' shared memory, in the order of the slices, so no partial sum goes to global memory.  Bound by
+// the multiply-adds, which are issued in pairs (fma.rn.f32x2, the same rounding), and by what they read from shared memory
+// (128 bytes a clock reach the registers, however many lanes want the same): 8 rows x 8 features a thread.  Both operands
+// wait in shared memory turned to [input][row], double-buffered; columns are exchanged by a pattern of the input's index, so
+// that neither the turned stores nor the 16-byte reads meet in a bank.  The next stage comes by cp.async into slots that only
+// the copying thread reads, so it needs no registers meanwhile and four CTAs fit an SM.  (300 rows, 11008 features of 2048:
+// 409 us with the next stage in registers, two CTAs an SM and a tile split only where that filled the last wave better; 305
+// now, 44 TFLOP/s.  Every value of A twice in shared memory instead of a move for each pair of features, or 64 x 256 tiles:
+// 347 and 327 us at best.)
 #define TL_BM 64
 #define TL_BN 128
+#define TL_NH (TL_BN / 64)               // groups of four features a thread
 #define TL_BK 16
 #define TL_THREADS 128
+#define TL_SMEM (3 * TL_BK * (TL_BM + TL_BN) > TL_BM * TL_BN ? 12 * TL_BK * (TL_BM + TL_BN) : 4 * TL_BM * TL_BN)
 
 __device__ __forceinline__ void fma2(float2& d, const float2 a, const float2 b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;"
@@ -225,151 +230,115 @@ __device__ __forceinline__ void fma2(float2& d, const float2 a, const float2 b) 
         : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
 }
 
-template <typename TC, bool SPLIT>
-__device__ __forceinline__ void gemm_f32_tile(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw,
-                                              TC* __restrict__ C, long ldc, int M, int N, int K, int slice) {
-    constexpr int STAGE = TL_BK * (TL_BM + TL_BN);
-    __shared__ __align__(16) float smem[SPLIT ? (2 * STAGE > TL_BM * TL_BN ? 2 * STAGE : TL_BM * TL_BN) : 2 * STAGE];
+template <typename TC>
+__global__ void __cluster_dims__(1, 1, GS_SLICES) __launch_bounds__(TL_THREADS, 4)
+    gemm_f32_tile_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw, TC* __restrict__ C,
+                         long ldc, int M, int N, int K, int slice) {
+    constexpr int A_FLOATS = TL_BK * TL_BM, STAGE = A_FLOATS + TL_BK * TL_BN, PIECES = (TL_BM + TL_BN) / 32;
+    extern __shared__ __align__(16) float tl_smem[];                    // two stages and the copies' slots; the tile's sums
+    float4(*raw)[TL_THREADS] = reinterpret_cast<float4(*)[TL_THREADS]>(tl_smem + 2 * STAGE);
+    pdl_wait();
+    pdl_trigger();
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int m0 = blockIdx.y * TL_BM, n0 = blockIdx.x * TL_BN;
-    const int k_begin = SPLIT ? min(K, (int)blockIdx.z * slice) : 0;
-    const int k_end = SPLIT ? min(K, k_begin + slice) : K;
-    // this thread's 16-byte pieces of a stage: rows lr, lr + 32, ... of A (two) and W (four), inputs 4 lk .. 4 lk + 3
+    const int k_begin = min(K, (int)blockIdx.z * slice), k_end = min(K, k_begin + slice);
+    // this thread's 16-byte pieces of a stage: rows lr, lr + 32, ... of A (two) and W, inputs 4 lk .. 4 lk + 3
     const int lr = tid >> 2, lk = tid & 3;
-    const float* src[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i)
-        src[i] = (i < 2 ? A + (long)min(m0 + lr + 32 * i, M - 1) * lda : W + (long)min(n0 + lr + 32 * (i - 2), N - 1) * ldw) + lk * 4;
-    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float4 next[6];
     auto fetch = [&](int k0) {
-        const bool in = k0 + lk * 4 < k_end;
+        const int k = k0 + lk * 4;
+        const bool in = k < k_end;
 #pragma unroll
-        for (int i = 0; i < 6; ++i) next[i] = in ? *reinterpret_cast<const float4*>(src[i] + k0) : zero;
+        for (int i = 0; i < PIECES; ++i) {
+            const int row = i < 2 ? m0 + lr + 32 * i : n0 + lr + 32 * (i - 2);
+            const bool there = in && row < (i < 2 ? M : N);             // else zeroes, and nothing is read
+            const float* src = i < 2 ? A + (long)row * lda : W + (long)row * ldw;
+            sk_cp16(reinterpret_cast<float*>(&raw[i][tid]), there ? src + k : A, there);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto put = [&](int buf) {
+    auto turn = [&](int buf) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        float* a_s = tl_smem + buf * STAGE;
 #pragma unroll
-        for (int i = 0; i < 6; ++i) {
-            constexpr int PA = TL_BM, PW = TL_BN;
-            const int pitch = i < 2 ? PA : PW;
-            float* d = smem + buf * STAGE + (i < 2 ? 0 : TL_BK * TL_BM) + lk * 4 * pitch + ((lr + 32 * (i < 2 ? i : i - 2)) ^ (lk << 3));
-            d[0] = next[i].x, d[pitch] = next[i].y, d[2 * pitch] = next[i].z, d[3 * pitch] = next[i].w;
+        for (int i = 0; i < PIECES; ++i) {
+            const float4 v = raw[i][tid];
+            const int pitch = i < 2 ? TL_BM : TL_BN;
+            float* d = a_s + (i < 2 ? 0 : A_FLOATS) + lk * 4 * pitch + ((lr + 32 * (i < 2 ? i : i - 2)) ^ (lk << 3));
+            d[0] = v.x, d[pitch] = v.y, d[2 * pitch] = v.z, d[3 * pitch] = v.w;
         }
     };
-    float2 acc[8][4], total[SPLIT ? 1 : 8][4];                          // 8 rows x 4 pairs of features
+    float2 acc[8][2 * TL_NH];                                           // 8 rows x pairs of features
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            acc[i][j] = make_float2(0.0f, 0.0f);
-            if (!SPLIT) total[i][j] = make_float2(0.0f, 0.0f);
-        }
+        for (int j = 0; j < 2 * TL_NH; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
     if (k_begin < k_end) {
         fetch(k_begin);
-        put(0);
+        turn(0);
+        if (k_begin + TL_BK < k_end) fetch(k_begin + TL_BK);
     }
     __syncthreads();
-    int buf = 0, left = slice;
+    int buf = 0;
     for (int k0 = k_begin; k0 < k_end; k0 += TL_BK) {
-        const bool more = k0 + TL_BK < k_end;
-        if (more) fetch(k0 + TL_BK);
-        const float* a_s = smem + buf * STAGE;
-        const float* w_s = a_s + TL_BK * TL_BM;
+        if (k0 + TL_BK < k_end) {
+            turn(buf ^ 1);
+            if (k0 + 2 * TL_BK < k_end) fetch(k0 + 2 * TL_BK);          // (its slots have been read: their values are stored)
+        }
+        const float* a_s = tl_smem + buf * STAGE;
+        const float* w_s = a_s + A_FLOATS;
 #pragma unroll
         for (int kk = 0; kk < TL_BK; ++kk) {
             const int x = (kk >> 2) << 3;
+            float2 b[2 * TL_NH];
+#pragma unroll
+            for (int h = 0; h < TL_NH; ++h) {
+                const float4 v = *reinterpret_cast<const float4*>(w_s + kk * TL_BN + h * 64 + ((tx * 4) ^ x));
+                b[2 * h] = make_float2(v.x, v.y), b[2 * h + 1] = make_float2(v.z, v.w);
+            }
             const float4 a0 = *reinterpret_cast<const float4*>(a_s + kk * TL_BM + ((ty * 4) ^ x));
             const float4 a1 = *reinterpret_cast<const float4*>(a_s + kk * TL_BM + 32 + ((ty * 4) ^ x));
-            const float4 b0 = *reinterpret_cast<const float4*>(w_s + kk * TL_BN + ((tx * 4) ^ x));
-            const float4 b1 = *reinterpret_cast<const float4*>(w_s + kk * TL_BN + 64 + ((tx * 4) ^ x));
-            const float2 b[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w), make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
             const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const float2 aa = make_float2(a[i], a[i]);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) fma2(acc[i][j], aa, b[j]);
+                for (int j = 0; j < 2 * TL_NH; ++j) fma2(acc[i][j], aa, b[j]);
             }
         }
-        if (!SPLIT) {
-            left -= TL_BK;
-            if (left == 0 || !more) {                                   // the slice is complete
-                left = slice;
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        total[i][j].x += acc[i][j].x;
-                        total[i][j].y += acc[i][j].y;
-                        acc[i][j] = make_float2(0.0f, 0.0f);
-                    }
-            }
-        }
-        if (more) put(buf ^ 1);
         __syncthreads();
         buf ^= 1;
     }
-    auto store = [&](int m, int n, const float4 v) {                    // four features of one row
-        if (m >= M) return;
-        TC* c = C + (long)m * ldc + n;
-        const float x[4] = {v.x, v.y, v.z, v.w};
-        if (sizeof(TC) == 4 && n + 4 <= N && ((uintptr_t)c & 15) == 0) {
-            *reinterpret_cast<float4*>(c) = v;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int h = 0; h < TL_NH; ++h)
+            *reinterpret_cast<float4*>(tl_smem + ((i >> 2) * 32 + ty * 4 + (i & 3)) * TL_BN + h * 64 + tx * 4) =
+                make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x, acc[i][2 * h + 1].y);
+    cluster.sync();
+    // an eighth of the tile's rows are this CTA's to add up: four features a thread
+#pragma unroll
+    for (int e = tid; e < TL_BM / GS_SLICES * TL_BN / 4; e += TL_THREADS) {
+        const int r = (int)blockIdx.z * (TL_BM / GS_SLICES) + e / (TL_BN / 4), c = e % (TL_BN / 4) * 4;
+        float sum[4] = {};
+#pragma unroll
+        for (int z = 0; z < GS_SLICES; ++z) {
+            const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(tl_smem, z) + r * TL_BN + c);
+            sum[0] += v.x, sum[1] += v.y, sum[2] += v.z, sum[3] += v.w;
+        }
+        const int m = m0 + r, n = n0 + c;
+        if (m >= M) continue;
+        TC* out = C + (long)m * ldc + n;
+        if (sizeof(TC) == 4 && n + 4 <= N && ((uintptr_t)out & 15) == 0) {
+            *reinterpret_cast<float4*>(out) = make_float4(sum[0], sum[1], sum[2], sum[3]);
         } else {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (n + j < N) c[j] = from_f32<TC>(x[j]);
+                if (n + j < N) out[j] = from_f32<TC>(sum[j]);
         }
-    };
-    if constexpr (!SPLIT) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                store(m0 + (i >> 2) * 32 + ty * 4 + (i & 3), n0 + h * 64 + tx * 4,
-                      make_float4(total[i][2 * h].x, total[i][2 * h].y, total[i][2 * h + 1].x, total[i][2 * h + 1].y));
-    } else {
-        namespace cg = cooperative_groups;
-        cg::cluster_group cluster = cg::this_cluster();
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                *reinterpret_cast<float4*>(smem + ((i >> 2) * 32 + ty * 4 + (i & 3)) * TL_BN + h * 64 + tx * 4) =
-                    make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x, acc[i][2 * h + 1].y);
-        cluster.sync();
-        // 8 rows x 128 features of the tile are this CTA's to add up: four features a thread
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int r = (int)blockIdx.z * (TL_BM / GS_SLICES) + half * 4 + (tid >> 5), c = (tid & 31) * 4;
-            float4 sum = zero;
-#pragma unroll
-            for (int z = 0; z < GS_SLICES; ++z) {
-                const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(smem, z) + r * TL_BN + c);
-                sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
-            }
-            store(m0 + r, n0 + c, sum);
-        }
-        cluster.sync();                                                 // no CTA leaves while another reads its sums
     }
-}
-
-template <typename TC>
-__global__ void __launch_bounds__(TL_THREADS, 2) gemm_f32_tile_kernel(const float* __restrict__ A, long lda,
-                                                               const float* __restrict__ W, long ldw, TC* __restrict__ C,
-                                                               long ldc, int M, int N, int K, int slice) {
-    pdl_wait();
-    pdl_trigger();
-    gemm_f32_tile<TC, false>(A, lda, W, ldw, C, ldc, M, N, K, slice);
-}
-
-template <typename TC>
-__global__ void __cluster_dims__(1, 1, GS_SLICES) __launch_bounds__(TL_THREADS, 2)
-    gemm_f32_tile_split_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw,
-                               TC* __restrict__ C, long ldc, int M, int N, int K, int slice) {
-    pdl_wait();
-    pdl_trigger();
-    gemm_f32_tile<TC, true>(A, lda, W, ldw, C, ldc, M, N, K, slice);
+    cluster.sync();                                                     // no CTA leaves while another reads its sums
 }
 
 // ------------------------------------------------------------ host side
@@ -383,8 +352,7 @@ static int gs_skinny(const float* A, long lda, const float* W, long ldw, TC* C, 
 }
 
 // Float operands that 16-byte loads can read.  Up to 16 rows W's bytes decide and the skinny kernel streams them; above,
-// the multiply-adds do.  A tile is split over a cluster when that fills the SMs better: what is compared is the waves of
-// CTAs (two an SM) times the inputs that a CTA goes through, a split CTA paying about 40 inputs' time for the exchange.
+// the multiply-adds do (17 rows, 2048 x 2048: 31 us in tiles; the skinny kernel takes 14.5 for each 16 rows).
 template <typename TC>
 static int gs_f32(const float* A, long lda, const float* W, long ldw, TC* C, long ldc, int M, int N, int K, int sms,
                   int constant_w, cudaStream_t stream) {
@@ -393,17 +361,21 @@ static int gs_f32(const float* A, long lda, const float* W, long ldw, TC* C, lon
     if (M <= 4) return gs_skinny<TC, 4>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
     if (M <= 8) return gs_skinny<TC, 8>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
     if (M <= 16) return gs_skinny<TC, 16>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
-    const int slice = gs_slice(K);
-    dim3 grid((N + TL_BN - 1) / TL_BN, (M + TL_BM - 1) / TL_BM);
+    dim3 grid((N + TL_BN - 1) / TL_BN, (M + TL_BM - 1) / TL_BM, GS_SLICES);
     if (grid.y > 65535) return (int)cudaErrorInvalidValue;
-    const long tiles = (long)grid.x * grid.y, slots = 2L * sms;
-    const long whole = (tiles + slots - 1) / slots * K;
-    const long split = (tiles * GS_SLICES + slots - 1) / slots * (slice + 40);
-    if (split < whole) {
-        grid.z = GS_SLICES;
-        return fl_launch(gemm_f32_tile_split_kernel<TC>, grid, dim3(TL_THREADS), 0, stream, A, lda, W, ldw, C, ldc, M, N, K, slice);
-    }
-    return fl_launch(gemm_f32_tile_kernel<TC>, grid, dim3(TL_THREADS), 0, stream, A, lda, W, ldw, C, ldc, M, N, K, slice);
+    // Four CTAs fit an SM, and the clusters of a product of few tiles would be packed so, beside idle SMs: more shared memory
+    // than they use keeps one, two or three an SM where that many hold all tiles (100 x 2048 x 2048: 36.4 us so packed, 31.8
+    // two an SM).  A cluster lies within a GPC: at one CTA an SM they reach 3 of 4 SMs (of 16 tiles one waits for another to
+    // end: 17 x 2048 x 2048 took 39.6 us), at two or three 7 of 8.
+    int smem = TL_SMEM;
+    for (int each = 1; each < 4; ++each)
+        if ((long)grid.x * grid.y * GS_SLICES <= (each == 1 ? sms * 3L / 4 : (long)sms * each * 7 / 8)) {
+            smem = 228 * 1024 / (each + 1) - 1024 + 128;                // (each CTA takes 1 KB more than it asks for)
+            break;
+        }
+    cudaError_t err = cudaFuncSetAttribute(gemm_f32_tile_kernel<TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024);
+    if (err != cudaSuccess) return (int)err;
+    return fl_launch(gemm_f32_tile_kernel<TC>, grid, dim3(TL_THREADS), smem, stream, A, lda, W, ldw, C, ldc, M, N, K, gs_slice(K));
 }
 
 // constant_w: no kernel that may still run when this one is launched writes W (which is then read ahead of it).

@@ -67,3 +67,20 @@ def test_prompt_attention_over_rows_of_keys_and_values(size, heads, kv_heads, pa
     ops.sink_attention_rows(q, alone, cache, bt, step, heads, kv_heads, size, size ** -0.5, s, page, False, g)
     single = starts[2]
     assert not bool(alone[single].any()) and torch.equal(alone[:single], got[:single]) and torch.equal(alone[single + 1:], got[single + 1:])
+
+
+@pytest.mark.parametrize("m,n,k", [(17, 4, 4), (64, 130, 36), (65, 1664, 260), (66, 1800, 264), (200, 1700, 520), (400, 1300, 2048), (257, 2500, 300)])
+def test_products_of_32_bits_in_tiles(m, n, k):
+    """One to four CTAs an SM, slices that are short or empty, rows and features that are not there (whose neighbours in memory
+    are not finite): bit for bit what the kernel for any operands gives."""
+    torch.manual_seed(m + n + k)
+    a, w = torch.full((m + 40, k), float("nan"), device="cuda"), torch.full((n + 140, k), float("nan"), device="cuda")
+    a[:m], w[:n] = torch.randn(m, k, device="cuda"), torch.randn(n, k, device="cuda")
+    got = torch.full((m + 1, n + 3), 7.0, device="cuda")
+    ops.gemm_simt(a[:m], w[:n], got[:m, :n])
+    odd = torch.empty(m * (k + 1), device="cuda").view(m, k + 1)[:, 1:]
+    odd.copy_(a[:m])
+    want = torch.empty(m, n, device="cuda")
+    ops.gemm_simt(odd, w[:n], want)
+    assert torch.equal(got[:m, :n], want)
+    assert bool((got[m] == 7).all()) and bool((got[:, n:] == 7).all())
