@@ -102,21 +102,25 @@ __global__ void __launch_bounds__(256, 4) gemm_simt_kernel(const TA* __restrict_
 }
 
 // ------------------------------------------------------------ up to 16 rows
-// A CTA of 64 threads serves 8 x RT features: thread (slice s, row r) sums slice s of features r, r + 8, ... for all MT
+// A CTA of 64 threads serves 16 features: thread (slice s, row r) sums slice s of features r and r + 8 for all MT
 // rows of A.  W and A pass through a ring of shared-memory stages, 32 inputs of every slice each, filled by 16-byte
-// cp.async: what bounds the product is the stream of W, so the ring keeps 3 of 4 stages (24 KB a CTA, several CTAs an
+// cp.async: what bounds the product is the stream of W, so the ring keeps 2 or 3 stages (16 KB of W each, two or three CTAs an
 // SM) in flight, and where the caller says that no kernel writes W (constant_w) its first stages are asked for before the
 // preceding kernel has ended.  A staged row of W is padded
-// to 36 floats: the eight lanes of a quarter warp, on eight rows, then read all 32 banks.  MT rows of A are read
-// (rows past M repeat the last one and are not written).  RT = 2 above four rows of A, so that a value of A that has
-// been read from shared memory serves two features.
+// to 36 floats: the eight lanes of a quarter warp, on eight rows, then read all 32 banks.  A value of A that has been read
+// from shared memory serves two features: with one, the reads of A kept more shared memory busy than W did (11008 features
+// of 2048, out of a cold cache: 21.7, 22.2, 29.1 and 25.0 us for 1 to 4 rows; 19.1, 20.1, 21.0 and 21.2 now, 4.2 to 4.7 TB/s
+// of W; 2048 features 6.1 to 8.0, now 5.6 to 6.4).  A third stage in flight costs four rows 5 to 10 % on many features, as
+// one CTA an SM fewer fits, and gains one or two rows up to 7 % on few.  Rows past M are zeroes up to four rows (3 rows took
+// longer than 4 when they repeated the last one), and repeat the last one above, where leaving them out costs 2 to 4 % of the
+// products that have them all; they are not written.
 #define SK_BK 32
 #define SK_PITCH 36
 
 template <int MT> struct Skinny {
-    static constexpr int RT = MT > 4 ? 2 : 1;
+    static constexpr int RT = 2;
     static constexpr int R = 8 * RT;
-    static constexpr int STAGES = MT > 8 ? 3 : 4;
+    static constexpr int STAGES = MT > 8 || MT == 4 ? 3 : 4;
     static constexpr int A_PITCH = MT * SK_BK + 4;                     // floats of a slice's rows of A
     static constexpr int W_FLOATS = GS_SLICES * R * SK_PITCH;
     static constexpr int STAGE_FLOATS = W_FLOATS + GS_SLICES * A_PITCH;
@@ -150,7 +154,10 @@ __global__ void __launch_bounds__(64) gemm_f32_skinny_kernel(const float* __rest
         const int k = s * slice + t * SK_BK + row * 4;
         float* dst = sk_smem + (t % STAGES) * L::STAGE_FLOATS + L::W_FLOATS + s * L::A_PITCH + row * 4;
 #pragma unroll
-        for (int m = 0; m < MT; ++m) sk_cp16(dst + m * SK_BK, k < K ? A + (long)min(m, M - 1) * lda + k : A, k < K);
+        for (int m = 0; m < MT; ++m) {
+            const bool in = k < K && (MT > 4 || m < M);
+            sk_cp16(dst + m * SK_BK, in ? A + (long)(MT > 4 ? min(m, M - 1) : m) * lda + k : A, in);
+        }
     };
     if (constant_w)
         for (int t = 0; t < STAGES - 1 && t < n_st; ++t) load_w(t);
