@@ -39,3 +39,15 @@ def test_a_prompt_beside_decoding_requests_does_not_lengthen_their_splits(monkey
     assert plans[0] == plans[1] == plans[2]
     keys, splits = plans[0]
     assert keys * splits >= 400 + 40 * 23 + 1 and keys * (splits - 1) < 400 + 40 * 23 + 1
+
+
+@pytest.mark.parametrize("lens,heads,single,pays", [([(0, 2048)], 16, False, True), ([(1500, 8)], 4, False, True), ([(0, 4)], 16, False, False),
+                                                    ([(0, 8)] * 20, 32, False, False), ([(0, 100)] * 8, 32, False, True),
+                                                    ([(700, 1)] * 16 + [(0, 4)], 16, False, False), ([(700, 1)] * 16, 16, True, True),
+                                                    ([], 16, False, True)])
+def test_prompt_attention_over_rows_goes_where_it_is_faster(lens, heads, single, pays):
+    """Measured sides of the rule; single tokens count only where the kernel serves them; a step without lengths is accepted."""
+    from fastllm_py_b200.native.ops import _sink_rows_pay
+
+    step = SimpleNamespace(q_lens=[q for _, q in lens], ctx_lens=[c for c, _ in lens]) if lens else SimpleNamespace()
+    assert _sink_rows_pay(step, heads, single, 148) is pays
