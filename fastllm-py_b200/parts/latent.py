@@ -167,18 +167,39 @@ class LatentAttention(Part):
         return step.plans.get(self.plan_key)
 
     def _prompts(self, step, n_tokens: int, page_size: int) -> bool:
-        """Whether a step without splits goes to the prompt kernel: it takes eight neighbouring tokens of a request at a
-        time at the price of 3.4 single tokens in the other kernel where both fill the GPU (2048 tokens: 413 us against
-        971), so it is the faster one until half of its rows stay empty.  A tile of keys alone takes it as long as the other
-        (4.6 us with a latent of 512), or longer (3.6 against 2.9 with 256, which leaves the other room for more blocks an
-        SM): with few blocks the other kernel is as fast (128 tokens of 16 heads behind 1000: 153 us both) or faster (256:
-        128 us against 103; level at 384 tokens).  The results are the same."""
+        """Whether a step without splits goes to the prompt kernel, which takes eight neighbouring tokens of a request at a
+        time.  The results are the same.
+
+        A latent of 512: a tile of 32 keys takes it 2.15 us and the other kernel 4.6 (6.6 where two of its blocks share an
+        SM), its start 10.7 us against 4 (6), and two of its blocks (one for either half of the value columns) stand on an SM
+        each, two of the other's on one.  128 tokens of 16 heads behind 1000 others take 87 us against 163, 16 requests of 4
+        behind 500 43 against 75; 20 prompts of 8 tokens 14.4 against 11.8, 60 of 3 with 32 heads 27 against 19.
+
+        Up to 256 the prompt kernel's tile takes 3.6 us against 2.9, and the other has room for more blocks an SM: with few
+        blocks that one is the faster (128 tokens of 16 heads behind 1000: 128 us against 103; level at 384 tokens), with
+        many the prompt kernel until half of its rows stay empty.  Captured steps serve many lengths and take this rule too."""
         if not step.q_lens or not ops.latent_prompt_takes(self.ctx.dtype, self.rank, self.rot, self.heads, page_size):
             return False
-        blocks = n_tokens * -(-self.heads // 16)                          # the other kernel's
-        if 2 * blocks <= (2 if self.rank > 256 else 5) * ops.sm_count(self.ctx.device):
-            return False
-        return 4 * sum(-(-q // 8) for q in step.q_lens) <= n_tokens       # four of eight rows at least
+        of_heads, sms = -(-self.heads // 16), ops.sm_count(self.ctx.device)
+        blocks = n_tokens * of_heads                                      # the other kernel's
+        ctx_lens = getattr(step, "ctx_lens", None)
+        if self.rank <= 256 or not ctx_lens or getattr(step, "for_graph", False):
+            if 2 * blocks <= (2 if self.rank > 256 else 5) * sms:
+                return False
+            return 4 * sum(-(-q // 8) for q in step.q_lens) <= n_tokens   # four of eight rows at least
+        start, a_tile = (4.0, 4.6) if blocks <= sms else (6.0, 6.6)
+        groups, tiles, longest, other_tiles = 0, 0.0, 0, 0.0
+        for q, ctx in zip(step.q_lens, ctx_lens):
+            last = ctx + q if self.window is None else min(ctx + q, self.window + 8)
+            mean = last if self.window is not None and ctx >= self.window else min(last, ctx + (q + 1) / 2)
+            n = -(-q // 8)
+            groups += n
+            tiles += n * (mean + 16) / 32
+            other_tiles += q * (mean + 16) / 32
+            longest = max(longest, -(-last // 32))
+        here = max(-(-2 * groups * of_heads // sms) * (10.7 + 2.15 * tiles / groups), 10.7 + 2.15 * longest)
+        other = max(-(-blocks // (2 * sms)) * (start + a_tile * other_tiles / n_tokens), start + a_tile * longest)
+        return here < other
 
     def _partials(self, n_tokens: int, n_splits: int):
         return scratch.get(self.ctx.device, self.SCRATCH, n_tokens * self.heads * n_splits * (self.rank + 2))

@@ -51,3 +51,23 @@ def test_prompt_attention_over_rows_goes_where_it_is_faster(lens, heads, single,
 
     step = SimpleNamespace(q_lens=[q for _, q in lens], ctx_lens=[c for c, _ in lens]) if lens else SimpleNamespace()
     assert _sink_rows_pay(step, heads, single, 148) is pays
+
+
+@pytest.mark.parametrize("lens,heads,pays", [([(0, 8)] * 20, 16, False), ([(0, 8)] * 20, 32, True), ([(0, 3)] * 60, 32, False), ([(0, 37)] * 8, 32, True),
+                                             ([(0, 64)], 16, False), ([(0, 128)], 16, True), ([(1000, 64)], 16, True),
+                                             ([(500, 4)] * 16, 16, True), ([(100, 1)] * 140, 16, False)])
+def test_latent_prompt_kernel_where_it_is_faster(lens, heads, pays, monkeypatch):
+    """Measured sides of the rule for a latent of 512; without the lengths behind, and under capture, the rule by rows."""
+    from fastllm_py_b200.parts import latent
+
+    monkeypatch.setattr(latent.ops, "latent_prompt_takes", lambda *a: True)
+    monkeypatch.setattr(latent.ops, "sm_count", lambda device: 148)
+    part = object.__new__(latent.LatentAttention)
+    part.rank, part.rot, part.heads, part.window, part.ctx = 512, 64, heads, None, SimpleNamespace(dtype=None, device=None)
+    n = sum(q for _, q in lens)
+    step = SimpleNamespace(q_lens=[q for _, q in lens], ctx_lens=[c for c, _ in lens])
+    assert part._prompts(step, n, 16) is pays
+    rows = 4 * sum(-(-q // 8) for q in step.q_lens) <= n and n * heads // 16 > 148
+    assert part._prompts(SimpleNamespace(q_lens=step.q_lens), n, 16) is rows
+    step.for_graph = True
+    assert part._prompts(step, n, 16) is rows
