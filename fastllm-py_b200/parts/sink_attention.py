@@ -131,7 +131,10 @@ class SinkAttention(Part):
         """(library, defines) pairs compiled for this part's sizes, so that a model's first load builds them beside
         its other libraries."""
         takes = self.ctx.device.type == "cuda" and ops.sink_tc_takes(self.ctx.dtype, self.dim, self.vdim)
-        return [ops.sink_tc_library(self.dim, self.vdim)] if takes else []
+        if not takes:
+            return []
+        rows = ops.sink_rows_takes(self.dim, self.vdim, self.window, self.keep_first, self.softcap, None, None, self.ctx.page_size)
+        return [ops.sink_tc_library(self.dim, self.vdim)] + ([("attention_prefill_tc", {"HEAD_DIM": self.dim})] if rows else [])
 
     def reserve(self, limits):
         for lin in (self.qkv, self.o):
@@ -139,7 +142,8 @@ class SinkAttention(Part):
                 lin.reserve(self.ctx.dtype, limits.max_tokens)
         if self.ctx.device.type == "cuda" and ops.sink_tc_takes(self.ctx.dtype, self.dim, self.vdim):
             from ..native.build import load_library
-            load_library(*ops.sink_tc_library(self.dim, self.vdim))        # built now, not inside the first step
+            for library in self.native_builds():
+                load_library(*library)                        # built now, not inside the first step
         if self.ctx.device.type == "cuda" and self._splits_single_tokens():
             longest = -(-limits.max_model_len // 1024) * 1024
             self._partials(min(limits.max_tokens, limits.max_requests),
