@@ -108,64 +108,51 @@ def decode_splits(max_seq_len: int, split_keys: int = DECODE_SPLIT) -> int:
     return max(1, -(-max_seq_len // split_keys))
 
 
-def _decode_time(groups: int, longest: int, mean: int, split: int, slots: int, head_dim: int) -> float:
+def _decode_time(groups: int, length: int, split: int, slots: int, head_dim: int) -> float:
     """Modelled microseconds of the decode kernel and its merge for `groups` (token, key/value
-    head) pairs of up to `longest` keys, `mean` on average, cut every `split` keys: the larger of the time to stream
+    head) pairs of `length` keys each, cut every `split` keys: the larger of the time to stream
     the keys and values (6.9 TB/s at best, a little less with short splits, and a last split that
     leaves warps of its CTA idle streams that much slower) and the time the CTAs take in rounds
     of `slots` (a CTA by itself: 4 us and 22 ns a key; a last split shorter than the others is
     as long as its busiest warp, a quarter of a split), plus the merge, which reads split after
-    split.  Lengths that differ are taken as evenly spread to both sides of their mean."""
+    split."""
     scale = head_dim / 128.0
-    lengths = [longest] if mean >= longest else \
-        [max(1, 2 * mean - longest + (longest - max(1, 2 * mean - longest)) * (2 * i + 1) // 16) for i in range(8)]
-    share = groups / len(lengths)
-    stream = whole = short = 0.0
-    for length in lengths:
-        n = -(-length // split)
-        last = length - (n - 1) * split
-        busy = min(1.0, -(-4 * last // split) / 4.0)        # share of its four warps that a last, shorter split keeps busy
-        stream += share * ((n - 1) * split + last / busy) * 4.0 * head_dim / (6.9e6 * split / (split + 16.0))
-        whole += share * (n - 1)                            # CTAs of whole splits, in rounds of `slots`
-        short = max(short, 4.0 + min(split, 4 * last) * 0.022 * scale)
+    n = -(-length // split)
+    last = length - (n - 1) * split
+    busy = min(1.0, -(-4 * last // split) / 4.0)            # share of its four warps that a last, shorter split keeps busy
+    stream = groups * ((n - 1) * split + last / busy) * 4.0 * head_dim / (6.9e6 * split / (split + 16.0))
     alone = 4.0 + split * 0.022 * scale
-    rounds = -(-int(whole + 0.5) // slots)
-    left = max(0, groups - (rounds * slots - int(whole + 0.5)))   # short CTAs that find no place beside them
+    short = 4.0 + min(split, 4 * last) * 0.022 * scale
+    whole = groups * (n - 1)                                # CTAs of whole splits, in rounds of `slots`
+    rounds = -(-whole // slots)
+    left = max(0, groups - (rounds * slots - whole))        # short CTAs that find no place beside them
     in_rounds = rounds * alone + -(-left // slots) * short
-    return max(stream, in_rounds) + 0.2 * -(-longest // split)
+    return max(stream, in_rounds) + 0.2 * n
 
 
 @functools.lru_cache(maxsize=4096)
-def _decode_split_keys(n_tokens: int, kv_heads: int, high: int, mean_high: int, num_sms: int, head_dim: int) -> int:
-    slots = 3 * num_sms
-    groups = n_tokens * kv_heads
-    best_split, best_time = DECODE_SPLIT, None
-    for split in range(64, 1025, 64):
-        t = _decode_time(groups, high - 255, mean_high - 255, split, slots, head_dim) + \
-            _decode_time(groups, high, mean_high, split, slots, head_dim)
-        if best_time is None or t < best_time:
-            best_split, best_time = split, t
-    return best_split
-
-
 def decode_split_keys(n_tokens: int, kv_heads: int, max_seq_len: int, num_sms: int = 148,
-                      head_dim: int = 128, mean_seq_len: int | None = None) -> int:
+                      head_dim: int = 128) -> int:
     """Keys per split for a launch, a multiple of 64 up to 1024: the one a small model of the
-    kernel's time likes best, for sequences of up to `max_seq_len` keys, `mean_seq_len` on average (None: all as long).
-    One CTA serves one (token, key/value head, split); three CTAs
+    kernel's time likes best.  One CTA serves one (token, key/value head, split); three CTAs
     fit an SM, so CTAs run in rounds of 3 x SMs.  Constants fitted to measurements on B200
     (batch 1 to 64, 300 to 4000 keys): the pick is within a few percent of the best there,
     where a fixed 256 keys was 11 % off on average (few CTAs: a round and a bit of small ones
     is worse than one round of larger ones; many: the longer the split the better it streams).
-    With lengths that differ the longest alone says too little: 24 requests of 360 to 1440 keys over 16 key/value heads take
-    49 us with the 1024 keys that suit 24 of 1950, and 39 with 512; over nine batches the picks are 2 % off the best.
 
     The answer is the same for all lengths of a stretch of 256 (the model is asked about both
-    ends of the stretch, of the longest and of the mean), so that a sequence that grows changes its split, and with it the
+    ends of the stretch), so that a sequence that grows changes its split, and with it the
     rounding of its result and the shape of a captured step, every 256 tokens at most."""
+    slots = 3 * num_sms
+    groups = n_tokens * kv_heads
     high = -(-max(max_seq_len, 1) // 256) * 256
-    mean_high = high if mean_seq_len is None else min(high, -(-max(mean_seq_len, 1) // 256) * 256)
-    return _decode_split_keys(n_tokens, kv_heads, high, mean_high, num_sms, head_dim)
+    low = high - 255
+    best_split, best_time = DECODE_SPLIT, None
+    for split in range(64, 1025, 64):
+        t = _decode_time(groups, low, split, slots, head_dim) + _decode_time(groups, high, split, slots, head_dim)
+        if best_time is None or t < best_time:
+            best_split, best_time = split, t
+    return best_split
 
 
 def decode_attention(q, out, cache_tensor, block_table, tok_req, positions, tok_list, n_list, heads,

@@ -89,10 +89,9 @@ class Attention(Part):
         if fast is None or step.n_decode_tokens == 0:
             step.plans[self.plan_key] = (0, 1)             # no launch of that kernel: one answer, one graph key
             return
-        lens = [c + 1 for c, q in zip(step.ctx_lens, step.q_lens) if q == 1] or [step.max_seq_len]
-        longest = max(lens)                                # (a prompt beside them is the other kernel's)
+        longest = step.max_seq_len
         keys = fast.decode_split_keys(step.n_decode_tokens, self.kv_heads, longest, fast.num_sms(self.ctx.device),
-                                      self.head_dim, sum(lens) // len(lens))
+                                      self.head_dim)
         if step.for_graph:
             longest = -(-longest // 1024) * 1024
         step.plans[self.plan_key] = (keys, fast.decode_splits(longest, keys))

@@ -1,44 +1,32 @@
-"""How the decode kernel's keys are split, with sequences of unequal lengths."""
+"""What the host decides per step: how the decode kernel's keys are split, and which kernel serves prompts."""
 from types import SimpleNamespace
 
 import pytest
 
-from fastllm_py_b200.native.attention import decode_split_keys
 
-
-@pytest.mark.parametrize("n,kv_heads,longest", [(1, 16, 1), (1, 16, 513), (8, 32, 2049), (64, 8, 1258), (24, 16, 1442), (200, 1, 70000)])
-def test_split_of_unequal_lengths(n, kv_heads, longest):
-    equal = decode_split_keys(n, kv_heads, longest)
-    assert decode_split_keys(n, kv_heads, longest, mean_seq_len=longest) == equal
-    assert decode_split_keys(n, kv_heads, longest, mean_seq_len=10 * longest) == equal       # (a mean cannot exceed the longest)
-    for mean in (1, longest // 3 + 1, longest // 2 + 1):
-        keys = decode_split_keys(n, kv_heads, longest, mean_seq_len=mean)
-        assert keys % 64 == 0 and 64 <= keys <= 1024
-        stretch = -(-mean // 256) * 256                     # one answer for all means of a stretch of 256
-        assert keys == decode_split_keys(n, kv_heads, longest, mean_seq_len=stretch) \
-            == decode_split_keys(n, kv_heads, longest, mean_seq_len=max(1, stretch - 255))
-
-
-def test_a_prompt_beside_decoding_requests_does_not_lengthen_their_splits(monkeypatch):
-    """The plan of a mixed step looks at the requests with one token only."""
+@pytest.mark.parametrize("lens", [[300 + 37 * i for i in range(64)], [5, 1900], [360 + 45 * i for i in range(24)]])
+def test_split_follows_the_longest_sequence_only(lens, monkeypatch):
+    """The split decides how a token's sums are rounded, and which captured step runs it: a batch that grows keeps it for 256
+    tokens, and the lengths of shorter neighbours do not enter."""
     from fastllm_py_b200.native import attention as fast
     from fastllm_py_b200.parts.attention import Attention
 
     part = object.__new__(Attention)
-    part.heads = part.kv_heads = 16
-    part.head_dim, part.ctx = 128, SimpleNamespace(device="cpu")
+    part.heads, part.kv_heads, part.head_dim, part.ctx = 16, 8, 128, SimpleNamespace(device="cpu")
     monkeypatch.setattr(Attention, "_fast", lambda self: fast)
     monkeypatch.setattr(fast, "num_sms", lambda device: 148)
-    plans = []
-    for extra in ([], [(0, 488)], [(1500, 450)]):
-        lens = [(400 + 40 * i, 1) for i in range(24)] + extra
-        step = SimpleNamespace(n_decode_tokens=24, for_graph=False, plans={}, ctx_lens=[c for c, _ in lens], q_lens=[q for _, q in lens],
-                               max_seq_len=max(c + q for c, q in lens))
+
+    def plan(ctx_lens):
+        step = SimpleNamespace(n_decode_tokens=len(ctx_lens), for_graph=True, plans={}, ctx_lens=ctx_lens, q_lens=[1] * len(ctx_lens),
+                               max_seq_len=max(ctx_lens) + 1)
         Attention.plan_step(part, step)
-        plans.append(step.plans[part.plan_key])
-    assert plans[0] == plans[1] == plans[2]
-    keys, splits = plans[0]
-    assert keys * splits >= 400 + 40 * 23 + 1 and keys * (splits - 1) < 400 + 40 * 23 + 1
+        return step.plans[part.plan_key]
+
+    grown = [plan([c + k for c in lens]) for k in range(1024)]
+    assert sum(a != b for a, b in zip(grown, grown[1:])) <= 4
+    assert plan(lens) == plan([1] * (len(lens) - 1) + [max(lens)]) == plan([max(lens)] * len(lens))
+    keys, splits = plan(lens)
+    assert keys == fast.decode_split_keys(len(lens), 8, max(lens) + 1) and keys * splits >= max(lens) + 1
 
 
 @pytest.mark.parametrize("lens,heads,single,pays", [([(0, 2048)], 16, False, True), ([(1500, 8)], 4, False, True), ([(0, 4)], 16, False, False),
