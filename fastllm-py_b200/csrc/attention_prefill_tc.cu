@@ -144,6 +144,13 @@ __device__ __forceinline__ void ft_ld32(uint32_t taddr, uint32_t* r) {
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void ft_ld4(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void ft_st2(uint32_t taddr, uint32_t a, uint32_t b) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(taddr), "r"(a), "r"(b) : "memory");
+}
 __device__ __forceinline__ void ft_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void ft_st32(uint32_t taddr, const uint32_t* r) {
     asm volatile(
@@ -174,10 +181,10 @@ __device__ __forceinline__ uint64_t ft_desc_kmajor(uint32_t saddr) {
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
            ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-// MN-major operand (the contiguous axis is N): 64-element blocks of N are FT_ATOM_BYTES apart
+// MN-major operand (the contiguous axis is N): 64-element blocks of N are `atom` bytes apart
 // (leading offset), groups of 8 K rows 1024 bytes apart (stride offset).
-__device__ __forceinline__ uint64_t ft_desc_mnmajor(uint32_t saddr) {
-    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(FT_ATOM_BYTES >> 4) << 16) |
+__device__ __forceinline__ uint64_t ft_desc_mnmajor(uint32_t saddr, uint32_t atom) {
+    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(atom >> 4) << 16) |
            ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 // float accumulator, bfloat16 operands; b_mn: B is MN-major
@@ -193,11 +200,15 @@ __device__ __forceinline__ float ft_ex2(float x) {
 }
 __device__ __forceinline__ float ft_weight(float a, float b) { return (a == -CUDART_INF_F) ? 0.0f : exp2f(a - b); }
 
-struct FtSmem {
+// ROWS (see the kernel): blocks of 64 keys, and stages for as much of the SM's shared memory as leaves room for one CTA.
+template <bool ROWS> struct FtSmem {
+    static constexpr int BN = ROWS ? 64 : FT_BN;                       // keys of a block
+    static constexpr int STAGES = ROWS ? (HEAD_DIM == 128 ? 5 : 6) : FT_STAGES;
+    static constexpr int ATOM = BN * 128;                              // bytes of 64 columns of a block
     static constexpr int Q_BYTES = FT_ATOMS * FT_ATOM_BYTES;
-    static constexpr int KV_BYTES = FT_ATOMS * FT_ATOM_BYTES;          // one of K or V, one stage
-    static constexpr int TILES = Q_BYTES + 2 * FT_STAGES * KV_BYTES;
-    static constexpr int BAR_SLOTS = 24 + 4 * FT_STAGES;               // 8-byte slots: barriers and the like
+    static constexpr int KV_BYTES = FT_ATOMS * ATOM;                   // one of K or V, one stage
+    static constexpr int TILES = Q_BYTES + 2 * STAGES * KV_BYTES;
+    static constexpr int BAR_SLOTS = 24 + 4 * STAGES;                  // 8-byte slots: barriers and the like
     static constexpr int BARS = BAR_SLOTS * 8 + 2 * FT_PARTS * 128 * 4; // ... then the parts' maxima (two rounds)
     // The tiles want a 1024-byte boundary.  Where they fill the SM's shared memory to within a KB
     // there is no room to round up to one: the kernel then counts on the dynamic shared memory
@@ -209,35 +220,42 @@ struct FtSmem {
 
 // ROWS: a cache row holds a token's key and its value (k | v, pages [n_kv_heads][page_size][2 HEAD_DIM]); `sink` ([heads], or
 // null) is a term exp(sink) of each head's denominator, and `gate` (or null) multiplies a row's result by the sigmoid of its
-// gate, `gate_cols` numbers a head (one, or one a channel), before it is rounded.
+// gate, `gate_cols` numbers a head (one, or one a channel), before it is rounded.  Such layers are served by two kernels, by
+// the lengths of a step, so this one makes the sums of the other (sink_attention_tc.cu), one by one: blocks of 64 keys at
+// multiples of 64 of the absolute position, a rescaling at every block where a row's maximum moved, scores scaled and weights
+// made by the same instructions, four partial sums of a row's weights (keys 2c and 2c + 1 of every eight), values in K steps
+// of 16 from the first to the last.  The results are the same bit for bit.
 template <bool ROWS>
 __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
     bf16* __restrict__ out, long out_ld, int page_size, int kv_rows_total, const int* __restrict__ block_table,
     int bt_stride, const int* __restrict__ req_start, const int* __restrict__ req_ctx,
     const int* __restrict__ req_qlen, int n_requests, int include_single, int n_heads, int n_kv_heads,
-    int window, float scale_log2e, int* __restrict__ status, const float* __restrict__ sink, const bf16* __restrict__ gate,
+    int window, float scale, int* __restrict__ status, const float* __restrict__ sink, const bf16* __restrict__ gate,
     long gate_ld, int gate_cols) {
+    using L = FtSmem<ROWS>;
+    constexpr int BN = L::BN, STAGES = L::STAGES;
+    const float scale_log2e = scale * 1.4426950408889634f;
     extern __shared__ __align__(1024) unsigned char ft_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)ft_raw + 1023) & ~(uintptr_t)1023);
-    if (base + FtSmem::TILES + FtSmem::BARS > ft_raw + FtSmem::TOTAL) {       // uniform over the CTA
+    if (base + L::TILES + L::BARS > ft_raw + L::TOTAL) {       // uniform over the CTA
         if (threadIdx.x == 0) atomicCAS(status, 0, FT_ERR_SMEM);
         return;
     }
     unsigned char* q_s = base;
-    unsigned char* k_s = q_s + FtSmem::Q_BYTES;                        // [stage][atom][128 rows][128 B]
-    unsigned char* v_s = k_s + FT_STAGES * FtSmem::KV_BYTES;
-    uint64_t* bars = (uint64_t*)(base + FtSmem::TILES);
+    unsigned char* k_s = q_s + L::Q_BYTES;                        // [stage][atom][128 rows][128 B]
+    unsigned char* v_s = k_s + STAGES * L::KV_BYTES;
+    uint64_t* bars = (uint64_t*)(base + L::TILES);
     uint64_t* q_full = bars + 0;
-    uint64_t* k_full = bars + 24;                                      // [FT_STAGES]
-    uint64_t* k_empty = k_full + FT_STAGES;
+    uint64_t* k_full = bars + 24;                                      // [STAGES]
+    uint64_t* k_empty = k_full + STAGES;
     uint64_t* s_full = bars + 5;                                       // [2]
     uint64_t* p_full = bars + 9;                                       // [2]
     uint64_t* o_done = bars + 11;                                      // [2] P V of block i is done: barrier i & 1, phase i >> 1
     uint32_t* tmem_slot = (uint32_t*)(bars + 13);
     uint64_t* x_bar = bars + 14;                                       // the softmax threads' exchange point
-    uint64_t* v_full = k_empty + FT_STAGES;
-    uint64_t* v_empty = v_full + FT_STAGES;
+    uint64_t* v_full = k_empty + STAGES;
+    uint64_t* v_empty = v_full + STAGES;
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     volatile int* never = (volatile int*)(bars + 15);                  // stays 0: for waits that must not be cut short
 
@@ -267,7 +285,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
     const int rows_here = min(FT_BM, q_len - row0);
     const int pos_first = ctx + row0, pos_last = ctx + row0 + rows_here - 1;
     const int lo_tile = window > 0 ? max(0, pos_first - window + 1) : 0;
-    const int kb_begin = lo_tile / FT_BN, kb_end = pos_last / FT_BN + 1;
+    const int kb_begin = lo_tile / BN, kb_end = pos_last / BN + 1;
     const int n_blocks = kb_end - kb_begin;
 
     // ---- the producers' side of a block: one box of a page and 64 columns per lane.  A block of 128 keys is
@@ -279,22 +297,22 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
     auto issue_block = [&](int i) {
         unsigned char* ring = is_v ? v_s : k_s;
         const int* bt = block_table + (long)req * bt_stride;
-        const int n_ops = (FT_BN / page_size) * FT_ATOMS;
-        const int s = i % FT_STAGES;
-        if (lane == 0) ft_bar_expect(&full[s], FtSmem::KV_BYTES);
+        const int box = min(page_size, BN), n_ops = (BN / box) * FT_ATOMS;
+        const int s = i % STAGES;
+        if (lane == 0) ft_bar_expect(&full[s], L::KV_BYTES);
         __syncwarp();
-        const int key0 = (kb_begin + i) * FT_BN;
+        const int key0 = (kb_begin + i) * BN;
         for (int op = lane; op < n_ops; op += 32) {
             const int p = op / FT_ATOMS, a = op % FT_ATOMS;
-            const int first_key = key0 + p * page_size;
-            const int last_key = first_key + page_size - 1;
-            // a page wholly outside what this tile may see is fetched from beyond the tensor: zeros
+            const int first_key = key0 + p * box;
+            const int last_key = first_key + box - 1;
+            // a page (or the part of one that lies in the block) wholly outside what this tile may see is fetched from beyond the tensor: zeros
             int row = kv_rows_total;
             if (first_key <= pos_last && last_key >= lo_tile) {
                 const long pg = bt[first_key / page_size];
-                row = (int)((ROWS ? pg * n_kv_heads + kvh : (pg * 2 + is_v) * n_kv_heads + kvh) * page_size);
+                row = (int)((ROWS ? pg * n_kv_heads + kvh : (pg * 2 + is_v) * n_kv_heads + kvh) * page_size) + (ROWS ? first_key % page_size : 0);
             }
-            const int off = s * FtSmem::KV_BYTES + a * FT_ATOM_BYTES + p * page_size * 128;
+            const int off = s * L::KV_BYTES + a * L::ATOM + p * box * 128;
             ft_tma_2d(ring + off, &map_kv, &full[s], a * 64 + (ROWS ? is_v * HEAD_DIM : 0), row);
         }
     };
@@ -303,19 +321,19 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
     // memory then hides: tensor memory, the other barriers, a look at the error word.  A tile with many blocks
     // sends for a whole ring at once; for a short one that only put the queries, which are wanted first, behind
     // three blocks of keys and values (measured: 2048 tokens 76 us against 70, 8192 tokens 693 against 744).
-    const int early = n_blocks > 32 ? FT_STAGES : 1;
+    const int early = n_blocks * BN > 32 * FT_BN ? STAGES : FT_BN / BN;
     int issued = 0;
     if (producer) {
         if (lane == 0) {
             if (!is_v) ft_bar_init(q_full, 1);
-            for (int s = 0; s < FT_STAGES; ++s) {
+            for (int s = 0; s < STAGES; ++s) {
                 ft_bar_init(&full[s], 1);
                 ft_bar_init(&empty[s], 1);
             }
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             if (!is_v) {
-                ft_bar_expect(q_full, FtSmem::Q_BYTES);
+                ft_bar_expect(q_full, L::Q_BYTES);
                 for (int a = 0; a < FT_ATOMS; ++a)
                     ft_tma_2d(q_s + a * FT_ATOM_BYTES, &map_q, q_full, h * HEAD_DIM + a * 64, tok0);
             }
@@ -345,7 +363,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
     __syncthreads();
     ft_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t tmem_s = tmem;                                      // two S buffers: columns 0 and 128
+    const uint32_t tmem_s = tmem;                                      // two S buffers: columns 0 and BN
     const uint32_t tmem_o = tmem + 256;                                // O: HEAD_DIM columns, accumulated over the blocks
 
 #define FT_GIVE_UP()                                                             \
@@ -361,32 +379,32 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
         // P V, and their way through TMA showed.
         int i = issued;
         for (; i < n_blocks && !*abort_flag; ++i) {
-            if (!ft_warp_wait(&empty[i % FT_STAGES], ((uint32_t)(i / FT_STAGES) & 1u) ^ 1u, abort_flag)) FT_GIVE_UP();
+            if (!ft_warp_wait(&empty[i % STAGES], ((uint32_t)(i / STAGES) & 1u) ^ 1u, abort_flag)) FT_GIVE_UP();
             issue_block(i);
         }
         if (*abort_flag) {
             // leaving early: the copies still on their way must land before the shared memory goes to
             // another CTA (the wait is bounded like every other)
-            for (int k = max(0, i - FT_STAGES); k < i; ++k)
-                ft_warp_wait(&full[k % FT_STAGES], (uint32_t)(k / FT_STAGES) & 1u, never);
+            for (int k = max(0, i - STAGES); k < i; ++k)
+                ft_warp_wait(&full[k % STAGES], (uint32_t)(k / STAGES) & 1u, never);
             if (!is_v && lane == 0) ft_wait(q_full, 0, never);
         }
     } else if (warp == FT_MMA_WARP) {
         if (lane == 0 && !*abort_flag) {
             // ---- MMA issuer.  The tensor core runs what this thread issues in order, so S(i + 2),
             // which goes where S(i) and then P(i) were, follows P V of block i without a barrier.
-            constexpr uint32_t idesc_s = ft_idesc(FT_BM, FT_BN, 0);
+            constexpr uint32_t idesc_s = ft_idesc(FT_BM, BN, 0);
             constexpr uint32_t idesc_o = ft_idesc(FT_BM, HEAD_DIM, 1);
             auto issue_s = [&](int i) -> bool {                        // S(i) = Q K(i)^T into S buffer i & 1
-                const int s = i & 1, ks = i % FT_STAGES;
-                if (!ft_wait(&k_full[ks], (uint32_t)(i / FT_STAGES) & 1u, abort_flag)) return false;
+                const int s = i & 1, ks = i % STAGES;
+                if (!ft_wait(&k_full[ks], (uint32_t)(i / STAGES) & 1u, abort_flag)) return false;
                 ft_fence_after();
-                const uint32_t qa = ft_smem(q_s), ka = ft_smem(k_s + ks * FtSmem::KV_BYTES);
+                const uint32_t qa = ft_smem(q_s), ka = ft_smem(k_s + ks * L::KV_BYTES);
 #pragma unroll
                 for (int k = 0; k < HEAD_DIM / 16; ++k) {
-                    const uint32_t off = (uint32_t)((k >> 2) * FT_ATOM_BYTES + (k & 3) * 32);
-                    ft_mma(tmem_s + (uint32_t)(s * FT_BN), ft_desc_kmajor(qa + off), ft_desc_kmajor(ka + off),
-                           idesc_s, k > 0 ? 1u : 0u);
+                    const uint32_t off = (uint32_t)((k & 3) * 32), atom = (uint32_t)(k >> 2);
+                    ft_mma(tmem_s + (uint32_t)(s * BN), ft_desc_kmajor(qa + atom * FT_ATOM_BYTES + off),
+                           ft_desc_kmajor(ka + atom * L::ATOM + off), idesc_s, k > 0 ? 1u : 0u);
                 }
                 ft_commit(&k_empty[ks]);            // the key stage is free once these MMAs have read it
                 ft_commit(&s_full[s]);
@@ -399,25 +417,25 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
                 // p_full of block i - 1 (a round ago) says the softmax has read that S, and P V of block
                 // i - 1 was issued before this
                 if (i + 1 < n_blocks && !issue_s(i + 1)) { ok = false; break; }
-                const int b = i & 1, vs = i % FT_STAGES;
-                if (!ft_wait(&v_full[vs], (uint32_t)(i / FT_STAGES) & 1u, abort_flag)) { ok = false; break; }
+                const int b = i & 1, vs = i % STAGES;
+                if (!ft_wait(&v_full[vs], (uint32_t)(i / STAGES) & 1u, abort_flag)) { ok = false; break; }
                 if (ROWS && i == n_blocks - 1) {
                     // what the last page holds behind the tile's last key may be anything, and a weight of zero does not
                     // make a value that is not finite vanish: those rows become zeros
-                    const int from = pos_last + 1 - (kb_begin + i) * FT_BN, to = (from + page_size - 1) / page_size * page_size;
+                    const int from = pos_last + 1 - (kb_begin + i) * BN, box = min(page_size, BN), to = (from + box - 1) / box * box;
                     for (int a = 0; a < FT_ATOMS; ++a)
                         for (int o = from * 128; o < to * 128; o += 16)
-                            *reinterpret_cast<uint4*>(v_s + vs * FtSmem::KV_BYTES + a * FT_ATOM_BYTES + o) = make_uint4(0u, 0u, 0u, 0u);
+                            *reinterpret_cast<uint4*>(v_s + vs * L::KV_BYTES + a * L::ATOM + o) = make_uint4(0u, 0u, 0u, 0u);
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 }
                 if (!ft_wait(&p_full[b], (uint32_t)(i >> 1) & 1u, abort_flag)) { ok = false; break; }
                 ft_fence_after();
                 // O (+)= P(i) V(i): A = P from tensor memory (rows in the lanes, 16 keys = 8 columns of
                 // bfloat16 pairs, at the start of S buffer b); B = V: MN-major, 16 keys = two 8-row groups
-                const uint32_t pa = tmem_s + (uint32_t)(b * FT_BN), va = ft_smem(v_s + vs * FtSmem::KV_BYTES);
+                const uint32_t pa = tmem_s + (uint32_t)(b * BN), va = ft_smem(v_s + vs * L::KV_BYTES);
 #pragma unroll
-                for (int k = 0; k < FT_BN / 16; ++k)
-                    ft_mma_ts(tmem_o, pa + (uint32_t)(k * 8), ft_desc_mnmajor(va + (uint32_t)(k * 16 * 128)), idesc_o,
+                for (int k = 0; k < BN / 16; ++k)
+                    ft_mma_ts(tmem_o, pa + (uint32_t)(k * 8), ft_desc_mnmajor(va + (uint32_t)(k * 16 * 128), L::ATOM), idesc_o,
                               (i > 0 || k > 0) ? 1u : 0u);
                 ft_commit(&v_empty[vs]);
                 ft_commit(&o_done[b]);              // O holds the blocks up to i
@@ -437,12 +455,13 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
         const int pos_r = ctx + row0 + r;
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
         // [round parity][part][row]: a round's values stay untouched while the next round's are written
-        float* part_max_all = reinterpret_cast<float*>(bars + FtSmem::BAR_SLOTS);
+        float* part_max_all = reinterpret_cast<float*>(bars + L::BAR_SLOTS);
         float m_run = -CUDART_INF_F, l_run = 0.0f;           // m_run: the maximum the scale in use is based on
         if (ROWS && sink != nullptr) {                       // the running maximum and sum start from the sink's term
             m_run = sink[h] * 1.4426950408889634f;
             l_run = part == 0 ? 1.0f : 0.0f;
         }
+        float l_odd = 0.0f;                                  // ROWS: l_run is for keys 0 and 1 of the thread's fours, this for the others
         bool ok = !*abort_flag;
         for (int i = 0; i < n_blocks && ok; ++i) {
             const int sb = i & 1;
@@ -452,6 +471,67 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
             if (i > 1 && !ft_warp_wait(&o_done[i & 1], (uint32_t)((i - 2) >> 1) & 1u, abort_flag)) FT_GIVE_UP();
             if (!ft_warp_wait(&s_full[sb], (uint32_t)(i >> 1) & 1u, abort_flag)) FT_GIVE_UP();
             ft_fence_after();
+            // O holds blocks 0 .. i - 1 once P V of block i - 1 is complete.  The whole warp reads,
+            // scales and writes its rows back (rows that keep their scale by 1): the loads and
+            // stores of tensor memory are warp-wide instructions.
+            auto rescale_o = [&](float corr) -> bool {
+                if (!ft_warp_wait(&o_done[(i - 1) & 1], (uint32_t)((i - 1) >> 1) & 1u, abort_flag)) return false;
+                ft_fence_after();
+#pragma unroll
+                for (int c = 0; c < FT_OD; c += 32) {
+                    uint32_t w[32];
+                    const uint32_t o_addr = tmem_o + lane_base + (uint32_t)(part * FT_OD + c);
+                    ft_ld32(o_addr, w);
+                    ft_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) w[j] = __float_as_uint(__uint_as_float(w[j]) * corr);
+                    ft_st32(o_addr, w);
+                }
+                return true;
+            };
+            if constexpr (ROWS) {
+                // of every eight keys four are this thread's, so that a row's partial sums are those of the other kernel
+                uint32_t w[32];
+#pragma unroll
+                for (int g = 0; g < 8; ++g) ft_ld4(tmem_s + (uint32_t)(sb * BN + g * 8 + part * 4) + lane_base, w + g * 4);
+                ft_ld_wait();
+                const int key0 = i * BN + part * 4;
+                const bool all_seen = i * BN + BN - 1 <= pos_r;
+                float x[32], mx = -CUDART_INF_F;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    const bool seen = all_seen || key0 + (j >> 2) * 8 + (j & 3) <= pos_r;
+                    x[j] = seen ? __fmul_rn(__fmul_rn(__uint_as_float(w[j]), scale), 1.4426950408889634f) : -CUDART_INF_F;
+                    mx = fmaxf(mx, x[j]);
+                }
+                float* part_max = part_max_all + sb * (FT_PARTS * 128);
+                part_max[part * 128 + r] = mx;
+                ft_warp_arrive(x_bar);                                    // past it S may be overwritten by P
+                if (!ft_warp_wait(x_bar, (uint32_t)i & 1u, abort_flag)) FT_GIVE_UP();
+                const float m_new = fmaxf(m_run, fmaxf(part_max[r], part_max[128 + r]));
+                const float corr = ft_weight(m_run, m_new);
+                m_run = m_new;
+                l_run *= corr;
+                l_odd *= corr;
+                uint32_t packed[16];
+#pragma unroll
+                for (int c = 0; c < 16; ++c) {
+                    const float p0 = ft_weight(x[2 * c], m_new), p1 = ft_weight(x[2 * c + 1], m_new);
+                    float& l = c & 1 ? l_odd : l_run;
+                    l += p0;
+                    l += p1;
+                    const __nv_bfloat162 b = __floats2bfloat162_rn(p0, p1);
+                    packed[c] = *reinterpret_cast<const uint32_t*>(&b);
+                }
+#pragma unroll
+                for (int g = 0; g < 8; ++g)
+                    ft_st2(tmem_s + (uint32_t)(sb * BN + g * 4 + part * 2) + lane_base, packed[2 * g], packed[2 * g + 1]);
+                if (i > 0 && __any_sync(0xffffffffu, corr != 1.0f) && !rescale_o(corr)) FT_GIVE_UP();
+                ft_st_wait();
+                ft_fence_before();
+                ft_warp_arrive(&p_full[sb]);
+                continue;
+            }
             const int key0 = (kb_begin + i) * FT_BN + part * FT_KP;      // first key of this thread's part
             const uint32_t s_addr = tmem_s + (uint32_t)(sb * FT_BN + part * FT_KP) + lane_base;
             const bool all_seen = (key0 + FT_KP - 1 <= pos_r) && (window <= 0 || key0 > pos_r - window);
@@ -492,23 +572,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
                 l_run *= corr;
                 m_run = m_new;
             }
-            if (any_rescale && i > 0) {
-                // O holds blocks 0 .. i - 1 once P V of block i - 1 is complete.  The whole warp reads,
-                // scales and writes its rows back (rows that keep their scale by 1): the loads and
-                // stores of tensor memory are warp-wide instructions.
-                if (!ft_warp_wait(&o_done[(i - 1) & 1], (uint32_t)((i - 1) >> 1) & 1u, abort_flag)) FT_GIVE_UP();
-                ft_fence_after();
-#pragma unroll
-                for (int c = 0; c < FT_OD; c += 32) {
-                    uint32_t w[32];
-                    const uint32_t o_addr = tmem_o + lane_base + (uint32_t)(part * FT_OD + c);
-                    ft_ld32(o_addr, w);
-                    ft_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) w[j] = __float_as_uint(__uint_as_float(w[j]) * corr);
-                    ft_st32(o_addr, w);
-                }
-            }
+            if (any_rescale && i > 0 && !rescale_o(corr)) FT_GIVE_UP();
             const float neg_m = (m_run == -CUDART_INF_F) ? 0.0f : -m_run;      // an empty row: every p below is 0
             float l4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             uint32_t packed[FT_KP / 2];
@@ -536,22 +600,18 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
             ft_fence_after();
         }
         float* part_sum = part_max_all + (n_blocks & 1) * (FT_PARTS * 128);
-        part_sum[part * 128 + r] = l_run;
+        part_sum[part * 128 + r] = ROWS ? l_run + l_odd : l_run;
         ft_warp_arrive(x_bar);
         const bool met = ft_warp_wait(x_bar, (uint32_t)n_blocks & 1u, abort_flag);
         float l_row = part_sum[r];
 #pragma unroll
         for (int q = 1; q < FT_PARTS; ++q) l_row += part_sum[q * 128 + r];
         if (met && ok && !*abort_flag && n_blocks > 0) {
-            float inv = 1.0f / l_row;
+            const float inv = 1.0f / l_row;
+            const bool by_channel = gate_cols > 1;            // else one number for the head
             const bf16* gate_row = nullptr;
-            if (ROWS && gate != nullptr && r < rows_here) {
-                gate_row = gate + (long)(tok0 + r) * gate_ld;
-                if (gate_cols == 1) {
-                    inv *= 1.0f / (1.0f + expf(-__bfloat162float(gate_row[h])));
-                    gate_row = nullptr;
-                }
-            }
+            if (ROWS && gate != nullptr && r < rows_here)
+                gate_row = gate + (long)(tok0 + r) * gate_ld + (long)h * gate_cols + (by_channel ? part * FT_OD : 0);
             bf16* dst = out + (long)(tok0 + r) * out_ld + (long)h * HEAD_DIM + part * FT_OD;
 #pragma unroll
             for (int c = 0; c < FT_OD; c += 32) {
@@ -567,9 +627,9 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
                         for (int e = 0; e < 4; ++e) {
                             float f0 = __uint_as_float(w[d + 2 * e]) * inv, f1 = __uint_as_float(w[d + 2 * e + 1]) * inv;
                             if (ROWS && gate_row != nullptr) {
-                                const bf16* gc = gate_row + h * HEAD_DIM + part * FT_OD + c + d + 2 * e;
-                                f0 *= 1.0f / (1.0f + expf(-__bfloat162float(gc[0])));
-                                f1 *= 1.0f / (1.0f + expf(-__bfloat162float(gc[1])));
+                                const int at = by_channel ? c + d + 2 * e : 0;
+                                f0 = f0 / (1.0f + expf(-__bfloat162float(gate_row[at])));
+                                f1 = f1 / (1.0f + expf(-__bfloat162float(gate_row[by_channel ? at + 1 : 0])));
                             }
                             wp[e] = __floats2bfloat162_rn(f0, f1);
                         }
@@ -636,12 +696,13 @@ static int ft_launch(const void* q, long q_ld, void* out, long out_ld, const voi
     CUtensorMap map_q, map_kv;
     int rc = ft_make_map(&map_q, q, n_tokens, (long)n_heads * HEAD_DIM, q_ld, FT_BM);
     if (rc) return rc;
-    rc = ft_make_map(&map_kv, cache, kv_rows, ROWS ? 2 * HEAD_DIM : HEAD_DIM, ROWS ? 2 * HEAD_DIM : HEAD_DIM, page_size);
+    rc = ft_make_map(&map_kv, cache, kv_rows, ROWS ? 2 * HEAD_DIM : HEAD_DIM, ROWS ? 2 * HEAD_DIM : HEAD_DIM,
+                     page_size < FtSmem<ROWS>::BN ? page_size : FtSmem<ROWS>::BN);
     if (rc) return rc;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             FtSmem::TOTAL);
+                                             FtSmem<ROWS>::TOTAL);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
@@ -649,9 +710,9 @@ static int ft_launch(const void* q, long q_ld, void* out, long out_ld, const voi
     if (max_tiles > 65535) return (int)cudaErrorInvalidValue;
     dim3 grid(n_heads, max_tiles);                 // heads fastest: every head's late (long) tiles start first
     // plain stream order (no programmatic overlap): this kernel takes all of an SM's tensor memory
-    attention_prefill_tc_kernel<ROWS><<<grid, FT_THREADS, FtSmem::TOTAL, stream>>>(
+    attention_prefill_tc_kernel<ROWS><<<grid, FT_THREADS, FtSmem<ROWS>::TOTAL, stream>>>(
         map_q, map_kv, (bf16*)out, out_ld, page_size, (int)kv_rows, block_table, bt_stride, req_start, req_ctx,
-        req_qlen, n_requests, include_single, n_heads, n_kv_heads, window, scale * 1.4426950408889634f, status, sink,
+        req_qlen, n_requests, include_single, n_heads, n_kv_heads, window, scale, status, sink,
         (const bf16*)gate, gate_ld, gate_cols);
     return fl_launch_status();
 }

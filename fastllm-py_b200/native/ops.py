@@ -860,7 +860,7 @@ def sink_rows_takes(dim: int, vdim: int, window, keep_first, cap, rel, chunk, pa
 
 
 def sink_attention_rows(q, out, cache, block_table, step, heads, kv_heads, size, scale, sink, page_size, include_single, gate):
-    """`sink_attention_tc` for layers that `sink_rows_takes`, on tcgen05 in tiles of 128 rows."""
+    """`sink_attention_mma` for layers that `sink_rows_takes`, on tcgen05 in tiles of 128 rows: the same bits."""
     from .gemm_tc import status_word
 
     fn = _fn("attention_prefill_tc", "fl_attention_prefill_rows",
@@ -873,19 +873,9 @@ def sink_attention_rows(q, out, cache, block_table, step, heads, kv_heads, size,
               *_gate_args(gate, out, heads, size), _ptr(status_word(q.device)), _stream()), "attention_prefill_rows")
 
 
-def sink_attention_tc(q, out, cache, block_table, step, heads, kv_heads, dim, vdim, window, keep_first, scale, cap,
-                      bucket_of, rel, sink, page_size, include_single=True, chunk=None, gate=None):
-    """`sink_attention_simt` on tensor cores: q, cache and out bfloat16; one build per (dim, vdim); 64 rows of a
-    request and one head per block, single tokens as tiles of one row (left out with include_single=False).  Prompts of
-    layers that `sink_rows_takes` go to tcgen05 in tiles of 128 rows."""
-    _require_cuda(q, out, cache, block_table, bucket_of, rel, sink, gate)
-    if q.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
-        raise KernelError("sink_attention_tc: q, cache and out must be bfloat16")
-    if sink_rows_takes(dim, vdim, window, keep_first, cap, rel, chunk, page_size) and cache.is_contiguous() \
-            and _ld(q) % 8 == 0 and _ld(out) % 8 == 0 and (q.data_ptr() | out.data_ptr() | cache.data_ptr()) % 16 == 0 \
-            and _sink_rows_pay(step, heads, include_single, sm_count(q.device)):
-        sink_attention_rows(q, out, cache, block_table, step, heads, kv_heads, dim, scale, sink, page_size, include_single, gate)
-        return
+def sink_attention_mma(q, out, cache, block_table, step, heads, kv_heads, dim, vdim, window, keep_first, scale, cap,
+                       bucket_of, rel, sink, page_size, include_single=True, chunk=None, gate=None):
+    """`sink_attention_simt` on mma.sync: one build per (dim, vdim); 64 rows of a request and one head per block."""
     name, defines = sink_tc_library(dim, vdim)
     fn = _fn(name, "fl_sink_attention_tc", [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_int, c_void_p, c_int,
                                             c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
@@ -896,6 +886,22 @@ def sink_attention_tc(q, out, cache, block_table, step, heads, kv_heads, dim, vd
               q.shape[0], int(include_single), heads, kv_heads, int(window or 0), int(keep_first or 0), int(chunk or 0),
               float(scale), float(cap or 0.0), _ptr(bucket_of), 0 if bucket_of is None else bucket_of.numel(), _ptr(rel), _ptr(sink),
               *_gate_args(gate, out, heads, vdim), _stream()), "sink_attention_tc")
+
+
+def sink_attention_tc(q, out, cache, block_table, step, heads, kv_heads, dim, vdim, window, keep_first, scale, cap,
+                      bucket_of, rel, sink, page_size, include_single=True, chunk=None, gate=None):
+    """`sink_attention_simt` on tensor cores: q, cache and out bfloat16; single tokens as tiles of one row (left out with
+    include_single=False).  Layers that `sink_rows_takes` go to the faster one of two kernels, which give the same bits."""
+    _require_cuda(q, out, cache, block_table, bucket_of, rel, sink, gate)
+    if q.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
+        raise KernelError("sink_attention_tc: q, cache and out must be bfloat16")
+    if sink_rows_takes(dim, vdim, window, keep_first, cap, rel, chunk, page_size) and cache.is_contiguous() \
+            and _ld(q) % 8 == 0 and _ld(out) % 8 == 0 and (q.data_ptr() | out.data_ptr() | cache.data_ptr()) % 16 == 0 \
+            and _sink_rows_pay(step, heads, include_single, sm_count(q.device)):
+        sink_attention_rows(q, out, cache, block_table, step, heads, kv_heads, dim, scale, sink, page_size, include_single, gate)
+        return
+    sink_attention_mma(q, out, cache, block_table, step, heads, kv_heads, dim, vdim, window, keep_first, scale, cap, bucket_of,
+                       rel, sink, page_size, include_single, chunk, gate)
 
 
 SINK_SPLIT = 128                 # keys of one split of the single-token kernel

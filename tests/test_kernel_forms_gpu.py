@@ -69,6 +69,51 @@ def test_prompt_attention_over_rows_of_keys_and_values(size, heads, kv_heads, pa
     assert not bool(alone[single].any()) and torch.equal(alone[:single], got[:single]) and torch.equal(alone[single + 1:], got[single + 1:])
 
 
+def prompts_over_rows(lens, size, heads, kv_heads, page, seed):
+    """Queries, a cache of rows k | v in shuffled pages and a step for requests of (cached, new) tokens."""
+    torch.manual_seed(seed)
+    per = [-(-(c + m) // page) for c, m in lens]
+    cache = torch.randn(sum(per), kv_heads, page, 2 * size, device="cuda").to(torch.bfloat16)
+    order = torch.randperm(sum(per), device="cuda").to(torch.int32)
+    bt = torch.zeros(len(lens), max(per), dtype=torch.int32, device="cuda")
+    for r, n in enumerate(per):
+        bt[r, :n] = order[sum(per[:r]):sum(per[:r]) + n]
+    starts = [sum(m for _, m in lens[:r]) for r in range(len(lens) + 1)]
+    step = SimpleNamespace(req_start=i32(starts), req_ctx=i32([c for c, _ in lens]), req_qlen=i32([m for _, m in lens]),
+                           n_requests=len(lens), q_lens=[m for _, m in lens], ctx_lens=[c for c, _ in lens])
+    return torch.randn(starts[-1], heads * size, device="cuda").to(torch.bfloat16), cache, bt, step
+
+
+@pytest.mark.parametrize("size,heads,kv_heads,page", [(128, 4, 2, 16), (64, 6, 3, 8), (128, 2, 1, 64), (64, 2, 2, 128)])
+@pytest.mark.parametrize("sink,gate", [(None, None), (1.0, "head"), (60.0, "channel"), (-60.0, None)])
+def test_both_prompt_kernels_over_rows_give_the_same_bits(size, heads, kv_heads, page, sink, gate):
+    """Prompts of a few tokens and of many key blocks (the ring goes round; more than 64 blocks are asked for at once), at
+    positions that are and are not multiples of 64, sinks far above and far below the scores; against float64 the
+    weights' and the result's rounding to bfloat16, 2^-9 of the largest value each."""
+    lens = [(0, 300), (4300, 150), (130, 129), (63, 66), (64, 128), (1, 1), (700, 1), (0, 2), (500, 17), (0, 2)]
+    q, cache, bt, step = prompts_over_rows(lens, size, heads, kv_heads, page, size + heads)
+    n, scale = q.shape[0], 3 * size ** -0.5
+    g = None if gate is None else torch.randn(n, heads if gate == "head" else heads * size, device="cuda").to(torch.bfloat16)
+    s = None if sink is None else torch.randn(heads, device="cuda") + sink
+    want, got = torch.empty_like(q), torch.zeros_like(q)
+    ops.sink_attention_mma(q, want, cache, bt, step, heads, kv_heads, size, size, None, 0, scale, None, None, None, s, page, gate=g)
+    ops.sink_attention_rows(q, got, cache, bt, step, heads, kv_heads, size, scale, s, page, True, g)
+    assert torch.equal(got, want)
+    start = 0
+    for r, (c, m) in enumerate(lens):
+        kv = cache[bt[r, :-(-(c + m) // page)].long()].permute(1, 0, 2, 3).reshape(kv_heads, -1, 2 * size)[:, :c + m].double()
+        kv = kv.repeat_interleave(heads // kv_heads, 0)
+        scores = q[start:start + m].view(m, heads, size).transpose(0, 1).double() @ kv[..., :size].transpose(1, 2) * scale
+        scores += torch.full((m, c + m), float("-inf"), device="cuda", dtype=torch.double).triu(c + 1)
+        extra = torch.full((heads, m, 1), float("-inf"), device="cuda", dtype=torch.double) if s is None else s.double().view(-1, 1, 1).expand(-1, m, 1)
+        ref = (torch.cat([scores, extra], -1).softmax(-1)[..., :-1] @ kv[..., size:]).transpose(0, 1).reshape(m, heads * size)
+        if g is not None:
+            gate_of = g[start:start + m].double().sigmoid()
+            ref = ref * (gate_of.repeat_interleave(size, 1) if gate == "head" else gate_of)
+        assert float((got[start:start + m].double() - ref).abs().max()) <= 2 ** -8 * float(kv[..., size:].abs().max())
+        start += m
+
+
 @pytest.mark.parametrize("m,n,k", [(17, 4, 4), (64, 130, 36), (65, 1664, 260), (66, 1800, 264), (200, 1700, 520), (400, 1300, 2048), (257, 2500, 300)])
 def test_products_of_32_bits_in_tiles(m, n, k):
     """One to four CTAs an SM, slices that are short or empty, rows and features that are not there (whose neighbours in memory
