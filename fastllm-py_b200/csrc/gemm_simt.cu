@@ -117,10 +117,10 @@ __global__ void __launch_bounds__(256, 4) gemm_simt_kernel(const TA* __restrict_
 #define SK_BK 32
 #define SK_PITCH 36
 
-template <int MT> struct Skinny {
-    static constexpr int RT = 2;
+template <int MT, int RT_> struct Skinny {
+    static constexpr int RT = RT_;
     static constexpr int R = 8 * RT;
-    static constexpr int STAGES = MT > 8 || MT == 4 ? 3 : 4;
+    static constexpr int STAGES = RT == 2 && (MT > 8 || MT == 4) ? 3 : 4;
     static constexpr int A_PITCH = MT * SK_BK + 4;                     // floats of a slice's rows of A
     static constexpr int W_FLOATS = GS_SLICES * R * SK_PITCH;
     static constexpr int STAGE_FLOATS = W_FLOATS + GS_SLICES * A_PITCH;
@@ -132,12 +132,12 @@ __device__ __forceinline__ void sk_cp16(float* smem, const float* gmem, bool val
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(valid ? 16 : 0) : "memory");
 }
 
-template <typename TC, int MT>
+template <typename TC, int MT, int RT_>
 __global__ void __launch_bounds__(64) gemm_f32_skinny_kernel(const float* __restrict__ A, long lda,
                                                              const float* __restrict__ W, long ldw,
                                                              TC* __restrict__ C, long ldc, int M, int N, int K, int slice,
                                                              int constant_w) {
-    using L = Skinny<MT>;
+    using L = Skinny<MT, RT_>;
     constexpr int RT = L::RT, R = L::R, STAGES = L::STAGES;
     extern __shared__ __align__(16) float sk_smem[];
     const int tid = threadIdx.x, row = tid & 7, s = tid >> 3;
@@ -214,15 +214,15 @@ __global__ void __launch_bounds__(64) gemm_f32_skinny_kernel(const float* __rest
 }
 
 // ------------------------------------------------------------ more rows
-// A cluster of GS_SLICES CTAs shares a tile of 64 rows x TL_BN features; each sums one slice, and each adds up an eighth of
-// the rows from the others' shared memory, in the order of the slices, so no partial sum goes to global memory.  Bound by
+// SPLIT: a cluster of GS_SLICES CTAs shares a tile of 64 rows x TL_BN features; each sums one slice, and each adds up an eighth
+// of the rows from the others' shared memory, in the order of the slices, so no partial sum goes to global memory.  Else one CTA
+// sums the slices of a tile one after the other, which is the faster form where a slice is short (see gs_f32).  Bound by
 // the multiply-adds, which are issued in pairs (fma.rn.f32x2, the same rounding), and by what they read from shared memory
 // (128 bytes a clock reach the registers, however many lanes want the same): 8 rows x 8 features a thread.  Both operands
 // wait in shared memory turned to [input][row], double-buffered; columns are exchanged by a pattern of the input's index, so
 // that neither the turned stores nor the 16-byte reads meet in a bank.  The next stage comes by cp.async into slots that only
-// the copying thread reads, so it needs no registers meanwhile and four CTAs fit an SM.  (300 rows, 11008 features of 2048:
-// 409 us with the next stage in registers, two CTAs an SM and a tile split only where that filled the last wave better; 305
-// now, 44 TFLOP/s.  Every value of A twice in shared memory instead of a move for each pair of features, or 64 x 256 tiles:
+// the copying thread reads, so it needs no registers meanwhile and four CTAs of a split tile fit an SM.  (300 rows, 11008
+// features of 2048: 409 us with the next stage in registers and two CTAs an SM; 305 now, 44 TFLOP/s.  Every value of A twice in shared memory instead of a move for each pair of features, or 64 x 256 tiles:
 // 347 and 327 us at best.)
 #define TL_BM 64
 #define TL_BN 128
@@ -237,18 +237,15 @@ __device__ __forceinline__ void fma2(float2& d, const float2 a, const float2 b) 
         : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
 }
 
-template <typename TC>
-__global__ void __cluster_dims__(1, 1, GS_SLICES) __launch_bounds__(TL_THREADS, 4)
-    gemm_f32_tile_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw, TC* __restrict__ C,
-                         long ldc, int M, int N, int K, int slice) {
+template <typename TC, bool SPLIT>
+__device__ __forceinline__ void gemm_f32_tile(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw,
+                                              TC* __restrict__ C, long ldc, int M, int N, int K, int slice) {
     constexpr int A_FLOATS = TL_BK * TL_BM, STAGE = A_FLOATS + TL_BK * TL_BN, PIECES = (TL_BM + TL_BN) / 32;
     extern __shared__ __align__(16) float tl_smem[];                    // two stages and the copies' slots; the tile's sums
     float4(*raw)[TL_THREADS] = reinterpret_cast<float4(*)[TL_THREADS]>(tl_smem + 2 * STAGE);
-    pdl_wait();
-    pdl_trigger();
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int m0 = blockIdx.y * TL_BM, n0 = blockIdx.x * TL_BN;
-    const int k_begin = min(K, (int)blockIdx.z * slice), k_end = min(K, k_begin + slice);
+    const int k_begin = SPLIT ? min(K, (int)blockIdx.z * slice) : 0, k_end = SPLIT ? min(K, k_begin + slice) : K;
     // this thread's 16-byte pieces of a stage: rows lr, lr + 32, ... of A (two) and W, inputs 4 lk .. 4 lk + 3
     const int lr = tid >> 2, lk = tid & 3;
     auto fetch = [&](int k0) {
@@ -274,18 +271,21 @@ __global__ void __cluster_dims__(1, 1, GS_SLICES) __launch_bounds__(TL_THREADS, 
             d[0] = v.x, d[pitch] = v.y, d[2 * pitch] = v.z, d[3 * pitch] = v.w;
         }
     };
-    float2 acc[8][2 * TL_NH];                                           // 8 rows x pairs of features
+    float2 acc[8][2 * TL_NH], total[SPLIT ? 1 : 8][2 * TL_NH];          // 8 rows x pairs of features
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 2 * TL_NH; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+        for (int j = 0; j < 2 * TL_NH; ++j) {
+            acc[i][j] = make_float2(0.0f, 0.0f);
+            if (!SPLIT) total[i][j] = make_float2(0.0f, 0.0f);
+        }
     if (k_begin < k_end) {
         fetch(k_begin);
         turn(0);
         if (k_begin + TL_BK < k_end) fetch(k_begin + TL_BK);
     }
     __syncthreads();
-    int buf = 0;
+    int buf = 0, left = slice;
     for (int k0 = k_begin; k0 < k_end; k0 += TL_BK) {
         if (k0 + TL_BK < k_end) {
             turn(buf ^ 1);
@@ -312,50 +312,119 @@ __global__ void __cluster_dims__(1, 1, GS_SLICES) __launch_bounds__(TL_THREADS, 
                 for (int j = 0; j < 2 * TL_NH; ++j) fma2(acc[i][j], aa, b[j]);
             }
         }
+        if (!SPLIT) {
+            left -= TL_BK;
+            if (left == 0 || k0 + TL_BK >= k_end) {                     // the slice is complete
+                left = slice;
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 2 * TL_NH; ++j) {
+                        total[i][j].x += acc[i][j].x;
+                        total[i][j].y += acc[i][j].y;
+                        acc[i][j] = make_float2(0.0f, 0.0f);
+                    }
+            }
+        }
         __syncthreads();
         buf ^= 1;
     }
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int h = 0; h < TL_NH; ++h)
-            *reinterpret_cast<float4*>(tl_smem + ((i >> 2) * 32 + ty * 4 + (i & 3)) * TL_BN + h * 64 + tx * 4) =
-                make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x, acc[i][2 * h + 1].y);
-    cluster.sync();
-    // an eighth of the tile's rows are this CTA's to add up: four features a thread
-#pragma unroll
-    for (int e = tid; e < TL_BM / GS_SLICES * TL_BN / 4; e += TL_THREADS) {
-        const int r = (int)blockIdx.z * (TL_BM / GS_SLICES) + e / (TL_BN / 4), c = e % (TL_BN / 4) * 4;
-        float sum[4] = {};
-#pragma unroll
-        for (int z = 0; z < GS_SLICES; ++z) {
-            const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(tl_smem, z) + r * TL_BN + c);
-            sum[0] += v.x, sum[1] += v.y, sum[2] += v.z, sum[3] += v.w;
-        }
-        const int m = m0 + r, n = n0 + c;
-        if (m >= M) continue;
+    auto store = [&](int m, int n, const float (&v)[4]) {               // four features of one row
+        if (m >= M) return;
         TC* out = C + (long)m * ldc + n;
         if (sizeof(TC) == 4 && n + 4 <= N && ((uintptr_t)out & 15) == 0) {
-            *reinterpret_cast<float4*>(out) = make_float4(sum[0], sum[1], sum[2], sum[3]);
+            *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
         } else {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-                if (n + j < N) out[j] = from_f32<TC>(sum[j]);
+                if (n + j < N) out[j] = from_f32<TC>(v[j]);
         }
+    };
+    if constexpr (!SPLIT) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int h = 0; h < TL_NH; ++h) {
+                const float v[4] = {total[i][2 * h].x, total[i][2 * h].y, total[i][2 * h + 1].x, total[i][2 * h + 1].y};
+                store(m0 + (i >> 2) * 32 + ty * 4 + (i & 3), n0 + h * 64 + tx * 4, v);
+            }
+    } else {
+        namespace cg = cooperative_groups;
+        cg::cluster_group cluster = cg::this_cluster();
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int h = 0; h < TL_NH; ++h)
+                *reinterpret_cast<float4*>(tl_smem + ((i >> 2) * 32 + ty * 4 + (i & 3)) * TL_BN + h * 64 + tx * 4) =
+                    make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x, acc[i][2 * h + 1].y);
+        cluster.sync();
+        // an eighth of the tile's rows are this CTA's to add up: four features a thread
+#pragma unroll
+        for (int e = tid; e < TL_BM / GS_SLICES * TL_BN / 4; e += TL_THREADS) {
+            const int r = (int)blockIdx.z * (TL_BM / GS_SLICES) + e / (TL_BN / 4), c = e % (TL_BN / 4) * 4;
+            float sum[4] = {};
+#pragma unroll
+            for (int z = 0; z < GS_SLICES; ++z) {
+                const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(tl_smem, z) + r * TL_BN + c);
+                sum[0] += v.x, sum[1] += v.y, sum[2] += v.z, sum[3] += v.w;
+            }
+            store(m0 + r, n0 + c, sum);
+        }
+        cluster.sync();                                                 // no CTA leaves while another reads its sums
     }
-    cluster.sync();                                                     // no CTA leaves while another reads its sums
+}
+
+template <typename TC, int EACH>
+__global__ void __cluster_dims__(1, 1, GS_SLICES) __launch_bounds__(TL_THREADS, EACH)
+    gemm_f32_tile_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw, TC* __restrict__ C,
+                         long ldc, int M, int N, int K, int slice) {
+    pdl_wait();
+    pdl_trigger();
+    gemm_f32_tile<TC, true>(A, lda, W, ldw, C, ldc, M, N, K, slice);
+}
+
+template <typename TC>
+__global__ void __launch_bounds__(TL_THREADS, 2)
+    gemm_f32_whole_tile_kernel(const float* __restrict__ A, long lda, const float* __restrict__ W, long ldw, TC* __restrict__ C,
+                               long ldc, int M, int N, int K, int slice) {
+    pdl_wait();
+    pdl_trigger();
+    gemm_f32_tile<TC, false>(A, lda, W, ldw, C, ldc, M, N, K, slice);
 }
 
 // ------------------------------------------------------------ host side
-template <typename TC, int MT>
+template <typename TC, int MT, int RT = 2>
 static int gs_skinny(const float* A, long lda, const float* W, long ldw, TC* C, long ldc, int M, int N, int K, int constant_w, cudaStream_t stream) {
-    using L = Skinny<MT>;
-    auto kernel = gemm_f32_skinny_kernel<TC, MT>;
+    using L = Skinny<MT, RT>;
+    auto kernel = gemm_f32_skinny_kernel<TC, MT, RT>;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
     if (err != cudaSuccess) return (int)err;
     return fl_launch(kernel, dim3((N + L::R - 1) / L::R), dim3(64), L::SMEM, stream, A, lda, W, ldw, C, ldc, M, N, K, gs_slice(K), constant_w);
+}
+
+template <typename TC, int EACH>
+static int gs_split(dim3 grid, int smem, const float* A, long lda, const float* W, long ldw, TC* C, long ldc, int M, int N, int K, int slice,
+                    cudaStream_t stream) {
+    auto kernel = gemm_f32_tile_kernel<TC, EACH>;
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024);
+    if (err != cudaSuccess) return (int)err;
+    return fl_launch(kernel, grid, dim3(TL_THREADS), smem, stream, A, lda, W, ldw, C, ldc, M, N, K, slice);
+}
+
+// The time of a product in whole and in split tiles, microseconds, fitted to 220 products of 17 to 2048 rows, 64 to 32000
+// features and 16 to 5504 inputs.  Whole tiles, two an SM: 0.094 us an input for a round of them (0.06 where there is one an
+// SM).  Split ones, four CTAs an SM: 0.19 us an input of a slice, and 6 us for a round's start and exchange, which is what a
+// slice of 32 inputs costs too: 2048 x 2048 x 64 takes 60 us split and 15 whole, 500 x 2048 x 128 19 and 9.6, 1024 x 32000 x 256
+// 469 and 349; 300 x 2048 x 256 14 and 18, 300 x 5504 x 2048 162 and 201.  The choice is right or within 3 %.
+static double gs_whole_us(long tiles, int K, int sms) {
+    const long rest = tiles % (2 * sms);
+    const double round = 3.0 + 0.0935 * K;
+    return tiles / (2 * sms) * round + (rest == 0 ? 0.0 : rest <= sms ? 1.7 + 0.06 * K : round);
+}
+static double gs_split_us(long tiles, int slice, int sms) {
+    const long ctas = tiles * GS_SLICES, rest = ctas % (4 * sms);
+    if (ctas <= sms * 7 / 4) return 1.5 + 0.011 * ctas + 0.098 * slice;          // all at once, two an SM at most
+    return 3.0 + (2.9 + 0.188 * slice) * (ctas / (4 * sms) + (rest + sms - 1) / sms * 0.25);
 }
 
 // Float operands that 16-byte loads can read.  Up to 16 rows W's bytes decide and the skinny kernel streams them; above,
@@ -370,19 +439,19 @@ static int gs_f32(const float* A, long lda, const float* W, long ldw, TC* C, lon
     if (M <= 16) return gs_skinny<TC, 16>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
     dim3 grid((N + TL_BN - 1) / TL_BN, (M + TL_BM - 1) / TL_BM, GS_SLICES);
     if (grid.y > 65535) return (int)cudaErrorInvalidValue;
+    const int slice = gs_slice(K);
+    if (gs_whole_us((long)grid.x * grid.y, K, sms) < gs_split_us((long)grid.x * grid.y, slice, sms)) {
+        grid.z = 1;
+        return fl_launch(gemm_f32_whole_tile_kernel<TC>, grid, dim3(TL_THREADS), TL_SMEM, stream, A, lda, W, ldw, C, ldc, M, N, K, slice);
+    }
     // Four CTAs fit an SM, and the clusters of a product of few tiles would be packed so, beside idle SMs: more shared memory
     // than they use keeps one, two or three an SM where that many hold all tiles (100 x 2048 x 2048: 36.4 us so packed, 31.8
-    // two an SM).  A cluster lies within a GPC: at one CTA an SM they reach 3 of 4 SMs (of 16 tiles one waits for another to
-    // end: 17 x 2048 x 2048 took 39.6 us), at two or three 7 of 8.
-    int smem = TL_SMEM;
+    // two an SM), and there they may use more registers (29.8).  A cluster lies within a GPC: at one CTA an SM they reach 3 of 4
+    // SMs (of 16 tiles one waits for another to end: 17 x 2048 x 2048 took 39.6 us), at two or three 7 of 8.
     for (int each = 1; each < 4; ++each)
-        if ((long)grid.x * grid.y * GS_SLICES <= (each == 1 ? sms * 3L / 4 : (long)sms * each * 7 / 8)) {
-            smem = 228 * 1024 / (each + 1) - 1024 + 128;                // (each CTA takes 1 KB more than it asks for)
-            break;
-        }
-    cudaError_t err = cudaFuncSetAttribute(gemm_f32_tile_kernel<TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024);
-    if (err != cudaSuccess) return (int)err;
-    return fl_launch(gemm_f32_tile_kernel<TC>, grid, dim3(TL_THREADS), smem, stream, A, lda, W, ldw, C, ldc, M, N, K, gs_slice(K));
+        if ((long)grid.x * grid.y * GS_SLICES <= (each == 1 ? sms * 3L / 4 : (long)sms * each * 7 / 8))
+            return gs_split<TC, 3>(grid, 228 * 1024 / (each + 1) - 1024 + 128, A, lda, W, ldw, C, ldc, M, N, K, slice, stream);
+    return gs_split<TC, 4>(grid, TL_SMEM, A, lda, W, ldw, C, ldc, M, N, K, slice, stream);      // (a CTA takes 1 KB more than it asks for)
 }
 
 // constant_w: no kernel that may still run when this one is launched writes W (which is then read ahead of it).

@@ -129,3 +129,19 @@ def test_products_of_32_bits_in_tiles(m, n, k):
     ops.gemm_simt(odd, w[:n], want)
     assert torch.equal(got[:m, :n], want)
     assert bool((got[m] == 7).all()) and bool((got[:, n:] == 7).all())
+
+
+@pytest.mark.parametrize("m,n,k", [(17, 2048, 16), (300, 2048, 64), (65, 8200, 72), (1100, 300, 100), (200, 2050, 260), (70, 32000, 256), (513, 4100, 516)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_products_of_32_bits_in_whole_tiles(m, n, k, dtype):
+    """Tiles that one CTA sums, slice after slice (few inputs, or many tiles): bit for bit the kernel for any operands."""
+    torch.manual_seed(m + n + k)
+    a, w = torch.randn(m, k, device="cuda"), torch.randn(n, k, device="cuda")
+    got = torch.full((m + 1, n + 3), 7.0, device="cuda", dtype=dtype)
+    ops.gemm_simt(a, w, got[:m, :n])
+    odd = torch.empty(m * (k + 1), device="cuda").view(m, k + 1)[:, 1:]
+    odd.copy_(a)
+    want = torch.empty(m, n, device="cuda", dtype=dtype)
+    ops.gemm_simt(odd, w, want)
+    assert torch.equal(got[:m, :n], want)
+    assert bool((got[m] == 7).all()) and bool((got[:, n:] == 7).all())
