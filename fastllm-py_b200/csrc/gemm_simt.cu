@@ -17,7 +17,7 @@
 //   gemm_f32_tile_kernel    float operands, more rows: bound by the multiply-adds
 //   gemm_simt_kernel        any operand types, alignments and batches
 // The last one served everything before: 350 us a product for 4 rows and 590 us for 300 rows of a layer with 2048 and
-// 5504 columns (10 TFLOP/s); the others take 7 to 25 us (2.3 to 3.7 TB/s of W, out of a cold cache) and 67 to 305 us (37
+// 5504 columns (10 TFLOP/s); the others take 6 to 21 us (2.7 to 4.3 TB/s of W, out of a cold cache) and 67 to 305 us (37
 // to 44 TFLOP/s).
 #include <cooperative_groups.h>
 
@@ -102,12 +102,12 @@ __global__ void __launch_bounds__(256, 4) gemm_simt_kernel(const TA* __restrict_
 }
 
 // ------------------------------------------------------------ up to 16 rows
-// A CTA of 64 threads serves 16 features: thread (slice s, row r) sums slice s of features r and r + 8 for all MT
+// A CTA of 64 threads serves 8 x RT features: thread (slice s, row r) sums slice s of features r, r + 8, ... for all MT
 // rows of A.  W and A pass through a ring of shared-memory stages, 32 inputs of every slice each, filled by 16-byte
 // cp.async: what bounds the product is the stream of W, so the ring keeps 2 or 3 stages (16 KB of W each, two or three CTAs an
 // SM) in flight, and where the caller says that no kernel writes W (constant_w) its first stages are asked for before the
 // preceding kernel has ended.  A staged row of W is padded
-// to 36 floats: the eight lanes of a quarter warp, on eight rows, then read all 32 banks.  A value of A that has been read
+// to 36 floats: the eight lanes of a quarter warp, on eight rows, then read all 32 banks.  With RT = 2 a value of A that has been read
 // from shared memory serves two features: with one, the reads of A kept more shared memory busy than W did (11008 features
 // of 2048, out of a cold cache: 21.7, 22.2, 29.1 and 25.0 us for 1 to 4 rows; 19.1, 20.1, 21.0 and 21.2 now, 4.2 to 4.7 TB/s
 // of W; 2048 features 6.1 to 8.0, now 5.6 to 6.4).  A third stage in flight costs four rows 5 to 10 % on many features, as
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(64) gemm_f32_skinny_kernel(const float* __rest
         float* dst = sk_smem + (t % STAGES) * L::STAGE_FLOATS + L::W_FLOATS + s * L::A_PITCH + row * 4;
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
-            const bool in = k < K && (MT > 4 || m < M);
+            const bool in = k < K && (MT != 4 || m < M);                // (below, M is MT)
             sk_cp16(dst + m * SK_BK, in ? A + (long)(MT > 4 ? min(m, M - 1) : m) * lda + k : A, in);
         }
     };
@@ -393,13 +393,25 @@ __global__ void __launch_bounds__(TL_THREADS, 2)
 }
 
 // ------------------------------------------------------------ host side
-template <typename TC, int MT, int RT = 2>
+template <typename TC, int MT, int RT>
 static int gs_skinny(const float* A, long lda, const float* W, long ldw, TC* C, long ldc, int M, int N, int K, int constant_w, cudaStream_t stream) {
     using L = Skinny<MT, RT>;
     auto kernel = gemm_f32_skinny_kernel<TC, MT, RT>;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
     if (err != cudaSuccess) return (int)err;
     return fl_launch(kernel, dim3((N + L::R - 1) / L::R), dim3(64), L::SMEM, stream, A, lda, W, ldw, C, ldc, M, N, K, gs_slice(K), constant_w);
+}
+
+// Features a CTA: two for a thread (RT = 2, above), but one where that leaves SMs idle or busy unevenly.  What is compared is the
+// features that the busiest SM gets.  Up to two rows, out of a cold cache: 256 of 2048 inputs 3.6 us with one and 4.2 with two,
+// 5504 11.6 and 12.4, 2048 6.2 and 5.5, 32256 60.8 and 48.7.  From three rows on two are the better ones as soon as every SM
+// has some (1024 of 2048 4.8 and 5.7 us, 2048 6.7 and 6.4, 5504 15.5 and 12.9).
+template <typename TC, int MT>
+static int gs_few_rows(const float* A, long lda, const float* W, long ldw, TC* C, long ldc, int M, int N, int K, int sms, int constant_w,
+                       cudaStream_t stream) {
+    const int one = ((N + 7) / 8 + sms - 1) / sms, two = 2 * (((N + 15) / 16 + sms - 1) / sms);
+    if (one < two && (MT <= 2 || one == 1)) return gs_skinny<TC, MT, 1>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
+    return gs_skinny<TC, MT, 2>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
 }
 
 template <typename TC, int EACH>
@@ -432,11 +444,11 @@ static double gs_split_us(long tiles, int slice, int sms) {
 template <typename TC>
 static int gs_f32(const float* A, long lda, const float* W, long ldw, TC* C, long ldc, int M, int N, int K, int sms,
                   int constant_w, cudaStream_t stream) {
-    if (M <= 1) return gs_skinny<TC, 1>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
-    if (M <= 2) return gs_skinny<TC, 2>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
-    if (M <= 4) return gs_skinny<TC, 4>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
-    if (M <= 8) return gs_skinny<TC, 8>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
-    if (M <= 16) return gs_skinny<TC, 16>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
+    if (M <= 1) return gs_few_rows<TC, 1>(A, lda, W, ldw, C, ldc, M, N, K, sms, constant_w, stream);
+    if (M <= 2) return gs_few_rows<TC, 2>(A, lda, W, ldw, C, ldc, M, N, K, sms, constant_w, stream);
+    if (M <= 4) return gs_few_rows<TC, 4>(A, lda, W, ldw, C, ldc, M, N, K, sms, constant_w, stream);
+    if (M <= 8) return gs_skinny<TC, 8, 2>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
+    if (M <= 16) return gs_skinny<TC, 16, 2>(A, lda, W, ldw, C, ldc, M, N, K, constant_w, stream);
     dim3 grid((N + TL_BN - 1) / TL_BN, (M + TL_BM - 1) / TL_BM, GS_SLICES);
     if (grid.y > 65535) return (int)cudaErrorInvalidValue;
     const int slice = gs_slice(K);

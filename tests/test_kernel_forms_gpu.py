@@ -145,3 +145,20 @@ def test_products_of_32_bits_in_whole_tiles(m, n, k, dtype):
     ops.gemm_simt(odd, w, want)
     assert torch.equal(got[:m, :n], want)
     assert bool((got[m] == 7).all()) and bool((got[:, n:] == 7).all())
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4])
+@pytest.mark.parametrize("n,k", [(1, 4), (255, 2052), (1184, 260), (1185, 260), (2500, 36), (5504, 100)])
+def test_products_of_32_bits_of_few_rows(m, n, k):
+    """Eight and sixteen features a CTA: bit for bit the kernel for any operands; rows that are not there are not read."""
+    torch.manual_seed(m + n + k)
+    a, w = torch.full((m + 3, k), float("nan"), device="cuda"), torch.randn(n, k, device="cuda")
+    a[:m] = torch.randn(m, k, device="cuda")
+    got = torch.full((m + 1, n + 3), 7.0, device="cuda")
+    ops.gemm_simt(a[:m], w, got[:m, :n], constant_w=True)
+    odd = torch.empty(m * (k + 1), device="cuda").view(m, k + 1)[:, 1:]
+    odd.copy_(a[:m])
+    want = torch.empty(m, n, device="cuda")
+    ops.gemm_simt(odd, w, want)
+    assert torch.equal(got[:m, :n], want)
+    assert bool((got[m] == 7).all()) and bool((got[:, n:] == 7).all())
