@@ -209,7 +209,7 @@ template <bool ROWS> struct FtSmem {
     static constexpr int KV_BYTES = FT_ATOMS * ATOM;                   // one of K or V, one stage
     static constexpr int TILES = Q_BYTES + 2 * STAGES * KV_BYTES;
     static constexpr int BAR_SLOTS = 24 + 4 * STAGES;                  // 8-byte slots: barriers and the like
-    static constexpr int BARS = BAR_SLOTS * 8 + 2 * FT_PARTS * 128 * 4; // ... then the parts' maxima (two rounds)
+    static constexpr int BARS = BAR_SLOTS * 8 + (ROWS ? 4 : 2) * FT_PARTS * 128 * 4;   // ... then the parts' maxima (two rounds; ROWS: and sums)
     // The tiles want a 1024-byte boundary.  Where they fill the SM's shared memory to within a KB
     // there is no room to round up to one: the kernel then counts on the dynamic shared memory
     // starting on such a boundary (it has no static shared memory) and reports FT_ERR_SMEM instead
@@ -462,6 +462,31 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
             l_run = part == 0 ? 1.0f : 0.0f;
         }
         float l_odd = 0.0f;                                  // ROWS: l_run is for keys 0 and 1 of the thread's fours, this for the others
+        // 32 columns of this thread's part of the row, from column c, with the row's sum
+        auto write_row = [&](const uint32_t (&w)[32], int c, float l_row) {
+            const float inv = 1.0f / l_row;
+            const bool by_channel = gate_cols > 1;            // else one number for the head
+            const bf16* gate_row = nullptr;
+            if (ROWS && gate != nullptr)
+                gate_row = gate + (long)(tok0 + r) * gate_ld + (long)h * gate_cols + (by_channel ? part * FT_OD : 0);
+            bf16* dst = out + (long)(tok0 + r) * out_ld + (long)h * HEAD_DIM + part * FT_OD;
+#pragma unroll
+            for (int d = 0; d < 32; d += 8) {
+                uint4 o4;
+                __nv_bfloat162* wp = reinterpret_cast<__nv_bfloat162*>(&o4);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float f0 = __uint_as_float(w[d + 2 * e]) * inv, f1 = __uint_as_float(w[d + 2 * e + 1]) * inv;
+                    if (ROWS && gate_row != nullptr) {
+                        const int at = by_channel ? c + d + 2 * e : 0;
+                        f0 = f0 / (1.0f + expf(-__bfloat162float(gate_row[at])));
+                        f1 = f1 / (1.0f + expf(-__bfloat162float(gate_row[by_channel ? at + 1 : 0])));
+                    }
+                    wp[e] = __floats2bfloat162_rn(f0, f1);
+                }
+                *reinterpret_cast<uint4*>(dst + c + d) = o4;
+            }
+        };
         bool ok = !*abort_flag;
         for (int i = 0; i < n_blocks && ok; ++i) {
             const int sb = i & 1;
@@ -473,8 +498,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
             ft_fence_after();
             // O holds blocks 0 .. i - 1 once P V of block i - 1 is complete.  The whole warp reads,
             // scales and writes its rows back (rows that keep their scale by 1): the loads and
-            // stores of tensor memory are warp-wide instructions.
-            auto rescale_o = [&](float corr) -> bool {
+            // stores of tensor memory are warp-wide instructions.  Rows that are `over` have seen their last block and are written.
+            auto rescale_o = [&](float corr, bool over, float l_row) -> bool {
                 if (!ft_warp_wait(&o_done[(i - 1) & 1], (uint32_t)((i - 1) >> 1) & 1u, abort_flag)) return false;
                 ft_fence_after();
 #pragma unroll
@@ -483,6 +508,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
                     const uint32_t o_addr = tmem_o + lane_base + (uint32_t)(part * FT_OD + c);
                     ft_ld32(o_addr, w);
                     ft_ld_wait();
+                    if (ROWS && over) write_row(w, c, l_row);
 #pragma unroll
                     for (int j = 0; j < 32; ++j) w[j] = __float_as_uint(__uint_as_float(w[j]) * corr);
                     ft_st32(o_addr, w);
@@ -505,7 +531,9 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
                     mx = fmaxf(mx, x[j]);
                 }
                 float* part_max = part_max_all + sb * (FT_PARTS * 128);
+                float* part_l = part_max + 2 * FT_PARTS * 128;
                 part_max[part * 128 + r] = mx;
+                part_l[part * 128 + r] = l_run + l_odd;
                 ft_warp_arrive(x_bar);                                    // past it S may be overwritten by P
                 if (!ft_warp_wait(x_bar, (uint32_t)i & 1u, abort_flag)) FT_GIVE_UP();
                 const float m_new = fmaxf(m_run, fmaxf(part_max[r], part_max[128 + r]));
@@ -526,7 +554,11 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
 #pragma unroll
                 for (int g = 0; g < 8; ++g)
                     ft_st2(tmem_s + (uint32_t)(sb * BN + g * 4 + part * 2) + lane_base, packed[2 * g], packed[2 * g + 1]);
-                if (i > 0 && __any_sync(0xffffffffu, corr != 1.0f) && !rescale_o(corr)) FT_GIVE_UP();
+                // A row that sees no key of this block or of later ones is done here, before their values are added: a weight of
+                // zero does not make a value that is not finite vanish.
+                const bool over = i > 0 && r < rows_here && pos_r / BN + 1 == i;
+                if (i > 0 && __any_sync(0xffffffffu, corr != 1.0f || over) &&
+                    !rescale_o(corr, over, part_l[r] + part_l[128 + r])) FT_GIVE_UP();
                 ft_st_wait();
                 ft_fence_before();
                 ft_warp_arrive(&p_full[sb]);
@@ -572,7 +604,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
                 l_run *= corr;
                 m_run = m_new;
             }
-            if (any_rescale && i > 0 && !rescale_o(corr)) FT_GIVE_UP();
+            if (any_rescale && i > 0 && !rescale_o(corr, false, 0.0f)) FT_GIVE_UP();
             const float neg_m = (m_run == -CUDART_INF_F) ? 0.0f : -m_run;      // an empty row: every p below is 0
             float l4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             uint32_t packed[FT_KP / 2];
@@ -607,35 +639,13 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
 #pragma unroll
         for (int q = 1; q < FT_PARTS; ++q) l_row += part_sum[q * 128 + r];
         if (met && ok && !*abort_flag && n_blocks > 0) {
-            const float inv = 1.0f / l_row;
-            const bool by_channel = gate_cols > 1;            // else one number for the head
-            const bf16* gate_row = nullptr;
-            if (ROWS && gate != nullptr && r < rows_here)
-                gate_row = gate + (long)(tok0 + r) * gate_ld + (long)h * gate_cols + (by_channel ? part * FT_OD : 0);
-            bf16* dst = out + (long)(tok0 + r) * out_ld + (long)h * HEAD_DIM + part * FT_OD;
+            const bool mine = r < rows_here && (!ROWS || pos_r / BN + 1 == n_blocks);
 #pragma unroll
             for (int c = 0; c < FT_OD; c += 32) {
                 uint32_t w[32];
                 ft_ld32(tmem_o + lane_base + (uint32_t)(part * FT_OD + c), w);      // all lanes of the warp take part
                 ft_ld_wait();
-                if (r < rows_here) {
-#pragma unroll
-                    for (int d = 0; d < 32; d += 8) {
-                        uint4 o4;
-                        __nv_bfloat162* wp = reinterpret_cast<__nv_bfloat162*>(&o4);
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            float f0 = __uint_as_float(w[d + 2 * e]) * inv, f1 = __uint_as_float(w[d + 2 * e + 1]) * inv;
-                            if (ROWS && gate_row != nullptr) {
-                                const int at = by_channel ? c + d + 2 * e : 0;
-                                f0 = f0 / (1.0f + expf(-__bfloat162float(gate_row[at])));
-                                f1 = f1 / (1.0f + expf(-__bfloat162float(gate_row[by_channel ? at + 1 : 0])));
-                            }
-                            wp[e] = __floats2bfloat162_rn(f0, f1);
-                        }
-                        *reinterpret_cast<uint4*>(dst + c + d) = o4;
-                    }
-                }
+                if (mine) write_row(w, c, l_row);
             }
         }
     }

@@ -114,6 +114,25 @@ def test_both_prompt_kernels_over_rows_give_the_same_bits(size, heads, kv_heads,
         start += m
 
 
+@pytest.mark.parametrize("size,page", [(128, 16), (64, 128)])
+@pytest.mark.parametrize("ctx,at", [(0, 64), (0, 127), (48, 200), (37, 130), (64, 64)])
+def test_values_that_are_not_finite_reach_no_block_before_theirs(size, page, ctx, at):
+    """A row is done once the blocks of 64 keys that it sees are added up: an infinite value at position `at` leaves the rows of
+    earlier blocks as they are (where 16 rows do not cross into another block, also the rest is the other kernel's)."""
+    lens, heads = [(ctx, 300)], 2
+    q, cache, bt, step = prompts_over_rows(lens, size, heads, 1, page, ctx + at)
+    clean, got, want = torch.zeros_like(q), torch.zeros_like(q), torch.zeros_like(q)
+    args = (bt, step, heads, 1, size)
+    ops.sink_attention_rows(q, clean, cache, *args, size ** -0.5, None, page, True, None)
+    cache[int(bt[0, at // page]), 0, at % page, size:] = float("inf")
+    ops.sink_attention_rows(q, got, cache, *args, size ** -0.5, None, page, True, None)
+    ops.sink_attention_mma(q, want, cache, *args, size, None, 0, size ** -0.5, None, None, None, None, page)
+    before = at // 64 * 64 - ctx
+    assert before <= 0 or torch.equal(got[:before], clean[:before])
+    if ctx % 16 == 0:
+        assert torch.equal(got.isfinite(), want.isfinite()) and torch.equal(got.nan_to_num(), want.nan_to_num())
+
+
 @pytest.mark.parametrize("m,n,k", [(17, 4, 4), (64, 130, 36), (65, 1664, 260), (66, 1800, 264), (200, 1700, 520), (400, 1300, 2048), (257, 2500, 300)])
 def test_products_of_32_bits_in_tiles(m, n, k):
     """One to four CTAs an SM, slices that are short or empty, rows and features that are not there (whose neighbours in memory
