@@ -254,6 +254,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
     uint64_t* o_done = bars + 11;                                      // [2] P V of block i is done: barrier i & 1, phase i >> 1
     uint32_t* tmem_slot = (uint32_t*)(bars + 13);
     uint64_t* x_bar = bars + 14;                                       // the softmax threads' exchange point
+    uint64_t* z_full = bars + 16;                                      // the last block's values are cleared behind the last key
     uint64_t* v_full = k_empty + STAGES;
     uint64_t* v_empty = v_full + STAGES;
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
@@ -287,6 +288,11 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
     const int lo_tile = window > 0 ? max(0, pos_first - window + 1) : 0;
     const int kb_begin = lo_tile / BN, kb_end = pos_last / BN + 1;
     const int n_blocks = kb_end - kb_begin;
+    // ROWS: what the last page holds behind the tile's last key may be anything, and a weight of zero does not make a value that is
+    // not finite vanish: the values' producer warp clears rows clear_from .. clear_to - 1 of the last block
+    const int page_box = min(page_size, BN), clear_from = pos_last + 1 - (kb_end - 1) * BN;
+    const int clear_to = (clear_from + page_box - 1) / page_box * page_box;
+    const bool clears = ROWS && clear_from < clear_to;
 
     // ---- the producers' side of a block: one box of a page and 64 columns per lane.  A block of 128 keys is
     // pages x atoms boxes of a few KB; one lane issues one box (looking up its page itself), so a block's
@@ -297,22 +303,22 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
     auto issue_block = [&](int i) {
         unsigned char* ring = is_v ? v_s : k_s;
         const int* bt = block_table + (long)req * bt_stride;
-        const int box = min(page_size, BN), n_ops = (BN / box) * FT_ATOMS;
+        const int n_ops = (BN / page_box) * FT_ATOMS;
         const int s = i % STAGES;
         if (lane == 0) ft_bar_expect(&full[s], L::KV_BYTES);
         __syncwarp();
         const int key0 = (kb_begin + i) * BN;
         for (int op = lane; op < n_ops; op += 32) {
             const int p = op / FT_ATOMS, a = op % FT_ATOMS;
-            const int first_key = key0 + p * box;
-            const int last_key = first_key + box - 1;
+            const int first_key = key0 + p * page_box;
+            const int last_key = first_key + page_box - 1;
             // a page (or the part of one that lies in the block) wholly outside what this tile may see is fetched from beyond the tensor: zeros
             int row = kv_rows_total;
             if (first_key <= pos_last && last_key >= lo_tile) {
                 const long pg = bt[first_key / page_size];
                 row = (int)((ROWS ? pg * n_kv_heads + kvh : (pg * 2 + is_v) * n_kv_heads + kvh) * page_size) + (ROWS ? first_key % page_size : 0);
             }
-            const int off = s * L::KV_BYTES + a * L::ATOM + p * box * 128;
+            const int off = s * L::KV_BYTES + a * L::ATOM + p * page_box * 128;
             ft_tma_2d(ring + off, &map_kv, &full[s], a * 64 + (ROWS ? is_v * HEAD_DIM : 0), row);
         }
     };
@@ -348,6 +354,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
             ft_bar_init(&o_done[s], 1);
         }
         ft_bar_init(x_bar, FT_SOFTMAX_WARPS);
+        ft_bar_init(z_full, 1);
         *abort_flag = (*(volatile int*)status != 0) ? 1 : 0;
         *never = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -381,6 +388,19 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
         for (; i < n_blocks && !*abort_flag; ++i) {
             if (!ft_warp_wait(&empty[i % STAGES], ((uint32_t)(i / STAGES) & 1u) ^ 1u, abort_flag)) FT_GIVE_UP();
             issue_block(i);
+        }
+        if (clears && is_v && i == n_blocks) {
+            const int s = (n_blocks - 1) % STAGES;
+            if (ft_warp_wait(&full[s], (uint32_t)((n_blocks - 1) / STAGES) & 1u, abort_flag)) {
+                for (int a = 0; a < FT_ATOMS; ++a)
+                    for (int o = clear_from * 128 + lane * 16; o < clear_to * 128; o += 512)
+                        *reinterpret_cast<uint4*>(v_s + s * L::KV_BYTES + a * L::ATOM + o) = make_uint4(0u, 0u, 0u, 0u);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                ft_warp_arrive(z_full);
+            } else if (!*abort_flag) {
+                *abort_flag = 1;
+                atomicCAS(status, 0, FT_ERR_WAIT);
+            }
         }
         if (*abort_flag) {
             // leaving early: the copies still on their way must land before the shared memory goes to
@@ -419,15 +439,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
                 if (i + 1 < n_blocks && !issue_s(i + 1)) { ok = false; break; }
                 const int b = i & 1, vs = i % STAGES;
                 if (!ft_wait(&v_full[vs], (uint32_t)(i / STAGES) & 1u, abort_flag)) { ok = false; break; }
-                if (ROWS && i == n_blocks - 1) {
-                    // what the last page holds behind the tile's last key may be anything, and a weight of zero does not
-                    // make a value that is not finite vanish: those rows become zeros
-                    const int from = pos_last + 1 - (kb_begin + i) * BN, box = min(page_size, BN), to = (from + box - 1) / box * box;
-                    for (int a = 0; a < FT_ATOMS; ++a)
-                        for (int o = from * 128; o < to * 128; o += 16)
-                            *reinterpret_cast<uint4*>(v_s + vs * L::KV_BYTES + a * L::ATOM + o) = make_uint4(0u, 0u, 0u, 0u);
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                }
+                if (clears && i == n_blocks - 1 && !ft_wait(z_full, 0, abort_flag)) { ok = false; break; }
                 if (!ft_wait(&p_full[b], (uint32_t)(i >> 1) & 1u, abort_flag)) { ok = false; break; }
                 ft_fence_after();
                 // O (+)= P(i) V(i): A = P from tensor memory (rows in the lanes, 16 keys = 8 columns of
