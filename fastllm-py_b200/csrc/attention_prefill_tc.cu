@@ -46,15 +46,6 @@ static_assert(HEAD_DIM == 64 || HEAD_DIM == 128, "the tcgen05 prefill kernel tak
 #ifndef FT_PARTS
 #define FT_PARTS 2                         // softmax threads per query row
 #endif
-#define FT_KP (FT_BN / FT_PARTS)           // keys of a block per softmax thread
-#define FT_OD (HEAD_DIM / FT_PARTS)        // output columns per softmax thread
-static_assert(FT_OD % 32 == 0 && FT_KP % 32 == 0, "a softmax thread owns multiples of 32 keys and of 32 columns");
-#define FT_SOFTMAX_THREADS (128 * FT_PARTS)
-#define FT_SOFTMAX_WARPS (FT_SOFTMAX_THREADS / 32)
-#define FT_PRODUCER_WARP FT_SOFTMAX_WARPS                      // queries and keys
-#define FT_MMA_WARP (FT_SOFTMAX_WARPS + 1)
-#define FT_VPRODUCER_WARP (FT_SOFTMAX_WARPS + 2)              // values
-#define FT_THREADS ((FT_SOFTMAX_WARPS + 3) * 32)
 #define FT_ATOMS (HEAD_DIM / 64)           // 64-column swizzle atoms per row
 #define FT_ATOM_BYTES (128 * 128)          // 128 rows x 128 bytes
 #define FT_WAIT_LIMIT_NS 2000000000ull
@@ -148,6 +139,12 @@ __device__ __forceinline__ void ft_ld4(uint32_t taddr, uint32_t* r) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
 }
+__device__ __forceinline__ void ft_ld2(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void ft_st1(uint32_t taddr, uint32_t a) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(a) : "memory");
+}
 __device__ __forceinline__ void ft_st2(uint32_t taddr, uint32_t a, uint32_t b) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(taddr), "r"(a), "r"(b) : "memory");
 }
@@ -203,13 +200,15 @@ __device__ __forceinline__ float ft_weight(float a, float b) { return (a == -CUD
 // ROWS (see the kernel): blocks of 64 keys, and stages for as much of the SM's shared memory as leaves room for one CTA.
 template <bool ROWS> struct FtSmem {
     static constexpr int BN = ROWS ? 64 : FT_BN;                       // keys of a block
+    static constexpr int PARTS = ROWS && HEAD_DIM == 128 ? 4 : FT_PARTS;   // softmax threads per query row
+    static constexpr int SOFTMAX_WARPS = 4 * PARTS, THREADS = (SOFTMAX_WARPS + 3) * 32;
     static constexpr int STAGES = ROWS ? (HEAD_DIM == 128 ? 5 : 6) : FT_STAGES;
     static constexpr int ATOM = BN * 128;                              // bytes of 64 columns of a block
     static constexpr int Q_BYTES = FT_ATOMS * FT_ATOM_BYTES;
     static constexpr int KV_BYTES = FT_ATOMS * ATOM;                   // one of K or V, one stage
     static constexpr int TILES = Q_BYTES + 2 * STAGES * KV_BYTES;
     static constexpr int BAR_SLOTS = 24 + 4 * STAGES;                  // 8-byte slots: barriers and the like
-    static constexpr int BARS = BAR_SLOTS * 8 + (ROWS ? 4 : 2) * FT_PARTS * 128 * 4;   // ... then the parts' maxima (two rounds; ROWS: and sums)
+    static constexpr int BARS = BAR_SLOTS * 8 + (ROWS ? 4 : 2) * PARTS * 128 * 4;   // ... then the parts' maxima (two rounds; ROWS: and sums)
     // The tiles want a 1024-byte boundary.  Where they fill the SM's shared memory to within a KB
     // there is no room to round up to one: the kernel then counts on the dynamic shared memory
     // starting on such a boundary (it has no static shared memory) and reports FT_ERR_SMEM instead
@@ -226,7 +225,7 @@ template <bool ROWS> struct FtSmem {
 // made by the same instructions, four partial sums of a row's weights (keys 2c and 2c + 1 of every eight), values in K steps
 // of 16 from the first to the last.  The results are the same bit for bit.
 template <bool ROWS>
-__global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
+__global__ void __launch_bounds__(FtSmem<ROWS>::THREADS, 1) attention_prefill_tc_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
     bf16* __restrict__ out, long out_ld, int page_size, int kv_rows_total, const int* __restrict__ block_table,
     int bt_stride, const int* __restrict__ req_start, const int* __restrict__ req_ctx,
@@ -234,7 +233,11 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
     int window, float scale, int* __restrict__ status, const float* __restrict__ sink, const bf16* __restrict__ gate,
     long gate_ld, int gate_cols) {
     using L = FtSmem<ROWS>;
-    constexpr int BN = L::BN, STAGES = L::STAGES;
+    constexpr int BN = L::BN, STAGES = L::STAGES, PARTS = L::PARTS;
+    constexpr int KP = BN / PARTS, OD = HEAD_DIM / PARTS;              // a softmax thread's keys of a block, and output columns
+    static_assert(OD % 32 == 0 && (ROWS || KP % 32 == 0), "multiples of 32 columns; of 32 keys, where these are neighbours");
+    constexpr int PRODUCER_WARP = L::SOFTMAX_WARPS;                    // queries and keys
+    constexpr int MMA_WARP = PRODUCER_WARP + 1, VPRODUCER_WARP = PRODUCER_WARP + 2;   // (VPRODUCER: values)
     const float scale_log2e = scale * 1.4426950408889634f;
     extern __shared__ __align__(1024) unsigned char ft_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)ft_raw + 1023) & ~(uintptr_t)1023);
@@ -261,10 +264,10 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
     volatile int* never = (volatile int*)(bars + 15);                  // stays 0: for waits that must not be cut short
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool producer = warp == FT_PRODUCER_WARP || warp == FT_VPRODUCER_WARP;
+    const bool producer = warp == PRODUCER_WARP || warp == VPRODUCER_WARP;
     if (producer && lane == 0) {
         // the copies' descriptors are wanted first thing: ask for them while the tile is being worked out
-        if (warp == FT_PRODUCER_WARP) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&map_q) : "memory");
+        if (warp == PRODUCER_WARP) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&map_q) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&map_kv) : "memory");
     }
     // which request and which 128-row tile: blockIdx.y counts tiles, a request's last (longest) tile first
@@ -297,7 +300,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
     // ---- the producers' side of a block: one box of a page and 64 columns per lane.  A block of 128 keys is
     // pages x atoms boxes of a few KB; one lane issues one box (looking up its page itself), so a block's
     // copies leave together.
-    const int is_v = warp == FT_VPRODUCER_WARP ? 1 : 0;
+    const int is_v = warp == VPRODUCER_WARP ? 1 : 0;
     uint64_t* full = is_v ? v_full : k_full;
     uint64_t* empty = is_v ? v_empty : k_empty;
     auto issue_block = [&](int i) {
@@ -350,17 +353,17 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
     if (threadIdx.x == 0) {
         for (int s = 0; s < 2; ++s) {
             ft_bar_init(&s_full[s], 1);
-            ft_bar_init(&p_full[s], FT_SOFTMAX_WARPS);
+            ft_bar_init(&p_full[s], L::SOFTMAX_WARPS);
             ft_bar_init(&o_done[s], 1);
         }
-        ft_bar_init(x_bar, FT_SOFTMAX_WARPS);
+        ft_bar_init(x_bar, L::SOFTMAX_WARPS);
         ft_bar_init(z_full, 1);
         *abort_flag = (*(volatile int*)status != 0) ? 1 : 0;
         *never = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == FT_MMA_WARP) {
+    if (warp == MMA_WARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ft_smem(tmem_slot)),
                      "r"(512u)
                      : "memory");
@@ -409,7 +412,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
                 ft_warp_wait(&full[k % STAGES], (uint32_t)(k / STAGES) & 1u, never);
             if (!is_v && lane == 0) ft_wait(q_full, 0, never);
         }
-    } else if (warp == FT_MMA_WARP) {
+    } else if (warp == MMA_WARP) {
         if (lane == 0 && !*abort_flag) {
             // ---- MMA issuer.  The tensor core runs what this thread issues in order, so S(i + 2),
             // which goes where S(i) and then P(i) were, follows P V of block i without a barrier.
@@ -455,8 +458,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
             if (!ok && !*abort_flag) { *abort_flag = 1; atomicCAS(status, 0, FT_ERR_WAIT); }
         }
     } else {
-        // ---- softmax: FT_PARTS threads (r, r + 128, ...) share query row r; `part` says which
-        // FT_KP keys of a block and which FT_OD output columns a thread owns.  P goes back into
+        // ---- softmax: PARTS threads (r, r + 128, ...) share query row r; `part` says which
+        // KP keys of a block and which OD output columns a thread owns.  P goes back into
         // tensor memory, over the first half of the S it was made from, as the A operand of P V,
         // and O stays in tensor memory, where P V accumulates; it is rescaled (read, multiplied,
         // written back by these threads) only when a row's maximum has grown by more than 2^8
@@ -474,14 +477,18 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
             l_run = part == 0 ? 1.0f : 0.0f;
         }
         float l_odd = 0.0f;                                  // ROWS: l_run is for keys 0 and 1 of the thread's fours, this for the others
+        auto row_sum = [&](const float* sums) -> float {     // ROWS: pairs first, as the other kernel's lanes add them
+            if (PARTS == 4) return (sums[r] + sums[128 + r]) + (sums[2 * 128 + r] + sums[3 * 128 + r]);
+            return sums[r] + sums[128 + r];
+        };
         // 32 columns of this thread's part of the row, from column c, with the row's sum
         auto write_row = [&](const uint32_t (&w)[32], int c, float l_row) {
             const float inv = 1.0f / l_row;
             const bool by_channel = gate_cols > 1;            // else one number for the head
             const bf16* gate_row = nullptr;
             if (ROWS && gate != nullptr)
-                gate_row = gate + (long)(tok0 + r) * gate_ld + (long)h * gate_cols + (by_channel ? part * FT_OD : 0);
-            bf16* dst = out + (long)(tok0 + r) * out_ld + (long)h * HEAD_DIM + part * FT_OD;
+                gate_row = gate + (long)(tok0 + r) * gate_ld + (long)h * gate_cols + (by_channel ? part * OD : 0);
+            bf16* dst = out + (long)(tok0 + r) * out_ld + (long)h * HEAD_DIM + part * OD;
 #pragma unroll
             for (int d = 0; d < 32; d += 8) {
                 uint4 o4;
@@ -514,98 +521,112 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
             auto rescale_o = [&](float corr, bool over, float l_row) -> bool {
                 if (!ft_warp_wait(&o_done[(i - 1) & 1], (uint32_t)((i - 1) >> 1) & 1u, abort_flag)) return false;
                 ft_fence_after();
+                const uint32_t o_addr = tmem_o + lane_base + (uint32_t)(part * OD);
+                uint32_t w[OD / 32][32];
 #pragma unroll
-                for (int c = 0; c < FT_OD; c += 32) {
-                    uint32_t w[32];
-                    const uint32_t o_addr = tmem_o + lane_base + (uint32_t)(part * FT_OD + c);
-                    ft_ld32(o_addr, w);
-                    ft_ld_wait();
-                    if (ROWS && over) write_row(w, c, l_row);
+                for (int c = 0; c < OD / 32; ++c) ft_ld32(o_addr + (uint32_t)(c * 32), w[c]);
+                ft_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) w[j] = __float_as_uint(__uint_as_float(w[j]) * corr);
-                    ft_st32(o_addr, w);
+                for (int c = 0; c < OD / 32; ++c) {
+                    if (ROWS && over) write_row(w[c], c * 32, l_row);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) w[c][j] = __float_as_uint(__uint_as_float(w[c][j]) * corr);
+                    ft_st32(o_addr + (uint32_t)(c * 32), w[c]);
                 }
                 return true;
             };
             if constexpr (ROWS) {
-                // of every eight keys four are this thread's, so that a row's partial sums are those of the other kernel
-                uint32_t w[32];
+                // of every eight keys E (neighbours) are this thread's, so that a row's partial sums are those of the other kernel
+                constexpr int E = 8 / PARTS;
+                uint32_t w[KP];
 #pragma unroll
-                for (int g = 0; g < 8; ++g) ft_ld4(tmem_s + (uint32_t)(sb * BN + g * 8 + part * 4) + lane_base, w + g * 4);
-                ft_ld_wait();
-                const int key0 = i * BN + part * 4;
-                const bool all_seen = i * BN + BN - 1 <= pos_r;
-                float x[32], mx = -CUDART_INF_F;
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const bool seen = all_seen || key0 + (j >> 2) * 8 + (j & 3) <= pos_r;
-                    x[j] = seen ? __fmul_rn(__fmul_rn(__uint_as_float(w[j]), scale), 1.4426950408889634f) : -CUDART_INF_F;
-                    mx = fmaxf(mx, x[j]);
+                for (int g = 0; g < 8; ++g) {
+                    const uint32_t s_addr = tmem_s + (uint32_t)(sb * BN + g * 8 + part * E) + lane_base;
+                    if constexpr (E == 4) ft_ld4(s_addr, w + g * E);
+                    else ft_ld2(s_addr, w + g * E);
                 }
-                float* part_max = part_max_all + sb * (FT_PARTS * 128);
-                float* part_l = part_max + 2 * FT_PARTS * 128;
+                ft_ld_wait();
+                const int key0 = i * BN + part * E;
+                float x[KP], mx4[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+#pragma unroll
+                for (int j = 0; j < KP; ++j) x[j] = __fmul_rn(__fmul_rn(__uint_as_float(w[j]), scale), 1.4426950408889634f);
+                if (i * BN + BN - 1 > pos_r) {
+#pragma unroll
+                    for (int j = 0; j < KP; ++j)
+                        if (key0 + j / E * 8 + j % E > pos_r) x[j] = -CUDART_INF_F;
+                }
+#pragma unroll
+                for (int j = 0; j < KP; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], x[j]);
+                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+                float* part_max = part_max_all + sb * (PARTS * 128);
+                float* part_l = part_max + 2 * PARTS * 128;
                 part_max[part * 128 + r] = mx;
                 part_l[part * 128 + r] = l_run + l_odd;
                 ft_warp_arrive(x_bar);                                    // past it S may be overwritten by P
                 if (!ft_warp_wait(x_bar, (uint32_t)i & 1u, abort_flag)) FT_GIVE_UP();
-                const float m_new = fmaxf(m_run, fmaxf(part_max[r], part_max[128 + r]));
+                float m_new = fmaxf(m_run, part_max[r]);
+#pragma unroll
+                for (int q = 1; q < PARTS; ++q) m_new = fmaxf(m_new, part_max[q * 128 + r]);
                 const float corr = ft_weight(m_run, m_new);
                 m_run = m_new;
                 l_run *= corr;
                 l_odd *= corr;
-                uint32_t packed[16];
+                uint32_t packed[KP / 2];
 #pragma unroll
-                for (int c = 0; c < 16; ++c) {
+                for (int c = 0; c < KP / 2; ++c) {
                     const float p0 = ft_weight(x[2 * c], m_new), p1 = ft_weight(x[2 * c + 1], m_new);
-                    float& l = c & 1 ? l_odd : l_run;
+                    float& l = E == 4 && (c & 1) ? l_odd : l_run;
                     l += p0;
                     l += p1;
                     const __nv_bfloat162 b = __floats2bfloat162_rn(p0, p1);
                     packed[c] = *reinterpret_cast<const uint32_t*>(&b);
                 }
 #pragma unroll
-                for (int g = 0; g < 8; ++g)
-                    ft_st2(tmem_s + (uint32_t)(sb * BN + g * 4 + part * 2) + lane_base, packed[2 * g], packed[2 * g + 1]);
+                for (int g = 0; g < 8; ++g) {
+                    const uint32_t p_addr = tmem_s + (uint32_t)(sb * BN + g * 4 + part * E / 2) + lane_base;
+                    if constexpr (E == 4) ft_st2(p_addr, packed[2 * g], packed[2 * g + 1]);
+                    else ft_st1(p_addr, packed[g]);
+                }
                 // A row that sees no key of this block or of later ones is done here, before their values are added: a weight of
                 // zero does not make a value that is not finite vanish.
                 const bool over = i > 0 && r < rows_here && pos_r / BN + 1 == i;
                 if (i > 0 && __any_sync(0xffffffffu, corr != 1.0f || over) &&
-                    !rescale_o(corr, over, part_l[r] + part_l[128 + r])) FT_GIVE_UP();
+                    !rescale_o(corr, over, row_sum(part_l))) FT_GIVE_UP();
                 ft_st_wait();
                 ft_fence_before();
                 ft_warp_arrive(&p_full[sb]);
                 continue;
             }
-            const int key0 = (kb_begin + i) * FT_BN + part * FT_KP;      // first key of this thread's part
-            const uint32_t s_addr = tmem_s + (uint32_t)(sb * FT_BN + part * FT_KP) + lane_base;
-            const bool all_seen = (key0 + FT_KP - 1 <= pos_r) && (window <= 0 || key0 > pos_r - window);
-            uint32_t v[FT_KP];
+            const int key0 = (kb_begin + i) * FT_BN + part * KP;      // first key of this thread's part
+            const uint32_t s_addr = tmem_s + (uint32_t)(sb * FT_BN + part * KP) + lane_base;
+            const bool all_seen = (key0 + KP - 1 <= pos_r) && (window <= 0 || key0 > pos_r - window);
+            uint32_t v[KP];
 #pragma unroll
-            for (int c = 0; c < FT_KP; c += 32) ft_ld32(s_addr + (uint32_t)c, v + c);
+            for (int c = 0; c < KP; c += 32) ft_ld32(s_addr + (uint32_t)c, v + c);
             ft_ld_wait();
             if (!all_seen) {
 #pragma unroll
-                for (int j = 0; j < FT_KP; ++j) {
+                for (int j = 0; j < KP; ++j) {
                     const int key = key0 + j;
                     if (!(key <= pos_r && (window <= 0 || key > pos_r - window))) v[j] = 0xff800000u;   // -inf
                 }
             }
             float mx4[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
 #pragma unroll
-            for (int j = 0; j < FT_KP; j += 4) {
+            for (int j = 0; j < KP; j += 4) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) mx4[e] = fmaxf(mx4[e], __uint_as_float(v[j + e]));
             }
             const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
             // exchange the parts' maxima (one barrier among the softmax warps per block); past it
             // every softmax thread has its S in registers, so the S buffer may take P
-            float* part_max = part_max_all + (i & 1) * (FT_PARTS * 128);
+            float* part_max = part_max_all + (i & 1) * (PARTS * 128);
             part_max[part * 128 + r] = mx;
             ft_warp_arrive(x_bar);                                        // (an mbarrier: its wait can give up)
             if (!ft_warp_wait(x_bar, (uint32_t)i & 1u, abort_flag)) FT_GIVE_UP();
             float mx_row = part_max[r];
 #pragma unroll
-            for (int q = 1; q < FT_PARTS; ++q) mx_row = fmaxf(mx_row, part_max[q * 128 + r]);
+            for (int q = 1; q < PARTS; ++q) mx_row = fmaxf(mx_row, part_max[q * 128 + r]);
             const float m_new = fmaxf(m_run, mx_row * scale_log2e);
             // the row's threads decide alike: they see the same maxima
             const bool rescale = m_new > m_run + 8.0f || (m_run == -CUDART_INF_F && m_new != -CUDART_INF_F);
@@ -619,9 +640,9 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
             if (any_rescale && i > 0 && !rescale_o(corr, false, 0.0f)) FT_GIVE_UP();
             const float neg_m = (m_run == -CUDART_INF_F) ? 0.0f : -m_run;      // an empty row: every p below is 0
             float l4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            uint32_t packed[FT_KP / 2];
+            uint32_t packed[KP / 2];
 #pragma unroll
-            for (int c = 0; c < FT_KP / 2; ++c) {
+            for (int c = 0; c < KP / 2; ++c) {
                 const float p0 = ft_ex2(fmaf(__uint_as_float(v[2 * c]), scale_log2e, neg_m));
                 const float p1 = ft_ex2(fmaf(__uint_as_float(v[2 * c + 1]), scale_log2e, neg_m));
                 l4[c & 3] += p0 + p1;
@@ -629,10 +650,10 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
                 packed[c] = *reinterpret_cast<const uint32_t*>(&b);
             }
             l_run += (l4[0] + l4[1]) + (l4[2] + l4[3]);
-            // P(i): this thread's FT_KP keys as FT_KP / 2 columns of bfloat16 pairs
+            // P(i): this thread's KP keys as KP / 2 columns of bfloat16 pairs
 #pragma unroll
-            for (int c = 0; c < FT_KP / 2; c += 32)
-                ft_st32(tmem_s + (uint32_t)(sb * FT_BN + part * (FT_KP / 2) + c) + lane_base, packed + c);
+            for (int c = 0; c < KP / 2; c += 32)
+                ft_st32(tmem_s + (uint32_t)(sb * FT_BN + part * (KP / 2) + c) + lane_base, packed + c);
             ft_st_wait();
             ft_fence_before();
             ft_warp_arrive(&p_full[sb]);
@@ -643,19 +664,17 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
             if (!ok && !*abort_flag) { *abort_flag = 1; atomicCAS(status, 0, FT_ERR_WAIT); }
             ft_fence_after();
         }
-        float* part_sum = part_max_all + (n_blocks & 1) * (FT_PARTS * 128);
+        float* part_sum = part_max_all + (n_blocks & 1) * (PARTS * 128);
         part_sum[part * 128 + r] = ROWS ? l_run + l_odd : l_run;
         ft_warp_arrive(x_bar);
         const bool met = ft_warp_wait(x_bar, (uint32_t)n_blocks & 1u, abort_flag);
-        float l_row = part_sum[r];
-#pragma unroll
-        for (int q = 1; q < FT_PARTS; ++q) l_row += part_sum[q * 128 + r];
+        const float l_row = row_sum(part_sum);
         if (met && ok && !*abort_flag && n_blocks > 0) {
             const bool mine = r < rows_here && (!ROWS || pos_r / BN + 1 == n_blocks);
 #pragma unroll
-            for (int c = 0; c < FT_OD; c += 32) {
+            for (int c = 0; c < OD; c += 32) {
                 uint32_t w[32];
-                ft_ld32(tmem_o + lane_base + (uint32_t)(part * FT_OD + c), w);      // all lanes of the warp take part
+                ft_ld32(tmem_o + lane_base + (uint32_t)(part * OD + c), w);      // all lanes of the warp take part
                 ft_ld_wait();
                 if (mine) write_row(w, c, l_row);
             }
@@ -664,7 +683,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attention_prefill_tc_kernel(
 #undef FT_GIVE_UP
     ft_fence_before();
     __syncthreads();
-    if (warp == FT_MMA_WARP) {
+    if (warp == MMA_WARP) {
         ft_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
@@ -732,7 +751,7 @@ static int ft_launch(const void* q, long q_ld, void* out, long out_ld, const voi
     if (max_tiles > 65535) return (int)cudaErrorInvalidValue;
     dim3 grid(n_heads, max_tiles);                 // heads fastest: every head's late (long) tiles start first
     // plain stream order (no programmatic overlap): this kernel takes all of an SM's tensor memory
-    attention_prefill_tc_kernel<ROWS><<<grid, FT_THREADS, FtSmem<ROWS>::TOTAL, stream>>>(
+    attention_prefill_tc_kernel<ROWS><<<grid, FtSmem<ROWS>::THREADS, FtSmem<ROWS>::TOTAL, stream>>>(
         map_q, map_kv, (bf16*)out, out_ld, page_size, (int)kv_rows, block_table, bt_stride, req_start, req_ctx,
         req_qlen, n_requests, include_single, n_heads, n_kv_heads, window, scale, status, sink,
         (const bf16*)gate, gate_ld, gate_cols);

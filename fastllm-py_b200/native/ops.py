@@ -832,24 +832,30 @@ def sink_tc_library(dim: int, vdim: int):
     return "sink_attention_tc", {"SINK_DIM": dim, "SINK_VDIM": vdim}
 
 
-def _sink_rows_pay(step, heads: int, include_single: bool, sms: int) -> bool:
-    """Which of the two prompt kernels is the faster one: tcgen05 takes tiles of 128 tokens, one an SM, at about 7.5 us and 1.5
-    for every 128 keys, the other takes 64 tokens, three an SM, at 5.3 us and 3.4 for every 64 keys.  Many prompts (or
-    portions) of a few tokens go to the other one, as they fill no tile: 20 of 8 tokens with 16 heads take it 16.5 us against
-    28, one of 4 tokens 7.9 against 9.6; the 2048 tokens of one prompt 217 against 38, 64 tokens behind 1500 93 against 27."""
+def _sink_rows_pay(step, heads: int, include_single: bool, sms: int, size: int = 128) -> bool:
+    """Which of the two prompt kernels is the faster one.  tcgen05 takes tiles of 128 tokens, one an SM, at 7.3 us and 1.9 for
+    every 64 keys.  The other takes 64 tokens, at 6 us and 3.5 for every 64 keys where one stands on an SM alone, and 2 us and 3
+    for every 64 keys of each tile that shares one (heads of 64: 0.72 of that; portions of up to 16 tokens 2 us less).  Many
+    prompts of a few tokens go to the other one, as they fill no tile: 20 of 8 tokens with 16 heads of 128 take it 16.5 us
+    against 26, one of 4 tokens 7.8 against 8.4; one of 128 14.7 against 13.3, the 2048 tokens of one prompt 217 against 75, 64
+    tokens behind 1500 93 against 55.  Over 84 mixtures of prompts the choice costs up to 4 %, 12 % in one."""
     tiles = small_tiles = 0
-    keys = small_keys = 0.0                                   # that the tiles go through, in blocks of 128 (of 64)
+    keys = small_keys = longest = 0.0                         # blocks of 64 keys that the tiles go through; the longest one's
+    few = True
     for q, ctx in zip(getattr(step, "q_lens", ()), getattr(step, "ctx_lens", ())):
         if q == 1 and not include_single:
             continue
         n, m = -(-q // 128), -(-q // 64)
         tiles, small_tiles = tiles + n, small_tiles + m
-        keys += n * (ctx / 128 + (n + 1) / 2)
-        small_keys += m * (ctx / 64 + (m + 1) / 2)
+        keys += n * (n - 1) + m + n * ctx / 64
+        small_keys += m * (m + 1) / 2 + m * ctx / 64
+        longest = max(longest, ctx / 64 + m)
+        few = few and q <= 16
     if not tiles:
         return True                                           # (a step built by hand, without its lengths)
-    return -(-tiles * heads // sms) * (7.5 + 1.5 * keys / tiles) < \
-        -(-small_tiles * heads // (3 * sms)) * (5.3 + 3.4 * small_keys / small_tiles)
+    here = max(-(-tiles * heads // sms) * (7.3 + 1.9 * keys / tiles), 7.3 + 1.9 * longest)
+    other = max(1.0 + 3.5 * longest, -(-small_tiles * heads // sms) * (2.0 + 3.0 * small_keys / small_tiles)) + (3.0 if few else 5.0)
+    return here < other * (1.0 if size > 64 else 0.72)
 
 
 def sink_rows_takes(dim: int, vdim: int, window, keep_first, cap, rel, chunk, page_size: int) -> bool:
@@ -897,7 +903,7 @@ def sink_attention_tc(q, out, cache, block_table, step, heads, kv_heads, dim, vd
         raise KernelError("sink_attention_tc: q, cache and out must be bfloat16")
     if sink_rows_takes(dim, vdim, window, keep_first, cap, rel, chunk, page_size) and cache.is_contiguous() \
             and _ld(q) % 8 == 0 and _ld(out) % 8 == 0 and (q.data_ptr() | out.data_ptr() | cache.data_ptr()) % 16 == 0 \
-            and _sink_rows_pay(step, heads, include_single, sm_count(q.device)):
+            and _sink_rows_pay(step, heads, include_single, sm_count(q.device), dim):
         sink_attention_rows(q, out, cache, block_table, step, heads, kv_heads, dim, scale, sink, page_size, include_single, gate)
         return
     sink_attention_mma(q, out, cache, block_table, step, heads, kv_heads, dim, vdim, window, keep_first, scale, cap, bucket_of,
