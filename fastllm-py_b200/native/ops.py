@@ -895,15 +895,16 @@ def sink_attention_mma(q, out, cache, block_table, step, heads, kv_heads, dim, v
 
 
 def sink_attention_tc(q, out, cache, block_table, step, heads, kv_heads, dim, vdim, window, keep_first, scale, cap,
-                      bucket_of, rel, sink, page_size, include_single=True, chunk=None, gate=None):
+                      bucket_of, rel, sink, page_size, include_single=True, chunk=None, gate=None, rows=None):
     """`sink_attention_simt` on tensor cores: q, cache and out bfloat16; single tokens as tiles of one row (left out with
-    include_single=False).  Layers that `sink_rows_takes` go to the faster one of two kernels, which give the same bits."""
+    include_single=False).  Layers that `sink_rows_takes` go to the faster one of two kernels, which give the same bits:
+    `rows` says whether that is the one on tcgen05 (None: by the step's lengths; a part decides that in its plan)."""
     _require_cuda(q, out, cache, block_table, bucket_of, rel, sink, gate)
     if q.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
         raise KernelError("sink_attention_tc: q, cache and out must be bfloat16")
     if sink_rows_takes(dim, vdim, window, keep_first, cap, rel, chunk, page_size) and cache.is_contiguous() \
             and _ld(q) % 8 == 0 and _ld(out) % 8 == 0 and (q.data_ptr() | out.data_ptr() | cache.data_ptr()) % 16 == 0 \
-            and _sink_rows_pay(step, heads, include_single, sm_count(q.device), dim):
+            and (_sink_rows_pay(step, heads, include_single, sm_count(q.device), dim) if rows is None else rows):
         sink_attention_rows(q, out, cache, block_table, step, heads, kv_heads, dim, scale, sink, page_size, include_single, gate)
         return
     sink_attention_mma(q, out, cache, block_table, step, heads, kv_heads, dim, vdim, window, keep_first, scale, cap, bucket_of,

@@ -143,7 +143,8 @@ class LatentAttention(Part):
             longest = -(-limits.max_model_len // 1024) * 1024
             self._partials(min(most, limits.max_tokens), self._split(1, longest)[1])   # nothing grows under a graph
 
-    # ---- what the host decides per step: whether and how the tensor-core kernel splits the keys
+    # ---- what the host decides per step: whether and how the tensor-core kernel splits the keys, and whether the step goes to
+    # the kernel for prompts
     @property
     def plan_key(self):
         return ("latent_attention", self.heads, self.rank, self.rot, self.window)
@@ -161,7 +162,9 @@ class LatentAttention(Part):
         longest = step.max_seq_len
         if step.for_graph:                                    # a captured step serves many: cover the length rounded up
             longest = -(-longest // 1024) * 1024
-        step.plans[self.plan_key] = self._split(step.n_tokens, longest)
+        keys, splits = self._split(step.n_tokens, longest)
+        prompts = keys == 0 and self.ctx.device.type == "cuda" and self._prompts(step, step.n_tokens, self.ctx.page_size)
+        step.plans[self.plan_key] = (keys, splits, prompts)
 
     def graph_key(self, step):
         return step.plans.get(self.plan_key)
@@ -177,7 +180,8 @@ class LatentAttention(Part):
 
         Up to 256 the prompt kernel's tile takes 3.6 us against 2.9, and the other has room for more blocks an SM: with few
         blocks that one is the faster (128 tokens of 16 heads behind 1000: 128 us against 103; level at 384 tokens), with
-        many the prompt kernel until half of its rows stay empty.  Captured steps serve many lengths and take this rule too."""
+        many the prompt kernel until half of its rows stay empty.  Steps of single tokens, captured for many lengths, take this
+        rule too (and so the other kernel); of other captured steps the answer is part of the key."""
         if not step.q_lens or not ops.latent_prompt_takes(self.ctx.dtype, self.rank, self.rot, self.heads, page_size):
             return False
         of_heads, sms = -(-self.heads // 16), ops.sm_count(self.ctx.device)
@@ -236,8 +240,7 @@ class LatentAttention(Part):
         if tc:
             if self.plan_key not in step.plans:               # a step built by hand, not by the engine
                 self.plan_step(step)
-            keys, splits = step.plans[self.plan_key]
-            prompts = keys == 0 and self._prompts(step, n, cache.page_size)
+            keys, splits, prompts = step.plans[self.plan_key]
             if prompts:
                 ops.latent_prompt(q, mix, cache.tensor, cache.block_table, step.req_start, step.req_ctx, step.req_qlen, self.heads,
                                   self.rank, self.rot, self.window, self.scale, cache.page_size, self.sink)

@@ -133,8 +133,7 @@ class SinkAttention(Part):
         takes = self.ctx.device.type == "cuda" and ops.sink_tc_takes(self.ctx.dtype, self.dim, self.vdim)
         if not takes:
             return []
-        rows = ops.sink_rows_takes(self.dim, self.vdim, self.window, self.keep_first, self.softcap, None, None, self.ctx.page_size)
-        return [ops.sink_tc_library(self.dim, self.vdim)] + ([("attention_prefill_tc", {"HEAD_DIM": self.dim})] if rows else [])
+        return [ops.sink_tc_library(self.dim, self.vdim)] + ([("attention_prefill_tc", {"HEAD_DIM": self.dim})] if self._rows() else [])
 
     def reserve(self, limits):
         for lin in (self.qkv, self.o):
@@ -149,10 +148,15 @@ class SinkAttention(Part):
             self._partials(min(limits.max_tokens, limits.max_requests),
                            ops.sink_decode_splits(self.window, self.keep_first, longest)[0])   # nothing grows under a graph
 
-    # ---- what the host decides per step: how many blocks share a single token's keys
+    # ---- what the host decides per step: how many blocks share a single token's keys, and which kernel serves prompts
     @property
     def plan_key(self):
-        return ("sink_attention", self.heads, self.kv_heads, self.dim, self.vdim, self.window, self.keep_first)
+        return ("sink_attention", self.heads, self.kv_heads, self.dim, self.vdim, self.window, self.keep_first, self._rows())
+
+    def _rows(self) -> bool:
+        """Whether the prompt attention on tcgen05 may serve this layer."""
+        return self.ctx.device.type == "cuda" and ops.sink_tc_takes(self.ctx.dtype, self.dim, self.vdim) and             ops.sink_rows_takes(self.dim, self.vdim, self.window, self.keep_first, self.softcap, self.bias_rows, None,
+                                self.ctx.page_size)
 
     def _splits_single_tokens(self) -> bool:
         """bfloat16 steps give their single tokens to the split-key kernels (the 32-bit path keeps one kernel for every
@@ -160,13 +164,16 @@ class SinkAttention(Part):
         return self.ctx.dtype == torch.bfloat16 and ops.sink_decode_takes(self.heads, self.kv_heads, self.dim, self.vdim)
 
     def plan_step(self, step):
-        if not self._splits_single_tokens() or step.n_decode_tokens == 0:
-            step.plans[self.plan_key] = (1, 0)
+        """(splits of a single token's keys, those of the kept tokens among them, whether prompts go to tcgen05)"""
+        splits = self._splits_single_tokens() and step.n_decode_tokens > 0
+        rows = self._rows() and ops._sink_rows_pay(step, self.heads, not splits, ops.sm_count(self.ctx.device), self.dim)
+        if not splits:
+            step.plans[self.plan_key] = (1, 0, rows)
             return
         longest = step.max_seq_len
         if step.for_graph:                                    # a captured step serves many: cover the length rounded up
             longest = -(-longest // 1024) * 1024
-        step.plans[self.plan_key] = ops.sink_decode_splits(self.window, self.keep_first, longest)
+        step.plans[self.plan_key] = (*ops.sink_decode_splits(self.window, self.keep_first, longest), rows)
 
     def graph_key(self, step):
         return step.plans.get(self.plan_key)
@@ -191,10 +198,10 @@ class SinkAttention(Part):
         tc = ops.sink_tc_takes(dt, self.dim, self.vdim)       # bfloat16 and sizes the tensor-core kernel is built for
         # (where only the CUDA-core kernel serves prompt rows, a mixed step gives it every row)
         single = step.n_decode_tokens if self._splits_single_tokens() and (tc or step.n_decode_tokens == n) else 0
+        if self.plan_key not in step.plans:                   # a step built by hand, not by the engine
+            self.plan_step(step)
+        n_splits, kept_splits, rows = step.plans[self.plan_key]
         if single:                                            # single tokens: their keys split over blocks
-            if self.plan_key not in step.plans:               # a step built by hand, not by the engine
-                self.plan_step(step)
-            n_splits, kept_splits = step.plans[self.plan_key]
             ops.sink_decode(q, ctx, cache.tensor, cache.block_table, step.tok_req, step.positions, step.decode_tokens,
                             self._partials(single, n_splits), n_splits, kept_splits, self.heads, self.kv_heads,
                             self.dim, self.vdim, self.window, self.keep_first, self.scale, self.softcap, self.bucket_of,
@@ -204,7 +211,7 @@ class SinkAttention(Part):
         elif tc:
             ops.sink_attention_tc(q, ctx, cache.tensor, cache.block_table, step, self.heads, self.kv_heads, self.dim,
                                   self.vdim, self.window, self.keep_first, self.scale, self.softcap, self.bucket_of,
-                                  self.rel, self.sink, cache.page_size, include_single=not single)
+                                  self.rel, self.sink, cache.page_size, include_single=not single, rows=rows)
         else:
             ops.sink_attention_simt(q, ctx, cache.tensor, cache.block_table, step.tok_req, step.positions, self.heads,
                                     self.kv_heads, self.dim, self.vdim, self.window, self.keep_first, self.scale,

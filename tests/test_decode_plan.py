@@ -59,3 +59,37 @@ def test_latent_prompt_kernel_where_it_is_faster(lens, heads, pays, monkeypatch)
     assert part._prompts(SimpleNamespace(q_lens=step.q_lens), n, 16) is rows
     step.for_graph = True
     assert part._prompts(step, n, 16) is rows
+
+
+@pytest.mark.parametrize("kind", ["normed", "sink", "latent"])
+def test_the_prompt_kernel_is_part_of_a_captured_steps_key(kind, monkeypatch):
+    """Equal portions of a lone prompt are captured: one far behind must not replay the kernel that suited the first.  Decided
+    once a step, in its plan."""
+    import torch
+
+    from fastllm_py_b200.native import ops
+    from fastllm_py_b200.parts import latent, normed_attention, sink_attention
+
+    monkeypatch.setattr(ops, "sm_count", lambda device: 148)
+    monkeypatch.setattr(ops, "latent_prompt_takes", lambda *a: True)
+    monkeypatch.setattr(ops, "sink_decode_takes", lambda *a: True)
+    part = object.__new__({"normed": normed_attention.NormedAttention, "sink": sink_attention.SinkAttention,
+                           "latent": latent.LatentAttention}[kind])
+    part.ctx = SimpleNamespace(device=torch.device("cuda"), dtype=torch.bfloat16, page_size=16)
+    part.heads, part.kv_heads, part.dim, part.vdim, part.window, part.chunk = 16, 4, 128, 128, None, None
+    part.keep_first, part.softcap, part.bias_rows, part.rank, part.rot = 0, None, None, 512, 64
+
+    def key(ctx, q):
+        step = SimpleNamespace(plans={}, ctx_lens=[ctx], q_lens=[q], max_seq_len=ctx + q, n_tokens=q, n_decode_tokens=0, for_graph=False)
+        part.plan_step(step)
+        return part.graph_key(step)
+
+    q = 8 if kind != "latent" else 64
+    assert key(0, q) != key(3000, q) and key(0, q)[-1] is False
+    assert key(3000, q) == key(5000, q) and key(3000, q)[-1] is True
+    if kind == "sink":
+        part.softcap = 30.0
+        capped = part.plan_key
+        assert key(3000, q)[-1] is False                      # a layer that the kernel does not serve, with a plan of its own
+        part.softcap = None
+        assert part.plan_key != capped

@@ -181,3 +181,39 @@ def test_products_of_32_bits_of_few_rows(m, n, k):
     ops.gemm_simt(odd, w, want)
     assert torch.equal(got[:m, :n], want)
     assert bool((got[m] == 7).all()) and bool((got[:, n:] == 7).all())
+
+
+@pytest.mark.parametrize("kind", ["rows", "latent"])
+def test_a_captured_portion_runs_the_kernel_that_its_context_wants(kind, tmp_path, monkeypatch):
+    """Equal portions of lone prompts, first at their beginning until one is captured, then far behind: the step there does not
+    replay what was captured for the beginning."""
+    import kerirax_tiny as kx
+    from fastllm_py_b200 import Model, StepEntry
+
+    mixer = kx.pair(kx.left(16, 4, 128, 128, rot=16), kx.right(40, 16, 8, 4)) if kind == "rows" else kx.latent(16, 16, 64, 16, 512, 24)
+    raw = kx.config([(mixer, kx.dense(48))], vocab=97, width=40)
+    model = Model.load(kx.write(raw, kx.weights(raw, seed=2), tmp_path / "m"), dtype="bfloat16", page_size=16, max_tokens=16384,
+                       max_requests=4, max_batched_tokens=2048, max_model_len=4096, cuda_graph=True)
+    engine, portion, launched = model.engine, 8 if kind == "rows" else 64, []
+    for name in ("sink_attention_rows", "sink_attention_mma", "latent_prompt", "latent_attention_tc"):
+        monkeypatch.setattr(ops, name, lambda *a, _f=getattr(ops, name), _n=name, **kw: (launched.append(_n), _f(*a, **kw))[1])
+    near, far = ("sink_attention_mma", "sink_attention_rows") if kind == "rows" else ("latent_attention_tc", "latent_prompt")
+    tokens = [i % 97 for i in range(4000)]
+
+    def run(rid, at):
+        engine.begin(rid)
+        if at:
+            engine.step([StepEntry(rid, tokens[:at // 2], [])])
+            engine.step([StepEntry(rid, tokens[at // 2:at], [])])
+        launched.clear()
+        out = engine.step([StepEntry(rid, tokens[at:at + portion], [portion - 1])]).clone()
+        engine.end(rid)
+        return out, list(launched)
+
+    beginning = [run(f"a{i}", 0) for i in range(5)]
+    assert [names for _, names in beginning] == [[near]] * 3 + [[]] * 2          # (two eager, one captured, two replayed)
+    behind = [run(f"b{i}", 3000) for i in range(5)]
+    assert [names for _, names in behind] == [[far]] * 3 + [[]] * 2
+    for group in (beginning, behind):
+        assert all(torch.equal(out, group[0][0]) for out, _ in group)
+    engine.check_status()
