@@ -512,7 +512,8 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
         // ---- producer: a lane issues one box, the part of a page that lies in the tile x 64 columns
         const int* bt = block_table + (long)req * bt_stride;
         const int box = min(page_size, LT_KEYS), boxes = LT_KEYS / box;
-        if (lane == 0 && !*abort_flag) {
+        const bool sent = __shfl_sync(0xffffffffu, *abort_flag, 0) == 0;
+        if (lane == 0 && sent) {
             mbar_expect_tx(q_full, LP_SQ * LP_Q_ATOM);
             for (int a = 0; a < LP_SQ; ++a) lp_tma_3d(q_s + a * LP_Q_ATOM, &map_q, q_full, (LP_TQ + a) * 64, head0, tok0);
         }
@@ -536,6 +537,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
         }
         if (*abort_flag) {                                // copies on their way land before the memory goes to another CTA
             for (int k = max(0, i - LP_STAGES); k < i; ++k) lp_warp_wait(&k_full[k % LP_STAGES], (uint32_t)(k / LP_STAGES) & 1u, never);
+            if (sent) lp_warp_wait(q_full, 0, never);
         }
     } else if (warp == 9) {
         // ---- MMA issuer

@@ -96,3 +96,13 @@ def test_products_that_give_up_wait_for_their_copies(name, kernels):
         assert drain < body.index("dealloc", met) and ("cluster_sync_all" not in body or drain < body.index("cluster_sync_all", met))
         ring = body[body.index("int issued = 0;"):met]
         assert ring.count("++issued;\n") == 1 and ring.index("++issued;") < ring.index("if (++s ==")
+
+
+@pytest.mark.parametrize("name", ["latent_attention_tc.cu", "attention_prefill_tc.cu"])
+def test_attention_that_gives_up_waits_for_its_copies(name):
+    """The same in the attention kernels: the producer, where the abort flag is set, waits for the rings' fills and for the
+    queries, with waits that the flag does not cut short."""
+    text = (CSRC / name).read_text()
+    drain = re.search(r"if \(\*abort_flag\) \{[^}]*?for \(int k = max\(0, i - \w+\); k < i; \+\+k\)[^}]*\}", text).group(0)
+    filled = set(re.findall(r"expect(?:_tx)?\(&?(\w+)", text)) - {"uint64_t"}                # (not the wrapper itself)
+    assert filled and all(re.search(rf"wait\(&?{bar}\b[^;]*never\)", drain) for bar in filled), (filled, drain)
