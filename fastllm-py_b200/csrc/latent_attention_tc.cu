@@ -355,7 +355,16 @@ FL_API int fl_latent_attention_tc(const void* q, long q_ld, void* out, int out_d
 #define LP_STAGES 4
 #define LP_TOKENS 8
 #define LP_THREADS 320
-#define LP_SMEM (LP_SQ * LP_Q_ATOM + LP_STAGES * LP_STAGE_BYTES + 256 + 3 * 128 * 4 + 1024)
+// They come by TMA too: into the stages of the second to fourth tile, which are filled when the queries have left, where that
+// is room enough (rows of 512 and more elements), else into memory of their own.  (Read row by row from global memory, 16 of
+// every 1152 bytes a lane, they took 2 us more: 20 prompts of 20 tokens, 16 heads, 14.5 us.)
+#define LP_TQ_BYTES (LP_TQ * LP_Q_ATOM)
+#define LP_TQ_LENT (LP_TQ_BYTES <= 3 * LP_STAGE_BYTES)
+#define LP_TILES (LP_SQ * LP_Q_ATOM + LP_STAGES * LP_STAGE_BYTES + (LP_TQ_LENT ? 0 : LP_TQ_BYTES))
+#define LP_SMEM (LP_TILES + 256 + 3 * 128 * 4 + 1024)
+// Asked for: more than half of an SM's.  A second CTA would only wait there for tensor memory, while another SM may have none
+// (2048 tokens, 16 heads, a latent of 128: 151 us with two on an SM, 106 with one).
+#define LP_SMEM_ASKED (LP_SMEM > 116 * 1024 ? LP_SMEM : 116 * 1024)
 enum { LP_ERR_WAIT = 141 };
 static_assert(LP_SMEM <= 232448, "more shared memory than a CTA can have");
 static_assert(LT_SMEM <= LP_SQ * LP_Q_ATOM + LP_STAGES * LP_STAGE_BYTES, "tokens done again find room in the tiles' place");
@@ -423,7 +432,8 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
     extern __shared__ unsigned char lp_raw[];
     unsigned char* q_s = (unsigned char*)(((uintptr_t)lp_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* k_s = q_s + LP_SQ * LP_Q_ATOM;
-    uint64_t* bars = (uint64_t*)(k_s + LP_STAGES * LP_STAGE_BYTES);
+    unsigned char* t_s = k_s + (LP_TQ_LENT ? LP_STAGE_BYTES : LP_STAGES * LP_STAGE_BYTES);     // queries on their way to tensor memory
+    uint64_t* bars = (uint64_t*)(q_s + LP_TILES);
     uint64_t* q_full = bars;
     uint64_t* k_full = bars + 1;                          // [LP_STAGES]
     uint64_t* k_empty = k_full + LP_STAGES;
@@ -432,7 +442,8 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
     uint64_t* p_full = c_full + 2;                        // [2] weights written and accumulators rescaled
     uint64_t* o_done = p_full + 2;                        // [2] values of tile i are added up: barrier i & 1, phase i >> 1
     uint64_t* t_full = o_done + 2;                        // the queries in tensor memory are there
-    uint32_t* tmem_slot = (uint32_t*)(t_full + 1);
+    uint64_t* t_sent = t_full + 1;                        // and in shared memory before that
+    uint32_t* tmem_slot = (uint32_t*)(t_sent + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     volatile int* never = abort_flag + 1;                 // stays 0: for waits that must not be cut short
     volatile int* again = never + 1;                      // the tokens are done again
@@ -461,6 +472,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
         mbar_init(t_full, 8);
+        mbar_init(t_sent, 1);
         for (int s = 0; s < LP_STAGES; ++s) {
             mbar_init(&k_full[s], 1);
             mbar_init(&k_empty[s], 1);
@@ -491,21 +503,26 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
     };
     if (warp < 8) {
         // a row's queries for tensor memory, pairs of elements a column, every other atom by warps 4-7
-        const int r = threadIdx.x & 127;
-        const bf16* src = q + (long)(tok0 + (r >> 4)) * q_ld + (long)(head0 + (r & 15)) * LT_WIDTH;
-        const uint32_t dst = tmem_q + ((uint32_t)((warp & 3) * 32) << 16);
-#pragma unroll 1
-        for (int a = warp >> 2; a < LP_TQ; a += 2) {
-            uint4 w[8];
+        if (lp_warp_wait(t_sent, 0, abort_flag)) {
+            const int r = threadIdx.x & 127;
+            const uint32_t dst = tmem_q + ((uint32_t)((warp & 3) * 32) << 16);
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                w[j] = (r >> 4) < tokens ? reinterpret_cast<const uint4*>(src + a * 64)[j] : make_uint4(0u, 0u, 0u, 0u);
-            tmem_st16(dst + (uint32_t)(a * 32), reinterpret_cast<const uint32_t*>(w));
-            tmem_st16(dst + (uint32_t)(a * 32 + 16), reinterpret_cast<const uint32_t*>(w + 4));
+            for (int i = 0; i < (LP_TQ + 1) / 2; ++i) {
+                const int a = (warp >> 2) + 2 * i;
+                if (a >= LP_TQ) continue;
+                uint4 w[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j)               // (the pieces of a row lie in the swizzle's order)
+                    w[j] = *reinterpret_cast<const uint4*>(t_s + a * LP_Q_ATOM + r * 128 + ((j ^ (r & 7)) << 4));
+                tmem_st16(dst + (uint32_t)(a * 32), reinterpret_cast<const uint32_t*>(w));
+                tmem_st16(dst + (uint32_t)(a * 32 + 16), reinterpret_cast<const uint32_t*>(w + 4));
+            }
+            tmem_st_wait();
+            tc_fence_before();
+            lp_warp_arrive(t_full);
+        } else if (lane == 0) {
+            give_up();
         }
-        tmem_st_wait();
-        tc_fence_before();
-        lp_warp_arrive(t_full);
     }
 
     if (warp == 8) {
@@ -514,6 +531,8 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
         const int box = min(page_size, LT_KEYS), boxes = LT_KEYS / box;
         const bool sent = __shfl_sync(0xffffffffu, *abort_flag, 0) == 0;
         if (lane == 0 && sent) {
+            mbar_expect_tx(t_sent, LP_TQ_BYTES);
+            for (int a = 0; a < LP_TQ; ++a) lp_tma_3d(t_s + a * LP_Q_ATOM, &map_q, t_sent, a * 64, head0, tok0);
             mbar_expect_tx(q_full, LP_SQ * LP_Q_ATOM);
             for (int a = 0; a < LP_SQ; ++a) lp_tma_3d(q_s + a * LP_Q_ATOM, &map_q, q_full, (LP_TQ + a) * 64, head0, tok0);
         }
@@ -521,7 +540,8 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
         int i = 0;
         for (; i < n_tiles && !*abort_flag; ++i) {
             const int s = i % LP_STAGES;
-            if (!lp_warp_wait(&k_empty[s], ((uint32_t)(i / LP_STAGES) & 1u) ^ 1u, abort_flag)) {
+            const bool lent = LP_TQ_LENT && i == 1;       // (the queries must have left this stage and the next two)
+            if ((lent && !lp_warp_wait(t_full, 0, abort_flag)) || !lp_warp_wait(&k_empty[s], ((uint32_t)(i / LP_STAGES) & 1u) ^ 1u, abort_flag)) {
                 if (lane == 0) give_up();
                 break;
             }
@@ -538,6 +558,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) latent_prompt_kernel(
         if (*abort_flag) {                                // copies on their way land before the memory goes to another CTA
             for (int k = max(0, i - LP_STAGES); k < i; ++k) lp_warp_wait(&k_full[k % LP_STAGES], (uint32_t)(k / LP_STAGES) & 1u, never);
             if (sent) lp_warp_wait(q_full, 0, never);
+            if (sent) lp_warp_wait(t_sent, 0, never);
         }
     } else if (warp == 9) {
         // ---- MMA issuer
@@ -770,9 +791,9 @@ FL_API int fl_latent_prompt(const void* q, long q_ld, void* out, int out_dtype, 
     // plain stream order (no programmatic overlap): this kernel takes all of an SM's tensor memory
     const dim3 grid(n_tokens / LP_TOKENS + n_requests, heads / 16 * LP_HALVES);
     FL_DISPATCH(out_dtype, TO, {
-        rc = (int)cudaFuncSetAttribute(latent_prompt_kernel<TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, LP_SMEM);
+        rc = (int)cudaFuncSetAttribute(latent_prompt_kernel<TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, LP_SMEM_ASKED);
         if (rc) return rc;
-        latent_prompt_kernel<TO><<<grid, LP_THREADS, LP_SMEM, stream>>>(map_q, map_k, (const bf16*)q, q_ld, (TO*)out, out_ld,
+        latent_prompt_kernel<TO><<<grid, LP_THREADS, LP_SMEM_ASKED, stream>>>(map_q, map_k, (const bf16*)q, q_ld, (TO*)out, out_ld,
                                                                         (const bf16*)cache, heads, page_size, (int)cache_rows,
                                                                         block_table, bt_stride, req_start, req_ctx, req_qlen,
                                                                         n_requests, window, scale, sink, status);

@@ -217,3 +217,26 @@ def test_a_captured_portion_runs_the_kernel_that_its_context_wants(kind, tmp_pat
     for group in (beginning, behind):
         assert all(torch.equal(out, group[0][0]) for out, _ in group)
     engine.check_status()
+
+
+@pytest.mark.parametrize("rank,rot", [(64, 64), (128, 64), (256, 128), (256, 192), (512, 0)])
+@pytest.mark.parametrize("window", [None, 70])
+def test_latent_prompts_of_every_width(rank, rot, window):
+    """Queries that arrive in memory of their own (rows of up to seven pieces of 64) and in the later tiles' (eight), one tile and
+    several: bit for bit the kernel for single tokens."""
+    torch.manual_seed(rank + rot)
+    heads, page, width, lens = 16, 16, rank + rot, [(0, 5), (150, 9), (33, 40), (0, 200), (7, 1)]
+    per = [-(-(c + m) // page) for c, m in lens]
+    bt = torch.zeros(len(lens), max(per), dtype=torch.int32, device="cuda")
+    order = torch.randperm(sum(per), device="cuda").to(torch.int32)
+    for r, k in enumerate(per):
+        bt[r, :k] = order[sum(per[:r]):sum(per[:r]) + k]
+    cache = torch.randn(sum(per), page, width, device="cuda").to(torch.bfloat16)
+    starts = [sum(m for _, m in lens[:r]) for r in range(len(lens) + 1)]
+    n = starts[-1]
+    tok_req, positions = i32([r for r, (_, m) in enumerate(lens) for _ in range(m)]), i32([c + i for c, m in lens for i in range(m)])
+    q = (0.3 * torch.randn(n, heads * width, device="cuda")).to(torch.bfloat16)
+    want, got = (torch.zeros(n, heads * rank, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    ops.latent_attention_tc(q, want, cache, bt, tok_req, positions, heads, rank, rot, window, 0.1, page)
+    ops.latent_prompt(q, got, cache, bt, i32(starts), i32([c for c, _ in lens]), i32([m for _, m in lens]), heads, rank, rot, window, 0.1, page)
+    assert torch.equal(got, want)
