@@ -175,23 +175,26 @@ class LatentAttention(Part):
 
         A latent of 512: a tile of 32 keys takes it 2.15 us and the other kernel 4.6 (6.6 where two of its blocks share an
         SM), its start 10.7 us against 4 (6), and two of its blocks (one for either half of the value columns) stand on an SM
-        each, two of the other's on one.  128 tokens of 16 heads behind 1000 others take 87 us against 163, 16 requests of 4
-        behind 500 43 against 75; 20 prompts of 8 tokens 14.4 against 11.8, 60 of 3 with 32 heads 27 against 19.
+        each, two of the other's on one.  128 tokens of 16 heads behind 1000 others take 85 us against 162, 16 requests of 4
+        behind 500 43 against 75; 20 prompts of 8 tokens 12.6 against 11.9, 60 of 3 with 32 heads 27 against 19.
 
-        Up to 256 the prompt kernel's tile takes 3.6 us against 2.9, and the other has room for more blocks an SM: with few
-        blocks that one is the faster (128 tokens of 16 heads behind 1000: 128 us against 103; level at 384 tokens), with
-        many the prompt kernel until half of its rows stay empty.  Steps of single tokens, captured for many lengths, take this
-        rule too (and so the other kernel); of other captured steps the answer is part of the key."""
+        Up to 256 a tile's rows decide: 1.4 us a tile for rows of 128 elements, 1.75 for 320, against 1.5 and 2.75 where a
+        block of the other kernel has an SM to itself, and 0.4 and 1.15 for each of them where many share it, its start as long
+        as 0.9 of a tile; the prompt kernel's start is longer with many requests, among which a block looks for its own.  Rows of 320,
+        16 heads: 128 tokens behind 1000 73 us against 102, 37 tokens each of eight prompts 11.4 against 10.1; rows of 128:
+        57 against 54, 2048 tokens 98 against 217.
+
+        Steps of single tokens, captured for many lengths, take the other kernel, as do those whose rows would mostly stay
+        empty in a step built without its lengths; of other captured steps the answer is part of the key."""
         if not step.q_lens or not ops.latent_prompt_takes(self.ctx.dtype, self.rank, self.rot, self.heads, page_size):
             return False
         of_heads, sms = -(-self.heads // 16), ops.sm_count(self.ctx.device)
         blocks = n_tokens * of_heads                                      # the other kernel's
         ctx_lens = getattr(step, "ctx_lens", None)
-        if self.rank <= 256 or not ctx_lens or getattr(step, "for_graph", False):
+        if not ctx_lens or getattr(step, "for_graph", False):
             if 2 * blocks <= (2 if self.rank > 256 else 5) * sms:
                 return False
             return 4 * sum(-(-q // 8) for q in step.q_lens) <= n_tokens   # four of eight rows at least
-        start, a_tile = (4.0, 4.6) if blocks <= sms else (6.0, 6.6)
         groups, tiles, longest, other_tiles = 0, 0.0, 0, 0.0
         for q, ctx in zip(step.q_lens, ctx_lens):
             last = ctx + q if self.window is None else min(ctx + q, self.window + 8)
@@ -201,9 +204,16 @@ class LatentAttention(Part):
             tiles += n * (mean + 16) / 32
             other_tiles += q * (mean + 16) / 32
             longest = max(longest, -(-last // 32))
-        here = max(-(-2 * groups * of_heads // sms) * (10.7 + 2.15 * tiles / groups), 10.7 + 2.15 * longest)
-        other = max(-(-blocks // (2 * sms)) * (start + a_tile * other_tiles / n_tokens), start + a_tile * longest)
-        return here < other
+        tiles, other_tiles = tiles / groups, other_tiles / n_tokens       # a block's
+        if self.rank > 256:
+            start, a_tile, halves = 10.7, 2.15, 2
+            other_start, other_tile = (4.0, 4.6) if blocks <= sms else (6.0, 6.6)
+            other = max(-(-blocks // (2 * sms)) * (other_start + other_tile * other_tiles), other_start + other_tile * longest)
+        else:
+            start, a_tile, halves = 4.2 + 0.012 * self.width + 0.1 * len(step.q_lens), 1.2 + 0.00175 * self.width, 1
+            alone, shared = 0.75 + 0.0027 * self.width, 0.0039 * self.width - 0.1
+            other = 3.0 + max((other_tiles + 0.9) * (alone + shared * -(-blocks // sms)), longest * (alone + shared))
+        return max(-(-halves * groups * of_heads // sms) * (start + a_tile * tiles), start + a_tile * longest) < other
 
     def _partials(self, n_tokens: int, n_splits: int):
         return scratch.get(self.ctx.device, self.SCRATCH, n_tokens * self.heads * n_splits * (self.rank + 2))
