@@ -543,25 +543,30 @@ FL_API int fl_glu(const void* gu, int dtype, long gu_ld, void* out, long out_ld,
 //
 // One CTA a row; a thread's KEEP chunks of four neighbouring elements stay in registers, and all their loads (the slabs or
 // y, x, both weights) are issued before the first reduction, so a row costs one round trip to memory and two reductions, and
-// nothing is read twice.  A chunk that 16-byte loads cannot read (VEC false) is taken an element at a time; every form sums
+// nothing is read twice.  Where 16-byte loads cannot read a row (VEC false), a thread's four elements of a chunk are not
+// neighbours but 128 apart, so that the loads of a warp still are (2048 rows of 2050: 21.7 us as neighbours, 19.7 so; 16 slabs
+// of one row 10.0 and 8.2).  Every form sums
 // the squares in one order: element i belongs to chain i mod 512 of up to 512, a chain goes from its first element to its
 // last, and the chains are added as a block's threads are (32 by 32, then the groups).  A thread holds four chains, 128 of
 // them all; of a row that is too long for one thread's registers (over 4096), blocks of 128 threads take 2048 elements each and
-// hand the chains on (WIDE).  2048 rows of 2048 take 9.0 us (6.4 us of bytes out of
+// hand the chains on (WIDE; slabs of single elements already over 2048, as they find no registers else).  2048 rows of 2048 take 9.0 us (6.4 us of bytes out of
 // memory; an element at a time with the row in shared memory 18.4), 8 rows of 9 slabs 3.8 (6.1).
 #define SAND_CHAINS 512
 #define SAND_LONGEST 12256               // elements of a row
-template <bool PARTIAL, typename TD, typename TW, typename TO, int KEEP, bool VEC, bool WIDE>
-__global__ void __launch_bounds__(WIDE ? 768 : SAND_CHAINS / 4) sandwich_norm_kernel(
+template <bool PARTIAL, typename TD, typename TW, typename TO, int KEEP, bool VEC, int GROUPS>
+__global__ void __launch_bounds__(GROUPS * SAND_CHAINS / 4) sandwich_norm_kernel(
     float* __restrict__ x, long x_ld, const void* __restrict__ y, long y_ld, int splits, long split_stride,
     const TW* __restrict__ w_post, float eps_post, const TW* __restrict__ w_pre, float eps_pre, TO* __restrict__ out,
     long out_ld, int dim, const int* __restrict__ rows, int write_back) {
     pdl_wait();
     pdl_trigger();
     __shared__ float scratch[SAND_CHAINS / 32];
+    constexpr bool WIDE = GROUPS > 1;                       // groups of 128 threads, at most
     __shared__ float4 carry[WIDE ? SAND_CHAINS / 4 : 1];
     const int r = blockIdx.x, lane = threadIdx.x & 31, part = WIDE ? threadIdx.x / (SAND_CHAINS / 4) : 0;
-    const int own = threadIdx.x % (SAND_CHAINS / 4), i0 = own * 4 + part * KEEP * SAND_CHAINS;
+    const int own = threadIdx.x % (SAND_CHAINS / 4);
+    const int apart = VEC ? 1 : min((int)blockDim.x, SAND_CHAINS / 4);              // between a thread's four elements of a chunk
+    const int i0 = (VEC ? own * 4 : own) + part * KEEP * SAND_CHAINS;
     const long src = rows ? (long)rows[r] : (long)r;
     float* xr = x + src * x_ld;
     auto squares = [&](const float4 (&v)[KEEP]) {
@@ -589,15 +594,21 @@ __global__ void __launch_bounds__(WIDE ? 768 : SAND_CHAINS / 4) sandwich_norm_ke
         } else {
             chain();
         }
+        // 32 neighbouring chains are eight lanes' four, or one of the four of each of a warp's lanes
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1) {
+        for (int o = VEC ? 4 : 16; o > 0; o >>= 1) {
             s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
             s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
             s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
             s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
         }
         __syncthreads();                                // scratch may still be read from the call before
-        if ((lane & 7) == 0 && part == 0) scratch[own / 8] = (s.x + s.z) + (s.y + s.w);
+        if (VEC) {
+            if ((lane & 7) == 0 && part == 0) scratch[own / 8] = (s.x + s.z) + (s.y + s.w);
+        } else if (lane == 0 && part == 0) {
+            float* to = scratch + own / 32;
+            to[0] = s.x, to[apart / 32] = s.y, to[2 * (apart / 32)] = s.z, to[3 * (apart / 32)] = s.w;
+        }
         __syncthreads();
         return warp_sum(lane < min((int)blockDim.x, SAND_CHAINS / 4) / 8 ? scratch[lane] : 0.0f);
     };
@@ -607,9 +618,9 @@ __global__ void __launch_bounds__(WIDE ? 768 : SAND_CHAINS / 4) sandwich_norm_ke
         } else {
             using T = std::remove_cv_t<std::remove_reference_t<decltype(*p)>>;
             v.x = to_f32<T>(p[i]);
-            v.y = i + 1 < dim ? to_f32<T>(p[i + 1]) : 0.0f;
-            v.z = i + 2 < dim ? to_f32<T>(p[i + 2]) : 0.0f;
-            v.w = i + 3 < dim ? to_f32<T>(p[i + 3]) : 0.0f;
+            v.y = i + apart < dim ? to_f32<T>(p[i + apart]) : 0.0f;
+            v.z = i + 2 * apart < dim ? to_f32<T>(p[i + 2 * apart]) : 0.0f;
+            v.w = i + 3 * apart < dim ? to_f32<T>(p[i + 3 * apart]) : 0.0f;
         }
     };
     auto put = [&](auto* p, int i, const float4& v) {
@@ -618,9 +629,9 @@ __global__ void __launch_bounds__(WIDE ? 768 : SAND_CHAINS / 4) sandwich_norm_ke
         } else {
             using T = std::remove_cv_t<std::remove_reference_t<decltype(*p)>>;
             p[i] = from_f32<T>(v.x);
-            if (i + 1 < dim) p[i + 1] = from_f32<T>(v.y);
-            if (i + 2 < dim) p[i + 2] = from_f32<T>(v.z);
-            if (i + 3 < dim) p[i + 3] = from_f32<T>(v.w);
+            if (i + apart < dim) p[i + apart] = from_f32<T>(v.y);
+            if (i + 2 * apart < dim) p[i + 2 * apart] = from_f32<T>(v.z);
+            if (i + 3 * apart < dim) p[i + 3 * apart] = from_f32<T>(v.w);
         }
     };
     float4 sub[KEEP], sum[KEEP], post[KEEP], pre[KEEP];
@@ -637,7 +648,7 @@ __global__ void __launch_bounds__(WIDE ? 768 : SAND_CHAINS / 4) sandwich_norm_ke
     }
     if constexpr (PARTIAL) {
         const float* pr = static_cast<const float*>(y) + src * y_ld;
-        constexpr int BATCH = WIDE ? 1 : KEEP >= 8 ? 2 : KEEP == 4 ? 5 : 10;      // slabs on their way at once
+        constexpr int BATCH = GROUPS > 2 ? 1 : KEEP >= 8 ? 2 : KEEP == 4 ? 5 : 10;      // slabs on their way at once
         for (int z0 = 0; z0 < splits; z0 += BATCH) {
             float4 q[BATCH][KEEP];
 #pragma unroll
@@ -690,29 +701,31 @@ static int sandwich_launch(float* x, long x_ld, const void* y, long y_ld, int sp
                      vec4_ok(dim, w_post, 4, sizeof(TW)) &&
                      (out == nullptr || (vec4_ok(dim, w_pre, 4, sizeof(TW)) && vec4_ok(dim, out, out_ld, sizeof(TO))));
     const int chunks = (dim + SAND_CHAINS - 1) / SAND_CHAINS;           // a thread's
-    const int threads = chunks > 8 ? SAND_CHAINS / 4 * ((chunks + 3) / 4) : chunks > 1 ? SAND_CHAINS / 4 : (dim + 127) / 128 * 32;
-#define FL_SANDWICH(KEEP, VEC, WIDE)                                                                                                \
-    return fl_launch(sandwich_norm_kernel<PARTIAL, TD, TW, TO, KEEP, VEC, WIDE>, dim3(n_rows), dim3(threads), 0, stream, x, x_ld, y, \
-                     y_ld, splits, split_stride, (const TW*)w_post, eps_post, (const TW*)w_pre, eps_pre, (TO*)out, out_ld, dim,     \
+    const int groups = chunks > (vec || !PARTIAL ? 8 : 4) ? (chunks + 3) / 4 : 1;
+    const int threads = chunks > 1 ? SAND_CHAINS / 4 * groups : (dim + 127) / 128 * 32;
+#define FL_SANDWICH(KEEP, VEC, GROUPS)                                                                                                \
+    return fl_launch(sandwich_norm_kernel<PARTIAL, TD, TW, TO, KEEP, VEC, GROUPS>, dim3(n_rows), dim3(threads), 0, stream, x, x_ld, y, \
+                     y_ld, splits, split_stride, (const TW*)w_post, eps_post, (const TW*)w_pre, eps_pre, (TO*)out, out_ld, dim,       \
                      rows, rows ? 0 : 1)
     if (chunks <= 1) {
-        if (vec) FL_SANDWICH(1, true, false);
-        FL_SANDWICH(1, false, false);
+        if (vec) FL_SANDWICH(1, true, 1);
+        FL_SANDWICH(1, false, 1);
     }
     if (chunks <= 2) {
-        if (vec) FL_SANDWICH(2, true, false);
-        FL_SANDWICH(2, false, false);
+        if (vec) FL_SANDWICH(2, true, 1);
+        FL_SANDWICH(2, false, 1);
     }
     if (chunks <= 4) {
-        if (vec) FL_SANDWICH(4, true, false);
-        FL_SANDWICH(4, false, false);
+        if (vec) FL_SANDWICH(4, true, 1);
+        FL_SANDWICH(4, false, 1);
     }
     if (chunks <= 8) {
-        if (vec) FL_SANDWICH(8, true, false);
-        FL_SANDWICH(8, false, false);
+        if (vec) FL_SANDWICH(8, true, 1);
+        if constexpr (PARTIAL) FL_SANDWICH(4, false, 2);
+        else FL_SANDWICH(8, false, 1);
     }
-    if (vec) FL_SANDWICH(4, true, true);
-    FL_SANDWICH(4, false, true);
+    if (vec) FL_SANDWICH(4, true, 6);
+    FL_SANDWICH(4, false, 6);
 #undef FL_SANDWICH
 }
 

@@ -240,3 +240,30 @@ def test_latent_prompts_of_every_width(rank, rot, window):
     ops.latent_attention_tc(q, want, cache, bt, tok_req, positions, heads, rank, rot, window, 0.1, page)
     ops.latent_prompt(q, got, cache, bt, i32(starts), i32([c for c, _ in lens]), i32([m for _, m in lens]), heads, rank, rot, window, 0.1, page)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dim,slabs", [(100, 2), (513, 6), (1028, 1), (2048, 9), (2050, 16), (4096, 11), (8192, 5), (12256, 3)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_norm_add_norm_of_partial_sums(dim, slabs, shift):
+    """Slabs in one batch and in several, chunks of a thread, rows over several groups of threads, accesses of 16 bytes and of one
+    element: the bits of the slabs added in order, rounded, and normed; `out` against float64 within its rounding (2^-9)."""
+    torch.manual_seed(dim + slabs)
+    rows, ld = 3, dim + 4
+    data = torch.empty(slabs * rows * ld + 1, device="cuda")[shift:shift + slabs * rows * ld].view(slabs, rows, ld)
+    data.copy_(torch.randn(slabs, rows, ld, device="cuda"))
+    partial = SimpleNamespace(data=data, splits=slabs, split_stride=rows * ld, ld=ld, check=lambda: None)
+    wa, wb = (1 + 0.2 * torch.randn(2, dim, device="cuda")).to(torch.bfloat16)
+    x = torch.randn(rows, dim, device="cuda")
+    y = torch.zeros(rows, dim, device="cuda")
+    for z in range(slabs):
+        y += data[z, :, :dim]
+    y = y.to(torch.bfloat16)
+    got_x, want_x = x.clone(), x.clone()
+    got, want = (torch.empty(rows, dim, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    ops.sandwich_norm_partial(got_x, partial, wa, 1e-5, wb, 1e-6, got)
+    ops.sandwich_norm(want_x, y, wa, 1e-5, wb, 1e-6, want)
+    assert torch.equal(got_x, want_x) and torch.equal(got, want)
+    yd = y.double()
+    total = x.double() + yd / torch.sqrt((yd * yd).mean(-1, keepdim=True) + 1e-5) * wa.double()
+    ref = total / torch.sqrt((total * total).mean(-1, keepdim=True) + 1e-6) * wb.double()
+    assert float(((got.double() - ref).abs() / ref.abs().clamp_min(1e-3)).max()) <= 2 ** -8   # (2^-9, and sums of 32 bits)
