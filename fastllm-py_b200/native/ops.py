@@ -904,6 +904,7 @@ def sink_attention_tc(q, out, cache, block_table, step, heads, kv_heads, dim, vd
         raise KernelError("sink_attention_tc: q, cache and out must be bfloat16")
     if sink_rows_takes(dim, vdim, window, keep_first, cap, rel, chunk, page_size) and cache.is_contiguous() \
             and _ld(q) % 8 == 0 and _ld(out) % 8 == 0 and (q.data_ptr() | out.data_ptr() | cache.data_ptr()) % 16 == 0 \
+            and q.shape[0] // 128 + step.n_requests <= 65535 \
             and (_sink_rows_pay(step, heads, include_single, sm_count(q.device), dim) if rows is None else rows):
         sink_attention_rows(q, out, cache, block_table, step, heads, kv_heads, dim, scale, sink, page_size, include_single, gate)
         return

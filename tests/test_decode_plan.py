@@ -93,3 +93,21 @@ def test_the_prompt_kernel_is_part_of_a_captured_steps_key(kind, monkeypatch):
         assert key(3000, q)[-1] is False                      # a layer that the kernel does not serve, with a plan of its own
         part.softcap = None
         assert part.plan_key != capped
+
+
+@pytest.mark.parametrize("requests,rows", [(65535, True), (65536, False)])
+def test_more_tiles_than_a_grid_holds_stay_with_the_other_kernel(requests, rows, monkeypatch):
+    """The tiles of 128 tokens are a grid's y, which the other kernel's are not: no step is refused for them."""
+    import torch
+
+    from fastllm_py_b200.native import ops
+
+    called = []
+    monkeypatch.setattr(ops, "_require_cuda", lambda *a: None)
+    monkeypatch.setattr(ops, "sm_count", lambda device: 148)
+    monkeypatch.setattr(ops, "sink_attention_rows", lambda *a: called.append(True))
+    monkeypatch.setattr(ops, "sink_attention_mma", lambda *a: called.append(False))
+    q = torch.empty(64, 256, dtype=torch.bfloat16)
+    ops.sink_attention_tc(q, q, torch.empty(4, 1, 16, 256, dtype=torch.bfloat16), None, SimpleNamespace(n_requests=requests), 2, 1, 128, 128,
+                          None, 0, 1.0, None, None, None, None, 16)
+    assert called == [rows]
