@@ -179,8 +179,9 @@ __global__ void delta_tail_kernel(const T* __restrict__ proj, long ld, float* __
 // the recurrence do nothing else, a warp of them being alone on its scheduler.  In shared memory
 // a part's k (and q) elements are contiguous and parts are DPT + 4 floats apart, so a thread fetches them
 // four at a time without bank conflicts.
-// What bounds a long prompt: the chain from one token's u to the next one's.  2048 tokens, 16 heads of 128 x 128: 310 us,
-// 151 ns a token; 676 us with the fetches and q . k on the same threads (156 instructions a token and warp, a fifth of the
+// What bounds a long prompt: 2048 tokens, 16 heads of 128 x 128 take 310 us, 151 ns a token.  Without the reads of shared
+// memory it would be 242 us, without the sums across lanes 233, without both 200: no part of it alone (sums over the state
+// two tokens ahead, a shorter chain with more instructions, took 342).  676 us with the fetches and q . k on the same threads (156 instructions a token and warp, a fifth of the
 // time at the barrier behind the two warps that fetched) and one multiply-add an element.
 // Registers are kept to what lets two blocks of 32 columns share an SM: several requests' prompts bring more blocks than SMs
 // (8 x 100 tokens, 16 heads of 128 x 128: 121 us with one block an SM, 96 with two).

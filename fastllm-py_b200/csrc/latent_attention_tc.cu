@@ -316,7 +316,7 @@ FL_API int fl_latent_attention_tc(const void* q, long q_ld, void* out, int out_d
 // ----------------------------------------------------------------- prompts: tcgen05
 // Eight neighbouring tokens of a request x 16 heads are the 128 rows of tcgen05.mma, where the kernel above has 16 rows of
 // mma.sync: a cache row that has been fetched serves 8 tokens.  (Prompt of 2048 tokens, 16 heads, rank 512, window 1024:
-// 971 us with mma.sync, which fetched 1.8 GB of rows from L2 and kept its tensor cores 4 % busy, 228 us so.)  The sums are the other
+// 971 us with mma.sync, which fetched 1.8 GB of rows from L2 and kept its tensor cores 4 % busy, 224 us so.)  The sums are the other
 // kernel's, one by one: the same tiles of 32 keys, scores and value sums in K steps of 16 from the first to the last, the
 // weights' sums in the same tree, a rescaling at every tile where the maximum moved (where it did not, the other kernel
 // multiplies by one), so results are the same bit for bit.
